@@ -1,0 +1,76 @@
+"""The GEMM that streams the weights past few rows (gemm_stream.cu) at the edges of its tiles, K slices
+and of the rule that picks it, against a 64-bit product."""
+import math
+
+import pytest
+import torch
+
+from vllm_gcu_b200.ops import _native, ref
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _status_clean():
+    yield
+    if torch.cuda.is_available():
+        _native.check_status()
+
+
+# rows around the multiples of 16 and the two row tiles; widths with a ragged last tile of 128, fewer
+# tiles than SMs (K split over 2 .. 8 CTAs) and more; K with a ragged last block of 64, K blocks that
+# the slices do not share evenly, and fewer blocks than a split takes
+SHAPES = [(1, 8, 8), (1, 4096, 4096), (3, 136, 72), (15, 200, 1000), (16, 128, 4160), (17, 640, 5120),
+          (32, 6144, 4096), (31, 28672, 512), (32, 19072, 264), (33, 6144, 4096), (64, 2112, 7168),
+          (65, 4096, 4160), (128, 8192, 4096), (129, 4096, 4104), (256, 2048, 4096), (250, 72, 14336)]
+
+
+@pytest.mark.parametrize("M,N,K", SHAPES)
+def test_every_epilogue(M, N, K):
+    from vllm_gcu_b200.ops import cuda as C
+    assert C._stream_pays(M, N, K)
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    wide = torch.randn(M, K + 8, device="cuda", generator=g).to(torch.bfloat16)
+    a = wide[:, :K]                                    # rows with a pitch
+    b = torch.randn(N, K, device="cuda", generator=g).div_(math.sqrt(K)).to(torch.bfloat16)
+    bias = torch.randn(N, device="cuda", generator=g).to(torch.bfloat16)
+    want = a.double() @ b.double().t()
+    # fp32 sums of K products in any order, |sum of |products|| about 0.8 for unit rows
+    sums = K * 2.0 ** -24
+
+    def close(got, exact, scale=1.0):
+        half_step = 2.0 ** -8 if got.dtype == torch.bfloat16 else 2.0 ** -23
+        err = (got.double() - exact).abs()
+        assert bool((err <= half_step * exact.abs() + scale * sums + 1e-30).all()), err.max()
+
+    out = torch.full((M, N + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    C.gemm_bf16(a, b, out=out[:, :N])
+    close(out[:, :N], want)
+    assert bool((out[:, N:] == 7.0).all())
+    assert torch.equal(C.gemm_bf16(a, b), out[:, :N])      # the order of the sums is fixed
+    close(C.gemm_bf16(a, b, epilogue=C.EPI_FP32), want)
+    close(C.gemm_bf16(a, b, bias=bias), want + bias.double())
+    # d relu2 = 2 |x| dx; the approximate exponentials of the gated forms are good to 1e-6 of |x|
+    close(C.gemm_bf16(a, b, epilogue=C.EPI_RELU2), want.clamp(min=0).square(), 2 * 6)
+    close(C.gemm_bf16(a, b, epilogue=C.EPI_GELU), torch.nn.functional.gelu(want), 2)
+    if N % 64 == 0:
+        parts = want.view(M, N // 64, 2, 32)
+        for epi, act in ((C.EPI_SILU_MUL, torch.nn.functional.silu),
+                         (C.EPI_GELU_MUL, lambda x: torch.nn.functional.gelu(x, approximate="tanh"))):
+            exact = (act(parts[:, :, 0]) * parts[:, :, 1]).reshape(M, N // 2)
+            close(C.gemm_bf16(a, b, epilogue=epi), exact, 2 * 6 + 6 * 6e-6 / sums)
+
+
+def test_captured_in_a_graph():
+    from vllm_gcu_b200.ops import cuda as C
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(5, 512, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(1024, 512, device="cuda", generator=g).to(torch.bfloat16)
+    want = ref.gemm(x, w, out_dtype=torch.float32)
+    out, side, graph = C.gemm_bf16(x, w), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=side):
+        C.gemm_bf16(x, w, out=out)
+    out.zero_()
+    graph.replay()
+    assert (out.float() - want).abs().max() <= 2.0 ** -8 * want.abs().max()

@@ -1,0 +1,379 @@
+// Weight-only quantised GEMM for decode-sized activations:
+//   C[M, N] = A[M, K] * dequant(W)[N, K]^T,  M <= 256, W stored as 4-bit or 8-bit integers with
+// per-group scales: w = q * scale - zs (zs = zero point * scale), groups of g along K.
+//
+// Replaces the reference's `gptq_gemm` / `awq_gemm` ops on the decode path
+// (vllm_gcu/kernels/quantization/awq.py:70-118, gptq.py:95-164).  The layer is bound by its packed
+// bytes (4 bit: 0.53 bytes a weight) and, close behind, by the instructions that de-quantise them:
+// 4.75 per pair of weights, 14 us for the 218 M weights of a Llama-3-8B layer on 148 SMs, 17 us for
+// their bytes at copy bandwidth.
+//
+// The operands are swapped, as in gemm_stream.cu: 128 weight rows are the M side of tcgen05.mma and the
+// activation rows its N side.  TMA brings packed tiles of 128 rows x 128 bytes into a ring; a thread
+// owns one weight row, de-quantises 64 of its weights in registers (4 bit: bf16 pair arithmetic with a
+// single rounding) and stores them into tensor memory, from where tcgen05.mma takes its A operand: no
+// shared-memory stores and no proxy fence per tile, which held the former kernel (bf16 tiles of 64 x 64
+// built in shared memory) at 0.3 us a tile.  Activations come by TMA into a ring of their own.  K is
+// split over a cluster of CTAs that add their partial sums through shared memory (stream.cuh).
+//
+// Roles (384 threads): warp 0 TMA of packed weights, warp 1 tcgen05.mma, warp 2 TMA of activations,
+// warp 3 owner of tensor memory, warps 4..7 and 8..11 de-quantise the even and the odd blocks of 64
+// (warp w can reach the lanes 32 (w mod 4) .. + 31); warps 4..7 move the accumulators out.  Every wait
+// is bounded.
+#include "stream.cuh"
+
+namespace b200 {
+namespace wna16s {
+
+using namespace b200::stream;
+
+constexpr unsigned int kKernelId = 71;
+constexpr int kThreads = 384;
+constexpr int kPackedBytes = BW * 128;   // a packed tile
+constexpr int kMaxPacked = 8, kMaxX = 16;
+constexpr int kBufs = 4;                 // de-quantised blocks in tensor memory, 32 columns each
+
+struct Args {
+  const __nv_bfloat16* scales;    // [N, K / g]
+  const __nv_bfloat16* zs;        // [N, K / g]
+  const __nv_bfloat16* bias;      // optional [N]
+  __nv_bfloat16* C;
+  long long ldc;
+  int M, N, K, g_shift;
+  int rows;                       // activation rows, a multiple of 16
+  int splits, packed_stages, x_stages;
+  unsigned int* status;
+};
+
+// D[tmem] (+)= A[tmem] * B[smem]: lane = row of A, a column = two neighbouring bf16 of its K.
+__device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint64_t desc_b, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "}\n"
+      :
+      : "r"(d), "r"(a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// 8 nibbles, low one first -> 4 bf16 pairs q * s - z.  0x4300 | q is the bf16 number 128 + q, the
+// subtraction of 128 is exact and the fused multiply-add rounds once.  The pairs come out as (0, 4),
+// (1, 5), (2, 6), (3, 7); two byte permutes per four restore the order.
+__device__ __forceinline__ void dequant8(uint32_t q, __nv_bfloat162 s2, __nv_bfloat162 nz2,
+                                         uint32_t* w) {
+  const __nv_bfloat162 k128 = __float2bfloat162_rn(128.0f);
+  uint32_t t[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const uint32_t bits = ((q >> (4 * e)) & 0x000F000Fu) | 0x43004300u;
+    const __nv_bfloat162 v =
+        __hfma2(__hsub2(*reinterpret_cast<const __nv_bfloat162*>(&bits), k128), s2, nz2);
+    t[e] = *reinterpret_cast<const uint32_t*>(&v);
+  }
+  w[0] = __byte_perm(t[0], t[1], 0x5410);
+  w[1] = __byte_perm(t[2], t[3], 0x5410);
+  w[2] = __byte_perm(t[0], t[1], 0x7632);
+  w[3] = __byte_perm(t[2], t[3], 0x7632);
+}
+
+template <int BITS>
+__global__ void __launch_bounds__(kThreads, 2)
+    gemm_wna16_stream_kernel(const __grid_constant__ CUtensorMap tmW,
+                             const __grid_constant__ CUtensorMap tmA, const Args p) {
+  constexpr int kBlocks = BITS == 4 ? 4 : 2;          // blocks of 64 in a packed tile
+  constexpr int kVec = BITS == 4 ? 2 : 4;             // 16-byte words of a row in a block
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* smem_x = smem + p.packed_stages * kPackedBytes;
+  const int x_bytes = p.rows * 128;
+  __shared__ uint64_t pfull[kMaxPacked], pempty[kMaxPacked], xfull[kMaxX], xempty[kMaxX];
+  __shared__ uint64_t afull[kBufs], aempty[kBufs], done_bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ volatile uint32_t abort_word;
+  volatile uint32_t* abort_flag = &abort_word;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int split = static_cast<int>(blockIdx.x);
+  const int n0 = static_cast<int>(blockIdx.y) * BW;
+  uint32_t acc_cols = 32;
+  while (acc_cols < static_cast<uint32_t>(p.rows)) acc_cols <<= 1;
+  const uint32_t cols = acc_cols <= 128 ? 256 : 512;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.packed_stages; ++s) {
+      mbar_init(&pfull[s], 1);
+      mbar_init(&pempty[s], 8);           // one arrival of every de-quantising warp
+    }
+    for (int s = 0; s < p.x_stages; ++s) {
+      mbar_init(&xfull[s], 1);
+      mbar_init(&xempty[s], 1);
+    }
+    for (int s = 0; s < kBufs; ++s) {
+      mbar_init(&afull[s], 4);
+      mbar_init(&aempty[s], 1);
+    }
+    mbar_init(&done_bar, 1);
+    abort_word = 0u;
+    mbar_fence_init();
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmA);
+  }
+  if (warp == 3) {
+    tmem_alloc(&tmem_slot, cols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot, tmem_a = tmem + acc_cols;
+
+  // this CTA's packed tiles, and its blocks of 64 (the last tile of a row may hold fewer)
+  const int total_blocks = p.K / 64;
+  const int total_tiles = (total_blocks + kBlocks - 1) / kBlocks;
+  const int t_lo = static_cast<int>(static_cast<long long>(split) * total_tiles / p.splits);
+  const int t_hi = static_cast<int>(static_cast<long long>(split + 1) * total_tiles / p.splits);
+  const int b_lo = t_lo * kBlocks;
+  const int blocks = min(t_hi * kBlocks, total_blocks) - b_lo;
+
+  if (warp == 0) {
+    if (elect_one()) {
+      int s = 0;
+      uint32_t phase = 0;
+      for (int t = t_lo; t < t_hi; ++t) {
+        if (!mbar_wait(&pempty[s], phase ^ 1u, p.status, kKernelId, 0x100u + s, abort_flag)) break;
+        mbar_expect_tx(&pfull[s], kPackedBytes);
+        tma_load_2d(smem + s * kPackedBytes, &tmW, &pfull[s], t * 128, n0);
+        if (++s == p.packed_stages) {
+          s = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+  } else if (warp == 2) {
+    if (elect_one()) {
+      int s = 0;
+      uint32_t phase = 0;
+      for (int b = 0; b < blocks; ++b) {
+        if (!mbar_wait(&xempty[s], phase ^ 1u, p.status, kKernelId, 0x200u + s, abort_flag)) break;
+        mbar_expect_tx(&xfull[s], x_bytes);
+        tma_load_2d(smem_x + s * x_bytes, &tmA, &xfull[s], (b_lo + b) * 64, 0);
+        if (++s == p.x_stages) {
+          s = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint32_t idesc = make_idesc(BW, p.rows, 1, 1);
+      int s = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int b = 0; b < blocks; ++b) {
+        const int buf = b % kBufs;
+        if (!mbar_wait(&xfull[s], phase, p.status, kKernelId, 0x300u + s, abort_flag) ||
+            !mbar_wait(&afull[buf], static_cast<uint32_t>(b / kBufs) & 1u, p.status, kKernelId,
+                       0x320u + buf, abort_flag)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint64_t xdesc = make_desc_k_sw128(smem_u32(smem_x + s * x_bytes));
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          umma_f16_ts(tmem, tmem_a + buf * 32 + k * 8, xdesc + static_cast<uint64_t>(k * 2), idesc,
+                      (b > 0 || k > 0) ? 1u : 0u);
+        umma_commit(&xempty[s]);
+        umma_commit(&aempty[buf]);
+        if (++s == p.x_stages) {
+          s = 0;
+          phase ^= 1u;
+        }
+      }
+      if (ok) umma_commit(&done_bar);
+    }
+  } else if (warp >= 4) {
+    const int q = warp & 3, group = (warp - 4) >> 2;
+    const int row = q * 32 + lane, n = n0 + row;
+    const uint32_t lane_addr = tmem_a + (static_cast<uint32_t>(q * 32) << 16);
+    const long long groups = p.K >> p.g_shift;
+    // rows past N hold zeros and are never stored: any scale will do
+    const __nv_bfloat16* srow = p.scales + (n < p.N ? n : 0) * groups;
+    const __nv_bfloat16* zrow = p.zs + (n < p.N ? n : 0) * groups;
+    const bool halves = p.g_shift < 6;                // groups of 32: two per block
+    __nv_bfloat16 sc[2], zz[2];                       // of the next block
+    auto fetch = [&](int b) {
+      const int g0 = ((b_lo + b) * 64) >> p.g_shift;
+      sc[0] = srow[g0];
+      zz[0] = zrow[g0];
+      if (halves) {
+        sc[1] = srow[g0 + 1];
+        zz[1] = zrow[g0 + 1];
+      }
+    };
+    if (group < blocks) fetch(group);
+    int s = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = t_lo; t < t_hi && ok; ++t) {
+      if (!mbar_wait(&pfull[s], phase, p.status, kKernelId, 0x400u + s, abort_flag)) break;
+      const uint8_t* tile = smem + s * kPackedBytes + row * 128;
+#pragma unroll 1
+      for (int c = group; c < kBlocks; c += 2) {
+        const int b = (t - t_lo) * kBlocks + c;
+        if (b >= blocks) break;
+        __nv_bfloat162 s2[2], nz2[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          s2[h] = __bfloat162bfloat162(h == 1 && halves ? sc[1] : sc[0]);
+          nz2[h] = __hneg2(__bfloat162bfloat162(h == 1 && halves ? zz[1] : zz[0]));
+        }
+        if (b + 2 < blocks) fetch(b + 2);
+        uint32_t w[32];
+#pragma unroll
+        for (int v = 0; v < kVec; ++v) {
+          const uint4 u = *reinterpret_cast<const uint4*>(tile + (((c * kVec + v) ^ (row & 7)) << 4));
+          const uint32_t words[4] = {u.x, u.y, u.z, u.w};
+          if constexpr (BITS == 4) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) dequant8(words[j], s2[v], nz2[v], w + v * 16 + j * 4);
+          } else {
+            const float fs = __bfloat162float(s2[v >> 1].x), fz = __bfloat162float(nz2[v >> 1].x);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint32_t x = words[j];
+              w[v * 8 + j * 2] = pack_bf16x2(fmaf(static_cast<float>(x & 0xFFu), fs, fz),
+                                             fmaf(static_cast<float>((x >> 8) & 0xFFu), fs, fz));
+              w[v * 8 + j * 2 + 1] = pack_bf16x2(fmaf(static_cast<float>((x >> 16) & 0xFFu), fs, fz),
+                                                 fmaf(static_cast<float>(x >> 24), fs, fz));
+            }
+          }
+        }
+        const int buf = b % kBufs;
+        if (!mbar_wait(&aempty[buf], (static_cast<uint32_t>(b / kBufs) & 1u) ^ 1u, p.status, kKernelId,
+                       0x420u + buf, abort_flag)) {
+          ok = false;
+          break;
+        }
+        __syncwarp();
+        tc_fence_after();
+        tmem_st_32x32(lane_addr + buf * 32, w);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&afull[buf]);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&pempty[s]);
+      if (++s == p.packed_stages) {
+        s = 0;
+        phase ^= 1u;
+      }
+    }
+    __syncwarp();
+    // every ring slot has been consumed when done_bar completes, so the partial sums take their place
+    // (the other de-quantising group has read its last packed tile before its last block was multiplied)
+    if (group == 0) {
+      ok = mbar_wait(&done_bar, 0u, p.status, kKernelId, 0x500u, abort_flag);
+      __syncwarp();
+      tc_fence_after();
+      if (ok) park_sums(tmem, reinterpret_cast<float*>(smem), q, lane, p.M);
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  if (p.splits > 1) cluster_arrive_wait();
+  else __syncthreads();
+  if (abort_word == 0u)
+    sum_rows<false>(smem, split, p.splits, warp, kThreads / 32, lane, p.M, [&](int r, float4 v) {
+      const int col = n0 + 4 * lane;
+      __nv_bfloat16* out = p.C + static_cast<long long>(r) * p.ldc + col;
+      float f[4] = {v.x, v.y, v.z, v.w};
+      if (col + 4 <= p.N && (p.ldc & 3) == 0) {
+        if (p.bias != nullptr)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) f[i] += __bfloat162float(p.bias[col + i]);
+        *reinterpret_cast<uint2*>(out) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
+        return;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (col + i < p.N)
+          out[i] = __float2bfloat16(
+              f[i] + (p.bias != nullptr ? __bfloat162float(p.bias[col + i]) : 0.0f));
+    });
+  // nobody leaves while another CTA may still read its partial sums
+  if (p.splits > 1) cluster_arrive_wait();
+  else __syncthreads();
+  if (warp == 3) tmem_dealloc(tmem, cols);
+}
+
+template <int BITS>
+static int launch(const CUtensorMap& tmW, const CUtensorMap& tmA, Args a, cudaStream_t stream) {
+  static AtOnce table = {};
+  const int* at_once = clusters_at_once(table, gemm_wna16_stream_kernel<BITS>, kThreads);
+  if (at_once == nullptr) return -20;
+  const int tiles = (a.N + BW - 1) / BW;
+  const int packed = (a.K / 64 + (BITS == 4 ? 3 : 1)) / (BITS == 4 ? 4 : 2);
+  const Split sp = plan_split(tiles, packed, 1, at_once);
+  // above 128 rows accumulators and de-quantised blocks fill the tensor memory of an SM
+  const int per_sm = a.rows > 128 ? 1 : sp.per_sm;
+  a.splits = sp.splits;
+  if (per_sm == 1 && sp.per_sm == 2)
+    while (a.splits > 1 && at_once[a.splits] < tiles) --a.splits;
+  a.packed_stages = per_sm == 2 ? 3 : 6;
+  const int room = (per_sm == 2 ? kSmemLimit / 2 - 1024 : kSmemLimit) - 1024;
+  a.x_stages = (room - a.packed_stages * kPackedBytes) / (a.rows * 128);
+  if (a.x_stages > kMaxX) a.x_stages = kMaxX;
+  const int ring = a.packed_stages * kPackedBytes + a.x_stages * a.rows * 128;
+  const int sums = a.rows * BW * 4;
+  const int bytes = (ring > sums ? ring : sums) + 1024;
+  if (a.x_stages < 2 || bytes > kSmemLimit) return -20;
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = launch_config(a.splits, tiles, kThreads, bytes, attr, stream);
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, gemm_wna16_stream_kernel<BITS>, tmW, tmA, a));
+}
+
+}  // namespace wna16s
+}  // namespace b200
+
+// A [M, K] bf16 (row pitch lda), qw [N, K / 2] (low nibble = even k) or [N, K] for 8 bit, scales / zs
+// [N, K / g], C [M, N] bf16.  Returns -20 when the shape is outside what the kernel covers (M > 256,
+// K % 64, group size not a power of two >= 32, misaligned pointers): callers de-quantise and use the
+// bf16 GEMM.
+B200_API int b200_gemm_wna16(const void* A, long long lda, const void* qw, const void* scales,
+                             const void* zs, const void* bias, void* C, long long ldc, int M,
+                             int N, int K, int g, int bits, void* stream) {
+  using namespace b200;
+  using namespace b200::wna16s;
+  if (M <= 0 || N <= 0) return 0;
+  if (M > 256 || K <= 0 || (K % 64) != 0 || g < 32 || (g & (g - 1)) != 0 || (K % g) != 0 ||
+      (bits != 4 && bits != 8) || (lda % 8) != 0 ||
+      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(qw)) & 15))
+    return -20;
+  Args a;
+  a.rows = (M + 15) / 16 * 16;
+  const uint64_t kbytes = static_cast<uint64_t>(bits == 4 ? K / 2 : K);
+  CUtensorMap tmW, tmA;
+  int r = encode_tmap_2d(&tmW, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, qw, static_cast<uint64_t>(N), kbytes,
+                         kbytes, BW, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r != 0) return r < 0 ? -6 : r;
+  r = encode_tmap_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, static_cast<uint64_t>(M),
+                     static_cast<uint64_t>(K), static_cast<uint64_t>(lda) * 2, a.rows, 64,
+                     CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r != 0) return r < 0 ? -6 : r;
+  a.scales = static_cast<const __nv_bfloat16*>(scales);
+  a.zs = static_cast<const __nv_bfloat16*>(zs);
+  a.bias = static_cast<const __nv_bfloat16*>(bias);
+  a.C = static_cast<__nv_bfloat16*>(C);
+  a.ldc = ldc;
+  a.M = M; a.N = N; a.K = K;
+  a.g_shift = 31 - __builtin_clz(static_cast<unsigned>(g));
+  a.status = status_ptr();
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  return bits == 4 ? launch<4>(tmW, tmA, a, s) : launch<8>(tmW, tmA, a, s);
+}

@@ -105,6 +105,22 @@ def _wide2_pays(M: int, Nn: int) -> bool:
     return eff2 * 1.15 >= eff1
 
 
+def _stream_pays(M: int, Nn: int, K: int) -> bool:
+    """Shapes for which the kernel that streams the weights past few rows (gemm_stream.cu) is taken.
+    Measured against the other kernels, us at rows x N x K: up to 32 rows it always wins (1 x 28672
+    x 4096 40.5 : 50.9, 16 x 7168 x 2048 9.7 : 15.0); up to 64 where a CTA has enough K to itself (64
+    x 4096 x 14336 24.6 : 29.5, 64 x 6144 x 4096 14.8 : 16.5, but 64 x 7168 x 2048 11.6 : 10.6); up
+    to 128 for few weight tiles, beyond which the tiles of 256 weight rows read the activations less
+    often (128 x 4096 x 4096 13.5 : 16.2, 128 x 7168 x 16384 48 : 54, but 128 x 28672 x 4096 52 : 50);
+    up to 256 for even fewer (256 x 4096 x 14336 35.5 : 43.9, 256 x 2048 x 4096 12.5 : 16.0, but 256 x
+    6144 x 4096 24 : 20)."""
+    if M <= 32:
+        return True
+    if K < 4096:
+        return False
+    return M <= 64 or (M <= 128 and Nn <= 8192) or (M <= 256 and Nn <= 4096)
+
+
 def _skinny_workspace(device: torch.device):
     """Per (device, stream) split-K workspace: fp32 partial sums + zeroed counters."""
     key = (device.index, torch.cuda.current_stream(device).cuda_stream)
@@ -191,6 +207,15 @@ def _gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = N
             y = ungated_act(y, "relu2" if epilogue == EPI_RELU2 else "gelu")
         out.copy_(y)
         return out
+    if (M <= 256 and epilogue != EPI_RESIDUAL and (epilogue not in _GATED or Nn % 64 == 0)
+            and _stream_pays(M, Nn, K)):
+        rc = N.lib().b200_gemm_stream(ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out),
+                                      out.stride(0), M, Nn, K, ptr(bias), epilogue, stream_ptr())
+        N.launch_count += 1
+        if rc == 0:
+            return out
+        if rc != -20:
+            raise N.NativeError(f"b200_gemm_stream failed with code {rc}")
     if (USE_PAIR_GEMM and PAIR_MIN_M <= M < WIDE2_MIN_M and Nn % 256 == 0 and K % 64 == 0
             and epilogue in _PAIR_EPI
             and -(-M // 256) * (Nn // 256) >= PAIR_MIN_TILES):
