@@ -1,4 +1,4 @@
-"""Times the fused de-quantising GEMM (csrc/gemm_wna16.cu) against de-quantise + bf16 GEMM on
+"""Times the fused de-quantising GEMM (csrc/gemm_wna16_stream.cu) against de-quantise + bf16 GEMM on
 the decode shapes of Llama-3-8B (CUDA events; each shape cycles through enough weight copies
 to exceed L2).
 

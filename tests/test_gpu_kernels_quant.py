@@ -135,7 +135,7 @@ def test_weight_dequant_and_quant_linear(C):
 @pytest.mark.parametrize("M,N,K,g", [(1, 256, 512, 128), (37, 200, 1024, 64), (128, 4096, 4096, 128),
                                      (256, 1024, 2048, 32), (200, 96, 256, 256)])
 def test_fused_wna16_gemm_matches_dequant_reference(C, bits, M, N, K, g):
-    """De-quantising GEMM (gemm_wna16.cu) against fp32 matmul on the de-quantised weights;
+    """De-quantising GEMM (gemm_wna16_stream.cu) against fp32 matmul on the de-quantised weights;
     the weights the kernel builds in shared memory are the ones the stand-alone kernel writes."""
     torch.manual_seed(bits * 100 + M)
     dev = "cuda"

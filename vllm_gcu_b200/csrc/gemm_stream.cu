@@ -19,18 +19,16 @@
 // Roles (192 threads): warp 0 TMA, warp 1 tcgen05.mma and the owner of tensor memory, warps 2..5
 // move the accumulators to shared memory; all six add up and store.  Every wait is bounded; on a
 // wait that runs out the CTA still passes both cluster barriers and leaves.
-#include "common.cuh"
+#include "stream.cuh"
 
 namespace b200 {
 namespace stream {
 
 constexpr unsigned int kKernelId = 70;
-constexpr int BW = 128;                 // weight rows of a tile
 constexpr int kRowBytes = 128;          // bytes of a row in a K block (the swizzle width)
 constexpr int kThreads = 192;
 constexpr int kWBytes = BW * kRowBytes;
 constexpr int kMaxStages = 16;
-constexpr int kMaxSplits = 8;
 
 // as in the other GEMMs of this library
 enum Epi : int {
@@ -49,28 +47,6 @@ struct Args {
   int epi;
   unsigned int* status;
 };
-
-__device__ __forceinline__ void cluster_arrive_wait() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t peer_addr(uint32_t local, uint32_t rank) {
-  uint32_t out;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(local), "r"(rank));
-  return out;
-}
-__device__ __forceinline__ float4 ld_peer4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ float2 ld_peer2(uint32_t addr) {
-  float2 v;
-  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
-  return v;
-}
 
 __global__ void __launch_bounds__(kThreads)
     gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW,
@@ -167,86 +143,49 @@ __global__ void __launch_bounds__(kThreads)
     const int q = warp & 3;
     const bool ok = mbar_wait(&done_bar, 0u, p.status, kKernelId, 0x300u, abort_flag);
     tc_fence_after();
-    if (ok) {
-      float* part = reinterpret_cast<float*>(smem) + q * 32 + lane;
-      const int used = min(p.M - m0, p.rows);
-#pragma unroll 1
-      for (int c = 0; c < used; c += 32) {
-        uint32_t r[32];
-        tmem_ld_32x32(tmem + (static_cast<uint32_t>(q * 32) << 16) + c, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (c + i < used) part[(c + i) * BW] = __uint_as_float(r[i]);
-      }
-    }
+    if (ok)
+      park_sums(tmem, reinterpret_cast<float*>(smem), q, lane, min(p.M - m0, p.rows));
   }
   __syncwarp();
   tc_fence_before();
   if (p.splits > 1) cluster_arrive_wait();
   else __syncthreads();
 
-  // ---------------- sum over the cluster; this CTA owns the rows split, split + splits, ... ---------
-  // all peers' values of a row are on their way before the first is added (a remote load takes some
-  // 250 ns: one after the other they cost 3 us at 128 rows); added up in the order of the K slices
+  // ---------------- sum over the cluster ----------------
   if (abort_word == 0u) {
     const int used = min(p.M - m0, p.rows);
-    const bool gated = p.epi == kSiluMul || p.epi == kGeluMul;
-    // gate and up rows of the weights alternate in blocks of 32: 64 outputs per tile
-    const int c2 = 2 * lane, gate = (c2 >> 5) * 64 + (c2 & 31);
-    const uint32_t own = smem_u32(smem) + (gated ? gate : 4 * lane) * 4;
-    uint32_t peer[kMaxSplits];
-#pragma unroll
-    for (int s = 0; s < kMaxSplits; ++s)
-      peer[s] = s < p.splits ? (p.splits > 1 ? peer_addr(own, s) : own) : 0u;
-    for (int r = split + warp * p.splits; r < used; r += 6 * p.splits) {
-      const long long row = m0 + r;
-      float4 x[kMaxSplits];
-#pragma unroll
-      for (int s = 0; s < kMaxSplits; ++s) {
-        if (s >= p.splits) continue;
-        const uint32_t a = peer[s] + r * (BW * 4);
-        if (gated) {
-          const float2 g = ld_peer2(a), u = ld_peer2(a + 128);
-          x[s] = make_float4(g.x, g.y, u.x, u.y);
-        } else {
-          x[s] = ld_peer4(a);
-        }
-      }
-      float4 v = x[0];
-#pragma unroll
-      for (int s = 1; s < kMaxSplits; ++s) {
-        if (s >= p.splits) continue;
-        v.x += x[s].x; v.y += x[s].y; v.z += x[s].z; v.w += x[s].w;
-      }
-      if (gated) {
-        if ((n0 >> 1) + c2 < (p.N >> 1)) {
-          const uint32_t o = p.epi == kSiluMul
-                                 ? pack_bf16x2(gated_f<false>(v.x, v.z), gated_f<false>(v.y, v.w))
-                                 : pack_bf16x2(gated_f<true>(v.x, v.z), gated_f<true>(v.y, v.w));
-          *reinterpret_cast<uint32_t*>(static_cast<__nv_bfloat16*>(p.C) + row * p.ldc + (n0 >> 1) +
-                                       c2) = o;
-        }
-        continue;
-      }
+    if (p.epi == kSiluMul || p.epi == kGeluMul) {
+      const int col = (n0 >> 1) + 2 * lane;
+      sum_rows<true>(smem, split, p.splits, warp, kThreads / 32, lane, used, [&](int r, float4 v) {
+        if (col >= (p.N >> 1)) return;
+        const uint32_t o = p.epi == kSiluMul
+                               ? pack_bf16x2(gated_f<false>(v.x, v.z), gated_f<false>(v.y, v.w))
+                               : pack_bf16x2(gated_f<true>(v.x, v.z), gated_f<true>(v.y, v.w));
+        *reinterpret_cast<uint32_t*>(static_cast<__nv_bfloat16*>(p.C) +
+                                     static_cast<long long>(m0 + r) * p.ldc + col) = o;
+      });
+    } else {
       const int col = n0 + 4 * lane;
-      if (col >= p.N) continue;
-      if (p.epi == kFp32) {
-        *reinterpret_cast<float4*>(static_cast<float*>(p.C) + row * p.ldc + col) = v;
-        continue;
-      }
-      if (p.epi == kBias) {
-        v.x += __bfloat162float(p.bias[col]);
-        v.y += __bfloat162float(p.bias[col + 1]);
-        v.z += __bfloat162float(p.bias[col + 2]);
-        v.w += __bfloat162float(p.bias[col + 3]);
-      } else if (p.epi == kRelu2) {
-        v = make_float4(relu2_f(v.x), relu2_f(v.y), relu2_f(v.z), relu2_f(v.w));
-      } else if (p.epi == kGelu) {
-        v = make_float4(gelu_f(v.x), gelu_f(v.y), gelu_f(v.z), gelu_f(v.w));
-      }
-      *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.C) + row * p.ldc + col) =
-          make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+      sum_rows<false>(smem, split, p.splits, warp, kThreads / 32, lane, used, [&](int r, float4 v) {
+        if (col >= p.N) return;
+        const long long at = static_cast<long long>(m0 + r) * p.ldc + col;
+        if (p.epi == kFp32) {
+          *reinterpret_cast<float4*>(static_cast<float*>(p.C) + at) = v;
+          return;
+        }
+        if (p.epi == kBias) {
+          v.x += __bfloat162float(p.bias[col]);
+          v.y += __bfloat162float(p.bias[col + 1]);
+          v.z += __bfloat162float(p.bias[col + 2]);
+          v.w += __bfloat162float(p.bias[col + 3]);
+        } else if (p.epi == kRelu2) {
+          v = make_float4(relu2_f(v.x), relu2_f(v.y), relu2_f(v.z), relu2_f(v.w));
+        } else if (p.epi == kGelu) {
+          v = make_float4(gelu_f(v.x), gelu_f(v.y), gelu_f(v.z), gelu_f(v.w));
+        }
+        *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.C) + at) =
+            make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+      });
     }
   }
   // nobody leaves while another CTA may still read its partial sums
@@ -259,84 +198,20 @@ struct Plan {
   int rows, row_tiles, splits, stages;
 };
 
-constexpr int kSmemLimit = 231424;      // of one CTA, 1 KB of it for the alignment of the ring
-
 static int smem_bytes(int rows, int stages) {
   const int ring = stages * (kWBytes + rows * kRowBytes), sums = rows * BW * 4;
   return (ring > sums ? ring : sums) + 1024;
 }
 
-static cudaLaunchConfig_t launch_config(int splits, int tiles, int bytes, cudaLaunchAttribute* attr,
-                                        cudaStream_t stream) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(splits, tiles);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = static_cast<size_t>(bytes);
-  cfg.stream = stream;
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = splits;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = splits > 1 ? 1 : 0;
-  return cfg;
-}
-
-// Clusters of every size that run at the same time with one CTA per SM (148, 74, 45, 33, 26, 22, 15,
-// 15 on a B200: a cluster lies within a group of SMs).  Filled once per device.
-static const int* clusters_at_once(int dev) {
-  static int table[64][kMaxSplits + 1] = {};
-  int* t = table[dev];
-  if (t[1] != 0) return t;
-  if (cudaFuncSetAttribute(gemm_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           kSmemLimit) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  for (int s = kMaxSplits; s >= 1; --s) {
-    cudaLaunchAttribute attr[1];
-    const cudaLaunchConfig_t cfg = launch_config(s, 512, kSmemLimit, attr, nullptr);
-    int n = 0;
-    if (s == 1) n = sm_count();
-    else if (cudaOccupancyMaxActiveClusters(&n, gemm_stream_kernel, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
-    }
-    t[s] = n > 0 || s > 1 ? n : 1;
-  }
-  return t;
-}
-
 // Up to 128 activation rows make one tile, more make tiles of 128 (a split of K costs 512 bytes per
 // row of traffic between the SMs, at about 25 GB/s per SM: it stays below what it saves up to there).
-// Weight tiles beyond the SM count: no split, two CTAs per SM, so that the last wave keeps half of
-// the SMs' rings full (28672 x 4096, 1 row: 40.5 us, 43.0 with one CTA per SM; copy bandwidth 35.9).
-// Fewer: the split that gives the most SMs something to do, one CTA per SM with a ring of 200 KB or two
-// with half of it (6144 x 4096, 48 tiles: two per SM and five slices 12.4 us, one and two slices
-// 12.7; 4096 x 4096, 32 tiles: one and four slices 9.8 us, two and six 10.1).
 static Plan make_plan(int M, int N, int K, const int* at_once) {
   Plan pl;
   pl.row_tiles = (M + 127) / 128;
   pl.rows = ((M + pl.row_tiles - 1) / pl.row_tiles + 15) / 16 * 16;
-  const int tiles = (N + BW - 1) / BW * pl.row_tiles, num_kb = (K + 63) / 64, sms = at_once[1];
-  int per_sm = 2;
-  pl.splits = 1;
-  if (tiles <= sms) {
-    per_sm = 1;
-    double best = 0.0;
-    for (int o = 1; o <= 2; ++o)
-      for (int s = 1; s <= kMaxSplits && s * 4 <= num_kb; ++s) {
-        if (s > 1 && o * at_once[s] < tiles) continue;
-        double use = static_cast<double>(tiles) * s / (o * sms);
-        if (o == 2 && s <= 4) use += 1e-6;           // the same use: two CTAs start sooner
-        if (use > best) {
-          best = use;
-          per_sm = o;
-          pl.splits = s;
-        }
-      }
-  }
-  const int room = (per_sm == 2 ? kSmemLimit / 2 - 1024 : kSmemLimit) - 1024;
+  const Split sp = plan_split((N + BW - 1) / BW * pl.row_tiles, (K + 63) / 64, 4, at_once);
+  pl.splits = sp.splits;
+  const int room = (sp.per_sm == 2 ? kSmemLimit / 2 - 1024 : kSmemLimit) - 1024;
   pl.stages = room / (kWBytes + pl.rows * kRowBytes);
   if (pl.stages > kMaxStages) pl.stages = kMaxStages;
   return pl;
@@ -364,9 +239,8 @@ B200_API int b200_gemm_stream(const void* A, long long lda, const void* W, long 
        reinterpret_cast<uintptr_t>(C)) & 15)
     return -3;
   if (epi == kBias && bias == nullptr) return -5;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -20;
-  const int* at_once = clusters_at_once(dev);
+  static AtOnce table = {};
+  const int* at_once = clusters_at_once(table, gemm_stream_kernel, kThreads);
   if (at_once == nullptr) return -20;
   const Plan pl = make_plan(M, N, K, at_once);
   const int bytes = smem_bytes(pl.rows, pl.stages);
@@ -390,7 +264,7 @@ B200_API int b200_gemm_stream(const void* A, long long lda, const void* W, long 
   a.status = status_ptr();
   cudaLaunchAttribute attr[1];
   const cudaLaunchConfig_t cfg =
-      launch_config(pl.splits, (N + BW - 1) / BW * pl.row_tiles, bytes, attr,
+      launch_config(pl.splits, (N + BW - 1) / BW * pl.row_tiles, kThreads, bytes, attr,
                     static_cast<cudaStream_t>(stream));
   return static_cast<int>(cudaLaunchKernelEx(&cfg, gemm_stream_kernel, tmW, tmA, a));
 }

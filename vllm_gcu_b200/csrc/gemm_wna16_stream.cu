@@ -59,24 +59,23 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint64_t des
       : "memory");
 }
 
-// 8 nibbles, low one first -> 4 bf16 pairs q * s - z.  0x4300 | q is the bf16 number 128 + q, the
-// subtraction of 128 is exact and the fused multiply-add rounds once.  The pairs come out as (0, 4),
-// (1, 5), (2, 6), (3, 7); two byte permutes per four restore the order.
+// 8 nibbles, low one first -> 4 bf16 pairs q * s - z.  A byte permute brings a byte's two nibbles to
+// the low ends of two halves; 0x4300 | q is the bf16 number 128 + q, the subtraction of 128 is exact and
+// the fused multiply-add rounds once.  (The integer pipe, half as wide as the others, is what bounds the
+// kernel: nine of these instructions a word here, eleven when four shifts and masks give the pairs
+// (0, 4), (1, 5), (2, 6), (3, 7) and four permutes restore the order.)
 __device__ __forceinline__ void dequant8(uint32_t q, __nv_bfloat162 s2, __nv_bfloat162 nz2,
                                          uint32_t* w) {
   const __nv_bfloat162 k128 = __float2bfloat162_rn(128.0f);
-  uint32_t t[4];
+  const uint32_t high = q >> 4;
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const uint32_t bits = ((q >> (4 * e)) & 0x000F000Fu) | 0x43004300u;
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t bits =
+        (__byte_perm(q, high, 0x4400u + 0x1111u * j) & 0x000F000Fu) | 0x43004300u;
     const __nv_bfloat162 v =
         __hfma2(__hsub2(*reinterpret_cast<const __nv_bfloat162*>(&bits), k128), s2, nz2);
-    t[e] = *reinterpret_cast<const uint32_t*>(&v);
+    w[j] = *reinterpret_cast<const uint32_t*>(&v);
   }
-  w[0] = __byte_perm(t[0], t[1], 0x5410);
-  w[1] = __byte_perm(t[2], t[3], 0x5410);
-  w[2] = __byte_perm(t[0], t[1], 0x7632);
-  w[3] = __byte_perm(t[2], t[3], 0x7632);
 }
 
 template <int BITS>
@@ -319,13 +318,17 @@ static int launch(const CUtensorMap& tmW, const CUtensorMap& tmA, Args a, cudaSt
   if (at_once == nullptr) return -20;
   const int tiles = (a.N + BW - 1) / BW;
   const int packed = (a.K / 64 + (BITS == 4 ? 3 : 1)) / (BITS == 4 ? 4 : 2);
-  const Split sp = plan_split(tiles, packed, 1, at_once);
-  // above 128 rows accumulators and de-quantised blocks fill the tensor memory of an SM
-  const int per_sm = a.rows > 128 ? 1 : sp.per_sm;
-  a.splits = sp.splits;
-  if (per_sm == 1 && sp.per_sm == 2)
-    while (a.splits > 1 && at_once[a.splits] < tiles) --a.splits;
-  a.packed_stages = per_sm == 2 ? 3 : 6;
+  // Bound by the de-quantising warps, so what counts is that every SM has the same share: two CTAs per
+  // SM and the largest split that one wave takes, down to two packed tiles a slice (four above 32 rows,
+  // where the sums of a slice cost more).  4096 x 14336 at 16 rows: eight slices 22.7 us, four 25.2; at
+  // 128 rows 29.2 and 29.5; 4096 x 4096 at 128 rows: eight 16.6, four 14.4; 6144 x 4096 at 16 rows in
+  // one wave (five) 15.0, in two (six) 19.5.  Above 128 rows accumulators and de-quantised blocks fill
+  // the tensor memory of an SM: one CTA.
+  const int per_sm = a.rows > 128 ? 1 : 2;
+  a.splits = 1;
+  for (int s = 2; s <= kMaxSplits; ++s)
+    if (packed >= s * (a.rows > 32 ? 4 : 2) && tiles <= at_once_for(at_once, s, per_sm)) a.splits = s;
+  a.packed_stages = per_sm == 2 ? 2 : 6;
   const int room = (per_sm == 2 ? kSmemLimit / 2 - 1024 : kSmemLimit) - 1024;
   a.x_stages = (room - a.packed_stages * kPackedBytes) / (a.rows * 128);
   if (a.x_stages > kMaxX) a.x_stages = kMaxX;

@@ -144,6 +144,11 @@ const int* clusters_at_once(AtOnce& table, Kernel kernel, int threads) {
 struct Split {
   int per_sm, splits;
 };
+// Clusters of s at the same time with `per_sm` CTAs per SM: two CTAs of a cluster may share an SM.
+inline int at_once_for(const int* at_once, int s, int per_sm) {
+  if (per_sm == 1) return at_once[s];
+  return (s & 1) ? 2 * at_once[s] : at_once[s / 2];
+}
 inline Split plan_split(int tiles, int blocks, int least, const int* at_once) {
   const int sms = at_once[1];
   if (tiles > sms) return {2, 1};
@@ -151,7 +156,7 @@ inline Split plan_split(int tiles, int blocks, int least, const int* at_once) {
   double most = 0.0;
   for (int o = 1; o <= 2; ++o)
     for (int s = 1; s <= kMaxSplits && s * least <= blocks; ++s) {
-      if (s > 1 && o * at_once[s] < tiles) continue;
+      if (s > 1 && at_once_for(at_once, s, o) < tiles) continue;
       double use = static_cast<double>(tiles) * s / (o * sms);
       if (o == 2 && s <= 4) use += 1e-6;             // the same use: two CTAs start sooner
       if (use > most) {

@@ -251,7 +251,7 @@ class WNA16LinearMethod(LinearMethod):
     """AWQ / GPTQ weight-only quantisation.  Device layout after loading: ``qw`` uint8
     ``[N, K/2]`` (two nibbles per byte, low = even k) or ``[N, K]`` for 8 bit, ``scales``
     and ``zs = zero * scale`` as ``[N, K/g]``.  On the GPU, inputs of up to 256 rows go
-    through the fused de-quantising GEMM (csrc/gemm_wna16.cu); larger ones de-quantise the
+    through the fused de-quantising GEMM (csrc/gemm_wna16_stream.cu); larger ones de-quantise the
     layer into a shared bf16 scratch and run the bf16 tcgen05 GEMM on it."""
 
     _scratch: dict = {}

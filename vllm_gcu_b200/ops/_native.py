@@ -168,8 +168,7 @@ class _Sigs:
                        F, F, I, I, I, I, I, I, I, P]
     b200_memory_step = [P, L, I, P, P, P, P, L, P, P, P, P, F, F, P, P, P, P, P, P, I, P, L, F, F,
                         I, I, I, I, I, I, P]
-    b200_gemm_wna16 = [P, L, P, P, P, P, P, L, I, I, I, I, I, P, P]
-    b200_gemm_wna16_workspace = [I, I, I]
+    b200_gemm_wna16 = [P, L, P, P, P, P, P, L, I, I, I, I, I, P]
     b200_gemm_wna16_grouped = [P, L, P, P, P, P, L, I, I, I, I, I, I, P, P, P, P]
     b200_sample = [P, L, I, I, I, P, P, P, P, P, L, P, P]
     b200_top_k_top_p = [P, L, I, I, I, P, P, P]

@@ -802,7 +802,7 @@ WNA16_FUSED_MAX_M = 256
 def gemm_wna16(x: torch.Tensor, qw: torch.Tensor, scales: torch.Tensor, zs: torch.Tensor,
                group: int, bits: int, bias: Optional[torch.Tensor] = None
                ) -> Optional[torch.Tensor]:
-    """Fused de-quantise + GEMM for decode-sized inputs (gemm_wna16.cu): ``x [M, K]`` bf16,
+    """Fused de-quantise + GEMM for decode-sized inputs (gemm_wna16_stream.cu): ``x [M, K]`` bf16,
     ``qw [N, K/2]`` (4 bit) or ``[N, K]`` (8 bit) uint8, ``scales`` / ``zs`` ``[N, K/g]`` bf16.
     Returns None when the shape is outside what the kernel covers."""
     M, K = x.shape
@@ -811,11 +811,9 @@ def gemm_wna16(x: torch.Tensor, qw: torch.Tensor, scales: torch.Tensor, zs: torc
             or x.stride(1) != 1):
         return None
     out = torch.empty((M, Nn), dtype=x.dtype, device=x.device)
-    nws = int(N.lib().b200_gemm_wna16_workspace(M, Nn, K))
-    ws = torch.empty(nws, dtype=torch.float32, device=x.device) if nws > 0 else None
     rc = N.lib().b200_gemm_wna16(ptr(x), x.stride(0), ptr(qw), ptr(scales), ptr(zs), ptr(bias),
                                  ptr(out), out.stride(0), M, Nn, K, int(group), int(bits),
-                                 ptr(ws), stream_ptr())
+                                 stream_ptr())
     N.launch_count += 1
     if rc == -20:
         return None
