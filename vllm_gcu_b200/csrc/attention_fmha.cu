@@ -75,6 +75,34 @@ struct Args {
   unsigned int* status;
 };
 
+// Sequence and query tile (of 128 rows) number `tile` of the step, by one warp: 32 sequences at a time,
+// all lanes load in parallel, prefix sum of the tile counts inside the warp.  -1: surplus tile.
+__device__ __forceinline__ void find_tile(const Args& a, int tile, int lane, int* seq, int* qt) {
+  int found = -1, base = 0;
+  *qt = 0;
+  for (int b0 = 0; b0 < a.B && found < 0; b0 += 32) {
+    const int b = b0 + lane;
+    int nt_b = 0;
+    if (b < a.B) nt_b = (a.cu_q[b + 1] - a.cu_q[b] + BQ - 1) / BQ;
+    int inc = nt_b;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, inc, d);
+      if (lane >= d) inc += n;
+    }
+    const int start = base + inc - nt_b;
+    const bool mine = nt_b > 0 && tile >= start && tile < start + nt_b;
+    const unsigned int vote = __ballot_sync(0xffffffffu, mine);
+    if (vote != 0u) {
+      const int src = __ffs(vote) - 1;
+      found = b0 + src;
+      *qt = tile - __shfl_sync(0xffffffffu, start, src);
+    }
+    base += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  *seq = found;
+}
+
 // HD below 128 uses the same tiles: the second 64-column half then carries columns of the next
 // head (or zeros) behind HD, which no contraction step and no store touches.
 // MODE 1 (shaped): soft cap, chunk and output columns of Args are in force.  The soft cap is
@@ -128,30 +156,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     tma_prefetch_desc(&tmV);
   }
   if (warp == 2) {
-    // which sequence and query tile this CTA works on: 32 sequences per step, all lanes load
-    // in parallel, prefix sum of the tile counts inside the warp
-    int found = -1, qt = 0, base = 0;
-    for (int b0 = 0; b0 < a.B && found < 0; b0 += 32) {
-      const int b = b0 + lane;
-      int nt_b = 0;
-      if (b < a.B) nt_b = (a.cu_q[b + 1] - a.cu_q[b] + BQ - 1) / BQ;
-      int inc = nt_b;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int n = __shfl_up_sync(0xffffffffu, inc, d);
-        if (lane >= d) inc += n;
-      }
-      const int start = base + inc - nt_b;
-      const bool mine = nt_b > 0 && static_cast<int>(blockIdx.x) >= start &&
-                        static_cast<int>(blockIdx.x) < start + nt_b;
-      const unsigned int vote = __ballot_sync(0xffffffffu, mine);
-      if (vote != 0u) {
-        const int src = __ffs(vote) - 1;
-        found = b0 + src;
-        qt = static_cast<int>(blockIdx.x) - __shfl_sync(0xffffffffu, start, src);
-      }
-      base += __shfl_sync(0xffffffffu, inc, 31);
-    }
+    int found, qt;
+    find_tile(a, static_cast<int>(blockIdx.x), lane, &found, &qt);
     if (lane == 0) {
       s_info[0] = found;
       s_info[1] = qt;
@@ -501,6 +507,14 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
 }
 
+}  // namespace fmha
+}  // namespace b200
+
+#include "attention_fmha_pair.cuh"
+
+namespace b200 {
+namespace fmha {
+
 // Tensor maps are cached per (base, rows, cols, box rows): the KV caches of a model never move.
 struct MapKey {
   const void* base;
@@ -564,6 +578,22 @@ static int launch(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensor
   return static_cast<int>(cudaGetLastError());
 }
 
+static int launch_pair(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
+                       const Args& a, int num_q_tiles, cudaStream_t s) {
+  static bool configured[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !configured[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(
+        fmha_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    configured[dev] = true;
+  }
+  dim3 grid(num_q_tiles, a.Hq / 2);
+  fmha_pair_kernel<<<grid, kThreads, kPairSmemBytes, s>>>(tmQ, tmK, tmV, a);
+  return static_cast<int>(cudaGetLastError());
+}
+
 }  // namespace fmha
 }  // namespace b200
 
@@ -620,6 +650,8 @@ B200_API int b200_fmha_prefill_sink(const void* q, long long ldq, void* out, lon
   } while (0)
   if (slopes != nullptr) B200_FMHA(2);
   if (softcap > 0.0f || chunk > 0 || OD != HD) B200_FMHA(1);
+  // query heads in pairs over one key head: both at once
+  if (HD == 128 && ((Hq / Hkv) & 1) == 0) return launch_pair(tmQ, tmK, tmV, a, num_q_tiles, s);
   B200_FMHA(0);
 #undef B200_FMHA
 }
