@@ -74,3 +74,70 @@ def test_captured_in_a_graph():
     out.zero_()
     graph.replay()
     assert (out.float() - want).abs().max() <= 2.0 ** -8 * want.abs().max()
+
+
+@pytest.mark.parametrize("kind,dtype", [(0, torch.float8_e4m3fn), (2, torch.int8)])
+@pytest.mark.parametrize("N,K", [(8, 16), (136, 144), (640, 5120), (4096, 4112), (19072, 272)])
+def test_eight_bit_operands(kind, dtype, N, K):
+    """One-byte operands with a scale per row and per column; K blocks are 128 wide here."""
+    from vllm_gcu_b200.ops import cuda as C
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+
+    def operand(rows):
+        if dtype == torch.int8:
+            return torch.randint(-127, 128, (rows, K + 16), device="cuda", generator=g).to(dtype)[:, :K]
+        return torch.randn(rows, K + 16, device="cuda", generator=g).to(dtype)[:, :K]
+    w = operand(N)
+    ws = torch.rand(N, device="cuda", generator=g) + 0.5
+    for M in (1, 16, 33, 128, 129, 256):
+        if not C._q8_stream_pays(M, N, K):
+            continue
+        x, xs = operand(M), torch.rand(M, device="cuda", generator=g) + 0.5
+        bias = torch.randn(N, device="cuda", generator=g).to(torch.bfloat16) if M % 2 else None
+        got = C.gemm_q8(x, w, xs, ws, bias, kind)
+        want = x.double() @ w.double().t() * xs.double()[:, None] * ws.double()
+        # fp8 products are exact in 32 bits and summed there (int8: exactly); three roundings of the scaled
+        # sum, then bf16
+        size = (x.double().abs() @ w.double().abs().t()) * xs.double()[:, None] * ws.double()
+        bound = 2.0 ** -8 * want.abs() + (K if kind == 0 else 4) * 2.0 ** -24 * size
+        if bias is not None:
+            want = want + bias.double()
+            bound = bound + 2.0 ** -8 * bias.double().abs()
+        assert bool(((got.double() - want).abs() <= bound + 1e-30).all()), M
+
+
+@pytest.mark.parametrize("act", ["silu_mul", "relu2", "gelu", ""])
+@pytest.mark.parametrize("E,N,K,counts", [
+    (1, 64, 8, [1]), (4, 128, 72, [0, 1, 16, 17]), (5, 320, 264, [128, 0, 129, 300, 2]),
+    (40, 192, 2048, [i % 7 for i in range(40)])])
+def test_experts(E, N, K, counts, act):
+    """Rows sorted by expert in tiles of 128: experts without rows, tiles with 1 .. 128 rows in use, several
+    tiles of one expert; the padding's rows stay as they were."""
+    from vllm_gcu_b200.ops import cuda as C
+    g = torch.Generator(device="cuda").manual_seed(E + N)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[:, None]
+    ids = ids[torch.randperm(len(ids), generator=torch.Generator().manual_seed(1))].to(torch.int32).cuda()
+    sid, eid, used, pos = C.moe_align(ids, E)
+    pairs, pos = ids.numel(), pos.long()
+    assert pairs <= C.GROUPED_STREAM_ROWS * E
+    x = torch.randn(pairs, K, device="cuda", generator=g).to(torch.bfloat16)
+    a = torch.full((sid.numel(), K), float("nan"), device="cuda", dtype=torch.bfloat16)
+    a[pos] = x
+    w = torch.randn(E, N, K, device="cuda", generator=g).div_(math.sqrt(K)).to(torch.bfloat16)
+    scale = torch.rand(sid.numel(), device="cuda", generator=g) if act == "" else None
+    gated = act == "silu_mul"
+    out = torch.full((sid.numel(), N // 2 if gated else N), 7.0, device="cuda", dtype=torch.bfloat16)
+    C.gemm_bf16_grouped(a, w, eid, used, silu_mul=gated, row_scale=scale, out=out,
+                        act="" if gated else act, sorted_ids=sid, pairs=pairs)
+    y = torch.einsum("pk,pnk->pn", x.double(), w[ids[:, 0].long()].double())
+    if gated:
+        parts = y.view(pairs, N // 64, 2, 32)
+        want = (torch.nn.functional.silu(parts[:, :, 0]) * parts[:, :, 1]).reshape(pairs, N // 2)
+    else:
+        want = y.clamp(min=0).square() if act == "relu2" else torch.nn.functional.gelu(y) \
+            if act == "gelu" else y * scale[pos].double()[:, None]
+    err = (out[pos].double() - want).abs()
+    assert bool((err <= 2.0 ** -8 * want.abs() + 12 * K * 2.0 ** -24 + 4e-5).all()), err.max()
+    rest = torch.ones(sid.numel(), dtype=torch.bool, device="cuda")
+    rest[pos] = False
+    assert bool((out[rest] == 7.0).all())

@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   if (p.splits > 1) cluster_arrive_wait();
   else __syncthreads();
   if (abort_word == 0u)
-    sum_rows<false>(smem, split, p.splits, warp, kThreads / 32, lane, p.M, [&](int r, float4 v) {
+    sum_rows<false, false>(smem, split, p.splits, warp, kThreads / 32, lane, p.M, [&](int r, float4 v) {
       const int col = n0 + 4 * lane;
       __nv_bfloat16* out = p.C + static_cast<long long>(r) * p.ldc + col;
       float f[4] = {v.x, v.y, v.z, v.w};

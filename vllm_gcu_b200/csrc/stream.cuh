@@ -52,9 +52,9 @@ __device__ __forceinline__ void park_sums(uint32_t tmem, float* sums, int q, int
 }
 
 // The rows that CTA `split` owns, four columns (GATED: two gate and two up columns, whose weight rows
-// alternate in blocks of 32) a lane, summed in the order of the K slices: store(row, lane, sums).  All
-// peers' values of a row are on their way before the first is added.
-template <bool GATED, typename Store>
+// alternate in blocks of 32) a lane, summed in the order of the K slices: store(row, sums).  All peers'
+// values of a row are on their way before the first is added.  WHOLE: the sums are 32-bit integers.
+template <bool GATED, bool WHOLE, typename Store>
 __device__ __forceinline__ void sum_rows(const void* smem, int split, int splits, int warp, int warps,
                                          int lane, int used, Store store) {
   const int gate = ((2 * lane) >> 5) * 64 + ((2 * lane) & 31);
@@ -80,8 +80,18 @@ __device__ __forceinline__ void sum_rows(const void* smem, int split, int splits
 #pragma unroll
     for (int s = 1; s < kMaxSplits; ++s) {
       if (s >= splits) continue;
-      v.x += x[s].x; v.y += x[s].y; v.z += x[s].z; v.w += x[s].w;
+      if constexpr (WHOLE) {
+        v.x = __int_as_float(__float_as_int(v.x) + __float_as_int(x[s].x));
+        v.y = __int_as_float(__float_as_int(v.y) + __float_as_int(x[s].y));
+        v.z = __int_as_float(__float_as_int(v.z) + __float_as_int(x[s].z));
+        v.w = __int_as_float(__float_as_int(v.w) + __float_as_int(x[s].w));
+      } else {
+        v.x += x[s].x; v.y += x[s].y; v.z += x[s].z; v.w += x[s].w;
+      }
     }
+    if constexpr (WHOLE)
+      v = make_float4(static_cast<float>(__float_as_int(v.x)), static_cast<float>(__float_as_int(v.y)),
+                      static_cast<float>(__float_as_int(v.z)), static_cast<float>(__float_as_int(v.w)));
     store(r, v);
   }
 }

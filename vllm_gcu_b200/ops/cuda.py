@@ -1341,6 +1341,12 @@ def moe_topk(gating: torch.Tensor, k: int, renormalize: bool, n_group: int = 1,
 
 
 GROUP_ROWS = 128        # rows of a tile of the grouped GEMM: one expert each
+#: Up to this many rows per expert on average the experts' weights are streamed past them (gemm_stream.cu)
+#: instead of row tiles of 128 that take their padding along (gemm_bf16.cu).  us of w13 + w2, both
+#: sides: 128 experts of 2048 x 768, 4 rows each 115 + 61 : 210 + 107, 64 rows 141 + 93 : 229 + 114, 256
+#: rows 275 + 226 : 340 + 221; 32 of 7168 x 2048, 32 rows 278 + 150 : 380 + 188, 256 rows 558 + 348 : 641
+#: + 483, 512 rows 1032 + 723 : 1089 + 676.
+GROUPED_STREAM_ROWS = 256
 
 
 def moe_align_cap(num_pairs: int, num_local_experts: int) -> int:
@@ -1367,17 +1373,29 @@ def moe_align(topk_ids: torch.Tensor, num_local_experts: int, cap: Optional[int]
 def gemm_bf16_grouped(a: torch.Tensor, w: torch.Tensor, expert_ids: torch.Tensor,
                       num_valid_rows: torch.Tensor, silu_mul: bool = False,
                       row_scale: Optional[torch.Tensor] = None,
-                      out: Optional[torch.Tensor] = None, act: str = "") -> torch.Tensor:
-    """a ``[M_cap, K]`` expert-sorted rows, w ``[E, N, K]``; ``act``: see :func:`ungated_act`."""
+                      out: Optional[torch.Tensor] = None, act: str = "",
+                      sorted_ids: Optional[torch.Tensor] = None, pairs: int = 0) -> torch.Tensor:
+    """a ``[M_cap, K]`` expert-sorted rows, w ``[E, N, K]``; ``act``: see :func:`ungated_act`.
+    ``sorted_ids [M_cap]`` of ``pairs`` (token, slot) pairs, as :func:`moe_align` gives them: the rows of
+    a tile's padding may then stay unwritten."""
     M_cap, K = a.shape
     E, Nn, _ = w.shape
     assert w.is_contiguous() and a.stride(1) == 1
     out_cols = Nn // 2 if silu_mul else Nn
     if out is None:
         out = torch.empty((M_cap, out_cols), device=a.device, dtype=torch.bfloat16)
+    epi = EPI_SILU_MUL if silu_mul else UNGATED_EPI.get(act, EPI_NONE)
+    if sorted_ids is not None and pairs <= GROUPED_STREAM_ROWS * E:
+        rc = N.lib().b200_gemm_stream_grouped(
+            ptr(a), a.stride(0), ptr(w), K, ptr(out), out.stride(0), M_cap, Nn, K, E, ptr(expert_ids),
+            ptr(num_valid_rows), ptr(sorted_ids), pairs, ptr(row_scale), epi, stream_ptr())
+        N.launch_count += 1
+        if rc == 0:
+            return out
+        if rc != -20:
+            raise N.NativeError(f"b200_gemm_stream_grouped failed with code {rc}")
     call("b200_gemm_bf16_grouped", ptr(a), a.stride(0), ptr(w), K, ptr(out), out.stride(0), M_cap,
-         Nn, K, E, ptr(expert_ids), ptr(num_valid_rows), ptr(row_scale),
-         EPI_SILU_MUL if silu_mul else UNGATED_EPI.get(act, EPI_NONE), stream_ptr())
+         Nn, K, E, ptr(expert_ids), ptr(num_valid_rows), ptr(row_scale), epi, stream_ptr())
     return out
 
 
@@ -1402,8 +1420,9 @@ def fused_experts(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_w: 
     row_w = torch.empty(cap, device=x.device, dtype=torch.float32)
     call("b200_moe_row_weights", ptr(sorted_ids), ptr(topk_w), ptr(npp), ptr(row_w), numel, cap,
          stream_ptr())
-    h = gemm_bf16_grouped(a_sorted, w13, expert_ids, npp, silu_mul=True)
-    y = gemm_bf16_grouped(h, w2, expert_ids, npp, row_scale=row_w)
+    pairs = dict(sorted_ids=sorted_ids, pairs=numel)
+    h = gemm_bf16_grouped(a_sorted, w13, expert_ids, npp, silu_mul=True, **pairs)
+    y = gemm_bf16_grouped(h, w2, expert_ids, npp, row_scale=row_w, **pairs)
     out = torch.empty((T, H), device=x.device, dtype=x.dtype)
     call("b200_moe_unpermute_sum", ptr(y), y.stride(0), ptr(pos_of), ptr(add),
          add.stride(0) if add is not None else 0, ptr(out), H, ptr(valid_tokens), T, k, H,
@@ -1429,8 +1448,9 @@ def input_weighted_experts(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor,
     call("b200_moe_permute_weighted", ptr(x), x.stride(0), ptr(topk_w), ptr(a_sorted), Hp,
          ptr(sorted_ids), ptr(npp), numel, k, H, Hp, cap, DTYPE_CODE[w13.dtype], stream_ptr())
     if w13.dtype == torch.bfloat16:
-        h = gemm_bf16_grouped(a_sorted, w13, expert_ids, npp, silu_mul=True)
-        return gemm_bf16_grouped(h, w2, expert_ids, npp), pos_of
+        ids = dict(sorted_ids=sorted_ids, pairs=T * k)
+        h = gemm_bf16_grouped(a_sorted, w13, expert_ids, npp, silu_mul=True, **ids)
+        return gemm_bf16_grouped(h, w2, expert_ids, npp, **ids), pos_of
     I = I2 // 2
     u = torch.empty((cap, I2), device=x.device, dtype=torch.float32)
     call("b200_grouped_gemm_f32", ptr(a_sorted), Hp, ptr(w13), ptr(u), I2, cap, I2, Hp, E,
@@ -1463,8 +1483,9 @@ def ungated_experts(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, topk_id
         call("b200_moe_permute_any", ptr(x), x.stride(0), ptr(a_sorted), Hp, ptr(sorted_ids),
              ptr(npp), numel, k, H, Hp, cap, DTYPE_CODE[x.dtype], stream_ptr())
     if x.dtype == torch.bfloat16:
-        h = gemm_bf16_grouped(a_sorted, w1, expert_ids, npp, act=act)
-        return gemm_bf16_grouped(h, w2, expert_ids, npp), pos_of
+        ids = dict(sorted_ids=sorted_ids, pairs=T * k)
+        h = gemm_bf16_grouped(a_sorted, w1, expert_ids, npp, act=act, **ids)
+        return gemm_bf16_grouped(h, w2, expert_ids, npp, **ids), pos_of
     h = torch.empty((cap, I), device=x.device, dtype=torch.float32)
     call("b200_grouped_gemm_f32", ptr(a_sorted), Hp, ptr(w1), ptr(h), I, cap, I, Hp, E,
          ptr(expert_ids), ptr(npp), stream_ptr())
@@ -1691,6 +1712,15 @@ def int8_dequant(q: torch.Tensor, scale: torch.Tensor, azp: Optional[torch.Tenso
     return out
 
 
+def _q8_stream_pays(M: int, Nn: int, K: int) -> bool:
+    """Shapes of 8-bit operands for which the weights are streamed past few rows (gemm_stream.cu)
+    instead of tiles of 128 x 128 (gemm_q8.cu).  us at rows x N x K, both sides: 128 x 28672 x 4096
+    32.4 : 37.0, 128 x 6144 x 4096 13.9 : 17.5; above 128 rows while a layer has few weight tiles: 256 x
+    4096 x 14336 23.1 : 33.6, 256 x 4096 x 4096 13.9 : 16.6, but 256 x 6144 x 4096 17.8 : 17.8, 256 x
+    28672 x 4096 51.3 : 49.1."""
+    return M <= 128 or (M <= 256 and Nn <= 4096)
+
+
 def gemm_q8(a: torch.Tensor, b: torch.Tensor, a_scale: torch.Tensor, b_scale: torch.Tensor,
             bias: Optional[torch.Tensor] = None, kind: int = 0,
             out: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -1706,6 +1736,16 @@ def gemm_q8(a: torch.Tensor, b: torch.Tensor, a_scale: torch.Tensor, b_scale: to
     b_scale = b_scale.contiguous()
     lds_a = a_scale.stride(0) if (kind == 1 and a_scale.dim() == 2) else 1
     lds_b = b_scale.stride(0) if (kind == 1 and b_scale.dim() == 2) else 1
+    if kind != 1 and _q8_stream_pays(M, Nn, K) \
+            and not (ptr(a) | ptr(b) | ptr(out)) & 15:
+        rc = N.lib().b200_gemm_stream_q8(ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out),
+                                         out.stride(0), M, Nn, K, ptr(a_scale), ptr(b_scale),
+                                         ptr(bias), kind, stream_ptr())
+        N.launch_count += 1
+        if rc == 0:
+            return out
+        if rc != -20:
+            raise N.NativeError(f"b200_gemm_stream_q8 failed with code {rc}")
     call("b200_gemm_q8", ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out), out.stride(0), M, Nn,
          K, ptr(a_scale), lds_a, ptr(b_scale), lds_b, ptr(bias), kind, stream_ptr())
     return out
