@@ -43,6 +43,9 @@ struct RopeCacheArgs {
   int is_neox;
   int cos_sin_fp32;
   int cache_fp8;   // 0: cache holds T, 1: fp8 e4m3, 2: int8 (symmetric)
+  const void* q_weight;    // optional [D]: RMS norm of every query / key head before its rotation
+  const void* k_weight;
+  float eps;
   unsigned int* status;
 };
 
@@ -66,6 +69,148 @@ __device__ __forceinline__ void rotate_head(T* x, const void* cs, long long cs_r
     x[i0] = from_f32<T>(a * c - b * s);
     x[i1] = from_f32<T>(b * c + a * s);
   }
+}
+
+// Eight columns of a cache row, as the cache stores them.
+template <typename T>
+__device__ __forceinline__ void store_cache8(const RopeCacheArgs& a, bool is_v, long long off,
+                                             const float (&f)[8]) {
+  void* cache = is_v ? a.v_cache : a.k_cache;
+  if (a.cache_fp8 == 0) {
+    vec8_store<T>(static_cast<T*>(cache) + off, f);
+    return;
+  }
+  const float inv = 1.0f / (is_v ? *a.v_scale : *a.k_scale);
+  uint2 pk;
+  uint8_t* b = reinterpret_cast<uint8_t*>(&pk);
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    if (a.cache_fp8 == 2)            // int8, symmetric (zero point 0)
+      b[u] = static_cast<uint8_t>(static_cast<int8_t>(
+          fminf(fmaxf(rintf(f[u] * inv), -128.0f), 127.0f)));
+    else
+      b[u] = f32_to_e4m3(f[u] * inv);
+  }
+  *reinterpret_cast<uint2*>(static_cast<uint8_t*>(cache) + off) = pk;
+}
+
+// Rotation of whole heads (pairs i, i + D / 2), with an RMS norm of every head in front if NORM, and the
+// write of keys and values to the cache, in one pass: a thread holds eight pairs, the LANES = D / 16
+// threads of a head sit side by side in a warp (the norm's sum needs no shared memory), rotated keys
+// go to the cache from registers, values pass by.  Bound by its bytes: 8192 tokens of 32 + 8 + 8 heads of
+// 128 in bf16 read and write 218 MB, 33 us at copy bandwidth; 48 us here, 71 in the kernel below, whose
+// threads load cosines one by one and read the rotated keys back behind a barrier.  With the norms 52 us,
+// where two norm kernels and two copies into dense rows took 115 more (4096 tokens, 32 + 4 heads).
+template <typename T, int LANES, bool NORM>
+__global__ void __launch_bounds__(256) rope_cache_heads_kernel(const RopeCacheArgs a) {
+  const int heads = a.Hq + 2 * a.Hkv;
+  const long long item = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  const long long row = item / LANES;
+  const int t = static_cast<int>(row / heads), h = static_cast<int>(row % heads);
+  const bool live = t < a.T;
+  const int i = static_cast<int>(item % LANES) * 8;
+  constexpr int kHalf = LANES * 8;
+  const bool is_v = h >= a.Hq + a.Hkv, is_q = h < a.Hq;
+  const int kv_head = is_v ? h - a.Hq - a.Hkv : h - a.Hq;
+  T* x = nullptr;
+  float lo[8] = {}, hi[8] = {};
+  if (live) {
+    // (values are only read)
+    x = is_q   ? static_cast<T*>(a.q) + static_cast<long long>(t) * a.ldq + h * (2 * kHalf)
+        : is_v ? const_cast<T*>(static_cast<const T*>(a.v)) + static_cast<long long>(t) * a.ldv +
+                     kv_head * (2 * kHalf)
+               : static_cast<T*>(a.k) + static_cast<long long>(t) * a.ldk + kv_head * (2 * kHalf);
+    vec8_load<T>(x + i, lo);
+    vec8_load<T>(x + kHalf + i, hi);
+  }
+  float scale = 1.0f;
+  if constexpr (NORM) {
+    float ss = 0.0f;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) ss += lo[u] * lo[u] + hi[u] * hi[u];
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    scale = rsqrtf(ss / (2 * kHalf) + a.eps);
+  }
+  if (!live) return;
+  if (!is_v) {
+    if constexpr (NORM) {
+      const T* w = static_cast<const T*>(is_q ? a.q_weight : a.k_weight);
+      float w0[8], w1[8];
+      vec8_load<T>(w + i, w0);
+      vec8_load<T>(w + kHalf + i, w1);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        lo[u] *= scale * w0[u];
+        hi[u] *= scale * w1[u];
+      }
+    }
+    const long long cs = a.positions[t] * (2 * kHalf) + i;
+    float c[8], s[8];
+    if (a.cos_sin_fp32) {
+      const float* tab = static_cast<const float*>(a.cos_sin) + cs;
+#pragma unroll
+      for (int u = 0; u < 8; u += 4) {
+        const float4 cc = *reinterpret_cast<const float4*>(tab + u);
+        const float4 sn = *reinterpret_cast<const float4*>(tab + kHalf + u);
+        c[u] = cc.x; c[u + 1] = cc.y; c[u + 2] = cc.z; c[u + 3] = cc.w;
+        s[u] = sn.x; s[u + 1] = sn.y; s[u + 2] = sn.z; s[u + 3] = sn.w;
+      }
+    } else {
+      vec8_load<T>(static_cast<const T*>(a.cos_sin) + cs, c);
+      vec8_load<T>(static_cast<const T*>(a.cos_sin) + cs + kHalf, s);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float p = lo[u], q = hi[u];
+      lo[u] = round_like<T>(p * c[u] - q * s[u]);
+      hi[u] = round_like<T>(q * c[u] + p * s[u]);
+    }
+    vec8_store<T>(x + i, lo);
+    vec8_store<T>(x + kHalf + i, hi);
+    if (is_q) return;
+  }
+  if (a.slot_mapping == nullptr) return;
+  const long long slot = a.slot_mapping[t];
+  if (slot < 0) return;              // padding token
+  if (slot >= a.num_slots) {
+    if (i == 0) report_status(a.status, kStatusBounds, kKernelId, static_cast<unsigned>(t));
+    return;
+  }
+  const long long off = slot * a.cache_slot_stride + kv_head * a.cache_head_stride + i;
+  store_cache8<T>(a, is_v, off, lo);
+  store_cache8<T>(a, is_v, off + kHalf, hi);
+}
+
+template <typename T, int LANES>
+static void launch_heads(const RopeCacheArgs& a, cudaStream_t s) {
+  const long long items = static_cast<long long>(a.T) * (a.Hq + 2 * a.Hkv) * LANES;
+  const unsigned blocks = static_cast<unsigned>((items + 255) / 256);
+  if (a.q_weight != nullptr) rope_cache_heads_kernel<T, LANES, true><<<blocks, 256, 0, s>>>(a);
+  else rope_cache_heads_kernel<T, LANES, false><<<blocks, 256, 0, s>>>(a);
+}
+
+// What the kernel above takes: query, key and value rows, whole heads of 64, 128 or 256 rotated, all of it
+// in vectors of 16 bytes (an 8-bit cache: 8).
+static bool heads_ok(const RopeCacheArgs& a) {
+  if (!a.is_neox || a.positions == nullptr || a.q == nullptr || a.k == nullptr || a.v == nullptr ||
+      a.rot_dim != a.D || (a.D != 64 && a.D != 128 && a.D != 256) || a.Hq <= 0 || a.Hkv <= 0)
+    return false;
+  if (((a.ldq | a.ldk | a.ldv) & 7) != 0 ||
+      ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) |
+        reinterpret_cast<uintptr_t>(a.v) | reinterpret_cast<uintptr_t>(a.cos_sin)) & 15))
+    return false;
+  if (a.slot_mapping == nullptr) return true;
+  const uintptr_t mask = a.cache_fp8 ? 7 : 15;
+  return ((a.cache_slot_stride | a.cache_head_stride) & 7) == 0 &&
+         ((reinterpret_cast<uintptr_t>(a.k_cache) | reinterpret_cast<uintptr_t>(a.v_cache)) & mask) == 0;
+}
+
+template <typename T>
+static void launch_heads_any(const RopeCacheArgs& a, cudaStream_t s) {
+  if (a.D == 64) launch_heads<T, 4>(a, s);
+  else if (a.D == 128) launch_heads<T, 8>(a, s);
+  else launch_heads<T, 16>(a, s);
 }
 
 template <typename T>
@@ -370,15 +515,18 @@ using namespace b200;
 using namespace b200::cache;
 
 // RoPE (+ cache write).  dtype 0 bf16 / 1 fp16.  Any of q / k / v / positions /
-// slot_mapping may be null to skip that part.  D must be a multiple of 8.
+// slot_mapping may be null to skip that part.  D must be a multiple of 8.  q_weight / k_weight (both or
+// neither): RMS norm of every query and key head over its D columns in front; -20 where the layout does
+// not allow it (nothing is written then).
 B200_API int b200_rope_cache_flash(void* q, long long ldq, void* k, long long ldk, const void* v,
                                    long long ldv, const long long* positions, const void* cos_sin,
                                    int cos_sin_fp32, int rot_dim, int is_neox,
                                    const long long* slot_mapping, void* k_cache, void* v_cache,
                                    long long cache_slot_stride, long long cache_head_stride,
                                    long long num_slots, int cache_fp8, const float* k_scale,
-                                   const float* v_scale, int T, int Hq, int Hkv, int D, int dtype,
-                                   void* stream) {
+                                   const float* v_scale, const void* q_weight,
+                                   const void* k_weight, float eps, int T, int Hq, int Hkv, int D,
+                                   int dtype, void* stream) {
   if (T <= 0) return 0;
   if ((D % 8) != 0 || (rot_dim % 2) != 0 || rot_dim > D) return -2;
   RopeCacheArgs a;
@@ -388,11 +536,18 @@ B200_API int b200_rope_cache_flash(void* q, long long ldq, void* k, long long ld
   a.cache_slot_stride = cache_slot_stride; a.cache_head_stride = cache_head_stride;
   a.num_slots = num_slots; a.T = T; a.Hq = Hq; a.Hkv = Hkv; a.D = D; a.rot_dim = rot_dim;
   a.is_neox = is_neox; a.cos_sin_fp32 = cos_sin_fp32; a.cache_fp8 = cache_fp8;
+  a.q_weight = q_weight; a.k_weight = k_weight; a.eps = eps;
   a.status = status_ptr();
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (dtype != 0 && dtype != 1) return -8;
+  if (heads_ok(a)) {
+    if (dtype == 0) launch_heads_any<__nv_bfloat16>(a, s);
+    else launch_heads_any<__half>(a, s);
+    return static_cast<int>(cudaGetLastError());
+  }
+  if (q_weight != nullptr) return -20;
   if (dtype == 0) rope_cache_flash_kernel<__nv_bfloat16><<<T, 256, 0, s>>>(a);
-  else if (dtype == 1) rope_cache_flash_kernel<__half><<<T, 256, 0, s>>>(a);
-  else return -8;
+  else rope_cache_flash_kernel<__half><<<T, 256, 0, s>>>(a);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -160,13 +160,19 @@ class PagedAttention(nn.Module):
         if kv_cache is None or md.is_dummy:
             # memory profile / keep-alive step of an idle rank: no cache, no attention
             return torch.zeros((T, Hq * D), dtype=qkv.dtype, device=qkv.device)
-        if self.q_norm is not None:     # per-head QK RMSNorm (Qwen3)
-            q = self.q_norm(q.reshape(T, Hq, D)).reshape(T, Hq * D)
-            k = self.k_norm(k.reshape(T, Hkv, D)).reshape(T, Hkv * D)
         k_cache, v_cache = kv_cache[0], kv_cache[1]
         if ops.use_native(qkv) and qkv.dtype in (torch.bfloat16, torch.float16):
             return self._forward_cuda(q, k, v, k_cache, v_cache, md)
+        q, k = self._head_norms(q, k)
         return self._forward_ref(q, k, v, k_cache, v_cache, md)
+
+    def _head_norms(self, q: torch.Tensor, k: torch.Tensor):
+        """Per-head QK RMSNorm (Qwen3)."""
+        if self.q_norm is None:
+            return q, k
+        T, D = q.shape[0], self.head_dim
+        return (self.q_norm(q.reshape(T, self.num_heads, D)).reshape(T, -1),
+                self.k_norm(k.reshape(T, self.num_kv_heads, D)).reshape(T, -1))
 
     def _rope_inputs(self, md: AttentionMetadata, T: int):
         """(positions, cos/sin table) of this step; with M-RoPE the table rows are gathered
@@ -204,9 +210,17 @@ class PagedAttention(nn.Module):
                                              device=q.device)
             ks_t, vs_t = self._scale_t[0:1], self._scale_t[1:2]
             kvq = (self.k_scale, self.v_scale, 0.0, 0.0)
-        C.rope_cache_flash(q, k, v, rope_pos, rope_table,
-                           rot.is_neox if rot is not None else True, D, md.slot_mapping,
-                           k_cache, v_cache, ks_t, vs_t)
+        rope = (rope_pos, rope_table, rot.is_neox if rot is not None else True, D, md.slot_mapping,
+                k_cache, v_cache, ks_t, vs_t)
+        # the norms of query and key heads run in the kernel that rotates them where both are plain RMS
+        # norms of one epsilon in the rows' type
+        qn, kn = self.q_norm, self.k_norm
+        fused = (qn is not None and type(qn) is RMSNorm and type(kn) is RMSNorm and qn.eps == kn.eps
+                 and qn.weight.dtype == q.dtype and kn.weight.dtype == q.dtype
+                 and C.rope_cache_flash(q, k, v, *rope, norms=(qn.weight, kn.weight, qn.eps)))
+        if not fused:
+            q, k = self._head_norms(q, k)
+            C.rope_cache_flash(q, k, v, *rope)
         out = torch.empty((T, Hq * D), dtype=q.dtype, device=q.device)
         nd = md.num_decode_tokens
         if (md.common_prefix_len > 0 and kvq is None and D in (64, 128) and not self.window

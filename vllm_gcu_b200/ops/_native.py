@@ -99,7 +99,7 @@ class _Sigs:
     b200_gemm_bf16 = [P, L, P, L, P, L, I, I, I, P, P, L, I, P]
     b200_norm = [P, L, P, L, P, P, P, L, P, P, P, I, I, F, I, I, I, P]
     b200_activation = [P, L, P, L, P, P, P, P, I, I, I, I, I, F, I, P]
-    b200_rope_cache_flash = [P, L, P, L, P, L, P, P, I, I, I, P, P, P, L, L, L, I, P, P,
+    b200_rope_cache_flash = [P, L, P, L, P, L, P, P, I, I, I, P, P, P, L, L, L, I, P, P, P, P, F,
                              I, I, I, I, I, P]
     b200_reshape_and_cache = [P, L, P, L, P, P, P, L, I, I, I, I, I, I, F, F, F, F, I, P]
     b200_mla_rope_cache = [P, L, L, P, L, L, P, L, P, P, P, L, L, P, P, P, P, P, P, P,

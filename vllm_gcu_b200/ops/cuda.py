@@ -356,9 +356,12 @@ def rope_cache_flash(q: Optional[torch.Tensor], k: Optional[torch.Tensor],
                      k_cache: Optional[torch.Tensor] = None,
                      v_cache: Optional[torch.Tensor] = None,
                      k_scale: Optional[torch.Tensor] = None,
-                     v_scale: Optional[torch.Tensor] = None) -> None:
+                     v_scale: Optional[torch.Tensor] = None,
+                     norms: Optional[tuple] = None) -> bool:
     """In-place RoPE on q ``[T, Hq*D]`` / k ``[T, Hkv*D]`` (views with a row stride are
-    fine) and paged write of k, v into ``[blocks, bs, Hkv, D]`` caches."""
+    fine) and paged write of k, v into ``[blocks, bs, Hkv, D]`` caches.  ``norms = (q_weight, k_weight,
+    eps)``: RMS norm of every query and key head in front (weights ``[D]`` of q's type); False, and
+    nothing is done, where the layout does not allow it."""
     ref_t = q if q is not None else k
     T = ref_t.shape[0]
     D = head_size
@@ -374,13 +377,21 @@ def rope_cache_flash(q: Optional[torch.Tensor], k: Optional[torch.Tensor],
         assert k_cache.stride(1) * bs == k_cache.stride(0), "slots must be evenly strided"
         slot_stride, head_stride, num_slots = k_cache.stride(1), k_cache.stride(2), nb * bs
         fp8 = 1 if k_cache.dtype == FP8 else (2 if k_cache.dtype == torch.int8 else 0)
-    call("b200_rope_cache_flash", ptr(q), q.stride(0) if q is not None else 0, ptr(k),
-         k.stride(0) if k is not None else 0, ptr(v), v.stride(0) if v is not None else 0,
-         ptr(positions), ptr(cos_sin),
-         int(cos_sin is not None and cos_sin.dtype == torch.float32),
-         cos_sin.shape[-1] if cos_sin is not None else 0, int(is_neox), ptr(slot_mapping),
-         ptr(k_cache), ptr(v_cache), slot_stride, head_stride, num_slots, fp8, ptr(k_scale),
-         ptr(v_scale), T, Hq, Hkv, D, DTYPE_CODE[ref_t.dtype], stream_ptr())
+    wq, wk, eps = norms or (None, None, 0.0)
+    rc = N.lib().b200_rope_cache_flash(
+        ptr(q), q.stride(0) if q is not None else 0, ptr(k), k.stride(0) if k is not None else 0,
+        ptr(v), v.stride(0) if v is not None else 0, ptr(positions), ptr(cos_sin),
+        int(cos_sin is not None and cos_sin.dtype == torch.float32),
+        cos_sin.shape[-1] if cos_sin is not None else 0, int(is_neox), ptr(slot_mapping),
+        ptr(k_cache), ptr(v_cache), slot_stride, head_stride, num_slots, fp8, ptr(k_scale),
+        ptr(v_scale), ptr(wq), ptr(wk), float(eps), T, Hq, Hkv, D, DTYPE_CODE[ref_t.dtype],
+        stream_ptr())
+    if rc == -20 and norms is not None:
+        return False
+    N.launch_count += 1
+    if rc != 0:
+        raise N.NativeError(f"b200_rope_cache_flash failed with code {rc}")
+    return True
 
 
 def reshape_and_cache(key, value, k_cache, v_cache, slot_mapping, k_scale=1.0, v_scale=1.0,
