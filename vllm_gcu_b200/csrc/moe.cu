@@ -165,6 +165,7 @@ struct AlignArgs {
   int* expert_ids;          // [cap / 128] expert of every tile, -1 beyond the valid tiles
   int* num_post_pad;        // [1]
   int* pos_of;              // [T * k] position of each pair, -1 if dropped
+  int* tile_rows;           // optional [cap / 128] rows of every tile that hold a pair
   int numel, k, num_local_experts, cap;
   unsigned int* status;
 };
@@ -213,6 +214,8 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const AlignArgs a) {
       e = lo;
     }
     a.expert_ids[b] = e;
+    if (a.tile_rows != nullptr)
+      a.tile_rows[b] = e < 0 ? 0 : min(kTileM, max(0, count[e] - (row - offset[e])));
   }
   __syncthreads();
   for (int i = threadIdx.x; i < a.numel; i += blockDim.x) {
@@ -229,14 +232,16 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const AlignArgs a) {
   }
 }
 
-// A_sorted[pos] = x[sorted_ids[pos] / k]; padding rows are zeroed.  One CTA per row.
+// A_sorted[pos] = x[sorted_ids[pos] / k]; padding rows are zeroed, or left as they are (zero_pads = 0) for
+// products that do not store them.  One CTA per row.
 template <typename T>
 __global__ void __launch_bounds__(256)
     moe_permute_kernel(const T* x, long long ldx, T* out, long long ldo, const int* sorted_ids,
-                       const int* num_post_pad, int numel, int k, int H) {
+                       const int* num_post_pad, int numel, int k, int H, int zero_pads) {
   const int pos = blockIdx.x;
   if (pos >= *num_post_pad) return;
   const int pair = sorted_ids[pos];
+  if (pair >= numel && !zero_pads) return;
   uint4* dst = reinterpret_cast<uint4*>(out + static_cast<long long>(pos) * ldo);
   const int nvec = H >> 3;
   if (pair >= numel) {
@@ -493,13 +498,13 @@ B200_API int b200_moe_topk(const void* gating, long long ldg, const float* bias,
 // cap must be a multiple of 128 and >= numel + num_local_experts * 127 rounded up.
 B200_API int b200_moe_align(const int* topk_ids, const int* expert_map, const int* valid_tokens,
                             int* sorted_ids, int* expert_ids, int* num_post_pad, int* pos_of,
-                            int numel, int k, int num_local_experts, int cap, void* stream) {
+                            int* tile_rows, int numel, int k, int num_local_experts, int cap, void* stream) {
   if (cap <= 0 || (cap % kTileM) != 0 || num_local_experts <= 0 || num_local_experts > 2048)
     return -2;
   AlignArgs a;
   a.topk_ids = topk_ids; a.expert_map = expert_map; a.valid_tokens = valid_tokens;
   a.sorted_ids = sorted_ids; a.expert_ids = expert_ids; a.num_post_pad = num_post_pad;
-  a.pos_of = pos_of; a.numel = numel; a.k = k; a.num_local_experts = num_local_experts;
+  a.pos_of = pos_of; a.tile_rows = tile_rows; a.numel = numel; a.k = k; a.num_local_experts = num_local_experts;
   a.cap = cap; a.status = status_ptr();
   const size_t smem = static_cast<size_t>(3 * num_local_experts + 1) * sizeof(int);
   moe_align_kernel<<<1, 1024, smem, static_cast<cudaStream_t>(stream)>>>(a);
@@ -508,18 +513,18 @@ B200_API int b200_moe_align(const int* topk_ids, const int* expert_map, const in
 
 B200_API int b200_moe_permute(const void* x, long long ldx, void* out, long long ldo,
                               const int* sorted_ids, const int* num_post_pad, int numel, int k,
-                              int H, int cap, int dtype, void* stream) {
+                              int H, int cap, int zero_pads, int dtype, void* stream) {
   if (cap <= 0) return 0;
   if ((H % 8) != 0) return -2;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == 0)
     moe_permute_kernel<__nv_bfloat16><<<cap, 256, 0, s>>>(
         static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_bfloat16*>(out), ldo,
-        sorted_ids, num_post_pad, numel, k, H);
+        sorted_ids, num_post_pad, numel, k, H, zero_pads);
   else if (dtype == 1)
     moe_permute_kernel<__half><<<cap, 256, 0, s>>>(static_cast<const __half*>(x), ldx,
                                                    static_cast<__half*>(out), ldo, sorted_ids,
-                                                   num_post_pad, numel, k, H);
+                                                   num_post_pad, numel, k, H, zero_pads);
   else
     return -8;
   return static_cast<int>(cudaGetLastError());

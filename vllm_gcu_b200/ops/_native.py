@@ -175,8 +175,8 @@ class _Sigs:
     b200_advance_step = [I, I, I, P, P, P, P, P, P, I, I, P]
     b200_feed_tokens = [P, P, P, P, I, P]
     b200_moe_topk = [P, L, P, P, P, I, I, I, I, I, I, I, F, P, I, P, P, I, P]
-    b200_moe_align = [P, P, P, P, P, P, P, I, I, I, I, P]
-    b200_moe_permute = [P, L, P, L, P, P, I, I, I, I, I, P]
+    b200_moe_align = [P, P, P, P, P, P, P, P, I, I, I, I, P]
+    b200_moe_permute = [P, L, P, L, P, P, I, I, I, I, I, I, P]
     b200_moe_permute_any = [P, L, P, L, P, P, I, I, I, I, I, I, P]
     b200_moe_permute_weighted = [P, L, P, P, L, P, P, I, I, I, I, I, I, P]
     b200_grouped_gemm_f32 = [P, L, P, P, L, I, I, I, I, P, P, P]
@@ -192,6 +192,8 @@ class _Sigs:
     b200_gemm_stream = [P, L, P, L, P, L, I, I, I, P, I, P]
     b200_gemm_stream_q8 = [P, L, P, L, P, L, I, I, I, P, P, P, I, P]
     b200_gemm_stream_grouped = [P, L, P, L, P, L, I, I, I, I, P, P, P, I, P, I, P]
+    b200_gemm_pair_rows = [P, L, P, L, P, L, I, I, I, P, I, I, P]
+    b200_gemm_pair_rows_grouped = [P, L, P, L, P, L, I, I, I, I, P, P, P, P, I, P]
     b200_gemm_pair = [P, L, P, L, P, L, I, I, I, P, I, P]
     b200_gemm_pair_split = [P, L, P, L, P, L, I, I, I, P, I, P, P, P]
     b200_gemm_pair_split_workspace = [P, P]

@@ -121,6 +121,23 @@ def _stream_pays(M: int, Nn: int, K: int) -> bool:
     return M <= 64 or (M <= 128 and Nn <= 8192) or (M <= 256 and Nn <= 4096)
 
 
+def _pair_rows(M: int, Nn: int) -> int:
+    """Rows of a tile of the pair kernel with the weights on the M side (gemm_pair_rows.cu), 0 where
+    another kernel is taken.  It pays for rows that would fill tiles of 256 badly, us at rows x N x K
+    against the other kernels: 301 x 28672 x 4096 76 : 89, 301 x 36864 x 7168 140 : 178, 301 x 6144 x 4096
+    22 : 28, 301 x 7168 x 2048 16 : 26, 384 x 28672 x 4096 83 : 93, 440 x 28672 x 4096 90 : 97, 440 x 6144 x
+    4096 23 : 29, but 512 x 28672 x 4096 101 : 98, 256 x 28672 x 4096 61 : 57.  And for enough weight
+    tiles: 301 x 5120 x 2048 17 : 16, 301 x 4096 x 4096 20 : 18.5, 301 x 4096 x 14336 52.7 : 51.  The rows go into
+    as few tiles as there can be, more while all tiles are one round of the pairs (301 x 6144 x 4096 in
+    tiles of 128 rows 22.1, of 160 22.9; 301 x 28672 x 4096 in tiles of 160 76, of 128 85)."""
+    tiles, w = -(-M // 256), -(-Nn // 256)
+    if tiles * 256 < 1.15 * M or w < 24:
+        return 0
+    while w * (tiles + 1) <= 74:
+        tiles += 1
+    return -(-(-(-M // tiles)) // 32) * 32
+
+
 def _skinny_workspace(device: torch.device):
     """Per (device, stream) split-K workspace: fp32 partial sums + zeroed counters."""
     key = (device.index, torch.cuda.current_stream(device).cuda_stream)
@@ -216,6 +233,18 @@ def _gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = N
             return out
         if rc != -20:
             raise N.NativeError(f"b200_gemm_stream failed with code {rc}")
+    if (USE_PAIR_GEMM and 256 < M < WIDE2_MIN_M and epilogue in _PAIR_EPI
+            and (epilogue not in _GATED or Nn % 64 == 0)):
+        rows = _pair_rows(M, Nn)
+        if rows:
+            rc = N.lib().b200_gemm_pair_rows(ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out),
+                                             out.stride(0), M, Nn, K, ptr(bias), epilogue, rows,
+                                             stream_ptr())
+            N.launch_count += 1
+            if rc == 0:
+                return out
+            if rc != -20:
+                raise N.NativeError(f"b200_gemm_pair_rows failed with code {rc}")
     if (USE_PAIR_GEMM and PAIR_MIN_M <= M < WIDE2_MIN_M and Nn % 256 == 0 and K % 64 == 0
             and epilogue in _PAIR_EPI
             and -(-M // 256) * (Nn // 256) >= PAIR_MIN_TILES):
@@ -1352,12 +1381,14 @@ def moe_topk(gating: torch.Tensor, k: int, renormalize: bool, n_group: int = 1,
 
 
 GROUP_ROWS = 128        # rows of a tile of the grouped GEMM: one expert each
-#: Up to this many rows per expert on average the experts' weights are streamed past them (gemm_stream.cu)
-#: instead of row tiles of 128 that take their padding along (gemm_bf16.cu).  us of w13 + w2, both
-#: sides: 128 experts of 2048 x 768, 4 rows each 115 + 61 : 210 + 107, 64 rows 141 + 93 : 229 + 114, 256
-#: rows 275 + 226 : 340 + 221; 32 of 7168 x 2048, 32 rows 278 + 150 : 380 + 188, 256 rows 558 + 348 : 641
-#: + 483, 512 rows 1032 + 723 : 1089 + 676.
-GROUPED_STREAM_ROWS = 256
+#: Up to this many rows per expert on average the experts' weights are streamed past them (gemm_stream.cu),
+#: beyond it pairs of CTAs take up to 256 rows of an expert (gemm_pair_rows.cu; the row tiles of 128 of
+#: gemm_bf16.cu remain for callers without the tiles' row counts).  us of w13 + w2, streamed : pairs :
+#: row tiles of 128, 128 experts of 2048 x 768, 4 rows each 119 + 63 : 131 + 67 : 205 + 106, 32 rows 130 +
+#: 79 : 138 + 72 : 208 + 106, 128 rows 177 + 132 : 159 + 96 : 244 + 138, 512 rows 500 + 429 : 472 + 361 :
+#: 535 + 438; 32 of 7168 x 2048, 16 rows 276 + 142 : 297 + 157 : 341 + 188, 64 rows 301 + 176 : 302 + 167 :
+#: 397 + 202, 256 rows 558 + 411 : 466 + 254 : 633 + 466, 2048 rows 3950 + 2392 : 3570 + 1567 : 4491 + 3449.
+GROUPED_STREAM_ROWS = 64
 
 
 def moe_align_cap(num_pairs: int, num_local_experts: int) -> int:
@@ -1366,8 +1397,10 @@ def moe_align_cap(num_pairs: int, num_local_experts: int) -> int:
 
 def moe_align(topk_ids: torch.Tensor, num_local_experts: int, cap: Optional[int] = None,
               expert_map: Optional[torch.Tensor] = None,
-              valid_tokens: Optional[torch.Tensor] = None):
-    """Returns (sorted_ids [cap], expert_ids [cap/128], num_post_pad [1], pos_of [T*k])."""
+              valid_tokens: Optional[torch.Tensor] = None,
+              tile_rows: Optional[torch.Tensor] = None):
+    """Returns (sorted_ids [cap], expert_ids [cap/128], num_post_pad [1], pos_of [T*k]);
+    ``tile_rows [cap/128]`` int32 takes the rows of every tile that are no padding."""
     T, k = topk_ids.shape
     numel = T * k
     cap = cap or moe_align_cap(numel, num_local_experts)
@@ -1377,7 +1410,8 @@ def moe_align(topk_ids: torch.Tensor, num_local_experts: int, cap: Optional[int]
     npp = torch.empty(1, device=dev, dtype=torch.int32)
     pos_of = torch.empty(max(numel, 1), device=dev, dtype=torch.int32)
     call("b200_moe_align", ptr(topk_ids), ptr(expert_map), ptr(valid_tokens), ptr(sorted_ids),
-         ptr(expert_ids), ptr(npp), ptr(pos_of), numel, k, num_local_experts, cap, stream_ptr())
+         ptr(expert_ids), ptr(npp), ptr(pos_of), ptr(tile_rows), numel, k, num_local_experts, cap,
+         stream_ptr())
     return sorted_ids, expert_ids, npp, pos_of
 
 
@@ -1385,10 +1419,12 @@ def gemm_bf16_grouped(a: torch.Tensor, w: torch.Tensor, expert_ids: torch.Tensor
                       num_valid_rows: torch.Tensor, silu_mul: bool = False,
                       row_scale: Optional[torch.Tensor] = None,
                       out: Optional[torch.Tensor] = None, act: str = "",
-                      sorted_ids: Optional[torch.Tensor] = None, pairs: int = 0) -> torch.Tensor:
+                      sorted_ids: Optional[torch.Tensor] = None, pairs: int = 0,
+                      tile_rows: Optional[torch.Tensor] = None) -> torch.Tensor:
     """a ``[M_cap, K]`` expert-sorted rows, w ``[E, N, K]``; ``act``: see :func:`ungated_act`.
-    ``sorted_ids [M_cap]`` of ``pairs`` (token, slot) pairs, as :func:`moe_align` gives them: the rows of
-    a tile's padding may then stay unwritten."""
+    ``sorted_ids [M_cap]`` of ``pairs`` (token, slot) pairs and ``tile_rows [M_cap / 128]``, as
+    :func:`moe_align` gives them: the rows of a tile's padding are then not read as such and may stay
+    unwritten."""
     M_cap, K = a.shape
     E, Nn, _ = w.shape
     assert w.is_contiguous() and a.stride(1) == 1
@@ -1405,6 +1441,15 @@ def gemm_bf16_grouped(a: torch.Tensor, w: torch.Tensor, expert_ids: torch.Tensor
             return out
         if rc != -20:
             raise N.NativeError(f"b200_gemm_stream_grouped failed with code {rc}")
+    elif tile_rows is not None:
+        rc = N.lib().b200_gemm_pair_rows_grouped(
+            ptr(a), a.stride(0), ptr(w), K, ptr(out), out.stride(0), M_cap, Nn, K, E, ptr(expert_ids),
+            ptr(num_valid_rows), ptr(tile_rows), ptr(row_scale), epi, stream_ptr())
+        N.launch_count += 1
+        if rc == 0:
+            return out
+        if rc != -20:
+            raise N.NativeError(f"b200_gemm_pair_rows_grouped failed with code {rc}")
     call("b200_gemm_bf16_grouped", ptr(a), a.stride(0), ptr(w), K, ptr(out), out.stride(0), M_cap,
          Nn, K, E, ptr(expert_ids), ptr(num_valid_rows), ptr(row_scale), epi, stream_ptr())
     return out
@@ -1424,14 +1469,16 @@ def fused_experts(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_w: 
     E = w13.shape[0]
     numel = T * k
     cap = moe_align_cap(numel, E)
-    sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap, expert_map, valid_tokens)
+    tile_rows = torch.empty(cap // GROUP_ROWS, device=x.device, dtype=torch.int32)
+    sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap, expert_map, valid_tokens,
+                                                    tile_rows)
     a_sorted = torch.empty((cap, H), device=x.device, dtype=x.dtype)
     call("b200_moe_permute", ptr(x), x.stride(0), ptr(a_sorted), H, ptr(sorted_ids), ptr(npp),
-         numel, k, H, cap, DTYPE_CODE[x.dtype], stream_ptr())
+         numel, k, H, cap, 0, DTYPE_CODE[x.dtype], stream_ptr())
     row_w = torch.empty(cap, device=x.device, dtype=torch.float32)
     call("b200_moe_row_weights", ptr(sorted_ids), ptr(topk_w), ptr(npp), ptr(row_w), numel, cap,
          stream_ptr())
-    pairs = dict(sorted_ids=sorted_ids, pairs=numel)
+    pairs = dict(sorted_ids=sorted_ids, pairs=numel, tile_rows=tile_rows)
     h = gemm_bf16_grouped(a_sorted, w13, expert_ids, npp, silu_mul=True, **pairs)
     y = gemm_bf16_grouped(h, w2, expert_ids, npp, row_scale=row_w, **pairs)
     out = torch.empty((T, H), device=x.device, dtype=x.dtype)
@@ -1454,12 +1501,13 @@ def input_weighted_experts(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor,
     E, I2, Hp = w13.shape
     numel = T * k
     cap = moe_align_cap(numel, E)
-    sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap)
+    tile_rows = torch.empty(cap // GROUP_ROWS, device=x.device, dtype=torch.int32)
+    sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap, tile_rows=tile_rows)
     a_sorted = torch.empty((cap, Hp), device=x.device, dtype=w13.dtype)
     call("b200_moe_permute_weighted", ptr(x), x.stride(0), ptr(topk_w), ptr(a_sorted), Hp,
          ptr(sorted_ids), ptr(npp), numel, k, H, Hp, cap, DTYPE_CODE[w13.dtype], stream_ptr())
     if w13.dtype == torch.bfloat16:
-        ids = dict(sorted_ids=sorted_ids, pairs=T * k)
+        ids = dict(sorted_ids=sorted_ids, pairs=T * k, tile_rows=tile_rows)
         h = gemm_bf16_grouped(a_sorted, w13, expert_ids, npp, silu_mul=True, **ids)
         return gemm_bf16_grouped(h, w2, expert_ids, npp, **ids), pos_of
     I = I2 // 2
@@ -1485,16 +1533,17 @@ def ungated_experts(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, topk_id
     E, I, Hp = w1.shape
     numel = T * k
     cap = moe_align_cap(numel, E)
-    sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap)
+    tile_rows = torch.empty(cap // GROUP_ROWS, device=x.device, dtype=torch.int32)
+    sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap, tile_rows=tile_rows)
     a_sorted = torch.empty((cap, Hp), device=x.device, dtype=x.dtype)
     if x.dtype == torch.bfloat16 and H == Hp and H % 8 == 0:
         call("b200_moe_permute", ptr(x), x.stride(0), ptr(a_sorted), Hp, ptr(sorted_ids), ptr(npp),
-             numel, k, H, cap, DTYPE_CODE[x.dtype], stream_ptr())
+             numel, k, H, cap, 1, DTYPE_CODE[x.dtype], stream_ptr())
     else:
         call("b200_moe_permute_any", ptr(x), x.stride(0), ptr(a_sorted), Hp, ptr(sorted_ids),
              ptr(npp), numel, k, H, Hp, cap, DTYPE_CODE[x.dtype], stream_ptr())
     if x.dtype == torch.bfloat16:
-        ids = dict(sorted_ids=sorted_ids, pairs=T * k)
+        ids = dict(sorted_ids=sorted_ids, pairs=T * k, tile_rows=tile_rows)
         h = gemm_bf16_grouped(a_sorted, w1, expert_ids, npp, act=act, **ids)
         return gemm_bf16_grouped(h, w2, expert_ids, npp, **ids), pos_of
     h = torch.empty((cap, I), device=x.device, dtype=torch.float32)
@@ -1545,7 +1594,7 @@ def fused_experts_fp8(x: torch.Tensor, w13: torch.Tensor, w13_scale: torch.Tenso
     sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap, expert_map, valid_tokens)
     a_sorted = torch.empty((cap, H), device=x.device, dtype=x.dtype)
     call("b200_moe_permute", ptr(x), x.stride(0), ptr(a_sorted), H, ptr(sorted_ids), ptr(npp),
-         numel, k, H, cap, DTYPE_CODE[x.dtype], stream_ptr())
+         numel, k, H, cap, 1, DTYPE_CODE[x.dtype], stream_ptr())
     row_w = torch.empty(cap, device=x.device, dtype=torch.float32)
     call("b200_moe_row_weights", ptr(sorted_ids), ptr(topk_w), ptr(npp), ptr(row_w), numel, cap,
          stream_ptr())
@@ -1616,7 +1665,7 @@ def fused_experts_wna16(x: torch.Tensor, q13: torch.Tensor, s13: torch.Tensor, z
     sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap, expert_map, valid_tokens)
     a_sorted = torch.empty((cap, H), device=x.device, dtype=x.dtype)
     call("b200_moe_permute", ptr(x), x.stride(0), ptr(a_sorted), H, ptr(sorted_ids), ptr(npp),
-         numel, k, H, cap, DTYPE_CODE[x.dtype], stream_ptr())
+         numel, k, H, cap, 1, DTYPE_CODE[x.dtype], stream_ptr())
     row_w = torch.empty(cap, device=x.device, dtype=torch.float32)
     call("b200_moe_row_weights", ptr(sorted_ids), ptr(topk_w), ptr(npp), ptr(row_w), numel, cap,
          stream_ptr())
@@ -1661,7 +1710,7 @@ def fused_experts_q8(x: torch.Tensor, w13: torch.Tensor, w13_scale: torch.Tensor
     sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap, expert_map, valid_tokens)
     a_sorted = torch.empty((cap, H), device=x.device, dtype=x.dtype)
     call("b200_moe_permute", ptr(x), x.stride(0), ptr(a_sorted), H, ptr(sorted_ids), ptr(npp),
-         numel, k, H, cap, DTYPE_CODE[x.dtype], stream_ptr())
+         numel, k, H, cap, 1, DTYPE_CODE[x.dtype], stream_ptr())
     row_w = torch.empty(cap, device=x.device, dtype=torch.float32)
     call("b200_moe_row_weights", ptr(sorted_ids), ptr(topk_w), ptr(npp), ptr(row_w), numel, cap,
          stream_ptr())
