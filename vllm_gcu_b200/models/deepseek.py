@@ -141,7 +141,7 @@ class MLAAttention(nn.Module):
         q_nope, q_pe = q[..., : self.nope], q[..., self.nope:]
         q_full = torch.empty((T, N, L + R), dtype=x.dtype, device=x.device)
         # latent query: q_nope x W_UK^T, written straight into the concatenated query
-        q_full[..., :L].copy_(torch.bmm(q_nope.transpose(0, 1), self.w_uk_t).transpose(0, 1))
+        torch.bmm(q_nope.transpose(0, 1), self.w_uk_t, out=q_full[..., :L].transpose(0, 1))
         if ops.use_native(x) and x.dtype in (torch.bfloat16, torch.float16):
             C.mla_rope_cache(q_pe, kv, md.positions, self.cos_sin_cache,
                              self.kv_a_layernorm.weight, cfg.rms_norm_eps, kv_cache,
@@ -173,9 +173,7 @@ class MLAAttention(nn.Module):
                     o_lat[nd + n_pf:] = 0
             elif nd < T:
                 o_lat[nd:] = 0
-            o = torch.bmm(o_lat.transpose(0, 1), self.w_uv).transpose(0, 1).reshape(
-                T, N * self.vdim)
-            return self.o_proj(o)
+            return self.o_proj(self._heads_out(o_lat))
         if nd > 0 and x.is_cuda:
             o_lat[:nd] = mla_decode_batched(q_full[:nd], kv_cache, md.block_tables[:nd],
                                             md.seq_lens[:nd], max(md.max_seq_len, 1), self.scale,
@@ -195,8 +193,13 @@ class MLAAttention(nn.Module):
                                                  self.scale, L)
             if t0 + n < T:
                 o_lat[t0 + n:] = 0
-        o = torch.bmm(o_lat.transpose(0, 1), self.w_uv).transpose(0, 1).reshape(T, N * self.vdim)
-        return self.o_proj(o)
+        return self.o_proj(self._heads_out(o_lat))
+
+    def _heads_out(self, o_lat: torch.Tensor) -> torch.Tensor:
+        """``[T, N, L]`` latent outputs -> ``[T, N * vdim]``; the product writes its rows in place."""
+        o = torch.empty((o_lat.shape[0], self.N, self.vdim), dtype=o_lat.dtype, device=o_lat.device)
+        torch.bmm(o_lat.transpose(0, 1), self.w_uv, out=o.transpose(0, 1))
+        return o.flatten(1)
 
 
 class DeepseekV3ForCausalLM(MoeDecoderLM):
