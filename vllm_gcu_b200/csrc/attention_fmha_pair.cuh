@@ -30,20 +30,6 @@ constexpr int kPairSmemBytes = kPairOffBar + 256 + 1024;
 constexpr uint32_t kPairColO = 256;               // scores of head h: 128 h, outputs 256 + 128 h
 static_assert(kPairSmemBytes <= 232448, "exceeds the shared memory of one CTA");
 
-// D[tmem] (+)= A[tmem] * B[smem]: lane = row of A, a column = two neighbouring bf16 of its K.
-__device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint64_t desc_b, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}\n"
-      :
-      : "r"(d), "r"(a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 __global__ void __launch_bounds__(kThreads, 1)
     fmha_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const Args a) {

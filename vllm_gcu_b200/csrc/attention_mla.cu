@@ -18,16 +18,25 @@
 //
 // A 128 x 512 fp32 output does not fit tensor memory next to the scores, so with L > 256 a tile
 // is worked on by two CTAs (neighbours in blockIdx.x): both compute the scores, each accumulates
-// its part of the output columns.  Shapes of the kernel, by what fits shared memory:
-//   QROWS = 128, two stages   two key tiles and a separate P buffer (W <= 384): loads, score
-//                MMAs of tile j + 1 and softmax of tile j overlap;
-//   QROWS = 128, one stage    one key tile; P in a buffer of its own, or (W = 576: Q takes 144 KB)
-//                in the chunks of the key tile that this CTA's part of V does not need, which
-//                are free once the score MMAs have completed;
+// its part of the output columns.  Two key tiles are in flight and P has a buffer of its own:
+// loads, score MMAs of tile j + 1 and softmax of tile j overlap.  What makes the room for it:
+//   QROWS = 128, W <= 384     nothing;
+//   QROWS = 128, W > 384      the first 384 columns of Q live in tensor memory, next to the output
+//                (256 columns) and one buffer of scores: 192 columns of two bf16 each.  (With all
+//                of Q in shared memory, 144 KB at W = 576, there was one key tile and its load,
+//                score MMAs, softmax and P V ran one after the other.)  The score MMAs read these
+//                columns without shared-memory traffic, which bounds them otherwise: 64 keys are
+//                few for 128 rows;
 //   QROWS = 32   tiles with at most 32 valid rows (decode with up to 32 heads per rank): only
 //                those rows of Q are loaded (the MMA still spans 128 rows and reads whatever
 //                follows in shared memory for the others; rows are independent and the
-//                surplus ones are never stored), which leaves room for two stages at any W.
+//                surplus ones are never stored).
+// A key tile is stored in groups of eight keys, every 64-wide chunk of a group 1 KB: one TMA copy
+// brings eight whole rows of the cache, eight copies a tile.
+// Measured (one key tile with 128 heads, 36 copies of 16 rows x 128 bytes a tile before): 256 requests x
+// 1152 keys, W 576, L 512: 128 heads 286 -> 189 us, 16 heads 219 -> 177; 4 x 2048 new tokens, 128 heads 6778
+// -> 4503 us = 519 TFLOP/s of useful work (the scores are computed twice: 794 in all).
+//
 // Long contexts are split over blockIdx.y; the partial results (normalised output +
 // log-sum-exp per row) are merged by mla_combine_kernel.  Whichever writes the result also applies
 // what a design may have at this point, in fp32: a learnt sink per head in the denominator and an
@@ -48,31 +57,32 @@ constexpr int BQ = 128;        // query rows (token, head) per tile
 constexpr int BKV = 64;        // keys per tile
 constexpr int kMaxL = 512;     // latent width = value width, at most
 constexpr int kMaxW = 576;     // key width, at most
-constexpr int kPage = 16;      // tokens per TMA copy
+constexpr int kPage = 16;      // tokens that are neighbours in the cache
+constexpr int kGroup = 8;      // tokens per TMA copy
+constexpr int kQTmem = 6;      // 64-wide chunks of Q in tensor memory, where they are there
 constexpr int kThreads = 320;
 constexpr int kKChunk = BKV * 128;        // [64 x 64] bf16: 8 KB
-constexpr uint32_t kColS = 0;      // one or two score buffers of 64 columns
-constexpr uint32_t kColO = 128;    // up to 256 columns of output
+constexpr uint32_t kColS = 0;      // one or two score buffers of 64 columns, then the output
+                                   // (up to 256 columns), then Q
 constexpr int kMaxSmem = 227 * 1024;
 
 // Shared memory of one CTA, offsets from a 1024-byte boundary.
 struct Lay {
   int off_k;        // key tiles
-  int off_p;        // probabilities, -1: inside the key tile
+  int off_p;        // probabilities
   int bytes;        // with the slack for the alignment
 };
 constexpr int kOffBar = 0;         // barriers first: Q may be read past its end
 constexpr int kOffX = 128;
 constexpr int kOffQ = 2048;
-static Lay make_lay(int qrows, int stages, int n_w, bool own_p) {
+static Lay make_lay(int qrows, int n_q, int n_w) {
   Lay l;
   const int q_chunk = qrows * 128;
-  l.off_k = kOffQ + n_w * q_chunk;
-  int end = l.off_k + stages * n_w * kKChunk;
-  l.off_p = own_p ? end : -1;
-  if (own_p) end += BQ * 128;
+  l.off_k = kOffQ + n_q * q_chunk;
+  l.off_p = l.off_k + 2 * n_w * kKChunk;
+  const int end = l.off_p + BQ * 128;
   // the 128-row MMA reads 16 KB from the start of every Q chunk: keep that inside the allocation
-  const int read_end = kOffQ + (n_w - 1) * q_chunk + BQ * 128;
+  const int read_end = kOffQ + (n_q - 1) * q_chunk + BQ * 128;
   l.bytes = (end > read_end ? end : read_end) + 1024;
   return l;
 }
@@ -84,6 +94,7 @@ __device__ __forceinline__ float ex2_approx(float x) {
 }
 
 struct Args {
+  const __nv_bfloat16* q;  // [T * N, 64 n_w]
   __nv_bfloat16* out;      // [T * N, L]
   float* ws_o;             // splits > 1: [splits, T * N, L] normalised partial outputs
   float* ws_lse;           // splits > 1: [splits, T * N] natural-log LSE (-inf: nothing seen)
@@ -110,7 +121,7 @@ __device__ __forceinline__ float head_gate(const __nv_bfloat16* gate, long long 
 
 // kResident CTAs share an SM: two where shared and tensor memory allow it (narrow latents, whose
 // tiles are too small to hide the latency of the chain loads -> scores -> softmax -> output)
-template <int QROWS, int kStages, int kResident>
+template <int QROWS, int kQT, int kResident>
 __global__ void __launch_bounds__(kThreads, kResident)
     mla_attn_kernel(const __grid_constant__ CUtensorMap tmQ,
                     const __grid_constant__ CUtensorMap tmK, const Args a) {
@@ -118,7 +129,13 @@ __global__ void __launch_bounds__(kThreads, kResident)
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   constexpr int kQChunk = QROWS * 128;
+  constexpr int kStages = 2;
+  constexpr int kSBufs = kQT > 0 ? 1 : 2;
+  constexpr uint32_t kColO = kColS + kSBufs * BKV;
+  constexpr uint32_t kColQ = kColO + 256;
+  static_assert(kColQ + kQT * 32 <= 512, "exceeds tensor memory");
   const int n_w = a.n_w;
+  const uint32_t group = static_cast<uint32_t>(n_w) * 1024;    // bytes of eight keys
   const int k_tile = n_w * kKChunk;            // bytes of one key tile
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kOffBar);
   uint64_t* q_full = bars;
@@ -146,7 +163,7 @@ __global__ void __launch_bounds__(kThreads, kResident)
   const int tq = BQ / a.N;                     // tokens per tile
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
+    mbar_init(q_full, kQT > 0 ? 9 : 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1);
       mbar_init(&k_empty[i], 1);
@@ -240,19 +257,14 @@ __global__ void __launch_bounds__(kThreads, kResident)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  // without a buffer of their own (one stage) the probabilities live in two chunks of the key
-  // tile that this CTA's part of V does not use
-  uint8_t* p_smem = a.off_p >= 0 ? smem + a.off_p
-                                 : smem + a.off_k + (half == 0 ? n_l0 : 0) * kKChunk;
+  uint8_t* p_smem = smem + a.off_p;
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    // (One thread issues the 36 copies of a key tile; issuing them from all lanes of the warp
-    // measured 25 % slower.)
     if (elect_one()) {
-      mbar_expect_tx(q_full, n_w * kQChunk);
-      for (int c = 0; c < n_w; ++c)
-        tma_load_2d(smem + kOffQ + c * kQChunk, &tmQ, q_full, c * 64, static_cast<int>(row0));
+      mbar_expect_tx(q_full, (n_w - kQT) * kQChunk);
+      for (int c = kQT; c < n_w; ++c)
+        tma_load_2d(smem + kOffQ + (c - kQT) * kQChunk, &tmQ, q_full, c * 64, static_cast<int>(row0));
       const int* bt = a.block_tables + static_cast<long long>(seq) * a.max_blocks;
       const int last_tok = seq_len - 1;
       for (int j = 0; j < nt; ++j) {
@@ -266,19 +278,19 @@ __global__ void __launch_bounds__(kThreads, kResident)
           const int tok = min(key0 + pg * kPage, last_tok);     // pages past the end: any valid page
           const int blk = bt[tok / a.block_size];
           const int y = blk * a.block_size + ((key0 + pg * kPage) % a.block_size);
-          for (int c = 0; c < n_w; ++c)
-            tma_load_2d(smem + a.off_k + st * k_tile + c * kKChunk + pg * (kPage * 128), &tmK,
-                        &k_full[st], c * 64, y);
+          for (int g = 0; g < kPage / kGroup; ++g)
+            tma_load_3d(smem + a.off_k + st * k_tile + (pg * (kPage / kGroup) + g) * group, &tmK,
+                        &k_full[st], 0, y + g * kGroup, 0);
         }
         // While this tile is worked on, pull the next one into L2: its load then pays an L2
-        // latency instead of an HBM latency (with one stage that load is on the critical path).
+        // latency instead of an HBM latency.
         if (j + 1 < nt) {
           const int nkey0 = (t0 + j + 1) * BKV;
           for (int pg = 0; pg < BKV / kPage; ++pg) {
             if (nkey0 + pg * kPage > last_tok) break;
             const int blk = bt[(nkey0 + pg * kPage) / a.block_size];
             const int y = blk * a.block_size + ((nkey0 + pg * kPage) % a.block_size);
-            for (int c = 0; c < n_w; ++c) tma_prefetch_2d(&tmK, c * 64, y);
+            for (int g = 0; g < kPage / kGroup; ++g) tma_prefetch_3d(&tmK, 0, y + g * kGroup, 0);
           }
         }
       }
@@ -295,37 +307,49 @@ __global__ void __launch_bounds__(kThreads, kResident)
         const uint32_t use = static_cast<uint32_t>(j / kStages);
         if (!mbar_wait(&k_full[st], use & 1u, a.status, kKernelId, 0x210u + st, abort_flag))
           return false;
-        if (kStages == 2 && j >= 2 &&
-            !mbar_wait(&s_empty[st], (use - 1u) & 1u, a.status, kKernelId, 0x230u + st, abort_flag))
+        if (j >= kSBufs &&
+            !mbar_wait(&s_empty[j % kSBufs], static_cast<uint32_t>(j / kSBufs - 1) & 1u, a.status,
+                       kKernelId, 0x230u + st, abort_flag))
           return false;
         tc_fence_after();
         const uint32_t k_addr = smem_u32(smem + a.off_k + st * k_tile);
+        const uint32_t col = tmem_base + kColS + j % kSBufs * BKV;
+        if constexpr (kQT > 0) {
+#pragma unroll
+          for (int c = 0; c < kQT; ++c) {
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks)
+              umma_f16_ts(col, tmem_base + kColQ + c * 32 + ks * 8,
+                          make_desc_k_sw128(k_addr + c * 1024, group) + static_cast<uint64_t>(ks * 2),
+                          kIdescS, (c > 0 || ks > 0) ? 1u : 0u);
+          }
+        }
 #pragma unroll 1
-        for (int c = 0; c < n_w; ++c) {
+        for (int c = kQT; c < n_w; ++c) {
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks)
-            umma_f16(tmem_base + kColS + st * BKV,
-                     make_desc_k_sw128(q_addr + c * kQChunk) + static_cast<uint64_t>(ks * 2),
-                     make_desc_k_sw128(k_addr + c * kKChunk) + static_cast<uint64_t>(ks * 2),
+            umma_f16(col, make_desc_k_sw128(q_addr + (c - kQT) * kQChunk) + static_cast<uint64_t>(ks * 2),
+                     make_desc_k_sw128(k_addr + c * 1024, group) + static_cast<uint64_t>(ks * 2),
                      kIdescS, (c > 0 || ks > 0) ? 1u : 0u);
         }
-        umma_commit(&s_full[st]);
+        umma_commit(&s_full[j % kSBufs]);
         return true;
       };
       bool ok = mbar_wait(q_full, 0, a.status, kKernelId, 0x200u, abort_flag);
       ok = ok && issue_s(0);
       for (int j = 0; ok && j < nt; ++j) {
-        // Two stages: the scores of tile j + 1 and P V of tile j are issued in whichever order
-        // their inputs arrive.  (The key tile j + 1 could only be requested after P V of tile
-        // j - 1 had finished; waiting for it first would hold back P V of tile j.)
-        bool s_pending = kStages == 2 && j + 1 < nt;
+        // The scores of tile j + 1 and P V of tile j are issued in whichever order their inputs
+        // arrive.  (The key tile j + 1 could only be requested after P V of tile j - 1 had
+        // finished; waiting for it first would hold back P V of tile j.)
+        bool s_pending = j + 1 < nt;
         const int st = j % kStages;
         if (s_pending) {
           const int st1 = (j + 1) % kStages;
           const uint32_t use1 = static_cast<uint32_t>((j + 1) / kStages);
+          const uint32_t s_phase = static_cast<uint32_t>((j + 1) / kSBufs - 1) & 1u;
           for (uint32_t it = 0; it < kMbarSpinLimit; ++it) {
             if (mbar_test(&k_full[st1], use1 & 1u) &&
-                (j + 1 < 2 || mbar_test(&s_empty[st1], (use1 - 1u) & 1u))) {
+                (j + 1 < kSBufs || mbar_test(&s_empty[(j + 1) % kSBufs], s_phase))) {
               ok = issue_s(j + 1);            // its waits return at once
               s_pending = false;
               break;
@@ -338,15 +362,15 @@ __global__ void __launch_bounds__(kThreads, kResident)
         if (!mbar_wait(p_full, j & 1, a.status, kKernelId, 0x220u, abort_flag)) break;
         tc_fence_after();
         const uint32_t k_addr = smem_u32(smem + a.off_k + st * k_tile);
-        const uint64_t vdesc = make_desc_mn_sw128(k_addr + c0 * kKChunk, kKChunk);
+        const uint64_t vdesc = make_desc_mn_sw128(k_addr + c0 * 1024, 1024, group);
 #pragma unroll
         for (int ks = 0; ks < BKV / 16; ++ks)
           umma_f16(tmem_base + kColO, make_desc_k_sw128(p_addr) + static_cast<uint64_t>(ks * 2),
-                   vdesc + static_cast<uint64_t>(ks) * (2048 >> 4), idesc_o,
+                   vdesc + static_cast<uint64_t>(ks) * (group >> 3), idesc_o,
                    (j > 0 || ks > 0) ? 1u : 0u);
         umma_commit(&k_empty[st]);
         umma_commit(o_done);
-        if ((kStages == 1 || s_pending) && j + 1 < nt) ok = issue_s(j + 1);
+        if (s_pending) ok = issue_s(j + 1);
       }
     }
   } else {
@@ -366,12 +390,33 @@ __global__ void __launch_bounds__(kThreads, kResident)
       if (a.sink != nullptr) sink2 = a.sink[head] * 1.4426950408889634f;
       gate = head_gate(a.gate, a.ldg, static_cast<long long>(q_start) + tok0 + tok, head);
     }
+    if constexpr (kQT > 0) {
+      // this row's half of the columns of Q that tensor memory takes
+      const bool there = row0 + r < rows_total;
+      const uint4* src = reinterpret_cast<const uint4*>(
+          a.q + (there ? row0 + r : row0) * (64 * n_w) + g * (kQT * 32));
+#pragma unroll
+      for (int c = 0; c < kQT / 2; ++c) {
+        uint32_t w[32];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const uint4 u = src[c * 8 + i];
+          w[4 * i] = there ? u.x : 0u; w[4 * i + 1] = there ? u.y : 0u;
+          w[4 * i + 2] = there ? u.z : 0u; w[4 * i + 3] = there ? u.w : 0u;
+        }
+        tmem_st_32x32(lane_addr + kColQ + (g * (kQT / 2) + c) * 32, w);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(q_full);
+    }
     float m_used = -INFINITY, l = 0.0f;
     float* xch = reinterpret_cast<float*>(smem + kOffX);    // [2][128]
     bool ok = true;
     for (int j = 0; j < nt; ++j) {
-      const int st = j % kStages;
-      if (ok && !mbar_wait(&s_full[st], static_cast<uint32_t>(j / kStages) & 1u, a.status,
+      const int st = j % kSBufs;
+      if (ok && !mbar_wait(&s_full[st], static_cast<uint32_t>(j / kSBufs) & 1u, a.status,
                            kKernelId, 0x300u + st, abort_flag))
         ok = false;
       tc_fence_after();
@@ -383,6 +428,9 @@ __global__ void __launch_bounds__(kThreads, kResident)
       if (ok) {
         tmem_ld_32x32(lane_addr + kColS + st * BKV + g * 32, v);
         tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_empty[st]);       // the scores of another tile may follow
         if (need_mask) {
 #pragma unroll
           for (int i = 0; i < 32; ++i)
@@ -420,18 +468,12 @@ __global__ void __launch_bounds__(kThreads, kResident)
       }
       l = l * alpha + rs;
       m_used = m_new;
-      if (kStages == 2) {
-        tc_fence_before();
-        __syncwarp();
-        if (ok && lane == 0) mbar_arrive(&s_empty[st]);
-        // the previous P V product must be complete before P is overwritten / O is rescaled
-        if (ok && j > 0 &&
-            !mbar_wait(o_done, (j - 1) & 1, a.status, kKernelId, 0x310u, abort_flag))
-          ok = false;
-        tc_fence_after();
-      }
-      // (One stage: the previous P V product is complete already, the key tile of this
-      // iteration was loaded only after it.)  Rescale the accumulator when the maximum rose.
+      // the previous P V product must be complete before P is overwritten / O is rescaled
+      if (ok && j > 0 &&
+          !mbar_wait(o_done, (j - 1) & 1, a.status, kKernelId, 0x310u, abort_flag))
+        ok = false;
+      tc_fence_after();
+      // Rescale the accumulator when the maximum rose.
       if (ok && j > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
 #pragma unroll 1
         for (int c = 0; c < nc; ++c) {
@@ -573,9 +615,13 @@ static int get_map(const void* base, unsigned long long rows, int W, int box_row
     }
   }
   CUtensorMap m;
-  int r = encode_tmap_2d(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, rows, W,
-                         static_cast<unsigned long long>(W) * 2, box_rows, 64,
-                         CU_TENSOR_MAP_SWIZZLE_128B);
+  const unsigned long long pitch = static_cast<unsigned long long>(W) * 2;
+  // the cache in whole rows, every 64-wide chunk of the box's rows by itself
+  const int r = cache_it ? encode_tmap_3d(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, W / 64, rows,
+                                          64, 128, pitch, W / 64, box_rows, 64,
+                                          CU_TENSOR_MAP_SWIZZLE_128B)
+                         : encode_tmap_2d(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, rows, W,
+                                          pitch, box_rows, 64, CU_TENSOR_MAP_SWIZZLE_128B);
   if (r != 0) return r;
   if (cache_it) {
     if (cache.size() > 4096) cache.clear();
@@ -591,19 +637,19 @@ static int get_map(const void* base, unsigned long long rows, int W, int box_row
 namespace b200 {
 namespace mla {
 
-template <int QROWS, int STAGES, int RESIDENT>
+template <int QROWS, int QT, int RESIDENT>
 static int launch(const CUtensorMap& tmQ, const CUtensorMap& tmK, const Args& a, dim3 grid,
                   int smem, cudaStream_t s) {
   static int configured[64] = {0};       // largest size allowed so far, per device
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && configured[dev] < smem) {
-    cudaError_t e = cudaFuncSetAttribute(mla_attn_kernel<QROWS, STAGES, RESIDENT>,
+    cudaError_t e = cudaFuncSetAttribute(mla_attn_kernel<QROWS, QT, RESIDENT>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
     configured[dev] = smem;
   }
-  mla_attn_kernel<QROWS, STAGES, RESIDENT><<<grid, kThreads, smem, s>>>(tmQ, tmK, a);
+  mla_attn_kernel<QROWS, QT, RESIDENT><<<grid, kThreads, smem, s>>>(tmQ, tmK, a);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -637,23 +683,17 @@ B200_API int b200_mla_attention(const void* q, void* out, const void* cache, lon
   // tiles with at most 32 valid rows (decode, up to 32 heads): the variant that loads only
   // those rows of Q and double-buffers the key tiles
   const bool small = cu_q == nullptr && N <= 32;
-  int stages = 2;
-  Lay lay = make_lay(small ? 32 : BQ, 2, n_w, true);
-  if (lay.bytes > kMaxSmem) {
-    stages = 1;
-    lay = make_lay(BQ, 1, n_w, true);
-    if (lay.bytes > kMaxSmem) {
-      if (n_l < 4) return -20;           // P needs two chunks outside the CTA's part of V
-      lay = make_lay(BQ, 1, n_w, false);
-    }
-  }
+  Lay lay = make_lay(small ? 32 : BQ, n_w, n_w);
+  const bool q_tmem = lay.bytes > kMaxSmem;
+  if (q_tmem) lay = make_lay(BQ, n_w - kQTmem, n_w);
   if (lay.bytes > kMaxSmem) return -20;
   CUtensorMap tmQ, tmK;
   int r = get_map(q, static_cast<unsigned long long>(T) * N, W, small ? 32 : BQ, false, &tmQ);
   if (r != 0) return r < 0 ? -6 : r;
-  r = get_map(cache, static_cast<unsigned long long>(num_slots), W, kPage, true, &tmK);
+  r = get_map(cache, static_cast<unsigned long long>(num_slots), W, kGroup, true, &tmK);
   if (r != 0) return r < 0 ? -6 : r;
   Args a;
+  a.q = static_cast<const __nv_bfloat16*>(q);
   a.out = static_cast<__nv_bfloat16*>(out);
   const long long rows_total = static_cast<long long>(T) * N;
   a.ws_o = workspace;
@@ -663,18 +703,18 @@ B200_API int b200_mla_attention(const void* q, void* out, const void* cache, lon
   a.block_size = block_size; a.splits = splits; a.scale = scale;
   a.L = L; a.n_w = n_w; a.n_l = n_l; a.halves = n_l > 4 ? 2 : 1;
   a.off_k = lay.off_k; a.off_p = lay.off_p;
-  a.tmem_cols = (a.halves == 2 ? (n_l + 1) / 2 : n_l) <= 2 ? 256 : 512;
+  a.tmem_cols = !q_tmem && (a.halves == 2 ? (n_l + 1) / 2 : n_l) <= 2 ? 256 : 512;
   a.sink = sink; a.gate = static_cast<const __nv_bfloat16*>(gate); a.ldg = ldg;
   a.status = status_ptr();
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   dim3 grid(num_tiles * a.halves, splits);
-  const bool pair = stages == 2 && a.tmem_cols == 256 && lay.bytes <= kMaxSmem / 2 - 1024;
+  const bool pair = a.tmem_cols == 256 && lay.bytes <= kMaxSmem / 2 - 1024;
   int e;
-  if (small) e = pair ? launch<32, 2, 2>(tmQ, tmK, a, grid, lay.bytes, s)
-                      : launch<32, 2, 1>(tmQ, tmK, a, grid, lay.bytes, s);
-  else if (stages == 2) e = pair ? launch<BQ, 2, 2>(tmQ, tmK, a, grid, lay.bytes, s)
-                                 : launch<BQ, 2, 1>(tmQ, tmK, a, grid, lay.bytes, s);
-  else e = launch<BQ, 1, 1>(tmQ, tmK, a, grid, lay.bytes, s);
+  if (small) e = pair ? launch<32, 0, 2>(tmQ, tmK, a, grid, lay.bytes, s)
+                      : launch<32, 0, 1>(tmQ, tmK, a, grid, lay.bytes, s);
+  else if (!q_tmem) e = pair ? launch<BQ, 0, 2>(tmQ, tmK, a, grid, lay.bytes, s)
+                             : launch<BQ, 0, 1>(tmQ, tmK, a, grid, lay.bytes, s);
+  else e = launch<BQ, kQTmem, 1>(tmQ, tmK, a, grid, lay.bytes, s);
   if (e != 0 || splits == 1) return e;
   mla_combine_kernel<<<static_cast<unsigned>(rows_total), L / 4, 0, s>>>(
       a.ws_o, a.ws_lse, a.out, rows_total, splits, L, N, a.sink, a.gate, ldg);

@@ -149,6 +149,13 @@ __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* m, int32_t x,
                : "memory");
 }
 
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* m, int32_t x, int32_t y, int32_t z) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];"
+               :
+               : "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
+
 __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m, uint64_t* bar,
                                             int32_t x, int32_t y, int32_t z) {
   asm volatile(
@@ -218,6 +225,19 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint6
       "}\n"
       :
       : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// 16-bit operands with A in tensor memory: lane = row of A, a column = two neighbours of its K.
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b,
+                                            uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "}\n"
+      :
+      : "r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // fp8 (e4m3 / e5m2) operands, fp32 accumulation, K = 32 per instruction.
@@ -322,11 +342,12 @@ __device__ __forceinline__ void fence_async_smem() {
 // rows form one 1024-byte swizzle atom; atoms follow each other along M/N
 // (stride byte offset 1024).  The tile base must be 1024-byte aligned; a K
 // step inside the atom is a plain byte advance of the start address.
-__device__ __forceinline__ uint64_t make_desc_k_sw128(uint32_t smem_addr) {
+__device__ __forceinline__ uint64_t make_desc_k_sw128(uint32_t smem_addr,
+                                                      uint32_t group_bytes = 1024) {
   uint64_t d = 0;
   d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);  // start address
   d |= static_cast<uint64_t>(1) << 16;                       // leading byte offset (unused)
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;               // stride byte offset
+  d |= static_cast<uint64_t>(group_bytes >> 4) << 32;        // stride byte offset: eight rows
   d |= static_cast<uint64_t>(1) << 46;                       // descriptor version (sm_100)
   d |= static_cast<uint64_t>(2) << 61;                       // SWIZZLE_128B
   return d;
@@ -334,15 +355,16 @@ __device__ __forceinline__ uint64_t make_desc_k_sw128(uint32_t smem_addr) {
 
 // Descriptor of an MN-major operand tile (the contraction index runs over rows of 128 bytes,
 // 64 elements of the M/N extent are contiguous in a row; this is how a [keys, head_dim] value
-// tile lands in shared memory under TMA SWIZZLE_128B).  Eight rows form a 1024-byte atom and
-// atoms follow each other along K (stride byte offset 1024); the next 64 elements of the M/N
-// extent start `mn_chunk_bytes` further (leading byte offset).  A step of 16 along K advances
-// the start address by 2048 bytes.  Needs the MN-major bit of the instruction descriptor.
-__device__ __forceinline__ uint64_t make_desc_mn_sw128(uint32_t smem_addr, uint32_t mn_chunk_bytes) {
+// tile lands in shared memory under TMA SWIZZLE_128B).  Eight rows form a 1024-byte atom; the
+// next eight along K start `group_bytes` further (stride byte offset), the next 64 elements of
+// the M/N extent `mn_chunk_bytes` further (leading byte offset).  A step of 16 along K advances
+// the start address by two groups.  Needs the MN-major bit of the instruction descriptor.
+__device__ __forceinline__ uint64_t make_desc_mn_sw128(uint32_t smem_addr, uint32_t mn_chunk_bytes,
+                                                       uint32_t group_bytes = 1024) {
   uint64_t d = 0;
   d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
   d |= static_cast<uint64_t>((mn_chunk_bytes >> 4) & 0x3FFFu) << 16;
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;
+  d |= static_cast<uint64_t>(group_bytes >> 4) << 32;
   d |= static_cast<uint64_t>(1) << 46;
   d |= static_cast<uint64_t>(2) << 61;
   return d;

@@ -45,20 +45,6 @@ struct Args {
   unsigned int* status;
 };
 
-// D[tmem] (+)= A[tmem] * B[smem]: lane = row of A, a column = two neighbouring bf16 of its K.
-__device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint64_t desc_b, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}\n"
-      :
-      : "r"(d), "r"(a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 // 8 nibbles, low one first -> 4 bf16 pairs q * s - z.  A byte permute brings a byte's two nibbles to
 // the low ends of two halves; 0x4300 | q is the bf16 number 128 + q, the subtraction of 128 is exact and
 // the fused multiply-add rounds once.  (The integer pipe, half as wide as the others, is what bounds the
