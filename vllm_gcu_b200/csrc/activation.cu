@@ -102,6 +102,8 @@ struct Args {
 
 template <typename T, int ACT, int MODE, int QUANT>
 __global__ void __launch_bounds__(512) act_kernel(const Args a) {
+  grid_release();
+  grid_wait();
   const int row = blockIdx.x;
   if (a.valid_rows != nullptr && row >= *a.valid_rows) return;
   const T* x = static_cast<const T*>(a.x) + static_cast<long long>(row) * a.ldx;
@@ -183,11 +185,11 @@ int launch_q(const Args& a, int quant, cudaStream_t s) {
   int threads = ((a.d >> 3) + 31) & ~31;
   threads = threads > 512 ? 512 : (threads < 32 ? 32 : threads);
   switch (quant) {
-    case kQNone: act_kernel<T, ACT, MODE, kQNone><<<a.T, threads, 0, s>>>(a); break;
-    case kQFp8Group128: act_kernel<T, ACT, MODE, kQFp8Group128><<<a.T, threads, 0, s>>>(a); break;
-    case kQFp8Static: act_kernel<T, ACT, MODE, kQFp8Static><<<a.T, threads, 0, s>>>(a); break;
-    case kQInt8Static: act_kernel<T, ACT, MODE, kQInt8Static><<<a.T, threads, 0, s>>>(a); break;
-    case kQInt8Asym: act_kernel<T, ACT, MODE, kQInt8Asym><<<a.T, threads, 0, s>>>(a); break;
+    case kQNone: return launch_overlapped(act_kernel<T, ACT, MODE, kQNone>, dim3(a.T), dim3(threads), 0, s, a);
+    case kQFp8Group128: return launch_overlapped(act_kernel<T, ACT, MODE, kQFp8Group128>, dim3(a.T), dim3(threads), 0, s, a);
+    case kQFp8Static: return launch_overlapped(act_kernel<T, ACT, MODE, kQFp8Static>, dim3(a.T), dim3(threads), 0, s, a);
+    case kQInt8Static: return launch_overlapped(act_kernel<T, ACT, MODE, kQInt8Static>, dim3(a.T), dim3(threads), 0, s, a);
+    case kQInt8Asym: return launch_overlapped(act_kernel<T, ACT, MODE, kQInt8Asym>, dim3(a.T), dim3(threads), 0, s, a);
     default: return -7;
   }
   return static_cast<int>(cudaGetLastError());

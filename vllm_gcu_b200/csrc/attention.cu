@@ -385,6 +385,8 @@ __global__ void __launch_bounds__(kThreads) paged_decode_kernel(const DecodeArgs
 
 template <typename T, int HD>
 __global__ void __launch_bounds__(128) decode_reduce_kernel(const DecodeArgs a) {
+  grid_release();
+  grid_wait();
   const int b = blockIdx.x, head = blockIdx.y;
   const long long base = (static_cast<long long>(b) * a.Hq + head) * a.num_splits;
   float M = -INFINITY;
@@ -661,8 +663,7 @@ int launch_decode(const DecodeArgs& a, cudaStream_t s) {
   kern<<<grid, kThreads, smem, s>>>(a);
   e = static_cast<int>(cudaGetLastError());
   if (e != 0 || a.num_splits <= 1) return e;
-  decode_reduce_kernel<T, HD><<<dim3(a.B, a.Hq), 128, 0, s>>>(a);
-  return static_cast<int>(cudaGetLastError());
+  return launch_overlapped(decode_reduce_kernel<T, HD>, dim3(a.B, a.Hq), dim3(128), 0, s, a);
 }
 
 template <typename T, int HD>
@@ -831,16 +832,15 @@ B200_API int b200_decode_reduce(void* out, long long ldo, float* tmp_out, float*
   a.num_splits = num_splits;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   dim3 grid(B, Hq);
-#define B200_RED(TT, H) decode_reduce_kernel<TT, H><<<grid, 128, 0, s>>>(a)
+#define B200_RED(TT, H) return launch_overlapped(decode_reduce_kernel<TT, H>, grid, dim3(128), 0, s, a)
   if (dtype == 0 && HD == 128) B200_RED(__nv_bfloat16, 128);
-  else if (dtype == 0 && HD == 64) B200_RED(__nv_bfloat16, 64);
-  else if (dtype == 0 && HD == 256) B200_RED(__nv_bfloat16, 256);
-  else if (dtype == 1 && HD == 128) B200_RED(__half, 128);
-  else if (dtype == 1 && HD == 64) B200_RED(__half, 64);
-  else if (dtype == 1 && HD == 256) B200_RED(__half, 256);
-  else return -8;
+  if (dtype == 0 && HD == 64) B200_RED(__nv_bfloat16, 64);
+  if (dtype == 0 && HD == 256) B200_RED(__nv_bfloat16, 256);
+  if (dtype == 1 && HD == 128) B200_RED(__half, 128);
+  if (dtype == 1 && HD == 64) B200_RED(__half, 64);
+  if (dtype == 1 && HD == 256) B200_RED(__half, 256);
 #undef B200_RED
-  return static_cast<int>(cudaGetLastError());
+  return -8;
 }
 
 // Prefill / chunked-prefill / prefix attention.  num_q_tiles must be

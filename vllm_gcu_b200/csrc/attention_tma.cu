@@ -98,6 +98,8 @@ __global__ void __launch_bounds__(kThreads)
   uint64_t* empty_bar = full_bar + kStages;
   volatile uint32_t* abort_flag = reinterpret_cast<uint32_t*>(empty_bar + kStages);
 
+  grid_release();
+  grid_wait();
   const int b = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
   const int G = a.Hq / a.Hkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -430,34 +432,36 @@ static int paged_decode_tma_impl(const void* q, long long ldq, void* out, long l
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   dim3 grid(B, Hkv, num_splits);
   static bool done0[64] = {false}, done1[64] = {false}, done2[64] = {false};
-  int dev = 0;
+  int dev = 0, e = 0;
   cudaGetDevice(&dev);
   if (shaped) {
     auto kern = paged_decode_tma_kernel<__nv_bfloat16, true>;
     if (dev >= 0 && dev < 64 && !done2[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) return static_cast<int>(e);
+      const cudaError_t set =
+          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      if (set != cudaSuccess) return static_cast<int>(set);
       done2[dev] = true;
     }
-    kern<<<grid, kThreads, smem, s>>>(tmK, tmV, a);
+    e = launch_overlapped(kern, grid, dim3(kThreads), smem, s, tmK, tmV, a);
   } else if (dtype == 0) {
     auto kern = paged_decode_tma_kernel<__nv_bfloat16, false>;
     if (dev >= 0 && dev < 64 && !done0[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) return static_cast<int>(e);
+      const cudaError_t set =
+          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      if (set != cudaSuccess) return static_cast<int>(set);
       done0[dev] = true;
     }
-    kern<<<grid, kThreads, smem, s>>>(tmK, tmV, a);
+    e = launch_overlapped(kern, grid, dim3(kThreads), smem, s, tmK, tmV, a);
   } else {
     auto kern = paged_decode_tma_kernel<__half, false>;
     if (dev >= 0 && dev < 64 && !done1[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) return static_cast<int>(e);
+      const cudaError_t set =
+          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      if (set != cudaSuccess) return static_cast<int>(set);
       done1[dev] = true;
     }
-    kern<<<grid, kThreads, smem, s>>>(tmK, tmV, a);
+    e = launch_overlapped(kern, grid, dim3(kThreads), smem, s, tmK, tmV, a);
   }
-  int e = static_cast<int>(cudaGetLastError());
   if (e != 0 || num_splits <= 1) return e;
   return b200_decode_reduce(out, ldo, tmp_out, tmp_lse, num_splits, B, Hq, HD, dtype, sink,
                             a.OD, stream);

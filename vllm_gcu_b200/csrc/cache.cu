@@ -103,6 +103,8 @@ __device__ __forceinline__ void store_cache8(const RopeCacheArgs& a, bool is_v, 
 // where two norm kernels and two copies into dense rows took 115 more (4096 tokens, 32 + 4 heads).
 template <typename T, int LANES, bool NORM>
 __global__ void __launch_bounds__(256) rope_cache_heads_kernel(const RopeCacheArgs a) {
+  grid_release();
+  grid_wait();
   const int heads = a.Hq + 2 * a.Hkv;
   const long long item = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   const long long row = item / LANES;
@@ -183,11 +185,12 @@ __global__ void __launch_bounds__(256) rope_cache_heads_kernel(const RopeCacheAr
 }
 
 template <typename T, int LANES>
-static void launch_heads(const RopeCacheArgs& a, cudaStream_t s) {
+static int launch_heads(const RopeCacheArgs& a, cudaStream_t s) {
   const long long items = static_cast<long long>(a.T) * (a.Hq + 2 * a.Hkv) * LANES;
   const unsigned blocks = static_cast<unsigned>((items + 255) / 256);
-  if (a.q_weight != nullptr) rope_cache_heads_kernel<T, LANES, true><<<blocks, 256, 0, s>>>(a);
-  else rope_cache_heads_kernel<T, LANES, false><<<blocks, 256, 0, s>>>(a);
+  return launch_overlapped(a.q_weight != nullptr ? rope_cache_heads_kernel<T, LANES, true>
+                                                 : rope_cache_heads_kernel<T, LANES, false>,
+                           dim3(blocks), dim3(256), 0, s, a);
 }
 
 // What the kernel above takes: query, key and value rows, whole heads of 64, 128 or 256 rotated, all of it
@@ -207,10 +210,10 @@ static bool heads_ok(const RopeCacheArgs& a) {
 }
 
 template <typename T>
-static void launch_heads_any(const RopeCacheArgs& a, cudaStream_t s) {
-  if (a.D == 64) launch_heads<T, 4>(a, s);
-  else if (a.D == 128) launch_heads<T, 8>(a, s);
-  else launch_heads<T, 16>(a, s);
+static int launch_heads_any(const RopeCacheArgs& a, cudaStream_t s) {
+  if (a.D == 64) return launch_heads<T, 4>(a, s);
+  if (a.D == 128) return launch_heads<T, 8>(a, s);
+  return launch_heads<T, 16>(a, s);
 }
 
 template <typename T>
@@ -541,9 +544,7 @@ B200_API int b200_rope_cache_flash(void* q, long long ldq, void* k, long long ld
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype != 0 && dtype != 1) return -8;
   if (heads_ok(a)) {
-    if (dtype == 0) launch_heads_any<__nv_bfloat16>(a, s);
-    else launch_heads_any<__half>(a, s);
-    return static_cast<int>(cudaGetLastError());
+    return dtype == 0 ? launch_heads_any<__nv_bfloat16>(a, s) : launch_heads_any<__half>(a, s);
   }
   if (q_weight != nullptr) return -20;
   if (dtype == 0) rope_cache_flash_kernel<__nv_bfloat16><<<T, 256, 0, s>>>(a);

@@ -122,6 +122,21 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
 }
 
 // ---------------------------------------------------------------------------
+// programmatic dependent launch
+// ---------------------------------------------------------------------------
+// A kernel launched with launch_overlapped (below) may start while the kernels in front of it in the
+// stream still run: launch, barrier and tensor-memory set-up and first instruction fetches, about 2 us of
+// a kernel, then overlap with their ends.  Every thread calls grid_wait() before it touches what they
+// write, and before it ends: it returns once they have completed and their stores are visible, so that
+// completion stays transitive along the stream.  grid_release() lets the next kernel start as soon as
+// every CTA has called it (or ended); a CTA that uses tensor memory calls it behind its allocation, else
+// a CTA of the next kernel might hold the columns that this one waits for.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// ---------------------------------------------------------------------------
 // TMA (tiled bulk tensor copies, never with cluster multicast)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
@@ -552,6 +567,23 @@ int encode_tmap_3d(CUtensorMap* out, CUtensorMapDataType dt, int elt_bytes, cons
                    CUtensorMapSwizzle swz);
 
 int sm_count();
+
+// Launch of a kernel that calls grid_wait().
+template <typename... P, typename... A>
+int launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                      A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
 
 // Device address of the status word of the current device (null on failure).
 unsigned int* status_ptr();

@@ -741,6 +741,8 @@ __global__ void __launch_bounds__(kThreadsFor<EPI>, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_release();
+  grid_wait();
 
   const int num_kb = (p.K + BK - 1) / BK;
   const int num_tiles = p.tiles_m * p.tiles_n;
@@ -1424,6 +1426,9 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const Args& a, cudaSt
   }
   const int tiles = a.tiles_m * a.tiles_n;
   const int grid = tiles < sm_count() ? tiles : sm_count();
+  if constexpr (!kPeerEpi<EPI> && EPI != kEpiGatherA)
+    return launch_overlapped(kern, dim3(grid), dim3(kThreadsFor<EPI>), L::kTotal, stream, tmA, tmB, a);
+  // (kernels that meet other ranks start when the stream is theirs)
   kern<<<grid, kThreadsFor<EPI>, L::kTotal, stream>>>(tmA, tmB, a);
   return static_cast<int>(cudaGetLastError());
 }

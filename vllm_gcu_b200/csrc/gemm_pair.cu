@@ -152,6 +152,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   cluster_sync_all();            // the other CTA's barriers exist before anything arrives there
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_release();
+  grid_wait();
   const int num_tiles = p.tiles_m * p.tiles_n;
 
   if (warp == 0) {
@@ -585,13 +587,15 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const Args& a, cudaSt
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = Smem::kTotal;
   cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = 2;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, a));
 }
 

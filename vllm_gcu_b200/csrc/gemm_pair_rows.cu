@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __shared__ volatile uint32_t abort_word, epi_abort;
   volatile uint32_t* abort_flag = &abort_word;
 
+  grid_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();                  // 0 = leader
   const int pair_id = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
@@ -151,6 +152,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   cluster_sync_all();            // the other CTA's barriers exist before anything arrives there
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
+  grid_release();
   const int num_kb = (p.K + 63) / 64;
   const int units = (GROUPED ? list_len : p.row_tiles) * ((p.N + 255) / 256);
 
@@ -324,12 +326,14 @@ static int launch(const CUtensorMap& tmW, const CUtensorMap& tmA, Args a, int un
   cfg.gridDim = dim3(2 * 74);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = kSmemBytes;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = 2;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (at_once[dev] == 0) {
     cudaError_t e =
@@ -343,6 +347,7 @@ static int launch(const CUtensorMap& tmW, const CUtensorMap& tmA, Args a, int un
   a.status = status_ptr();
   cfg.gridDim = dim3(2 * (units < at_once[dev] ? units : at_once[dev]));
   cfg.stream = stream;
+  cfg.numAttrs = 2;
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, tmW, tmA, a));
 }
 

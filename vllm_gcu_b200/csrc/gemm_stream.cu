@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(kThreads)
   // activation rows [m0, m0 + used) times weight rows [n0, n0 + 128) of a matrix from row w0 on
   int rows, used, m0, n0, w0, split, stages;
   if constexpr (GROUPED) {
+    grid_wait();
     m0 = static_cast<int>(blockIdx.y) * kGroupRows;
     if (m0 >= *p.num_rows) return;
     const int expert = p.expert_ids[blockIdx.y];
@@ -140,11 +141,22 @@ __global__ void __launch_bounds__(kThreads)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
+  grid_release();
 
   const int total_kb = (p.K + kCols - 1) / kCols;
   const int kb_lo = static_cast<int>(static_cast<long long>(split) * total_kb / splits);
   const int num_kb =
       static_cast<int>(static_cast<long long>(split + 1) * total_kb / splits) - kb_lo;
+
+  if constexpr (!GROUPED) {
+    // The first weight tiles come into L2 while the kernels in front still run (not into shared memory:
+    // nothing says that they do not write them)
+    if (threadIdx.x == 0)
+      for (int kb = 0; kb < num_kb && kb < stages; ++kb)
+        tma_prefetch_2d(&tmW, (kb_lo + kb) * kCols, n0);
+    __syncwarp();
+    grid_wait();
+  }
 
   if (warp == 0) {
     if (elect_one()) {
@@ -322,7 +334,7 @@ static int launch(const void* A, long long lda, const void* W, long long ldw, Ar
   if (r != 0) return r;
   p.rows = pl.rows; p.row_tiles = pl.row_tiles; p.splits = pl.splits; p.stages = pl.stages;
   p.status = status_ptr();
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   const cudaLaunchConfig_t cfg = launch_config(pl.splits, (p.N + BW - 1) / BW * pl.row_tiles, kThreads,
                                                bytes, attr, stream);
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, tmW, tmA, p));
@@ -428,6 +440,6 @@ B200_API int b200_gemm_stream_grouped(const void* A, long long lda, const void* 
     configured[dev] = true;
   }
   dim3 grid((N + BW - 1) / BW, M_cap / kGroupRows);
-  kernel<<<grid, kThreads, room, static_cast<cudaStream_t>(stream)>>>(tmW, tmA, a);
-  return static_cast<int>(cudaGetLastError());
+  return launch_overlapped(kernel, grid, dim3(kThreads), static_cast<size_t>(room),
+                           static_cast<cudaStream_t>(stream), tmW, tmA, a);
 }

@@ -55,6 +55,8 @@ __device__ __forceinline__ float load_gate(const void* p, long long i, int dtype
 
 // 4 warps per CTA, one token per warp.  Shared: per warp 2 * E floats.
 __global__ void __launch_bounds__(128) moe_topk_kernel(const TopkArgs a) {
+  grid_release();
+  grid_wait();
   extern __shared__ float sm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + warp;
@@ -171,6 +173,8 @@ struct AlignArgs {
 };
 
 __global__ void __launch_bounds__(1024) moe_align_kernel(const AlignArgs a) {
+  grid_release();
+  grid_wait();
   extern __shared__ int smi[];
   int* count = smi;                              // [E]
   int* offset = smi + a.num_local_experts;       // [E + 1] padded exclusive offsets
@@ -238,6 +242,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
     moe_permute_kernel(const T* x, long long ldx, T* out, long long ldo, const int* sorted_ids,
                        const int* num_post_pad, int numel, int k, int H, int zero_pads) {
+  grid_release();
+  grid_wait();
   const int pos = blockIdx.x;
   if (pos >= *num_post_pad) return;
   const int pair = sorted_ids[pos];
@@ -393,6 +399,8 @@ __global__ void __launch_bounds__(256)
     moe_unpermute_sum_kernel(const T* y, long long ldy, const int* pos_of, const T* add,
                              long long lda, T* out, long long ldo, const int* valid_tokens, int k,
                              int H, float alpha) {
+  grid_release();
+  grid_wait();
   const int t = blockIdx.x;
   if (valid_tokens != nullptr && t >= *valid_tokens) return;
   const int nvec = H >> 3;
@@ -421,6 +429,8 @@ __global__ void __launch_bounds__(256)
 // Per sorted row: the routing weight of its (token, slot) pair (0 for padding rows).
 __global__ void moe_row_weights_kernel(const int* sorted_ids, const float* topk_w,
                                        const int* num_post_pad, float* row_w, int numel, int cap) {
+  grid_release();
+  grid_wait();
   const int pos = blockIdx.x * blockDim.x + threadIdx.x;
   if (pos >= cap) return;
   float w = 0.0f;
@@ -491,8 +501,8 @@ B200_API int b200_moe_topk(const void* gating, long long ldg, const float* bias,
   a.n_group = n_group; a.topk_group = topk_group; a.R = R; a.sigmoid = sigmoid;
   a.renorm = renorm; a.scale = scale; a.dtype = dtype;
   const size_t smem = static_cast<size_t>(4) * 2 * E * sizeof(float);
-  moe_topk_kernel<<<(T + 3) / 4, 128, smem, static_cast<cudaStream_t>(stream)>>>(a);
-  return static_cast<int>(cudaGetLastError());
+  return launch_overlapped(moe_topk_kernel, dim3((T + 3) / 4), dim3(128), smem,
+                           static_cast<cudaStream_t>(stream), a);
 }
 
 // cap must be a multiple of 128 and >= numel + num_local_experts * 127 rounded up.
@@ -507,8 +517,8 @@ B200_API int b200_moe_align(const int* topk_ids, const int* expert_map, const in
   a.pos_of = pos_of; a.tile_rows = tile_rows; a.numel = numel; a.k = k; a.num_local_experts = num_local_experts;
   a.cap = cap; a.status = status_ptr();
   const size_t smem = static_cast<size_t>(3 * num_local_experts + 1) * sizeof(int);
-  moe_align_kernel<<<1, 1024, smem, static_cast<cudaStream_t>(stream)>>>(a);
-  return static_cast<int>(cudaGetLastError());
+  return launch_overlapped(moe_align_kernel, dim3(1), dim3(1024), smem,
+                           static_cast<cudaStream_t>(stream), a);
 }
 
 B200_API int b200_moe_permute(const void* x, long long ldx, void* out, long long ldo,
@@ -518,16 +528,15 @@ B200_API int b200_moe_permute(const void* x, long long ldx, void* out, long long
   if ((H % 8) != 0) return -2;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == 0)
-    moe_permute_kernel<__nv_bfloat16><<<cap, 256, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_bfloat16*>(out), ldo,
-        sorted_ids, num_post_pad, numel, k, H, zero_pads);
-  else if (dtype == 1)
-    moe_permute_kernel<__half><<<cap, 256, 0, s>>>(static_cast<const __half*>(x), ldx,
-                                                   static_cast<__half*>(out), ldo, sorted_ids,
-                                                   num_post_pad, numel, k, H, zero_pads);
-  else
-    return -8;
-  return static_cast<int>(cudaGetLastError());
+    return launch_overlapped(moe_permute_kernel<__nv_bfloat16>, dim3(cap), dim3(256), 0, s,
+                             static_cast<const __nv_bfloat16*>(x), ldx,
+                             static_cast<__nv_bfloat16*>(out), ldo, sorted_ids, num_post_pad, numel, k,
+                             H, zero_pads);
+  if (dtype == 1)
+    return launch_overlapped(moe_permute_kernel<__half>, dim3(cap), dim3(256), 0, s,
+                             static_cast<const __half*>(x), ldx, static_cast<__half*>(out), ldo,
+                             sorted_ids, num_post_pad, numel, k, H, zero_pads);
+  return -8;
 }
 
 // x [T, ldx], H columns; out rows [cap, ldo] of Ho >= H columns (zeros behind H); dtype 0 bf16,
@@ -605,9 +614,9 @@ B200_API int b200_moe_row_weights(const int* sorted_ids, const float* topk_w,
                                   const int* num_post_pad, float* row_w, int numel, int cap,
                                   void* stream) {
   if (cap <= 0) return 0;
-  moe_row_weights_kernel<<<(cap + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      sorted_ids, topk_w, num_post_pad, row_w, numel, cap);
-  return static_cast<int>(cudaGetLastError());
+  return launch_overlapped(moe_row_weights_kernel, dim3((cap + 255) / 256), dim3(256), 0,
+                           static_cast<cudaStream_t>(stream), sorted_ids, topk_w, num_post_pad, row_w,
+                           numel, cap);
 }
 
 B200_API int b200_moe_unpermute_sum(const void* y, long long ldy, const int* pos_of,
@@ -618,16 +627,16 @@ B200_API int b200_moe_unpermute_sum(const void* y, long long ldy, const int* pos
   if ((H % 8) != 0) return -2;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == 0)
-    moe_unpermute_sum_kernel<__nv_bfloat16><<<T, 256, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(y), ldy, pos_of, static_cast<const __nv_bfloat16*>(add),
-        lda, static_cast<__nv_bfloat16*>(out), ldo, valid_tokens, k, H, alpha);
-  else if (dtype == 1)
-    moe_unpermute_sum_kernel<__half><<<T, 256, 0, s>>>(
-        static_cast<const __half*>(y), ldy, pos_of, static_cast<const __half*>(add), lda,
-        static_cast<__half*>(out), ldo, valid_tokens, k, H, alpha);
-  else
-    return -8;
-  return static_cast<int>(cudaGetLastError());
+    return launch_overlapped(moe_unpermute_sum_kernel<__nv_bfloat16>, dim3(T), dim3(256), 0, s,
+                             static_cast<const __nv_bfloat16*>(y), ldy, pos_of,
+                             static_cast<const __nv_bfloat16*>(add), lda,
+                             static_cast<__nv_bfloat16*>(out), ldo, valid_tokens, k, H, alpha);
+  if (dtype == 1)
+    return launch_overlapped(moe_unpermute_sum_kernel<__half>, dim3(T), dim3(256), 0, s,
+                             static_cast<const __half*>(y), ldy, pos_of,
+                             static_cast<const __half*>(add), lda, static_cast<__half*>(out), ldo,
+                             valid_tokens, k, H, alpha);
+  return -8;
 }
 
 B200_API int b200_get_ep_indices(const int* topk_ids, int T, int k, int experts_per_rank, int ep,

@@ -113,6 +113,8 @@ struct Args {
 template <typename T, int QMODE, bool ADD>
 __global__ void __launch_bounds__(1024) rms_norm_kernel(const Args a) {
   __shared__ float red[32];
+  grid_release();
+  grid_wait();
   const int row = blockIdx.x;
   if (a.valid_rows != nullptr && row >= *a.valid_rows) return;
   const T* x = static_cast<const T*>(a.x) + static_cast<long long>(row) * a.ldx;
@@ -239,9 +241,9 @@ int launch2(const Args& a, bool add, cudaStream_t s) {
   if (threads > 1024) threads = 1024;
   if (threads < 32) threads = 32;
   if (add)
-    rms_norm_kernel<T, QMODE, true><<<a.T, threads, 0, s>>>(a);
+    return launch_overlapped(rms_norm_kernel<T, QMODE, true>, dim3(a.T), dim3(threads), 0, s, a);
   else
-    rms_norm_kernel<T, QMODE, false><<<a.T, threads, 0, s>>>(a);
+    return launch_overlapped(rms_norm_kernel<T, QMODE, false>, dim3(a.T), dim3(threads), 0, s, a);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -23,6 +23,8 @@ template <typename T, bool INT8>
 __global__ void __launch_bounds__(1024)
     per_token_quant_kernel(const T* x, long long ldx, uint8_t* out, long long ldo, float* scales,
                            const int* valid_rows, int H) {
+  grid_release();
+  grid_wait();
   __shared__ float red[32];
   const int row = blockIdx.x;
   if (valid_rows != nullptr && row >= *valid_rows) return;
@@ -136,14 +138,14 @@ B200_API int b200_per_token_quant(const void* x, long long ldx, void* out, long 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   uint8_t* o = static_cast<uint8_t*>(out);
 #define B200_PTQ(TT, I8) \
-  per_token_quant_kernel<TT, I8><<<T, threads, 0, s>>>(static_cast<const TT*>(x), ldx, o, ldo, scales, valid_rows, H)
+  return launch_overlapped(per_token_quant_kernel<TT, I8>, dim3(T), dim3(threads), 0, s, \
+                           static_cast<const TT*>(x), ldx, o, ldo, scales, valid_rows, H)
   if (dtype == 0 && kind == 0) B200_PTQ(__nv_bfloat16, false);
-  else if (dtype == 0 && kind == 1) B200_PTQ(__nv_bfloat16, true);
-  else if (dtype == 1 && kind == 0) B200_PTQ(__half, false);
-  else if (dtype == 1 && kind == 1) B200_PTQ(__half, true);
-  else return -8;
+  if (dtype == 0 && kind == 1) B200_PTQ(__nv_bfloat16, true);
+  if (dtype == 1 && kind == 0) B200_PTQ(__half, false);
+  if (dtype == 1 && kind == 1) B200_PTQ(__half, true);
 #undef B200_PTQ
-  return static_cast<int>(cudaGetLastError());
+  return -8;
 }
 
 // Dynamic per-tensor fp8: scale_out[0] = amax / 448.  `amax_ws` is one float of workspace.

@@ -190,6 +190,8 @@ struct Args {
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) sample_kernel(const Args a) {
+  grid_release();
+  grid_wait();
   // 32 KB shared by the replicated histogram of a full-row select (first 16 KB) and the
   // candidate list that replaces the row once top-k has cut it down.
   constexpr int kCap = 4096;
@@ -298,11 +300,11 @@ B200_API int b200_sample(const void* logits, long long ld, int B, int V, int dty
   a.top_p = top_p; a.noise = noise; a.seeds = seeds; a.out_ids = out_ids; a.ld = ld;
   a.step = step; a.B = B; a.V = V; a.mask_only = 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dtype == 0) sample_kernel<__nv_bfloat16><<<B, kThreads, 0, s>>>(a);
-  else if (dtype == 1) sample_kernel<__half><<<B, kThreads, 0, s>>>(a);
-  else if (dtype == 2) sample_kernel<float><<<B, kThreads, 0, s>>>(a);
-  else return -8;
-  return static_cast<int>(cudaGetLastError());
+  if (dtype < 0 || dtype > 2) return -8;
+  return b200::launch_overlapped(dtype == 0   ? sample_kernel<__nv_bfloat16>
+                                 : dtype == 1 ? sample_kernel<__half>
+                                              : sample_kernel<float>,
+                                 dim3(B), dim3(kThreads), 0, s, a);
 }
 
 // In-place top-k / top-p mask: entries outside the kept set become -inf.
@@ -315,9 +317,9 @@ B200_API int b200_top_k_top_p(void* logits, long long ld, int B, int V, int dtyp
   a.top_p = top_p; a.noise = nullptr; a.seeds = nullptr; a.out_ids = nullptr; a.ld = ld;
   a.step = 0; a.B = B; a.V = V; a.mask_only = 1;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dtype == 0) sample_kernel<__nv_bfloat16><<<B, kThreads, 0, s>>>(a);
-  else if (dtype == 1) sample_kernel<__half><<<B, kThreads, 0, s>>>(a);
-  else if (dtype == 2) sample_kernel<float><<<B, kThreads, 0, s>>>(a);
-  else return -8;
-  return static_cast<int>(cudaGetLastError());
+  if (dtype < 0 || dtype > 2) return -8;
+  return b200::launch_overlapped(dtype == 0   ? sample_kernel<__nv_bfloat16>
+                                 : dtype == 1 ? sample_kernel<__half>
+                                              : sample_kernel<float>,
+                                 dim3(B), dim3(kThreads), 0, s, a);
 }

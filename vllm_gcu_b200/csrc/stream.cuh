@@ -110,8 +110,10 @@ inline cudaLaunchConfig_t launch_config(int splits, int tiles, int threads, int 
   attr[0].val.clusterDim.x = splits;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = splits > 1 ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = splits > 1 ? attr : attr + 1;
+  cfg.numAttrs = splits > 1 ? 2 : 1;
   return cfg;
 }
 
@@ -132,8 +134,9 @@ const int* clusters_at_once(AtOnce& table, Kernel kernel, int threads) {
     return nullptr;
   }
   for (int s = kMaxSplits; s >= 1; --s) {
-    cudaLaunchAttribute attr[1];
-    const cudaLaunchConfig_t cfg = launch_config(s, 512, threads, kSmemLimit, attr, nullptr);
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = launch_config(s, 512, threads, kSmemLimit, attr, nullptr);
+    cfg.numAttrs = 1;                  // the cluster size alone counts here
     int n = 0;
     if (s == 1) n = sm_count();
     else if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
