@@ -122,8 +122,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         y = bt[min(key, last_tok) / a.block_size] * a.block_size + key % a.block_size;
       bool ok = true;
       for (int kv = 0; kv < 2 && ok; ++kv) {
-        ok = mbar_wait(&empty[slot], phase ^ 1u, a.status, kKernelId, 0x600u + slot, abort_flag);
-        __syncwarp();
+        ok = mbar_wait_warp(&empty[slot], phase ^ 1u, a.status, kKernelId, 0x600u + slot, abort_flag);
         if (ok) {
           if (lane == 0) mbar_expect_tx(&full[slot], kTile);
           __syncwarp();
@@ -210,8 +209,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     float m_used = -INFINITY, l = 0.0f;
     bool ok = true;
     for (int j = 0; j < nt; ++j) {
-      ok = mbar_wait(&s_full[h], j & 1, a.status, kKernelId, 0x640u + h, abort_flag);
-      __syncwarp();
+      ok = mbar_wait_warp(&s_full[h], j & 1, a.status, kKernelId, 0x640u + h, abort_flag);
       if (!ok) break;
       tc_fence_after();
       uint32_t v[4][32];
@@ -277,8 +275,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[h]);
     }
-    if (ok) ok = mbar_wait(&o_done[h], 0, a.status, kKernelId, 0x650u + h, abort_flag);
-    __syncwarp();
+    if (ok) ok = mbar_wait_warp(&o_done[h], 0, a.status, kKernelId, 0x650u + h, abort_flag);
     if (ok) {
       tc_fence_after();
       float den = l;

@@ -413,32 +413,28 @@ __global__ void __launch_bounds__(kThreads, kResident)
     }
     float m_used = -INFINITY, l = 0.0f;
     float* xch = reinterpret_cast<float*>(smem + kOffX);    // [2][128]
-    bool ok = true;
     for (int j = 0; j < nt; ++j) {
       const int st = j % kSBufs;
-      if (ok && !mbar_wait(&s_full[st], static_cast<uint32_t>(j / kSBufs) & 1u, a.status,
-                           kKernelId, 0x300u + st, abort_flag))
-        ok = false;
+      mbar_pass_warp(&s_full[st], static_cast<uint32_t>(j / kSBufs) & 1u, a.status, kKernelId, 0x300u + st,
+                     abort_flag);
       tc_fence_after();
       const int tile_key0 = (t0 + j) * BKV;
       const int key0 = tile_key0 + g * 32;
       const bool need_mask = valid_rows < BQ || tile_key0 + BKV - 1 > hi_first;
       uint32_t v[32];
       float mt = -INFINITY;
-      if (ok) {
-        tmem_ld_32x32(lane_addr + kColS + st * BKV + g * 32, v);
-        tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&s_empty[st]);       // the scores of another tile may follow
-        if (need_mask) {
+      tmem_ld_32x32(lane_addr + kColS + st * BKV + g * 32, v);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_empty[st]);       // the scores of another tile may follow
+      if (need_mask) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (key0 + i <= hi) mt = fmaxf(mt, __uint_as_float(v[i]));
-        } else {
+        for (int i = 0; i < 32; ++i)
+          if (key0 + i <= hi) mt = fmaxf(mt, __uint_as_float(v[i]));
+      } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) mt = fmaxf(mt, __uint_as_float(v[i]));
-        }
+        for (int i = 0; i < 32; ++i) mt = fmaxf(mt, __uint_as_float(v[i]));
       }
       xch[g * BQ + r] = mt;
       asm volatile("bar.sync 2, 256;" ::: "memory");
@@ -453,28 +449,24 @@ __global__ void __launch_bounds__(kThreads, kResident)
       const float mb = (m_new == -INFINITY ? 0.0f : m_new) * sl2;
       uint32_t pk[16];
       float rs = 0.0f;
-      if (ok) {
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float p0 = ex2_approx(fmaf(__uint_as_float(v[i]), sl2, -mb));
-          float p1 = ex2_approx(fmaf(__uint_as_float(v[i + 1]), sl2, -mb));
-          if (need_mask) {
-            if (key0 + i > hi) p0 = 0.0f;
-            if (key0 + i + 1 > hi) p1 = 0.0f;
-          }
-          rs += p0 + p1;
-          pk[i >> 1] = pack_bf16x2(p0, p1);
+      for (int i = 0; i < 32; i += 2) {
+        float p0 = ex2_approx(fmaf(__uint_as_float(v[i]), sl2, -mb));
+        float p1 = ex2_approx(fmaf(__uint_as_float(v[i + 1]), sl2, -mb));
+        if (need_mask) {
+          if (key0 + i > hi) p0 = 0.0f;
+          if (key0 + i + 1 > hi) p1 = 0.0f;
         }
+        rs += p0 + p1;
+        pk[i >> 1] = pack_bf16x2(p0, p1);
       }
       l = l * alpha + rs;
       m_used = m_new;
       // the previous P V product must be complete before P is overwritten / O is rescaled
-      if (ok && j > 0 &&
-          !mbar_wait(o_done, (j - 1) & 1, a.status, kKernelId, 0x310u, abort_flag))
-        ok = false;
+      if (j > 0) mbar_pass_warp(o_done, (j - 1) & 1, a.status, kKernelId, 0x310u, abort_flag);
       tc_fence_after();
       // Rescale the accumulator when the maximum rose.
-      if (ok && j > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
+      if (j > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
 #pragma unroll 1
         for (int c = 0; c < nc; ++c) {
           uint32_t o[32];
@@ -486,24 +478,22 @@ __global__ void __launch_bounds__(kThreads, kResident)
         }
         tmem_st_wait();
       }
-      if (ok) {
-        // P row = 64 keys = 128 bytes; this thread owns 16-byte chunks 4 g .. 4 g + 3,
-        // XOR-swizzled by row % 8
+      // P row = 64 keys = 128 bytes; this thread owns 16-byte chunks 4 g .. 4 g + 3,
+      // XOR-swizzled by row % 8
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-          uint4 u = make_uint4(pk[cc * 4], pk[cc * 4 + 1], pk[cc * 4 + 2], pk[cc * 4 + 3]);
-          *reinterpret_cast<uint4*>(p_smem + r * 128 + (((g * 4 + cc) ^ (r & 7)) << 4)) = u;
-        }
-        fence_async_smem();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(p_full);
+      for (int cc = 0; cc < 4; ++cc) {
+        uint4 u = make_uint4(pk[cc * 4], pk[cc * 4 + 1], pk[cc * 4 + 2], pk[cc * 4 + 3]);
+        *reinterpret_cast<uint4*>(p_smem + r * 128 + (((g * 4 + cc) ^ (r & 7)) << 4)) = u;
       }
+      fence_async_smem();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
     }
     xch[g * BQ + r] = l;
     asm volatile("bar.sync 2, 256;" ::: "memory");
     l += xch[(g ^ 1) * BQ + r];
-    if (ok && mbar_wait(o_done, (nt - 1) & 1, a.status, kKernelId, 0x320u, abort_flag)) {
+    if (mbar_wait_warp(o_done, (nt - 1) & 1, a.status, kKernelId, 0x320u, abort_flag)) {
       tc_fence_after();
       const long long grow = row0 + r;
       float inv = l > 0.0f ? 1.0f / l : 0.0f;

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int b = it & 1;
       const Unit x = unit_at<GROUPED>(p, list, u);
       const int n0 = x.n0 + static_cast<int>(rank) * kHalfW;
-      if (!mbar_wait(&tfull_bar[b], tphase[b], p.status, kKernelId, 0x400u + b, abort_flag))
+      if (!mbar_wait_warp(&tfull_bar[b], tphase[b], p.status, kKernelId, 0x400u + b, abort_flag))
         epi_abort = 1u;
       // (the four warps meet at barriers below, so they leave together)
       asm volatile("bar.sync 1, 128;" ::: "memory");

@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kThreads)
     // ---------------- accumulators -> shared memory, [activation row][weight row] ----------------
     // every stage has been consumed when done_bar completes, so the partial sums take their place
     const int q = warp & 3;
-    const bool ok = mbar_wait(&done_bar, 0u, p.status, kKernelId, 0x300u, abort_flag);
+    const bool ok = mbar_wait_warp(&done_bar, 0u, p.status, kKernelId, 0x300u, abort_flag);
     tc_fence_after();
     if (ok)
       park_sums(tmem, reinterpret_cast<float*>(smem), q, lane, used);

@@ -204,9 +204,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     if (group < blocks) fetch(group);
     int s = 0;
     uint32_t phase = 0;
-    bool ok = true;
-    for (int t = t_lo; t < t_hi && ok; ++t) {
-      if (!mbar_wait(&pfull[s], phase, p.status, kKernelId, 0x400u + s, abort_flag)) break;
+    for (int t = t_lo; t < t_hi; ++t) {
+      mbar_pass_warp(&pfull[s], phase, p.status, kKernelId, 0x400u + s, abort_flag);
       const uint8_t* tile = smem + s * kPackedBytes + row * 128;
 #pragma unroll 1
       for (int c = group; c < kBlocks; c += 2) {
@@ -240,12 +239,8 @@ __global__ void __launch_bounds__(kThreads, 2)
           }
         }
         const int buf = b % kBufs;
-        if (!mbar_wait(&aempty[buf], (static_cast<uint32_t>(b / kBufs) & 1u) ^ 1u, p.status, kKernelId,
-                       0x420u + buf, abort_flag)) {
-          ok = false;
-          break;
-        }
-        __syncwarp();
+        mbar_pass_warp(&aempty[buf], (static_cast<uint32_t>(b / kBufs) & 1u) ^ 1u, p.status, kKernelId,
+                       0x420u + buf, abort_flag);
         tc_fence_after();
         tmem_st_32x32(lane_addr + buf * 32, w);
         tmem_st_wait();
@@ -264,7 +259,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     // every ring slot has been consumed when done_bar completes, so the partial sums take their place
     // (the other de-quantising group has read its last packed tile before its last block was multiplied)
     if (group == 0) {
-      ok = mbar_wait(&done_bar, 0u, p.status, kKernelId, 0x500u, abort_flag);
+      const bool ok = mbar_wait_warp(&done_bar, 0u, p.status, kKernelId, 0x500u, abort_flag);
       // Not earlier: a next kernel that already holds its place takes issue slots from the de-quantising
       // warps (96 requests over eight layers 1642 us with the release in front, 1553 here, 1567 without).
       grid_release();
