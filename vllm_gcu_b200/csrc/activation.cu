@@ -184,15 +184,17 @@ template <typename T, int ACT, int MODE>
 int launch_q(const Args& a, int quant, cudaStream_t s) {
   int threads = ((a.d >> 3) + 31) & ~31;
   threads = threads > 512 ? 512 : (threads < 32 ? 32 : threads);
+  auto go = [&](void (*kernel)(Args)) {
+    return launch_overlapped(kernel, dim3(a.T), dim3(threads), 0, s, a);
+  };
   switch (quant) {
-    case kQNone: return launch_overlapped(act_kernel<T, ACT, MODE, kQNone>, dim3(a.T), dim3(threads), 0, s, a);
-    case kQFp8Group128: return launch_overlapped(act_kernel<T, ACT, MODE, kQFp8Group128>, dim3(a.T), dim3(threads), 0, s, a);
-    case kQFp8Static: return launch_overlapped(act_kernel<T, ACT, MODE, kQFp8Static>, dim3(a.T), dim3(threads), 0, s, a);
-    case kQInt8Static: return launch_overlapped(act_kernel<T, ACT, MODE, kQInt8Static>, dim3(a.T), dim3(threads), 0, s, a);
-    case kQInt8Asym: return launch_overlapped(act_kernel<T, ACT, MODE, kQInt8Asym>, dim3(a.T), dim3(threads), 0, s, a);
+    case kQNone: return go(act_kernel<T, ACT, MODE, kQNone>);
+    case kQFp8Group128: return go(act_kernel<T, ACT, MODE, kQFp8Group128>);
+    case kQFp8Static: return go(act_kernel<T, ACT, MODE, kQFp8Static>);
+    case kQInt8Static: return go(act_kernel<T, ACT, MODE, kQInt8Static>);
+    case kQInt8Asym: return go(act_kernel<T, ACT, MODE, kQInt8Asym>);
     default: return -7;
   }
-  return static_cast<int>(cudaGetLastError());
 }
 
 template <typename T>

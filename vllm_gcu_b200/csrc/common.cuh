@@ -587,6 +587,13 @@ int encode_tmap_3d(CUtensorMap* out, CUtensorMapDataType dt, int elt_bytes, cons
 
 int sm_count();
 
+// What a launch answered, for the caller.  A refused launch stays behind as the runtime's last error,
+// which a later launch would answer in its own name.
+inline int launch_code(cudaError_t e) {
+  if (e != cudaSuccess) cudaGetLastError();
+  return static_cast<int>(e);
+}
+
 // Launch of a kernel that calls grid_wait().
 template <typename... P, typename... A>
 int launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
@@ -601,7 +608,7 @@ int launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, 
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+  return launch_code(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
 }
 
 // Device address of the status word of the current device (null on failure).

@@ -596,7 +596,7 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const Args& a, cudaSt
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, a));
+  return launch_code(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, a));
 }
 
 template <int EPI>
@@ -625,7 +625,7 @@ int launch_split(const CUtensorMap& tmA, const CUtensorMap& tmB, const Args& a, 
   attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, a));
+  return launch_code(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, a));
 }
 
 // Pairs the device can co-schedule for the split kernel (its resource use equals that of

@@ -348,7 +348,7 @@ static int launch(const CUtensorMap& tmW, const CUtensorMap& tmA, Args a, int un
   cfg.gridDim = dim3(2 * (units < at_once[dev] ? units : at_once[dev]));
   cfg.stream = stream;
   cfg.numAttrs = 2;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, tmW, tmA, a));
+  return launch_code(cudaLaunchKernelEx(&cfg, kernel, tmW, tmA, a));
 }
 
 static int make_maps(const void* W, uint64_t w_rows, long long ldw, const void* A, uint64_t a_rows,

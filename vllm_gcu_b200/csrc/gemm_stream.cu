@@ -337,7 +337,7 @@ static int launch(const void* A, long long lda, const void* W, long long ldw, Ar
   cudaLaunchAttribute attr[2];
   const cudaLaunchConfig_t cfg = launch_config(pl.splits, (p.N + BW - 1) / BW * pl.row_tiles, kThreads,
                                                bytes, attr, stream);
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, tmW, tmA, p));
+  return launch_code(cudaLaunchKernelEx(&cfg, kernel, tmW, tmA, p));
 }
 
 }  // namespace stream

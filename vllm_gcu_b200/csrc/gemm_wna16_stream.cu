@@ -323,7 +323,7 @@ static int launch(const CUtensorMap& tmW, const CUtensorMap& tmA, Args a, cudaSt
   if (a.x_stages < 2 || bytes > kSmemLimit) return -20;
   cudaLaunchAttribute attr[2];
   const cudaLaunchConfig_t cfg = launch_config(a.splits, tiles, kThreads, bytes, attr, stream);
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, gemm_wna16_stream_kernel<BITS>, tmW, tmA, a));
+  return launch_code(cudaLaunchKernelEx(&cfg, gemm_wna16_stream_kernel<BITS>, tmW, tmA, a));
 }
 
 }  // namespace wna16s

@@ -240,11 +240,8 @@ int launch2(const Args& a, bool add, cudaStream_t s) {
   int threads = ((a.H >> 3) + 31) & ~31;
   if (threads > 1024) threads = 1024;
   if (threads < 32) threads = 32;
-  if (add)
-    return launch_overlapped(rms_norm_kernel<T, QMODE, true>, dim3(a.T), dim3(threads), 0, s, a);
-  else
-    return launch_overlapped(rms_norm_kernel<T, QMODE, false>, dim3(a.T), dim3(threads), 0, s, a);
-  return static_cast<int>(cudaGetLastError());
+  return launch_overlapped(add ? rms_norm_kernel<T, QMODE, true> : rms_norm_kernel<T, QMODE, false>,
+                           dim3(a.T), dim3(threads), 0, s, a);
 }
 
 template <typename T>
