@@ -1,5 +1,7 @@
 """Prefill attention of two heads at once (attention_fmha_pair.cuh) at the edges of its tiles, windows and
-rescaling, against attention in 64 bits; layouts around the rule that picks it."""
+rescaling, against attention in 64 bits; layouts around the rule that picks it.  Steps of fewer tiles of
+single heads than SMs go to the kernel for one head; a tile count far above the step's, which is an upper
+bound by contract, brings them to both."""
 import pytest
 import torch
 
@@ -55,7 +57,7 @@ def test_against_64_bits(new, cached, heads, kv_heads, window, causal, block, sp
     wide = torch.randn(sum(new), heads * 128 + 64, device="cuda", generator=gen).to(torch.bfloat16)
     q = wide[:, :heads * 128].unflatten(1, (heads, 128))
     tiles = [sum(-(-n // t) for n in new) for t in (64, 128)]
-    for extra in (0, 3):                               # the tile count is an upper bound
+    for extra in (0, 3, 150):                          # more tiles than the SMs of a B200
         out, lse = C.varlen_prefill(q, kc, vc, table, cu, lens, 128 ** -0.5, tiles[0] + extra,
                                     causal=causal, window=window, return_lse=True,
                                     num_q_tiles_128=tiles[1] + extra)
@@ -78,3 +80,30 @@ def test_against_64_bits(new, cached, heads, kv_heads, window, causal, block, sp
             bound = (2.0 ** -9 + size * 2.0 ** -18) * v.abs().max() + 2.0 ** -8 * want.abs()
             assert bool(((out[rows].double() - want).abs() <= bound).all())
             assert (lse[:, rows].double() - torch.logsumexp(s, -1)).abs().max() <= 1e-5 + size * 2.0 ** -18
+
+
+# one, two and six heads per key head: both kernels at the tile counts that the others above do not reach
+@pytest.mark.parametrize("heads,kv_heads", [(2, 2), (4, 2), (6, 1)])
+@pytest.mark.parametrize("window", [0, 70])
+def test_sinks(heads, kv_heads, window):
+    from vllm_gcu_b200.ops import cuda as C
+    gen = torch.Generator(device="cuda").manual_seed(heads)
+    new, cached, block = [130, 1], [100, 64], 16
+    kc, vc, table, cu, lens = _step(new, cached, kv_heads, block, gen, 1.0)
+    q = torch.randn(sum(new), heads, 128, device="cuda", generator=gen).to(torch.bfloat16)
+    sink = torch.randn(heads, device="cuda", generator=gen)
+    for extra in (0, 150):
+        out = C.fmha_prefill_sink(q, kc, vc, table, cu, lens, 128 ** -0.5, 3 + extra, sink, window=window)
+        for i, (n, c) in enumerate(zip(new, cached)):
+            rows = slice(int(cu[i]), int(cu[i + 1]))
+            used = table[i, :-(-(n + c) // block)].long()
+            k, v = (x[used].flatten(0, 1)[:n + c].double().repeat_interleave(heads // kv_heads, 1)
+                    for x in (kc, vc))
+            s = torch.einsum("qhd,khd->hqk", q[rows].double(), k) * 128 ** -0.5
+            pos, key = torch.arange(c, n + c, device="cuda")[:, None], torch.arange(n + c, device="cuda")
+            hidden = (key > pos) | (key <= pos - window if window else key < 0)
+            s = s.masked_fill(hidden, float("-inf"))
+            p = torch.softmax(torch.cat([s, sink.double()[:, None, None].expand(-1, n, 1)], -1), -1)
+            want = torch.einsum("hqk,khd->qhd", p[..., :-1], v)
+            bound = 2.0 ** -8 * (v.abs().max() + want.abs())
+            assert bool(((out[rows].double() - want).abs() <= bound).all())

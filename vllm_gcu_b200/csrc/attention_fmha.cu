@@ -650,8 +650,13 @@ B200_API int b200_fmha_prefill_sink(const void* q, long long ldq, void* out, lon
   } while (0)
   if (slopes != nullptr) B200_FMHA(2);
   if (softcap > 0.0f || chunk > 0 || OD != HD) B200_FMHA(1);
-  // query heads in pairs over one key head: both at once
-  if (HD == 128 && ((Hq / Hkv) & 1) == 0) return launch_pair(tmQ, tmK, tmV, a, num_q_tiles, s);
+  // Query heads in pairs over one key head: both at once, where one head per CTA would take more than one
+  // round of the SMs.  A CTA with two heads takes 1.3 to 1.5 times as long as one with one, us of both at
+  // the same call: 32 heads, 128 tokens 13.0 : 8.6, 301 tokens (96 CTAs of one head) 15.3 : 11.6, 512
+  // tokens (128) 18.8 : 13.7 and behind 8192 keys 150 : 117; but 64 heads, 301 tokens (192) 15.5 : 18.5, 32
+  // heads, 1024 tokens (256) 27.2 : 35.2 and 2048 tokens 73 : 88, eight chunks of 17 behind 1024 27.9 : 40.2.
+  if (HD == 128 && ((Hq / Hkv) & 1) == 0 && static_cast<long long>(num_q_tiles) * Hq > sm_count())
+    return launch_pair(tmQ, tmK, tmV, a, num_q_tiles, s);
   B200_FMHA(0);
 #undef B200_FMHA
 }
