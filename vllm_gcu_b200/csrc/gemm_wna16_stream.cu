@@ -40,7 +40,8 @@ struct Args {
   __nv_bfloat16* C;
   long long ldc;
   int M, N, K, g_shift;
-  int rows;                       // activation rows, a multiple of 16
+  int rows;                       // activation rows of a tile, a multiple of 16
+  int row_tiles;
   int splits, packed_stages, x_stages;
   unsigned int* status;
 };
@@ -64,7 +65,10 @@ __device__ __forceinline__ void dequant8(uint32_t q, __nv_bfloat162 s2, __nv_bfl
   }
 }
 
-template <int BITS>
+// SMALL: layers of few packed tiles, whose rows may be dealt out over blockIdx.z, and which set up before
+// they wait for the kernel in front (a twentieth of their time; the others gain as much with few rows, but
+// lose it with 96 and more: 128 x 4096 x 14336 of 8 bits 35.9 -> 38.5 us).
+template <int BITS, bool SMALL>
 __global__ void __launch_bounds__(kThreads, 2)
     gemm_wna16_stream_kernel(const __grid_constant__ CUtensorMap tmW,
                              const __grid_constant__ CUtensorMap tmA, const Args p) {
@@ -81,10 +85,12 @@ __global__ void __launch_bounds__(kThreads, 2)
   __shared__ volatile uint32_t abort_word;
   volatile uint32_t* abort_flag = &abort_word;
 
-  grid_wait();
+  if constexpr (!SMALL) grid_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int split = static_cast<int>(blockIdx.x);
   const int n0 = static_cast<int>(blockIdx.y) * BW;
+  const int m0 = SMALL ? static_cast<int>(blockIdx.z) * p.rows : 0;
+  const int used = SMALL ? min(p.M - m0, p.rows) : p.M;
   uint32_t acc_cols = 32;
   while (acc_cols < static_cast<uint32_t>(p.rows)) acc_cols <<= 1;
   const uint32_t cols = acc_cols <= 128 ? 256 : 512;
@@ -116,6 +122,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot, tmem_a = tmem + acc_cols;
+  if constexpr (SMALL) grid_wait();
 
   // this CTA's packed tiles, and its blocks of 64 (the last tile of a row may hold fewer)
   const int total_blocks = p.K / 64;
@@ -146,7 +153,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       for (int b = 0; b < blocks; ++b) {
         if (!mbar_wait(&xempty[s], phase ^ 1u, p.status, kKernelId, 0x200u + s, abort_flag)) break;
         mbar_expect_tx(&xfull[s], x_bytes);
-        tma_load_2d(smem_x + s * x_bytes, &tmA, &xfull[s], (b_lo + b) * 64, 0);
+        tma_load_2d(smem_x + s * x_bytes, &tmA, &xfull[s], (b_lo + b) * 64, m0);
         if (++s == p.x_stages) {
           s = 0;
           phase ^= 1u;
@@ -265,7 +272,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       grid_release();
       __syncwarp();
       tc_fence_after();
-      if (ok) park_sums(tmem, reinterpret_cast<float*>(smem), q, lane, p.M);
+      if (ok) park_sums(tmem, reinterpret_cast<float*>(smem), q, lane, used);
     }
   }
   __syncwarp();
@@ -273,9 +280,9 @@ __global__ void __launch_bounds__(kThreads, 2)
   if (p.splits > 1) cluster_arrive_wait();
   else __syncthreads();
   if (abort_word == 0u)
-    sum_rows<false, false>(smem, split, p.splits, warp, kThreads / 32, lane, p.M, [&](int r, float4 v) {
+    sum_rows<false, false>(smem, split, p.splits, warp, kThreads / 32, lane, used, [&](int r, float4 v) {
       const int col = n0 + 4 * lane;
-      __nv_bfloat16* out = p.C + static_cast<long long>(r) * p.ldc + col;
+      __nv_bfloat16* out = p.C + static_cast<long long>(m0 + r) * p.ldc + col;
       float f[4] = {v.x, v.y, v.z, v.w};
       if (col + 4 <= p.N && (p.ldc & 3) == 0) {
         if (p.bias != nullptr)
@@ -297,22 +304,50 @@ __global__ void __launch_bounds__(kThreads, 2)
 }
 
 template <int BITS>
-static int launch(const CUtensorMap& tmW, const CUtensorMap& tmA, Args a, cudaStream_t stream) {
-  static AtOnce table = {};
-  const int* at_once = clusters_at_once(table, gemm_wna16_stream_kernel<BITS>, kThreads);
-  if (at_once == nullptr) return -20;
+static int launch(const void* A, long long lda, const void* qw, Args a, cudaStream_t stream) {
   const int tiles = (a.N + BW - 1) / BW;
   const int packed = (a.K / 64 + (BITS == 4 ? 3 : 1)) / (BITS == 4 ? 4 : 2);
+  const bool small = packed <= 8;
+  static AtOnce table[2] = {};
+  auto kernel = small ? gemm_wna16_stream_kernel<BITS, true> : gemm_wna16_stream_kernel<BITS, false>;
+  const int* at_once = clusters_at_once(table[small], kernel, kThreads);
+  if (at_once == nullptr) return -20;
   // Bound by the de-quantising warps, so what counts is that every SM has the same share: two CTAs per
   // SM and the largest split that one wave takes, down to two packed tiles a slice (four above 32 rows,
   // where the sums of a slice cost more).  4096 x 14336 at 16 rows: eight slices 22.7 us, four 25.2; at
   // 128 rows 29.2 and 29.5; 4096 x 4096 at 128 rows: eight 16.6, four 14.4; 6144 x 4096 at 16 rows in
   // one wave (five) 15.0, in two (six) 19.5.  Above 128 rows accumulators and de-quantised blocks fill
   // the tensor memory of an SM: one CTA.
-  const int per_sm = a.rows > 128 ? 1 : 2;
+  a.row_tiles = 1;
+  a.rows = (a.M + 15) / 16 * 16;
   a.splits = 1;
   for (int s = 2; s <= kMaxSplits; ++s)
-    if (packed >= s * (a.rows > 32 ? 4 : 2) && tiles <= at_once_for(at_once, s, per_sm)) a.splits = s;
+    if (packed >= s * (a.rows > 32 ? 4 : 2) && tiles <= at_once_for(at_once, s, a.rows > 128 ? 1 : 2))
+      a.splits = s;
+  // Layers of few packed tiles leave most SMs idle that way.  With one CTA per SM a slice may have as
+  // little as one packed tile, and the rows may be dealt out as well (every tile de-quantises for itself):
+  // a CTA takes about as long for a packed tile, 1 us, as for moving out the sums of 50 rows, and two on an SM
+  // 1.7 times as long as one.  4 bits, in one tile of rows and slices as above : as here (: tiles of 64 x 64 built in
+  // shared memory), us: 64 x 512 x 512 7.7 : 4.9 (6.4), 256 x 512 x 512 12.6 : 5.0 (8.1), 256 x 1024 x
+  // 1024 15.5 : 6.4 (11.0), 128 x 4096 x 1024 12.0 : 7.7 (9.2), 256 x 2048 x 2048 15.0 : 9.2 (23).
+  if (small) {
+    auto cost = [&](int row_tiles, int rows, int splits) {
+      const int load = (tiles * row_tiles * splits + at_once[1] - 1) / at_once[1];
+      return ((packed + splits - 1) / splits + rows * 0.02) * (load > 1 ? 0.85 * load : 1.0);
+    };
+    double best = cost(1, a.rows, a.splits);
+    for (int t = 1; t <= 16; t *= 2) {
+      const int rows = ((a.M + t - 1) / t + 15) / 16 * 16;
+      for (int s = 1; s <= kMaxSplits && s <= packed; ++s)
+        if (tiles * t <= at_once[s] && cost(t, rows, s) < best) {
+          best = cost(t, rows, s);
+          a.rows = rows;
+          a.splits = s;
+        }
+    }
+    a.row_tiles = (a.M + a.rows - 1) / a.rows;
+  }
+  const int per_sm = a.rows > 128 ? 1 : 2;
   a.packed_stages = per_sm == 2 ? 2 : 6;
   const int room = (per_sm == 2 ? kSmemLimit / 2 - 1024 : kSmemLimit) - 1024;
   a.x_stages = (room - a.packed_stages * kPackedBytes) / (a.rows * 128);
@@ -321,9 +356,19 @@ static int launch(const CUtensorMap& tmW, const CUtensorMap& tmA, Args a, cudaSt
   const int sums = a.rows * BW * 4;
   const int bytes = (ring > sums ? ring : sums) + 1024;
   if (a.x_stages < 2 || bytes > kSmemLimit) return -20;
+  const uint64_t kbytes = static_cast<uint64_t>(BITS == 4 ? a.K / 2 : a.K);
+  CUtensorMap tmW, tmA;
+  int r = encode_tmap_2d(&tmW, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, qw, static_cast<uint64_t>(a.N), kbytes,
+                         kbytes, BW, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r == 0)
+    r = encode_tmap_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, static_cast<uint64_t>(a.M),
+                       static_cast<uint64_t>(a.K), static_cast<uint64_t>(lda) * 2, a.rows, 64,
+                       CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r != 0) return r < 0 ? -6 : r;
   cudaLaunchAttribute attr[2];
-  const cudaLaunchConfig_t cfg = launch_config(a.splits, tiles, kThreads, bytes, attr, stream);
-  return launch_code(cudaLaunchKernelEx(&cfg, gemm_wna16_stream_kernel<BITS>, tmW, tmA, a));
+  cudaLaunchConfig_t cfg = launch_config(a.splits, tiles, kThreads, bytes, attr, stream);
+  cfg.gridDim.z = a.row_tiles;
+  return launch_code(cudaLaunchKernelEx(&cfg, kernel, tmW, tmA, a));
 }
 
 }  // namespace wna16s
@@ -344,16 +389,6 @@ B200_API int b200_gemm_wna16(const void* A, long long lda, const void* qw, const
       ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(qw)) & 15))
     return -20;
   Args a;
-  a.rows = (M + 15) / 16 * 16;
-  const uint64_t kbytes = static_cast<uint64_t>(bits == 4 ? K / 2 : K);
-  CUtensorMap tmW, tmA;
-  int r = encode_tmap_2d(&tmW, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, qw, static_cast<uint64_t>(N), kbytes,
-                         kbytes, BW, 128, CU_TENSOR_MAP_SWIZZLE_128B);
-  if (r != 0) return r < 0 ? -6 : r;
-  r = encode_tmap_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, static_cast<uint64_t>(M),
-                     static_cast<uint64_t>(K), static_cast<uint64_t>(lda) * 2, a.rows, 64,
-                     CU_TENSOR_MAP_SWIZZLE_128B);
-  if (r != 0) return r < 0 ? -6 : r;
   a.scales = static_cast<const __nv_bfloat16*>(scales);
   a.zs = static_cast<const __nv_bfloat16*>(zs);
   a.bias = static_cast<const __nv_bfloat16*>(bias);
@@ -363,5 +398,5 @@ B200_API int b200_gemm_wna16(const void* A, long long lda, const void* qw, const
   a.g_shift = 31 - __builtin_clz(static_cast<unsigned>(g));
   a.status = status_ptr();
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  return bits == 4 ? launch<4>(tmW, tmA, a, s) : launch<8>(tmW, tmA, a, s);
+  return bits == 4 ? launch<4>(A, lda, qw, a, s) : launch<8>(A, lda, qw, a, s);
 }
