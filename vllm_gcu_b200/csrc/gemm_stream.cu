@@ -290,11 +290,22 @@ static int smem_bytes(int rows, int stages) {
 
 // Up to 128 activation rows make one tile, more make tiles of 128 (a split of K costs 512 bytes per
 // row of traffic between the SMs, at about 25 GB/s per SM: it stays below what it saves up to there).
+// Smaller ones where K is so short that it leaves no room for a split and SMs for more tiles: moving out
+// the sums is most of a tile's time then.  us with one tile of rows : as here (the kernels that went
+// before), 128 x 512 x 512 of 8 bits 10.9 : 4.0 (10.0), 256 x 1152 x 896 11.5 : 5.5 (11.1), 32 x 1024 x 128
+// of bf16 3.9 : 3.2 (3.5).  With a longer K it does not pay: 17 x 896 x 4864 5.3 : 6.6.
 static Plan make_plan(int M, int N, int blocks, const int* at_once) {
+  const int tiles = (N + BW - 1) / BW;
   Plan pl;
-  pl.row_tiles = (M + 127) / 128;
-  pl.rows = ((M + pl.row_tiles - 1) / pl.row_tiles + 15) / 16 * 16;
-  const Split sp = plan_split((N + BW - 1) / BW * pl.row_tiles, blocks, 4, at_once);
+  Split sp;
+  for (pl.row_tiles = (M + 127) / 128;; pl.row_tiles *= 2) {
+    const int used = (M + pl.row_tiles - 1) / pl.row_tiles;
+    pl.rows = (used + 15) / 16 * 16;
+    sp = plan_split(tiles * pl.row_tiles, blocks, 4, at_once);
+    const int ctas = tiles * pl.row_tiles * sp.splits;
+    if (blocks > 8 || pl.rows == 16 || (used > 24 ? 2 : 4) * ctas > at_once[1]) break;
+  }
+  pl.row_tiles = (M + pl.rows - 1) / pl.rows;
   pl.splits = sp.splits;
   const int room = (sp.per_sm == 2 ? kSmemLimit / 2 - 1024 : kSmemLimit) - 1024;
   pl.stages = room / (kWBytes + pl.rows * kRowBytes);

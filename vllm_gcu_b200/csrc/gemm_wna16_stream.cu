@@ -327,7 +327,7 @@ static int launch(const void* A, long long lda, const void* qw, Args a, cudaStre
   // Layers of few packed tiles leave most SMs idle that way.  With one CTA per SM a slice may have as
   // little as one packed tile, and the rows may be dealt out as well (every tile de-quantises for itself):
   // a CTA takes about as long for a packed tile, 1 us, as for moving out the sums of 50 rows, and two on an SM
-  // 1.7 times as long as one.  4 bits, in one tile of rows and slices as above : as here (: tiles of 64 x 64 built in
+  // 1.7 times as long as one.  4 bits, one tile of rows and slices as above : as here (tiles of 64 x 64 built in
   // shared memory), us: 64 x 512 x 512 7.7 : 4.9 (6.4), 256 x 512 x 512 12.6 : 5.0 (8.1), 256 x 1024 x
   // 1024 15.5 : 6.4 (11.0), 128 x 4096 x 1024 12.0 : 7.7 (9.2), 256 x 2048 x 2048 15.0 : 9.2 (23).
   if (small) {
