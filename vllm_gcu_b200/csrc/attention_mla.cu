@@ -33,9 +33,12 @@
 //                surplus ones are never stored).
 // A key tile is stored in groups of eight keys, every 64-wide chunk of a group 1 KB: one TMA copy
 // brings eight whole rows of the cache, eight copies a tile.
-// Measured (one key tile with 128 heads, 36 copies of 16 rows x 128 bytes a tile before): 256 requests x
-// 1152 keys, W 576, L 512: 128 heads 286 -> 189 us, 16 heads 219 -> 177; 4 x 2048 new tokens, 128 heads 6778
-// -> 4503 us = 519 TFLOP/s of useful work (the scores are computed twice: 794 in all).
+// Measured (one key tile with 128 heads, 36 copies of 16 rows x 128 bytes a tile before), W 576, L 512: 256
+// requests x 1152 keys, 128 heads 281 -> 167 us, 16 heads 214 -> 170; 128 requests x 128 keys, 128 heads
+// 27.7 -> 23.8; 2 x 1024 new tokens, 128 heads 980 -> 644 us = 454 TFLOP/s of useful work (the scores are
+// computed twice).  The columns of Q for tensor memory pass through the place of the second key tile:
+// read from global memory by the threads that own the rows they came 3 to 5 us later, which a context of
+// two key tiles does not get back (2 x 1024 new tokens 758, one request x 64 keys 13.5 against 10.0).
 //
 // Long contexts are split over blockIdx.y; the partial results (normalised output +
 // log-sum-exp per row) are merged by mla_combine_kernel.  Whichever writes the result also applies
@@ -80,7 +83,11 @@ static Lay make_lay(int qrows, int n_q, int n_w) {
   const int q_chunk = qrows * 128;
   l.off_k = kOffQ + n_q * q_chunk;
   l.off_p = l.off_k + 2 * n_w * kKChunk;
-  const int end = l.off_p + BQ * 128;
+  int end = l.off_p + BQ * 128;
+  if (n_q < n_w) {         // the other chunks of Q pass through the second key tile and what follows
+    const int staged = l.off_k + n_w * kKChunk + (n_w - n_q) * BQ * 128;
+    end = end > staged ? end : staged;
+  }
   // the 128-row MMA reads 16 KB from the start of every Q chunk: keep that inside the allocation
   const int read_end = kOffQ + (n_q - 1) * q_chunk + BQ * 128;
   l.bytes = (end > read_end ? end : read_end) + 1024;
@@ -94,7 +101,6 @@ __device__ __forceinline__ float ex2_approx(float x) {
 }
 
 struct Args {
-  const __nv_bfloat16* q;  // [T * N, 64 n_w]
   __nv_bfloat16* out;      // [T * N, L]
   float* ws_o;             // splits > 1: [splits, T * N, L] normalised partial outputs
   float* ws_lse;           // splits > 1: [splits, T * N] natural-log LSE (-inf: nothing seen)
@@ -145,6 +151,7 @@ __global__ void __launch_bounds__(kThreads, kResident)
   uint64_t* s_empty = bars + 7;     // [2]
   uint64_t* p_full = bars + 9;
   uint64_t* o_done = bars + 10;
+  uint64_t* q_staged = bars + 13;   // (behind the words below)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   int* s_info = reinterpret_cast<int*>(tmem_slot + 2);
@@ -164,6 +171,7 @@ __global__ void __launch_bounds__(kThreads, kResident)
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, kQT > 0 ? 9 : 1);
+    mbar_init(q_staged, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1);
       mbar_init(&k_empty[i], 1);
@@ -258,10 +266,16 @@ __global__ void __launch_bounds__(kThreads, kResident)
   const uint32_t tmem_base = *tmem_slot;
 
   uint8_t* p_smem = smem + a.off_p;
+  uint8_t* q_stage = smem + a.off_k + k_tile;      // chunks of Q on their way to tensor memory
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (elect_one()) {
+      if constexpr (kQT > 0) {
+        mbar_expect_tx(q_staged, kQT * kQChunk);
+        for (int c = 0; c < kQT; ++c)
+          tma_load_2d(q_stage + c * kQChunk, &tmQ, q_staged, c * 64, static_cast<int>(row0));
+      }
       mbar_expect_tx(q_full, (n_w - kQT) * kQChunk);
       for (int c = kQT; c < n_w; ++c)
         tma_load_2d(smem + kOffQ + (c - kQT) * kQChunk, &tmQ, q_full, c * 64, static_cast<int>(row0));
@@ -270,6 +284,8 @@ __global__ void __launch_bounds__(kThreads, kResident)
       for (int j = 0; j < nt; ++j) {
         const int st = j % kStages;
         const uint32_t use = static_cast<uint32_t>(j / kStages);
+        // the second tile takes the place that Q passes through
+        if (kQT > 0 && j == 1 && !mbar_wait(q_full, 0, a.status, kKernelId, 0x110u, abort_flag)) break;
         if (!mbar_wait(&k_empty[st], (use & 1u) ^ 1u, a.status, kKernelId, 0x100u + st, abort_flag))
           break;
         mbar_expect_tx(&k_full[st], k_tile);
@@ -391,20 +407,19 @@ __global__ void __launch_bounds__(kThreads, kResident)
       gate = head_gate(a.gate, a.ldg, static_cast<long long>(q_start) + tok0 + tok, head);
     }
     if constexpr (kQT > 0) {
-      // this row's half of the columns of Q that tensor memory takes
-      const bool there = row0 + r < rows_total;
-      const uint4* src = reinterpret_cast<const uint4*>(
-          a.q + (there ? row0 + r : row0) * (64 * n_w) + g * (kQT * 32));
+      // this row's half of the columns of Q that tensor memory takes (by TMA into shared memory first:
+      // read straight from global memory, a row a lane, they came 3 to 5 us later)
+      mbar_pass_warp(q_staged, 0, a.status, kKernelId, 0x330u, abort_flag);
 #pragma unroll
-      for (int c = 0; c < kQT / 2; ++c) {
+      for (int c = g * (kQT / 2); c < (g + 1) * (kQT / 2); ++c) {
+        const uint8_t* src = q_stage + c * kQChunk + r * 128;
         uint32_t w[32];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const uint4 u = src[c * 8 + i];
-          w[4 * i] = there ? u.x : 0u; w[4 * i + 1] = there ? u.y : 0u;
-          w[4 * i + 2] = there ? u.z : 0u; w[4 * i + 3] = there ? u.w : 0u;
+          const uint4 u = *reinterpret_cast<const uint4*>(src + ((i ^ (r & 7)) << 4));
+          w[4 * i] = u.x; w[4 * i + 1] = u.y; w[4 * i + 2] = u.z; w[4 * i + 3] = u.w;
         }
-        tmem_st_32x32(lane_addr + kColQ + (g * (kQT / 2) + c) * 32, w);
+        tmem_st_32x32(lane_addr + kColQ + c * 32, w);
       }
       tmem_st_wait();
       tc_fence_before();
@@ -683,7 +698,6 @@ B200_API int b200_mla_attention(const void* q, void* out, const void* cache, lon
   r = get_map(cache, static_cast<unsigned long long>(num_slots), W, kGroup, true, &tmK);
   if (r != 0) return r < 0 ? -6 : r;
   Args a;
-  a.q = static_cast<const __nv_bfloat16*>(q);
   a.out = static_cast<__nv_bfloat16*>(out);
   const long long rows_total = static_cast<long long>(T) * N;
   a.ws_o = workspace;
