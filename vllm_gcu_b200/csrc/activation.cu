@@ -102,7 +102,7 @@ struct Args {
 
 template <typename T, int ACT, int MODE, int QUANT>
 __global__ void __launch_bounds__(512) act_kernel(const Args a) {
-  grid_release();
+  grid_release_small();
   grid_wait();
   const int row = blockIdx.x;
   if (a.valid_rows != nullptr && row >= *a.valid_rows) return;

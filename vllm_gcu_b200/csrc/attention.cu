@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kThreads) paged_decode_kernel(const DecodeArgs
 
 template <typename T, int HD>
 __global__ void __launch_bounds__(128) decode_reduce_kernel(const DecodeArgs a) {
-  grid_release();
+  grid_release_small();
   grid_wait();
   const int b = blockIdx.x, head = blockIdx.y;
   const long long base = (static_cast<long long>(b) * a.Hq + head) * a.num_splits;

@@ -103,7 +103,7 @@ __device__ __forceinline__ void store_cache8(const RopeCacheArgs& a, bool is_v, 
 // where two norm kernels and two copies into dense rows took 115 more (4096 tokens, 32 + 4 heads).
 template <typename T, int LANES, bool NORM>
 __global__ void __launch_bounds__(256) rope_cache_heads_kernel(const RopeCacheArgs a) {
-  grid_release();
+  grid_release_small();
   grid_wait();
   const int heads = a.Hq + 2 * a.Hkv;
   const long long item = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;

@@ -154,6 +154,14 @@ __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;
 __device__ __forceinline__ void grid_release() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// The same for kernels of one or a few rows per CTA, in grids of at most 2048 CTAs; the next kernel starts as
+// the last CTAs end in larger ones.  Every CTA that executes the instruction takes 0.45 ns more of the grid's
+// time (norm of 16384 rows of 128 columns 17.9 us with it and 10.5 without, 48896 CTAs that place the rows
+// of a few tokens over 384 experts 51 and 27), and the next kernel gains about 2 us by it (three layers of
+// fp8 rows, norms and activations between GEMMs, 1024 rows 977 us with it and 1009 without, 256 rows 398 and 405).
+__device__ __forceinline__ void grid_release_small() {
+  if (static_cast<unsigned long long>(gridDim.x) * gridDim.y * gridDim.z <= 2048u) grid_release();
+}
 
 // ---------------------------------------------------------------------------
 // TMA (tiled bulk tensor copies, never with cluster multicast)

@@ -55,7 +55,7 @@ __device__ __forceinline__ float load_gate(const void* p, long long i, int dtype
 
 // 4 warps per CTA, one token per warp.  Shared: per warp 2 * E floats.
 __global__ void __launch_bounds__(128) moe_topk_kernel(const TopkArgs a) {
-  grid_release();
+  grid_release_small();
   grid_wait();
   extern __shared__ float sm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -173,7 +173,7 @@ struct AlignArgs {
 };
 
 __global__ void __launch_bounds__(1024) moe_align_kernel(const AlignArgs a) {
-  grid_release();
+  grid_release_small();
   grid_wait();
   extern __shared__ int smi[];
   int* count = smi;                              // [E]
@@ -242,7 +242,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
     moe_permute_kernel(const T* x, long long ldx, T* out, long long ldo, const int* sorted_ids,
                        const int* num_post_pad, int numel, int k, int H, int zero_pads) {
-  grid_release();
+  grid_release_small();
   grid_wait();
   const int pos = blockIdx.x;
   if (pos >= *num_post_pad) return;
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(256)
     moe_unpermute_sum_kernel(const T* y, long long ldy, const int* pos_of, const T* add,
                              long long lda, T* out, long long ldo, const int* valid_tokens, int k,
                              int H, float alpha) {
-  grid_release();
+  grid_release_small();
   grid_wait();
   const int t = blockIdx.x;
   if (valid_tokens != nullptr && t >= *valid_tokens) return;
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(256)
 // Per sorted row: the routing weight of its (token, slot) pair (0 for padding rows).
 __global__ void moe_row_weights_kernel(const int* sorted_ids, const float* topk_w,
                                        const int* num_post_pad, float* row_w, int numel, int cap) {
-  grid_release();
+  grid_release_small();
   grid_wait();
   const int pos = blockIdx.x * blockDim.x + threadIdx.x;
   if (pos >= cap) return;

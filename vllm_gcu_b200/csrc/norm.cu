@@ -113,7 +113,7 @@ struct Args {
 template <typename T, int QMODE, bool ADD>
 __global__ void __launch_bounds__(1024) rms_norm_kernel(const Args a) {
   __shared__ float red[32];
-  grid_release();
+  grid_release_small();
   grid_wait();
   const int row = blockIdx.x;
   if (a.valid_rows != nullptr && row >= *a.valid_rows) return;

@@ -23,7 +23,7 @@ template <typename T, bool INT8>
 __global__ void __launch_bounds__(1024)
     per_token_quant_kernel(const T* x, long long ldx, uint8_t* out, long long ldo, float* scales,
                            const int* valid_rows, int H) {
-  grid_release();
+  grid_release_small();
   grid_wait();
   __shared__ float red[32];
   const int row = blockIdx.x;

@@ -190,7 +190,7 @@ struct Args {
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) sample_kernel(const Args a) {
-  grid_release();
+  grid_release_small();
   grid_wait();
   // 32 KB shared by the replicated histogram of a full-row select (first 16 KB) and the
   // candidate list that replaces the row once top-k has cut it down.
