@@ -30,6 +30,35 @@ def _close(a, b, rtol, atol):
     assert bad == 0.0, f"{bad:.2%} out of tolerance, max err {err.max().item():.4g}"
 
 
+class _Calls:
+    """The native library, with the result of every call."""
+
+    def __init__(self, lib):
+        self._lib, self.seen = lib, []
+
+    def __getattr__(self, name):
+        fn = getattr(self._lib, name)
+
+        def call(*args):
+            rc = fn(*args)
+            self.seen.append((name, rc))
+            return rc
+        return call
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    c = _Calls(_native.lib())
+    monkeypatch.setattr(_native, "lib", lambda: c)
+    return c
+
+
+def _no_swapped_operands(C, monkeypatch):
+    """The rules that come first take no call (gemm_stream.cu, gemm_pair_rows.cu)."""
+    monkeypatch.setattr(C, "_stream_pays", lambda *a: False)
+    monkeypatch.setattr(C, "_pair_rows", lambda *a: 0)
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 128, 64), (256, 512, 4096), (1, 4096, 4096),
                                    (77, 6144, 4096), (333, 256, 200), (1024, 28672, 4096),
                                    (8192, 4096, 4096), (130, 136, 72)])
@@ -45,11 +74,12 @@ def test_gemm_bf16(C, M, N, K):
 @pytest.mark.parametrize("M,N,K", [(256, 6144, 4096), (256, 4096, 14336), (200, 4096, 4096),
                                    (129, 28672, 4096), (64, 2048, 2048), (7, 136, 72),
                                    (256, 128256, 1024), (128, 64, 8192), (256, 1024, 256)])
-def test_gemm_skinny_decode_shapes(C, M, N, K, monkeypatch):
+def test_gemm_skinny_decode_shapes(C, M, N, K, monkeypatch, calls):
     """Weight-streaming kernel for M <= 256 (column tile x K slice per CTA, split-K reduce):
     same result as the fp32 reference, also on repeated launches (the counters must come back
     to zero) and identical to the persistent-tile kernel within bf16 rounding."""
     assert C.USE_SKINNY_GEMM and M <= C.SKINNY_MAX_M
+    _no_swapped_operands(C, monkeypatch)
     monkeypatch.setattr(C, "USE_PAIR_GEMM", False)          # (wide shapes would go to CTA pairs)
     monkeypatch.setattr(C, "SKINNY_ALLOW_SPLIT", True)      # exercise the split-K path too
     a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
@@ -62,6 +92,8 @@ def test_gemm_skinny_decode_shapes(C, M, N, K, monkeypatch):
         if first is None:
             first = out.clone()
         assert torch.equal(out, first), "split-K reduction must be reproducible"
+    assert calls.seen == [("b200_gemm_skinny_workspace", 0)] * (len(calls.seen) - 3) \
+        + [("b200_gemm_skinny", 0)] * 3
     bias = torch.randn(N, device="cuda", dtype=torch.bfloat16)
     _close(C.gemm_bf16(a, b, bias=bias), want + bias.float(), 2e-2, 3e-2)
     if N % 256 == 0:
@@ -126,12 +158,13 @@ def test_gemm_cta_pair_large_m(C, M, N, K, mt, monkeypatch):
 @pytest.mark.parametrize("M,N,K,epi", [(256, 4096, 4096, 0), (256, 6144, 1024, 0),
                                        (200, 1024, 2048, 1), (512, 4096, 4096, 0),
                                        (130, 2048, 1024, 2)])
-def test_gemm_cta_pair_k_split(C, M, N, K, epi, monkeypatch):
+def test_gemm_cta_pair_k_split(C, M, N, K, epi, monkeypatch, calls):
     """K split of the CTA-pair kernel (one tile and K slice per pair, fp32 partial sums meet at
     a counter, every CTA reduces a row slice): off by default (measured slower than the
     weight-streaming kernel), kept correct: same result as the reference, bitwise equal on
     repeated launches (the counters return to zero)."""
     monkeypatch.setattr(C, "USE_PAIR_SPLIT", True)
+    _no_swapped_operands(C, monkeypatch)
     torch.manual_seed(M + N + K)
     a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
     b = (torch.randn(N, K, device="cuda") / math.sqrt(K)).to(torch.bfloat16)
@@ -147,6 +180,7 @@ def test_gemm_cta_pair_k_split(C, M, N, K, epi, monkeypatch):
     first = C.gemm_bf16(a, b, bias=bias, epilogue=epi)
     _close(first, want, 3e-2, 3e-2)
     assert torch.equal(C.gemm_bf16(a, b, bias=bias, epilogue=epi), first)
+    assert calls.seen[-2:] == [("b200_gemm_pair_split", 0)] * 2
     torch.cuda.synchronize()
     assert int(wsp[1].abs().sum()) == 0
     _native.check_status()
@@ -482,12 +516,13 @@ def test_advance_step(C):
 
 
 @pytest.mark.parametrize("M,N,K", [(64, 4096, 14336), (1, 4096, 4096), (100, 1024, 8192)])
-def test_skinny_gemm_two_kernel_k_split_matches_reference(M, N, K):
+def test_skinny_gemm_two_kernel_k_split_matches_reference(M, N, K, monkeypatch, calls):
     """Rows <= 128: wide column tiles with a K split whose fp32 partial sums are added by a
     second kernel (gemm_skinny.cu, ``make_plan2``), with and without a bias."""
     import ctypes
     from vllm_gcu_b200.ops import _native
     from vllm_gcu_b200.ops import cuda as C
+    _no_swapped_operands(C, monkeypatch)
     torch.manual_seed(M + N)
     x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
     w = torch.randn(N, K, device="cuda", dtype=torch.bfloat16) * 0.02
@@ -502,3 +537,22 @@ def test_skinny_gemm_two_kernel_k_split_matches_reference(M, N, K):
     _native.check_status()
     # twice the same: the summation order is fixed
     assert torch.equal(C.gemm_bf16(x, w), C.gemm_bf16(x, w))
+    assert [c for c in calls.seen if c[0].startswith("b200_gemm") and c[0] != "b200_gemm_skinny_workspace"] \
+        == [("b200_gemm_skinny", 0)] * 4
+
+
+@pytest.mark.parametrize("M,N,K,wide", [(33, 128, 2560, True), (128, 128, 2560, True),
+                                        (64, 512, 3584, False), (100, 1024, 3584, False)])
+def test_skinny_gemm_where_the_rules_leave_it(M, N, K, wide, calls):
+    """33 to 128 rows and a K below 4096 still go to the K split with a second kernel, results in 32 bits
+    among them."""
+    from vllm_gcu_b200.ops import cuda as C
+    torch.manual_seed(M + N)
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda") / math.sqrt(K)).to(torch.bfloat16)
+    want = x.double() @ w.double().t()
+    got = C.gemm_bf16(x, w, epilogue=C.EPI_FP32 if wide else C.EPI_NONE)
+    assert calls.seen[-1] == ("b200_gemm_skinny", 0)
+    # sums of K products in 32 bits, the result rounded to bf16
+    bound = K * 2.0 ** -24 * 0.8 + (2.0 ** -23 if wide else 2.0 ** -8) * want.abs()
+    assert bool(((got.double() - want).abs() <= bound).all())
