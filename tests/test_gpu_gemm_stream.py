@@ -22,7 +22,8 @@ def _status_clean():
 # the slices do not share evenly, and fewer blocks than a split takes
 SHAPES = [(1, 8, 8), (1, 4096, 4096), (3, 136, 72), (15, 200, 1000), (16, 128, 4160), (17, 640, 5120),
           (32, 6144, 4096), (31, 28672, 512), (32, 19072, 264), (33, 6144, 4096), (64, 2112, 7168),
-          (65, 4096, 4160), (128, 8192, 4096), (129, 4096, 4104), (256, 2048, 4096), (250, 72, 14336)]
+          (65, 4096, 4160), (128, 8192, 4096), (129, 4096, 4104), (256, 2048, 4096), (250, 72, 14336),
+          (32, 1024, 128), (27, 200, 512), (17, 8, 72)]       # K so short that rows go into more tiles
 
 
 @pytest.mark.parametrize("M,N,K", SHAPES)
