@@ -2,9 +2,10 @@
 captured in a CUDA graph and replayed (a single launch from Python costs more host time than
 these kernels take on the device), weights cycling through copies that exceed L2.
 
-Per shape: the kernel the dispatcher picks (persistent tiles, weight-streaming kernel, two-kernel
-K split for up to 128 rows), the same with the K split switched off, the CTA-pair kernel
-(one 256 x 256 tile per cluster of two, no K split) and torch.matmul (cuBLAS).
+Per shape: the kernel the dispatcher picks; what it picks without the kernels that have the weights on the
+M side (gemm_stream.cu, gemm_pair_rows.cu): persistent tiles, 256-wide column tiles, a two-kernel K split
+for up to 128 rows; the same with that K split switched off; the CTA-pair kernel (one 256 x 256 tile per
+cluster of two, no K split) and torch.matmul (cuBLAS).
 
 Usage: python benchmarks/kernels/bench_decode_gemm.py [--rows 256 128 64 16 1]
 """
@@ -46,8 +47,8 @@ def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--rows", type=int, nargs="+", default=[256, 128, 64, 16, 1])
     a = ap.parse_args()
-    keep = C.SKINNY_SPLIT2_MAX_M
-    print(f"{'rows':>5} {'layer':>8} {'N x K':>14} {'ours us':>8} {'no split us':>12} "
+    keep = C.SKINNY_SPLIT2_MAX_M, C._stream_pays, C._pair_rows
+    print(f"{'rows':>5} {'layer':>8} {'N x K':>14} {'ours us':>8} {'W on N us':>10} {'no split us':>12} "
           f"{'pair us':>8} {'cuBLAS us':>10}")
     for M in a.rows:
         for Nn, K, name in SHAPES:
@@ -56,11 +57,15 @@ def main():
                   for _ in range(copies)]
             x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
             out = torch.empty(M, Nn, device="cuda", dtype=torch.bfloat16)
-            C.SKINNY_SPLIT2_MAX_M = keep
-            t_ours = replay_time(lambda i: C.gemm_bf16(x, ws[i % copies], out=out))
+
+            def dispatched(i):
+                C.gemm_bf16(x, ws[i % copies], out=out)
+            t_ours = replay_time(dispatched)
+            C._stream_pays, C._pair_rows = (lambda *shape: False), (lambda *shape: 0)
+            t_n_side = replay_time(dispatched)
             C.SKINNY_SPLIT2_MAX_M = 0
-            t_nosplit = replay_time(lambda i: C.gemm_bf16(x, ws[i % copies], out=out))
-            C.SKINNY_SPLIT2_MAX_M = keep
+            t_nosplit = replay_time(dispatched)
+            C.SKINNY_SPLIT2_MAX_M, C._stream_pays, C._pair_rows = keep
 
             def pair(i):
                 w = ws[i % copies]
@@ -70,7 +75,8 @@ def main():
                 assert rc == 0, rc
             t_pair = replay_time(pair) if Nn % 256 == 0 else float("nan")
             t_ref = replay_time(lambda i: torch.matmul(x, ws[i % copies].t(), out=out))
-            print(f"{M:>5} {name:>8} {Nn:>7} x {K:<5} {t_ours:8.1f} {t_nosplit:12.1f} "
+            print(f"{M:>5} {name:>8} {Nn:>7} x {K:<5} {t_ours:8.1f} {t_n_side:10.1f} "
+                  f"{t_nosplit:12.1f} "
                   f"{t_pair:8.1f} {t_ref:10.1f}", flush=True)
             del ws
 

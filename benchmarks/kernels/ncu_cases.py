@@ -15,6 +15,11 @@ launches the kernel of interest a handful of times:
   python benchmarks/kernels/ncu_cases.py --case mla_decode     # latent attention, 128 heads
   python benchmarks/kernels/ncu_cases.py --case mla_decode_small  # latent attention, 16 heads
   python benchmarks/kernels/ncu_cases.py --case wna16_decode   # fused 4-bit de-quantising GEMM
+  python benchmarks/kernels/ncu_cases.py --case gemm_one_row   # 1 x 28672 x 4096 bf16
+  python benchmarks/kernels/ncu_cases.py --case gemm_prompt    # 301 x 28672 x 4096 bf16
+  python benchmarks/kernels/ncu_cases.py --case experts_decode   # 64 tokens, 8 of 128 experts, w13
+  python benchmarks/kernels/ncu_cases.py --case experts_prefill  # 4096 tokens, the same
+  python benchmarks/kernels/ncu_cases.py --case rope_heads     # 8192 tokens, 32 + 8 heads, head norms
 
 Capture (one GPU):
   ncu --set full --clock-control none -k regex:<kernel> -s 2 -c 2 -o <output dir>/<name> \
@@ -38,8 +43,10 @@ def main():
     a = ap.parse_args()
     dev = "cuda"
     torch.manual_seed(0)
-    if a.case in ("gemm_prefill", "gemm_decode"):
-        M, N, K = (8192, 4096, 4096) if a.case == "gemm_prefill" else (256, 4096, 14336)
+    gemms = {"gemm_prefill": (8192, 4096, 4096), "gemm_decode": (256, 4096, 14336),
+             "gemm_one_row": (1, 28672, 4096), "gemm_prompt": (301, 28672, 4096)}
+    if a.case in gemms:
+        M, N, K = gemms[a.case]
         x = torch.randn(M, K, device=dev, dtype=torch.bfloat16)
         w = torch.randn(N, K, device=dev, dtype=torch.bfloat16) * 0.02
         out = torch.empty(M, N, device=dev, dtype=torch.bfloat16)
@@ -168,6 +175,28 @@ def main():
         def fn():
             state["i"] += 1
             C.gemm_wna16(x, qws[state["i"] % 3], sc, zs, g, 4)
+    elif a.case in ("experts_decode", "experts_prefill"):
+        # the gated product of Qwen3-30B-A3B's experts: weights 805 MB, every expert in use
+        T, E, k, H, I = 64 if a.case == "experts_decode" else 4096, 128, 8, 2048, 768
+        w = torch.randn(E, 2 * I, H, device=dev, dtype=torch.bfloat16) * 0.02
+        ids = torch.rand(T, E, device=dev).topk(k, -1).indices.to(torch.int32)
+        cap = C.moe_align_cap(T * k, E)
+        used = torch.empty(cap // C.GROUP_ROWS, device=dev, dtype=torch.int32)
+        sid, eid, rows, _ = C.moe_align(ids, E, cap, tile_rows=used)
+        x = torch.randn(cap, H, device=dev, dtype=torch.bfloat16)
+        fn = lambda: C.gemm_bf16_grouped(x, w, eid, rows, silu_mul=True, sorted_ids=sid,  # noqa
+                                         pairs=T * k, tile_rows=used)
+    elif a.case == "rope_heads":
+        T, Hq, Hkv, D, bs = 8192, 32, 8, 128, 16
+        qkv = torch.randn(T, (Hq + 2 * Hkv) * D, device=dev, dtype=torch.bfloat16)
+        q, k, v = qkv.split([Hq * D, Hkv * D, Hkv * D], -1)
+        kc, vc = (torch.zeros(T // bs, bs, Hkv, D, device=dev, dtype=torch.bfloat16)
+                  for _ in range(2))
+        table = torch.randn(T, D, device=dev)
+        pos = torch.arange(T, device=dev)
+        w = torch.ones(D, device=dev, dtype=torch.bfloat16)
+        fn = lambda: C.rope_cache_flash(q, k, v, pos, table, True, D, pos, kc, vc,  # noqa: E731
+                                        norms=(w, w, 1e-5))
     else:
         raise SystemExit(f"unknown case {a.case}")
     for _ in range(a.iters):
