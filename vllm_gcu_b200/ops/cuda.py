@@ -7,6 +7,7 @@ kernels' own guards (status word, see ``_native.check_status``).
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional, Sequence
 
 import torch
@@ -95,13 +96,17 @@ _SKINNY_WS: dict = {}
 _SM_COUNT = 0
 
 
-def _wide2_pays(M: int, Nn: int) -> bool:
-    """256 x 256 tiles move a third less data per flop (measured +12 % on 8192 x 28672 x 4096)
-    but leave a larger ragged last wave; take them unless that costs more than it gains."""
+def _sms() -> int:
     global _SM_COUNT
     if _SM_COUNT == 0:
         _SM_COUNT = max(1, int(N.lib().b200_sm_count()))
-    sms = _SM_COUNT
+    return _SM_COUNT
+
+
+def _wide2_pays(M: int, Nn: int) -> bool:
+    """256 x 256 tiles move a third less data per flop (measured +12 % on 8192 x 28672 x 4096)
+    but leave a larger ragged last wave; take them unless that costs more than it gains."""
+    sms = _sms()
     t2 = -(-M // 256) * (Nn // 256)
     t1 = -(-M // 128) * (Nn // 256)
     eff2 = t2 / (-(-t2 // sms) * sms)
@@ -125,21 +130,45 @@ def _stream_pays(M: int, Nn: int, K: int) -> bool:
     return M <= 64 or (M <= 128 and Nn <= 8192) or (M <= 256 and Nn <= 4096)
 
 
-def _pair_rows(M: int, Nn: int) -> int:
+def _pair_rows(M: int, Nn: int, K: int = 4096) -> int:
     """Rows of a tile of the pair kernel with the weights on the M side (gemm_pair_rows.cu), 0 where
     another kernel is taken.  It pays for rows that would fill tiles of 256 badly, us at rows x N x K
-    against the other kernels: 301 x 28672 x 4096 76 : 89, 301 x 36864 x 7168 140 : 178, 301 x 6144 x 4096
-    22 : 28, 301 x 7168 x 2048 16 : 26, 384 x 28672 x 4096 83 : 93, 440 x 28672 x 4096 90 : 97, 440 x 6144 x
-    4096 23 : 29, but 512 x 28672 x 4096 101 : 98, 256 x 28672 x 4096 61 : 57.  And for enough weight
-    tiles: 301 x 5120 x 2048 17 : 16, 301 x 4096 x 4096 20 : 18.5, 301 x 4096 x 14336 52.7 : 51.  The rows go into
-    as few tiles as there can be, more while all tiles are one round of the pairs (301 x 6144 x 4096 in
-    tiles of 128 rows 22.1, of 160 22.9; 301 x 28672 x 4096 in tiles of 160 76, of 128 85)."""
+    against the other kernels: 301 x 28672 x 4096 82 : 104, 301 x 36864 x 7168 143 : 179, 301 x 6144 x 4096
+    22 : 27, 301 x 7168 x 2048 20 : 24, 544 x 28672 x 4096 102 : 130, 610 x 6144 x 4096 28.1 : 28.8, 800 x 7168 x
+    16384 185 : 210, 850 x 12288 x 5120 85 : 91, but 512 x 28672 x 4096 101 : 98, 256 x 28672 x 4096 61 : 57.
+    And for enough weight tiles: 301 x 5120 x 2048 17 : 16, 301 x 4096 x 4096 20 : 18.5, 301 x 4096 x 14336
+    52.7 : 51.  And where K is long enough for its way out, which is the dearer one, and the other kernel's
+    tiles do not fill their last wave better (_pair_rows_gain): 610 x 8192 x 1024 21.4 : 17.0, 800 x 6144 x 512
+    18.0 : 15.4, 384 x 6200 x 4096 25.2 : 21.2, 361 x 12040 x 256 17.1 : 10.9.  The rows go into as few tiles as
+    there can be, more while all tiles are one round of the pairs (301 x 6144 x 4096 in tiles of 128
+    rows 21.6, of 160 22.8; 301 x 28672 x 4096 in tiles of 160 82, of 128 90)."""
     tiles, w = -(-M // 256), -(-Nn // 256)
     if tiles * 256 < 1.15 * M or w < 24:
         return 0
-    while w * (tiles + 1) <= 74:
+    sms = _sms()
+    while w * (tiles + 1) <= sms // 2:
         tiles += 1
-    return -(-(-(-M // tiles)) // 32) * 32
+    rows = -(-(-(-M // tiles)) // 32) * 32
+    return rows if _pair_rows_gain(M, Nn, K, rows, sms) >= 0 else 0
+
+
+@functools.lru_cache(maxsize=1024)
+def _pair_rows_gain(M: int, Nn: int, K: int, rows: int, sms: int) -> float:
+    """us by which the pair kernel in tiles of ``rows`` rows is faster than the kernel that would run in
+    its place, estimated: rounds of the SMs times (K blocks times a rate, and the way out of a tile).
+    Fitted to 1216 shapes of 257 .. 890 rows, N 5889 .. 49152, K 256 .. 16384 on 148 SMs, where it takes 732 calls
+    at 0.86 of the other kernels' time (15 are slower by more than 3 %, all but one of them by less than
+    14 %) and leaves out 16 that it would make 5 % faster; without it 393 of the 1216 were slower by 3 to 65 %."""
+    kb = -(-K // 64)
+    rounds = -(-(-(-M // rows)) * -(-Nn // 256) // (sms // 2))
+    ours = 5.4 + rounds * (1.46 + rows * 0.0139 + kb * (0.137 + rows * 0.00055))
+    if Nn % 256 == 0 and K % 64 == 0:                  # tiles of 256 x 256 by pairs (gemm_pair.cu)
+        return 5.13 + -(-(-(-M // 256)) * (Nn // 256) // (sms // 2)) * (2.64 + kb * 0.324) - ours
+    # tiles of 128 rows and the width that gemm_bf16.cu picks
+    waves = {c: -(-(-(-M // 128)) * -(-Nn // c) // sms) for c in (256, 128, 96, 64)
+             if c != 256 or Nn % 256 == 0}
+    c = min(waves, key=lambda c: waves[c] * (c + 32))
+    return 2.96 + waves[c] * (c * 0.0202 + kb * (0.181 + c * 0.00039)) - ours
 
 
 def _skinny_workspace(device: torch.device):
@@ -239,7 +268,7 @@ def _gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = N
             raise N.NativeError(f"b200_gemm_stream failed with code {rc}")
     if (USE_PAIR_GEMM and 256 < M < WIDE2_MIN_M and epilogue in _PAIR_EPI
             and (epilogue not in _GATED or Nn % 64 == 0)):
-        rows = _pair_rows(M, Nn)
+        rows = _pair_rows(M, Nn, K)
         if rows:
             rc = N.lib().b200_gemm_pair_rows(ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out),
                                              out.stride(0), M, Nn, K, ptr(bias), epilogue, rows,
@@ -895,10 +924,7 @@ def mla_attention(q: torch.Tensor, cache: torch.Tensor, block_tables: torch.Tens
     B = block_tables.shape[0]
     if splits is None:
         ctas = max(num_tiles, 1) * (2 if L > 256 else 1)
-        global _SM_COUNT
-        if _SM_COUNT == 0:
-            _SM_COUNT = max(1, int(N.lib().b200_sm_count()))
-        slots = _SM_COUNT * (2 if L <= 128 else 1)       # narrow latents: two CTAs per SM
+        slots = _sms() * (2 if L <= 128 else 1)       # narrow latents: two CTAs per SM
         splits = max(1, min(slots // ctas, (max_seq_len + 255) // 256, 16))
     ws = None
     if splits > 1:
