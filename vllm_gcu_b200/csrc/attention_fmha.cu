@@ -72,6 +72,7 @@ struct Args {
   int chunk;               // > 0: keys of the query's own chunk of that many positions
   int OD;                  // output columns per head (the first of the HD)
   const float* slopes;     // biased kernels: [Hq], slope * (key - query position) joins the score
+  int rope_col;            // latent form: first shared key column in a row of the latent rows
   unsigned int* status;
 };
 
@@ -578,20 +579,68 @@ static int launch(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensor
   return static_cast<int>(cudaGetLastError());
 }
 
+// num_tiles pieces of 128 rows (latent: 256) for every pair of heads (latent: head)
+template <bool kLatent>
 static int launch_pair(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
-                       const Args& a, int num_q_tiles, cudaStream_t s) {
+                       const Args& a, int num_tiles, cudaStream_t s) {
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
     cudaError_t e = cudaFuncSetAttribute(
-        fmha_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
+        fmha_pair_kernel<kLatent>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
     if (e != cudaSuccess) return static_cast<int>(e);
     configured[dev] = true;
   }
-  dim3 grid(num_q_tiles, a.Hq / 2);
-  fmha_pair_kernel<<<grid, kThreads, kPairSmemBytes, s>>>(tmQ, tmK, tmV, a);
-  return static_cast<int>(cudaGetLastError());
+  const long long total = static_cast<long long>(num_tiles) * (kLatent ? a.Hq : a.Hq / 2);
+  if (total > 0x3fffffff) return -2;
+  const int grid = static_cast<int>(total < sm_count() ? total : sm_count());
+  return launch_overlapped(fmha_pair_kernel<kLatent>, dim3(grid), dim3(kPairThreads), kPairSmemBytes, s, tmQ,
+                           tmK, tmV, a, static_cast<int>(total));
+}
+
+// Rows of the paged latent cache, request after request: row k of request b is its key k; every request
+// starts at a multiple of 128 rows, and rows behind its last key are zeros (a tile of keys may reach over
+// them, and zeros times probability 0 are zeros whatever another request holds).  One warp per row.
+// Bound by memory: 2048 rows of 576 columns 3 us.
+__global__ void __launch_bounds__(256)
+    latent_rows_kernel(const uint4* cache, uint4* rows, const int* block_tables, const int* seq_lens, int B,
+                       int max_blocks, int block_size, int vecs, long long num_slots, int total,
+                       unsigned int* status) {
+  grid_release_small();
+  grid_wait();
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= total) return;
+  int base = 0, seq = -1, key = 0;
+  for (int b0 = 0; b0 < B && seq < 0; b0 += 32) {
+    const int len = b0 + lane < B ? seq_lens[b0 + lane] : 0;
+    const int room = (len + BKV - 1) / BKV * BKV;
+    int inc = room;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, inc, d);
+      if (lane >= d) inc += n;
+    }
+    const int start = base + inc - room;
+    const unsigned int vote = __ballot_sync(0xffffffffu, row >= start && row < start + room);
+    if (vote != 0u) {
+      const int src = __ffs(vote) - 1;
+      key = row - __shfl_sync(0xffffffffu, start, src);
+      seq = key < __shfl_sync(0xffffffffu, len, src) ? b0 + src : B;        // B: a row of zeros
+    }
+    base += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  long long slot = -1;
+  if (seq >= 0 && seq < B) {
+    slot = static_cast<long long>(block_tables[static_cast<long long>(seq) * max_blocks + key / block_size]) *
+               block_size + key % block_size;
+    if (slot < 0 || slot >= num_slots) {
+      if (lane == 0) report_status(status, kStatusBounds, kKernelId, static_cast<unsigned>(row));
+      slot = -1;
+    }
+  }
+  for (int i = lane; i < vecs; i += 32)
+    rows[static_cast<long long>(row) * vecs + i] = slot >= 0 ? cache[slot * vecs + i] : make_uint4(0, 0, 0, 0);
 }
 
 }  // namespace fmha
@@ -639,7 +688,7 @@ B200_API int b200_fmha_prefill_sink(const void* q, long long ldq, void* out, lon
   a.lse = lse; a.sink = sink; a.cu_q = cu_q; a.seq_lens = seq_lens; a.block_tables = block_tables;
   a.ldo = ldo; a.B = B; a.T = T; a.Hq = Hq; a.Hkv = Hkv; a.max_blocks = max_blocks;
   a.block_size = block_size; a.causal = causal; a.window = window; a.scale = scale;
-  a.softcap = softcap; a.chunk = chunk; a.OD = OD; a.slopes = slopes;
+  a.softcap = softcap; a.chunk = chunk; a.OD = OD; a.slopes = slopes; a.rope_col = 0;
   a.status = status_ptr();
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 #define B200_FMHA(MODE)                                                        \
@@ -651,12 +700,12 @@ B200_API int b200_fmha_prefill_sink(const void* q, long long ldq, void* out, lon
   if (slopes != nullptr) B200_FMHA(2);
   if (softcap > 0.0f || chunk > 0 || OD != HD) B200_FMHA(1);
   // Query heads in pairs over one key head: both at once, where one head per CTA would take more than one
-  // round of the SMs.  A CTA with two heads takes 1.3 to 1.5 times as long as one with one, us of both at
-  // the same call: 32 heads, 128 tokens 13.0 : 8.6, 301 tokens (96 CTAs of one head) 15.3 : 11.6, 512
-  // tokens (128) 18.8 : 13.7 and behind 8192 keys 150 : 117; but 64 heads, 301 tokens (192) 15.5 : 18.5, 32
-  // heads, 1024 tokens (256) 27.2 : 35.2 and 2048 tokens 73 : 88, eight chunks of 17 behind 1024 27.9 : 40.2.
+  // round of the SMs.  A CTA with two heads takes 1.1 to 1.25 times as long as one with one, us of both at
+  // the same call: 32 heads, 301 tokens (96 CTAs of one head) 14.4 : 12.5, 512 tokens (128) 17.7 : 14.5 and
+  // behind 8192 keys 145 : 121; but 64 heads, 301 tokens (192) 14.8 : 19.9, 32 heads, 1024 tokens (256) 27.2 :
+  // 37.0 and 2048 tokens 47 : 90, eight chunks of 17 behind 1024 28.6 : 42.5.
   if (HD == 128 && ((Hq / Hkv) & 1) == 0 && static_cast<long long>(num_q_tiles) * Hq > sm_count())
-    return launch_pair(tmQ, tmK, tmV, a, num_q_tiles, s);
+    return launch_pair<false>(tmQ, tmK, tmV, a, num_q_tiles, s);
   B200_FMHA(0);
 #undef B200_FMHA
 }
@@ -672,4 +721,50 @@ B200_API int b200_fmha_prefill(const void* q, long long ldq, void* out, long lon
                                 slot_stride, head_stride, num_slots, block_tables, max_blocks,
                                 block_size, B, T, num_q_tiles, Hq, Hkv, HD, scale, causal, window,
                                 dtype, nullptr, 0.0f, 0, nullptr, 0, stream);
+}
+
+// Rows of a paged latent cache [num_slots, W] (W a multiple of 8) for b200_latent_prefill: rows [total, W], total >=
+// the sum of seq_lens rounded up to 128 (rows behind them are zeros).
+B200_API int b200_latent_rows(const void* cache, void* rows, const int* block_tables, int max_blocks,
+                              int block_size, const int* seq_lens, int B, int W, long long num_slots,
+                              int total, void* stream) {
+  using namespace b200;
+  using namespace b200::fmha;
+  if (B <= 0 || total <= 0) return 0;
+  if (W <= 0 || W % 8 != 0 || ((reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(rows)) & 15))
+    return -20;
+  return launch_overlapped(latent_rows_kernel, dim3((total + 7) / 8), dim3(256), 0,
+                           static_cast<cudaStream_t>(stream), static_cast<const uint4*>(cache),
+                           static_cast<uint4*>(rows), block_tables, seq_lens, B, max_blocks, block_size, W / 8,
+                           num_slots, total, status_ptr());
+}
+
+// Causal latent attention over expanded keys and values, bf16.  q [T, N, 192] with row pitch ldq (128 columns,
+// then 64 rotated ones); kv [total, N * 256], the product of the latent part of `rows` and the up-projection (per
+// head 128 columns of the key, 128 of the value); rows [total, W] from b200_latent_rows with the shared
+// rotated key columns at W - 64; out [T, N * 128] with row pitch ldo.  num_tiles >= sum ceil(q_len / 256).
+// Returns -20 when the layout does not qualify.
+B200_API int b200_latent_prefill(const void* q, long long ldq, void* out, long long ldo, const int* cu_q,
+                                 const int* seq_lens, const void* kv, const void* rows, int W, int total,
+                                 int B, int T, int num_tiles, int N, float scale, void* stream) {
+  using namespace b200;
+  using namespace b200::fmha;
+  if (B <= 0 || T <= 0 || num_tiles <= 0 || N <= 0) return 0;
+  if (total <= 0 || W < 64 || W % 8 != 0 || ldq % 8 != 0 || ldo % 8 != 0 ||
+      ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out) |
+        reinterpret_cast<uintptr_t>(kv) | reinterpret_cast<uintptr_t>(rows)) & 15))
+    return -20;
+  CUtensorMap tmQ, tmKV, tmPe;
+  const unsigned long long n = static_cast<unsigned long long>(N), t = static_cast<unsigned long long>(total);
+  int r = get_map(q, static_cast<unsigned long long>(T), n * 192, static_cast<unsigned long long>(ldq) * 2, BQ,
+                  false, &tmQ);
+  if (r == 0) r = get_map(kv, t, n * 256, n * 512, BKV, false, &tmKV);
+  if (r == 0) r = get_map(rows, t, W, static_cast<unsigned long long>(W) * 2, BKV, false, &tmPe);
+  if (r != 0) return r < 0 ? -6 : r;
+  Args a = {};
+  a.out = static_cast<__nv_bfloat16*>(out);
+  a.cu_q = cu_q; a.seq_lens = seq_lens; a.ldo = ldo; a.B = B; a.T = T; a.Hq = N; a.Hkv = N; a.causal = 1;
+  a.scale = scale; a.rope_col = W - 64;
+  a.status = status_ptr();
+  return launch_pair<true>(tmQ, tmKV, tmPe, a, num_tiles, static_cast<cudaStream_t>(stream));
 }

@@ -139,6 +139,13 @@ class MLAAttention(nn.Module):
             kv = self.kv_a_proj_with_mqa(x)
         q = q.view(T, N, self.qk_dim)
         q_nope, q_pe = q[..., : self.nope], q[..., self.nope:]
+        nd = md.num_decode_tokens
+        B = md.num_decodes + md.num_prefills
+        if (USE_MLA_KERNEL and ops.use_native(x) and md.num_prefills > 0
+                and C.mla_attention_supported(q.new_empty((0, N, L + R)), kv_cache, L)):
+            o = self._forward_runs(q, kv, kv_cache, md)
+            if o is not None:
+                return self.o_proj(o)
         q_full = torch.empty((T, N, L + R), dtype=x.dtype, device=x.device)
         # latent query: q_nope x W_UK^T, written straight into the concatenated query
         torch.bmm(q_nope.transpose(0, 1), self.w_uk_t, out=q_full[..., :L].transpose(0, 1))
@@ -151,9 +158,7 @@ class MLAAttention(nn.Module):
                                              self.kv_a_layernorm.weight, cfg.rms_norm_eps,
                                              kv_cache, md.slot_mapping, L, cfg.rope_is_neox)
             q_full[..., L:] = q_rot
-        nd = md.num_decode_tokens
         o_lat = torch.empty((T, N, L), dtype=x.dtype, device=x.device)
-        B = md.num_decodes + md.num_prefills
         if (USE_MLA_KERNEL and ops.use_native(x)
                 and C.mla_attention_supported(q_full, kv_cache, L)):
             # tcgen05 kernel: decode rows (one token per request), then the multi-token
@@ -194,6 +199,53 @@ class MLAAttention(nn.Module):
             if t0 + n < T:
                 o_lat[t0 + n:] = 0
         return self.o_proj(self._heads_out(o_lat))
+
+    def _forward_runs(self, q: torch.Tensor, kv: torch.Tensor, kv_cache: torch.Tensor,
+                      md: AttentionMetadata) -> Optional[torch.Tensor]:
+        """Steps with prompts: attention of long ones over keys and values expanded by ``kv_b_proj``
+        (csrc/attention_fmha_pair.cuh), of decode rows and short ones over the latent rows.  None where no
+        request of the step is worth expanding."""
+        N, L, nd, first = self.N, self.L, md.num_decode_tokens, md.num_decodes
+        q_lens, seq_lens = md.q_lens_cpu[first:], md.seq_lens_cpu[first:]
+        w = self.kv_b_proj.weight
+        if not (len(q_lens) == len(seq_lens) == md.num_prefills and w.dtype == torch.bfloat16
+                and self.kv_b_proj.bias is None):
+            return None
+        runs = C.latent_prefill_plan(q_lens, seq_lens, N, L, self.nope, self.R, self.vdim)
+        if not any(wide for _, _, wide in runs):
+            return None
+        q_pe = q[..., self.nope:]
+        C.mla_rope_cache(q_pe, kv, md.positions, self.cos_sin_cache, self.kv_a_layernorm.weight,
+                         self.cfg.rms_norm_eps, kv_cache, md.slot_mapping, L,
+                         is_neox=self.cfg.rope_is_neox)
+        o = torch.empty((q.shape[0], N, self.vdim), dtype=q.dtype, device=q.device)
+        bt, sl, max_len, tq = md.block_tables, md.seq_lens, max(md.max_seq_len, 1), 128 // N
+
+        def absorbed(lo, hi, bt, sl, cu_q, tiles):
+            q_full = torch.empty((hi - lo, N, L + self.R), dtype=q.dtype, device=q.device)
+            torch.bmm(q[lo:hi, :, : self.nope].transpose(0, 1), self.w_uk_t,
+                      out=q_full[..., :L].transpose(0, 1))
+            q_full[..., L:].copy_(q_pe[lo:hi])
+            o_lat = C.mla_attention(q_full, kv_cache, bt, sl, cu_q, tiles, max_len, self.scale, L=L)
+            torch.bmm(o_lat.transpose(0, 1), self.w_uv, out=o[lo:hi].transpose(0, 1))
+
+        if nd > 0:
+            absorbed(0, nd, bt[:nd], sl[:nd], None, nd)
+        lo = nd
+        for a, b, wide in runs:
+            hi = lo + sum(q_lens[a:b])
+            cu = md.cu_q_prefill[a:b + 1]
+            place = bt[first + a:first + b], sl[first + a:first + b]
+            if wide:
+                C.latent_prefill(q[nd:], kv_cache, place[0], cu, place[1],
+                                 sum(-(-s // 128) * 128 for s in seq_lens[a:b]),
+                                 sum(-(-n // 256) for n in q_lens[a:b]), w, self.scale, o[nd:])
+            else:
+                absorbed(lo, hi, *place, cu - (lo - nd) if lo > nd else cu,
+                         sum(-(-n // tq) for n in q_lens[a:b]))
+            lo = hi
+        o[lo:] = 0
+        return o.flatten(1)
 
     def _heads_out(self, o_lat: torch.Tensor) -> torch.Tensor:
         """``[T, N, L]`` latent outputs -> ``[T, N * vdim]``; the product writes its rows in place."""

@@ -123,6 +123,8 @@ class _Sigs:
     b200_fmha_prefill = [P, L, P, L, P, P, P, P, P, L, L, L, P, I, I, I, I, I, I, I, I, F,
                          I, I, I, P]
     b200_merge_attn_states = [P, P, P, P, P, P, I, I, I, I, P]
+    b200_latent_rows = [P, P, P, I, I, P, I, I, L, I, P]
+    b200_latent_prefill = [P, L, P, L, P, P, P, P, I, I, I, I, I, I, F, P]
     b200_mla_attention = [P, P, P, L, P, P, P, I, I, I, I, I, I, I, I, I, P, F, P, P, L, P]
     b200_latent_cache = [P, L, P, F, P, L, I, P, P, P, P, I, I, I, I, I, I, I, I, I, P, L, P, P, L, P,
                          I, P]

@@ -940,6 +940,69 @@ def mla_attention(q: torch.Tensor, cache: torch.Tensor, block_tables: torch.Tens
     return out
 
 
+#: expanded keys and values of one launch of latent_prefill
+LATENT_PREFILL_BYTES = 1 << 30
+LATENT_PREFILL_MIN_ROWS = 64
+
+
+def _expanding_pays(q: int, s: int, num_heads: int) -> bool:
+    """Whether q new tokens at the end of s keys take less time with keys and values expanded per head.
+
+    Microseconds fitted to both forms, 16 and 128 heads: expanding costs every key 2 x 512 x 256 operations
+    and 1 KB per head, a query and key then 640 operations instead of 2176, and a pair of query tiles goes
+    through its key tiles one by one where the absorbed form splits them.  Measured, expanded : absorbed, 128
+    heads, 64 tokens 33 : 43, 2 x 1024 206 : 826, 64 behind 1024 cached ones 79 : 62, 128 behind 1024 80 : 107,
+    128 behind 4096 228 : 275, 512 behind 7680 626 : 1620; 16 heads, 256 tokens 30 : 42, 128 behind 4096 97 :
+    64, 384 behind 4096 113 : 152."""
+    h, pairs, tiles = num_heads / 128, q * (s - 0.5 * q), -(-s // 128)
+    expanded = 25 + 6.0 * tiles * h + max(1e-4 * pairs * h, 2.0 * tiles)
+    return q >= LATENT_PREFILL_MIN_ROWS and s >= q and expanded < 40 + 6e-4 * pairs * h
+
+
+def latent_prefill_plan(q_lens, seq_lens, num_heads: int, latent: int, nope: int, rope: int, vdim: int):
+    """Runs of neighbouring requests ``(first, end, expanded)`` of a step's multi-token requests: those whose
+    keys and values are worth expanding per head (``latent_prefill``), and the others (``mla_attention``).  The
+    expanded keys and values of a run stay within ``LATENT_PREFILL_BYTES``."""
+    runs: list[list] = []
+    room = 0
+    fits = (nope, rope, vdim) == (128, 64, 128) and latent % 64 == 0
+    limit = LATENT_PREFILL_BYTES // (num_heads * (nope + vdim) * 2)
+    for i, (q, s) in enumerate(zip(q_lens, seq_lens)):
+        keys = -(-s // 128) * 128
+        wide = fits and keys <= limit and _expanding_pays(q, s, num_heads)
+        if runs and runs[-1][2] == wide and (not wide or room + keys <= limit):
+            runs[-1][1] = i + 1
+        else:
+            runs.append([i, i + 1, wide])
+            room = 0
+        room += keys
+    return [tuple(r) for r in runs]
+
+
+def latent_prefill(q: torch.Tensor, cache: torch.Tensor, block_tables: torch.Tensor, cu_q: torch.Tensor,
+                   seq_lens: torch.Tensor, total: int, num_tiles: int, weight: torch.Tensor, scale: float,
+                   out: torch.Tensor) -> torch.Tensor:
+    """Causal latent attention over keys and values that ``weight [N * 256, L]`` (per head 128 rows of the key,
+    128 of the value) expands from the rows of ``cache [blocks, block_size, L + 64]``.  q ``[T, N, 192]`` (128
+    columns, 64 rotated ones), out ``[T, N, 128]``, both row-strided views; ``cu_q [B + 1]`` gives rows of
+    them.  ``total``: sum of the lengths rounded up to 128 each; ``num_tiles`` >= sum ceil(q_len / 256)."""
+    T, Nh, D = q.shape
+    nb, bs, W = cache.shape
+    L = weight.shape[1]
+    B = block_tables.shape[0]
+    assert (D == 192 and W == L + 64 and weight.shape[0] == Nh * 256 and cache.is_contiguous()
+            and q.dtype == out.dtype == cache.dtype == weight.dtype == torch.bfloat16
+            and q.stride(2) == out.stride(2) == 1 and q.stride(1) == D and out.stride(1) == 128
+            and block_tables.stride(1) == 1)
+    rows = torch.empty((total, W), dtype=cache.dtype, device=cache.device)
+    call("b200_latent_rows", ptr(cache), ptr(rows), ptr(block_tables), block_tables.stride(0), bs,
+         ptr(seq_lens), B, W, nb * bs, total, stream_ptr())
+    kv = gemm_bf16(rows[:, :L], weight)
+    call("b200_latent_prefill", ptr(q), q.stride(0), ptr(out), out.stride(0), ptr(cu_q), ptr(seq_lens),
+         ptr(kv), ptr(rows), W, total, B, T, num_tiles, Nh, float(scale), stream_ptr())
+    return out
+
+
 def latent_cache(kv: torch.Tensor, weight: torch.Tensor, eps: float, cache: torch.Tensor,
                  slot_mapping: torch.Tensor, x: Optional[torch.Tensor] = None,
                  state: Optional[torch.Tensor] = None, num_decodes: int = 0,
