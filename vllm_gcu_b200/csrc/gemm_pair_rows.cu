@@ -20,8 +20,13 @@
 // 28672 x 4096 76 us (89; 44 at the tensor cores' rate, 63 the vendor library), 6144 x 4096 22 (28), 36864 x
 // 7168 140 (178); 32 experts of 7168 x 2048 with 256 rows each, w13 466 us (633 in row tiles of 128; 321 at
 // the tensor cores' rate), w2 254 (466).
+// What held short K was the epilogue, 3000 cycles for 32 rows of a gated product (IEEE divisions that wait for
+// one another, four warps that meet three times a chunk) beside 512 of a K block's products.  Eight warps,
+// no divisions with branches, neighbours' exchange in place of a transposition: 128 experts, 4096 tokens of 8
+// (the same in equal shares): w13 1536 x 2048 260 (216) -> 220 (182), w2 2048 x 768 177 (149) -> 125 (106),
+// where the weights and rows take 150 and 90 at copy bandwidth.
 //
-// Roles (192 threads per CTA) and barriers as in gemm_pair.cu.
+// Roles (320 threads per CTA; eight epilogue warps) and barriers as in gemm_pair.cu.
 #include "pair.cuh"
 
 namespace b200 {
@@ -30,13 +35,13 @@ namespace pair_rows {
 using namespace b200::pair;
 
 constexpr unsigned int kKernelId = 72;
-constexpr int kThreads = 192;
+constexpr int kThreads = 320;
 constexpr int kHalfW = 128;              // weight rows of a CTA
 constexpr int kMaxRows = 256;            // activation rows of a tile
 constexpr int kStages = 6;
 constexpr int kWBytes = kHalfW * 128;
 constexpr int kStageBytes = kWBytes + kMaxRows / 2 * 128;
-constexpr int kChunk = 32 * kHalfW * 4;  // 32 activation rows on their way out
+constexpr int kChunk = 4 * 4096;         // gate and up values between the epilogue warps
 constexpr int kOffOut = kStages * kStageBytes;
 constexpr int kSmemBytes = kOffOut + kChunk + 1024;
 constexpr int kMaxList = 2048;           // row tiles of a grouped launch, in pairs
@@ -109,7 +114,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull_bar[b], 1);
-      mbar_init(&tempty_bar[b], 8);                         // four epilogue warps of each CTA
+      mbar_init(&tempty_bar[b], 16);                        // eight epilogue warps of each CTA
     }
     abort_word = 0u;
     epi_abort = 0u;
@@ -226,13 +231,18 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else {
     // ---------------- epilogue: this CTA's 128 weight rows, 32 activation rows at a time ----------------
-    const int q = warp & 3;
+    // Two sets of four warps take the chunks of 32 rows in turn.  A lane holds 32 rows of one column: two
+    // neighbours exchange one number for every two rows, and each stores two columns of one of them.
+    const int q = warp & 3, set = (warp - 2) >> 2;
     uint32_t tphase[2] = {0u, 0u};
     const uint32_t tempty_leader[2] = {map_to_cta(&tempty_bar[0], 0), map_to_cta(&tempty_bar[1], 0)};
     const bool gated = p.epi == kSiluMul || p.epi == kGeluMul;
-    // gate and up rows of the weights alternate in blocks of 32
-    const int gate = ((2 * lane) >> 5) * 64 + ((2 * lane) & 31);
-    float* out = reinterpret_cast<float*>(smem + kOffOut);
+    const bool odd_lane = (lane & 1) != 0;
+    // gate and up rows of the weights alternate in blocks of 32: of the lanes in quarters q and q ^ 1.  The
+    // first takes the first 16 rows of a chunk, the second the others.
+    const bool up = (q & 1) != 0;
+    const int pair_bar = 2 + set * 2 + (q >> 1);
+    float* xch = reinterpret_cast<float*>(smem + kOffOut) + (set * 2 + (q >> 1)) * 1024 + lane;
     int it = 0;
     for (int u = pair_id; u < units; u += num_pairs, ++it) {
       const int b = it & 1;
@@ -240,70 +250,94 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int n0 = x.n0 + static_cast<int>(rank) * kHalfW;
       if (!mbar_wait_warp(&tfull_bar[b], tphase[b], p.status, kKernelId, 0x400u + b, abort_flag))
         epi_abort = 1u;
-      // (the four warps meet at barriers below, so they leave together)
-      asm volatile("bar.sync 1, 128;" ::: "memory");
+      // (the warps meet at barriers below, so they leave together)
+      asm volatile("bar.sync 1, 256;" ::: "memory");
       if (epi_abort != 0u) break;
       tphase[b] ^= 1u;
       tc_fence_after();
-      for (int c = 0; c < x.used; c += 32) {
+      // first of the lane's two columns
+      const int col = (gated ? (n0 >> 1) + (q >> 1) * 32 : n0 + q * 32) + (lane & ~1);
+      const bool inside = col < (gated ? p.N >> 1 : p.N);
+      float bias0 = 0.0f, bias1 = 0.0f;
+      if (p.epi == kBias && inside) {
+        bias0 = __bfloat162float(p.bias[col]);
+        bias1 = __bfloat162float(p.bias[col + 1]);
+      }
+      const uint32_t acc = tmem + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(b * kMaxRows);
+      bool released = false;
+      for (int c = set * 32; c < x.used; c += 64) {
         uint32_t r[32];
-        tmem_ld_32x32(tmem + (static_cast<uint32_t>(q * 32) << 16) +
-                          static_cast<uint32_t>(b * kMaxRows + c), r);
+        tmem_ld_32x32(acc + c, r);
         float scales = 1.0f;             // of row c + lane
         if (GROUPED && p.row_scale != nullptr && c + lane < x.used)
           scales = p.row_scale[x.m0 + c + lane];
         tmem_ld_wait();
-        if (c > 0) asm volatile("bar.sync 1, 128;" ::: "memory");       // the last chunk has been read
-#pragma unroll
-        for (int i = 0; i < 32; ++i) out[i * kHalfW + q * 32 + lane] = __uint_as_float(r[i]);
-        if (c + 32 >= x.used) {
-          // the last chunk is out of tensor memory
+        if (c + 64 >= x.used) {          // the set's last chunk is out of tensor memory
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive_remote(tempty_leader[b]);
+          released = true;
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        // warp q stores the rows q, q + 4, ...; all eight are read before the first is stored
-        float4 v[8];
+        if (gated) {
+          asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");       // the last chunk has been read
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-          const float* src = out + (q + 4 * t) * kHalfW;
-          if (gated) {
-            const float2 g = *reinterpret_cast<const float2*>(src + gate);
-            const float2 up = *reinterpret_cast<const float2*>(src + gate + 32);
-            v[t] = make_float4(g.x, g.y, up.x, up.y);
+          for (int i = 0; i < 16; ++i) xch[(up ? 0 : 512) + i * 32] = __uint_as_float(up ? r[i] : r[16 + i]);
+          asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");
+          float f[16], g[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float own = __uint_as_float(up ? r[16 + i] : r[i]), other = xch[(up ? 512 : 0) + i * 32];
+            g[i] = up ? other : own;
+            f[i] = up ? own : other;
+          }
+          if (p.epi == kSiluMul) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) f[i] = gated_f<false>(g[i], f[i]);
           } else {
-            v[t] = *reinterpret_cast<const float4*>(src + 4 * lane);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) f[i] = gated_f<true>(g[i], f[i]);
           }
+          const int row = c + (up ? 16 : 0) + (odd_lane ? 1 : 0);
+          __nv_bfloat16* dst = p.C + static_cast<long long>(x.m0 + row) * p.ldc + col;
+#pragma unroll
+          for (int i = 0; i < 16; i += 2, dst += 2 * p.ldc) {
+            const float in = __shfl_xor_sync(0xffffffffu, odd_lane ? f[i] : f[i + 1], 1);
+            if (inside && row + i < x.used)
+              *reinterpret_cast<uint32_t*>(dst) =
+                  odd_lane ? pack_bf16x2(in, f[i + 1]) : pack_bf16x2(f[i], in);
+          }
+          continue;
         }
-        const int col = gated ? (n0 >> 1) + 2 * lane : n0 + 4 * lane;
-        __nv_bfloat16* dst = p.C + static_cast<long long>(x.m0 + c + q) * p.ldc + col;
-        const bool inside = col < (gated ? p.N >> 1 : p.N);
-        const int left = x.used - c - q;             // rows t with 4 t < left are in use
-        float bias[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if (p.epi == kBias && inside)
+        const int row = c + (odd_lane ? 1 : 0);
+        __nv_bfloat16* dst = p.C + static_cast<long long>(x.m0 + row) * p.ldc + col;
+        // (a loop for each activation: one with the choice inside takes 170 cycles a turn)
+        auto out = [&](auto act) {
+          float lo[16], hi[16];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) bias[e] = __bfloat162float(p.bias[col + e]);
-#pragma unroll
-        for (int t = 0; t < 8; ++t, dst += 4 * p.ldc) {
-          const float s = __shfl_sync(0xffffffffu, scales, q + 4 * t);
-          if (4 * t >= left || !inside) continue;
-          if (gated) {
-            *reinterpret_cast<uint32_t*>(dst) =
-                p.epi == kSiluMul
-                    ? pack_bf16x2(gated_f<false>(v[t].x, v[t].z), gated_f<false>(v[t].y, v[t].w))
-                    : pack_bf16x2(gated_f<true>(v[t].x, v[t].z), gated_f<true>(v[t].y, v[t].w));
-            continue;
+          for (int i = 0; i < 16; ++i) {
+            const float a0 = __uint_as_float(r[2 * i]), a1 = __uint_as_float(r[2 * i + 1]);
+            const float in = __shfl_xor_sync(0xffffffffu, odd_lane ? a0 : a1, 1);
+            lo[i] = odd_lane ? in : a0;
+            hi[i] = odd_lane ? a1 : in;
+            if (GROUPED) {
+              const float s = __shfl_sync(0xffffffffu, scales, 2 * i + (odd_lane ? 1 : 0));
+              lo[i] *= s;
+              hi[i] *= s;
+            }
           }
-          float f[4] = {v[t].x * s, v[t].y * s, v[t].z * s, v[t].w * s};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if (p.epi == kRelu2) f[e] = relu2_f(f[e]);
-            else if (p.epi == kGelu) f[e] = gelu_f(f[e]);
-            f[e] += bias[e];
-          }
-          *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
-        }
+          for (int i = 0; i < 16; ++i, dst += 2 * p.ldc)
+            if (inside && row + 2 * i < x.used)
+              *reinterpret_cast<uint32_t*>(dst) = pack_bf16x2(act(lo[i]) + bias0, act(hi[i]) + bias1);
+        };
+        if (p.epi == kRelu2) out([](float v) { return relu2_f(v); });
+        else if (p.epi == kGelu) out([](float v) { return gelu_f(v); });
+        else out([](float v) { return v; });
+      }
+      if (!released) {                   // a tile of up to 32 rows: nothing for the second set
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_remote(tempty_leader[b]);
       }
     }
   }
