@@ -28,3 +28,16 @@ def test_the_faster_side_is_taken(M, N, K, ratio, monkeypatch):
 def test_full_tiles_and_few_weight_tiles_go_elsewhere(M, monkeypatch):
     monkeypatch.setattr(C, "_SM_COUNT", 148)
     assert not C._pair_rows(M, 28672, 4096) and not C._pair_rows(301, 24 * 256 - 256, 4096)
+
+
+# us of tiles on pairs and of the kernel with 128-row tiles as measured: the rule takes the faster one
+@pytest.mark.parametrize("M,N,K,pair,other", [
+    (4096, 5120, 2048, 65.0, 85.4), (2945, 5120, 2048, 59.2, 78.8), (2433, 8192, 3072, 91.0, 111.1),
+    (3862, 2560, 14336, 243.9, 304.9), (7098, 10240, 11264, 1108.1, 1280.3), (1025, 14336, 4096, 96.6, 117.9),
+    (1375, 10240, 3072, 83.1, 80.1), (2118, 768, 4096, 29.5, 20.3), (1569, 3072, 256, 16.2, 13.1),
+    (3248, 512, 14336, 72.5, 52.6), (1065, 1024, 1536, 14.0, 9.2)])
+def test_pairs_or_tiles_of_128_rows(monkeypatch, M, N, K, pair, other):
+    monkeypatch.setattr(C, "_sms", lambda: 148)
+    C._pair_pays.cache_clear()
+    assert C._pair_pays(M, N, K) == (pair < other)
+    C._pair_pays.cache_clear()

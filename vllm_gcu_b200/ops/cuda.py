@@ -114,6 +114,21 @@ def _wide2_pays(M: int, Nn: int) -> bool:
     return eff2 * 1.15 >= eff1
 
 
+@functools.lru_cache(maxsize=1024)
+def _pair_pays(M: int, Nn: int, K: int) -> bool:
+    """Whether 256 x 256 tiles on CTA pairs (gemm_pair.cu) take less time from 1024 rows on than 128-row tiles
+    of the width that gemm_bf16.cu picks: rounds of the SMs times (K blocks times a rate, and the way out of
+    a tile), as in ``_pair_rows_gain``; beyond a few rounds the 128-row tiles take 1.2 times what those constants
+    say, at the power limit.  Of 110 timed shapes (799 .. 8192 rows, N 512 .. 28672, K 256 .. 14336) it is
+    wrong by more than 3 per cent for one (1962 x 2560 x 768 19.6 : 18.3); a rule by the share of a last wave
+    that tiles fill was for 26, by up to 1.4 (2945 x 5120 x 2048 59 : 79, 4096 x 5120 x 2048 65 : 85)."""
+    kb, sms = K // 64, _sms()
+    pair = 5.13 + -(-(-(-M // 256)) * (Nn // 256) // (sms // 2)) * (2.64 + kb * 0.324)
+    waves = {c: -(-(-(-M // 128)) * -(-Nn // c) // sms) for c in (256, 128, 96, 64)}
+    c = min(waves, key=lambda c: waves[c] * (c + 32))
+    return pair <= 1.13 * (2.96 + waves[c] * (c * 0.0202 + kb * (0.181 + c * 0.00039)))
+
+
 def _stream_pays(M: int, Nn: int, K: int) -> bool:
     """Shapes for which the kernel that streams the weights past few rows (gemm_stream.cu) is taken.
     Measured against the other kernels, us at rows x N x K: up to 32 rows it always wins (1 x 28672
@@ -319,8 +334,10 @@ def _gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = N
             return out
         if rc != -20:
             raise N.NativeError(f"b200_gemm_skinny failed with code {rc}")
-    if (USE_PAIR_GEMM and M >= WIDE2_MIN_M and Nn % 256 == 0 and K % 64 == 0
-            and epilogue in _PAIR_EPI and _wide2_pays(M, Nn)):
+    on_pairs = USE_PAIR_GEMM and Nn % 256 == 0 and K % 64 == 0 and epilogue in _PAIR_EPI
+    wide_pays = M >= WIDE2_MIN_M and Nn % 256 == 0 and (
+        _pair_pays(M, Nn, K) if on_pairs else _wide2_pays(M, Nn))
+    if on_pairs and wide_pays:
         # one 256 x 256 tile per pair of CTAs (gemm_pair.cu); -20 = shape or device not covered
         rc = N.lib().b200_gemm_pair(ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out),
                                     out.stride(0), M, Nn, K, ptr(bias), epilogue, stream_ptr())
@@ -329,8 +346,7 @@ def _gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = N
             return out
         if rc != -20:
             raise N.NativeError(f"b200_gemm_pair failed with code {rc}")
-    if (USE_WIDE2_GEMM and M >= WIDE2_MIN_M and Nn % 256 == 0
-            and epilogue in _WIDE_EPI and _wide2_pays(M, Nn)):
+    if USE_WIDE2_GEMM and wide_pays and epilogue in _WIDE_EPI:
         rc = N.lib().b200_gemm_wide2(ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out),
                                      out.stride(0), M, Nn, K, ptr(bias), epilogue, stream_ptr())
         N.launch_count += 1
