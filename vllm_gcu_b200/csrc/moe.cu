@@ -168,47 +168,113 @@ struct AlignArgs {
   int* num_post_pad;        // [1]
   int* pos_of;              // [T * k] position of each pair, -1 if dropped
   int* tile_rows;           // optional [cap / 128] rows of every tile that hold a pair
+  const float* topk_w;      // optional [T, k], with row_w [cap]: the weight of a row's pair, 0 for padding
+  float* row_w;
   int numel, k, num_local_experts, cap;
   unsigned int* status;
 };
 
+// Pairs sorted by expert, every expert from a tile of 128 rows on.  A cluster of CTAs shares the pairs (one CTA
+// takes a few hundred): counts in shared memory give every pair its rank among the CTA's pairs of an expert
+// at once, the CTAs read one another's counts, and each places its own pairs and its share of the tiles.
+// Bound by latency: 32768 pairs of 128 experts 36 us with one CTA, two passes of atomics and offsets added up by
+// one thread, 9.5 here.
 __global__ void __launch_bounds__(1024) moe_align_kernel(const AlignArgs a) {
   grid_release_small();
   grid_wait();
   extern __shared__ int smi[];
-  int* count = smi;                              // [E]
-  int* offset = smi + a.num_local_experts;       // [E + 1] padded exclusive offsets
-  int* cursor = offset + a.num_local_experts + 1;
   const int E = a.num_local_experts;
+  int* count = smi;                              // [E] of this CTA's pairs
+  int* base = count + E;                         // [E] of the pairs of the CTAs in front
+  int* sum = base + E;                           // [E] of all pairs
+  int* offset = sum + E;                         // [E + 1] padded exclusive offsets
+  int* warp_sum = offset + E + 1;                // [32]
+  uint32_t rank, ctas;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ctas));
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n = a.valid_tokens ? min(a.numel, *a.valid_tokens * a.k) : a.numel;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) { count[e] = 0; cursor[e] = 0; }
+  const int stride = static_cast<int>(ctas) * blockDim.x, first = static_cast<int>(rank) * blockDim.x + threadIdx.x;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+  auto expert_of = [&](int i) {
     int e = a.topk_ids[i];
     if (a.expert_map != nullptr) e = (e >= 0) ? a.expert_map[e] : -1;
-    if (e >= 0 && e < E) atomicAdd(&count[e], 1);
+    return e < E ? e : -1;
+  };
+  // the first pairs of a thread stay in registers, the ranks of others wait in pos_of
+  constexpr int kKeep = 4;
+  int expert[kKeep], place[kKeep];
+#pragma unroll
+  for (int c = 0; c < kKeep; ++c) expert[c] = first + c * stride < n ? expert_of(first + c * stride) : -1;
+#pragma unroll
+  for (int c = 0; c < kKeep; ++c) place[c] = expert[c] >= 0 ? atomicAdd(&count[expert[c]], 1) : -1;
+  for (int i = first + kKeep * stride; i < n; i += stride) {
+    const int e = expert_of(i);
+    a.pos_of[i] = e >= 0 ? atomicAdd(&count[e], 1) : -1;
   }
   __syncthreads();
+  if (ctas > 1) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+  // sums over the CTAs and padded offsets: a thread takes neighbouring experts
+  const int per = (E + static_cast<int>(blockDim.x) - 1) / static_cast<int>(blockDim.x);
+  int mine = 0;
+  for (int c = 0; c < per; ++c) {
+    const int e = static_cast<int>(threadIdx.x) * per + c;
+    if (e >= E) break;
+    int before = 0, all = 0;
+    for (uint32_t r = 0; r < ctas; ++r) {
+      int v = count[e];
+      if (ctas > 1) {
+        uint32_t addr;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(&count[e])), "r"(r));
+        asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+      }
+      if (r < rank) before += v;
+      all += v;
+    }
+    base[e] = before;
+    sum[e] = all;
+    mine += (all + kTileM - 1) / kTileM * kTileM;
+  }
+  // (the others may still read this CTA's counts: it leaves behind the wait at the end)
+  if (ctas > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  int inc = mine;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, d);
+    if (lane >= d) inc += v;
+  }
+  if (lane == 31) warp_sum[warp] = inc;
+  __syncthreads();
+  int at = inc - mine, total = 0;
+  for (int w = 0; w < static_cast<int>(blockDim.x) / 32; ++w) {
+    const int v = warp_sum[w];
+    if (w < warp) at += v;
+    total += v;
+  }
+  const bool fits = total <= a.cap;
+  if (!fits) total = 0;    // nothing valid: consumers skip every tile
+  for (int c = 0; c < per; ++c) {
+    const int e = static_cast<int>(threadIdx.x) * per + c;
+    if (e >= E) break;
+    offset[e] = fits ? at : 0;
+    at += (sum[e] + kTileM - 1) / kTileM * kTileM;
+  }
   if (threadIdx.x == 0) {
-    int off = 0;
-    for (int e = 0; e < E; ++e) {
-      offset[e] = off;
-      off += (count[e] + kTileM - 1) / kTileM * kTileM;
+    offset[E] = total;
+    if (rank == 0) {
+      if (!fits) report_status(a.status, kStatusBounds, kKernelId, static_cast<unsigned>(a.cap));
+      *a.num_post_pad = total;
     }
-    offset[E] = off;
-    if (off > a.cap) {
-      report_status(a.status, kStatusBounds, kKernelId, static_cast<unsigned>(off));
-      off = 0;  // nothing valid: consumers skip every tile
-      for (int e = 0; e <= E; ++e) offset[e] = 0;
-    }
-    *a.num_post_pad = off;
   }
   __syncthreads();
-  const int total = offset[E];
-  for (int i = threadIdx.x; i < a.cap; i += blockDim.x) a.sorted_ids[i] = a.numel;
-  for (int b = threadIdx.x; b < a.cap / kTileM; b += blockDim.x) {
+  // a warp writes a tile's padding
+  for (int b = static_cast<int>(rank) * (blockDim.x / 32) + warp; b < a.cap / kTileM; b += stride / 32) {
     const int row = b * kTileM;
-    int e = -1;
+    int e = -1, used = 0;
     if (row < total) {
       int lo = 0, hi = E;  // last e with offset[e] <= row
       while (hi - lo > 1) {
@@ -216,23 +282,49 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const AlignArgs a) {
         if (offset[mid] <= row) lo = mid; else hi = mid;
       }
       e = lo;
+      used = min(kTileM, max(0, sum[e] - (row - offset[e])));
     }
-    a.expert_ids[b] = e;
-    if (a.tile_rows != nullptr)
-      a.tile_rows[b] = e < 0 ? 0 : min(kTileM, max(0, count[e] - (row - offset[e])));
+    if (lane == 0) {
+      a.expert_ids[b] = e;
+      if (a.tile_rows != nullptr) a.tile_rows[b] = used;
+    }
+    for (int r = used + lane; r < kTileM; r += 32) {
+      a.sorted_ids[row + r] = a.numel;
+      if (a.row_w != nullptr) a.row_w[row + r] = 0.0f;
+    }
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < a.numel; i += blockDim.x) {
+  auto put = [&](int i, int e, int r) {
     int pos = -1;
-    if (i < n && total > 0) {
-      int e = a.topk_ids[i];
-      if (a.expert_map != nullptr) e = (e >= 0) ? a.expert_map[e] : -1;
-      if (e >= 0 && e < E) {
-        pos = offset[e] + atomicAdd(&cursor[e], 1);
-        a.sorted_ids[pos] = i;
-      }
+    if (e >= 0 && total > 0) {
+      pos = offset[e] + base[e] + r;
+      a.sorted_ids[pos] = i;
+      if (a.row_w != nullptr) a.row_w[pos] = a.topk_w[i];
     }
     a.pos_of[i] = pos;
+  };
+#pragma unroll
+  for (int c = 0; c < kKeep; ++c)
+    if (first + c * stride < a.numel) put(first + c * stride, expert[c], place[c]);
+  for (int i = first + kKeep * stride; i < a.numel; i += stride)
+    put(i, i < n ? expert_of(i) : -1, i < n ? a.pos_of[i] : 0);
+  if (ctas > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// A_sorted[pos_of[t, s]] = x[t] for every pair of a token, which is read once; rows of padding stay as they are,
+// for products that do not store them.  Against a CTA for every sorted row that there is room for: 4096
+// tokens of 8 experts, 2048 columns 52 -> 26 us
+template <typename T>
+__global__ void __launch_bounds__(256)
+    moe_scatter_kernel(const T* x, long long ldx, T* out, long long ldo, const int* pos_of, int k, int H) {
+  grid_release_small();
+  grid_wait();
+  const int t = blockIdx.x, nvec = H >> 3;
+  const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<long long>(t) * ldx);
+  const int* pos = pos_of + static_cast<long long>(t) * k;
+  for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
+    const uint4 u = src[v];
+    for (int s = 0; s < k; ++s)
+      if (pos[s] >= 0) reinterpret_cast<uint4*>(out + static_cast<long long>(pos[s]) * ldo)[v] = u;
   }
 }
 
@@ -426,21 +518,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Per sorted row: the routing weight of its (token, slot) pair (0 for padding rows).
-__global__ void moe_row_weights_kernel(const int* sorted_ids, const float* topk_w,
-                                       const int* num_post_pad, float* row_w, int numel, int cap) {
-  grid_release_small();
-  grid_wait();
-  const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pos >= cap) return;
-  float w = 0.0f;
-  if (pos < *num_post_pad) {
-    const int pair = sorted_ids[pos];
-    if (pair < numel) w = topk_w[pair];
-  }
-  row_w[pos] = w;
-}
-
 // get_ep_indices: one CTA; count[r] = #tokens with an expert on rank r, indices rank-major.
 __global__ void __launch_bounds__(1024)
     ep_indices_kernel(const int* topk_ids, int T, int k, int experts_per_rank, int ep,
@@ -506,19 +583,57 @@ B200_API int b200_moe_topk(const void* gating, long long ldg, const float* bias,
 }
 
 // cap must be a multiple of 128 and >= numel + num_local_experts * 127 rounded up.
+// topk_w and row_w (both or neither): see AlignArgs
 B200_API int b200_moe_align(const int* topk_ids, const int* expert_map, const int* valid_tokens,
                             int* sorted_ids, int* expert_ids, int* num_post_pad, int* pos_of,
-                            int* tile_rows, int numel, int k, int num_local_experts, int cap, void* stream) {
+                            int* tile_rows, const float* topk_w, float* row_w, int numel, int k,
+                            int num_local_experts, int cap, void* stream) {
   if (cap <= 0 || (cap % kTileM) != 0 || num_local_experts <= 0 || num_local_experts > 2048)
     return -2;
+  if ((topk_w == nullptr) != (row_w == nullptr)) return -2;
   AlignArgs a;
   a.topk_ids = topk_ids; a.expert_map = expert_map; a.valid_tokens = valid_tokens;
   a.sorted_ids = sorted_ids; a.expert_ids = expert_ids; a.num_post_pad = num_post_pad;
   a.pos_of = pos_of; a.tile_rows = tile_rows; a.numel = numel; a.k = k; a.num_local_experts = num_local_experts;
+  a.topk_w = topk_w; a.row_w = row_w;
   a.cap = cap; a.status = status_ptr();
-  const size_t smem = static_cast<size_t>(3 * num_local_experts + 1) * sizeof(int);
-  return launch_overlapped(moe_align_kernel, dim3(1), dim3(1024), smem,
-                           static_cast<cudaStream_t>(stream), a);
+  const size_t smem = static_cast<size_t>(4 * num_local_experts + 1 + 32) * sizeof(int);
+  cudaLaunchConfig_t cfg = {};
+  // one pair a thread up to eight CTAs
+  const int ctas = numel > 4096 ? 8 : numel > 2048 ? 4 : numel > 1024 ? 2 : 1;
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(1024);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = ctas;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = ctas > 1 ? 2 : 1;
+  return launch_code(cudaLaunchKernelEx(&cfg, moe_align_kernel, a));
+}
+
+// x [T, ldx], out rows [cap, ldo] of H columns; pos_of [T * k] as b200_moe_align gives it; dtype 0 bf16, 1 fp16
+B200_API int b200_moe_scatter(const void* x, long long ldx, void* out, long long ldo, const int* pos_of, int T,
+                              int k, int H, int dtype, void* stream) {
+  if (T <= 0) return 0;
+  if ((H % 8) != 0 || (ldx % 8) != 0 || (ldo % 8) != 0 || k <= 0 ||
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15))
+    return -2;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const dim3 block(H >= 2048 ? 256 : (H / 8 + 31) / 32 * 32);
+  if (dtype == 0)
+    return launch_overlapped(moe_scatter_kernel<__nv_bfloat16>, dim3(T), block, 0, s,
+                             static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_bfloat16*>(out), ldo,
+                             pos_of, k, H);
+  if (dtype == 1)
+    return launch_overlapped(moe_scatter_kernel<__half>, dim3(T), block, 0, s, static_cast<const __half*>(x), ldx,
+                             static_cast<__half*>(out), ldo, pos_of, k, H);
+  return -8;
 }
 
 B200_API int b200_moe_permute(const void* x, long long ldx, void* out, long long ldo,
@@ -608,15 +723,6 @@ B200_API int b200_ungated_rows_f32(const float* u, float* h, int rows, int I,
   else if (act == 10) ungated_rows_f32_kernel<true><<<rows, 256, 0, s>>>(u, h, I, num_valid_rows);
   else return -2;
   return static_cast<int>(cudaGetLastError());
-}
-
-B200_API int b200_moe_row_weights(const int* sorted_ids, const float* topk_w,
-                                  const int* num_post_pad, float* row_w, int numel, int cap,
-                                  void* stream) {
-  if (cap <= 0) return 0;
-  return launch_overlapped(moe_row_weights_kernel, dim3((cap + 255) / 256), dim3(256), 0,
-                           static_cast<cudaStream_t>(stream), sorted_ids, topk_w, num_post_pad, row_w,
-                           numel, cap);
 }
 
 B200_API int b200_moe_unpermute_sum(const void* y, long long ldy, const int* pos_of,

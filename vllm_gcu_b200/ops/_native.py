@@ -177,14 +177,14 @@ class _Sigs:
     b200_advance_step = [I, I, I, P, P, P, P, P, P, I, I, P]
     b200_feed_tokens = [P, P, P, P, I, P]
     b200_moe_topk = [P, L, P, P, P, I, I, I, I, I, I, I, F, P, I, P, P, I, P]
-    b200_moe_align = [P, P, P, P, P, P, P, P, I, I, I, I, P]
+    b200_moe_align = [P, P, P, P, P, P, P, P, P, P, I, I, I, I, P]
+    b200_moe_scatter = [P, L, P, L, P, I, I, I, I, P]
     b200_moe_permute = [P, L, P, L, P, P, I, I, I, I, I, I, P]
     b200_moe_permute_any = [P, L, P, L, P, P, I, I, I, I, I, I, P]
     b200_moe_permute_weighted = [P, L, P, P, L, P, P, I, I, I, I, I, I, P]
     b200_grouped_gemm_f32 = [P, L, P, P, L, I, I, I, I, P, P, P]
     b200_silu_mul_rows_f32 = [P, P, I, I, P, P]
     b200_ungated_rows_f32 = [P, P, I, I, P, I, P]
-    b200_moe_row_weights = [P, P, P, P, I, I, P]
     b200_moe_unpermute_sum = [P, L, P, P, L, P, L, P, I, I, I, F, I, P]
     b200_get_ep_indices = [P, I, I, I, I, P, P, P, P]
     b200_gemm_bf16_grouped = [P, L, P, L, P, L, I, I, I, I, P, P, P, I, P]

@@ -1507,9 +1507,11 @@ def moe_align_cap(num_pairs: int, num_local_experts: int) -> int:
 def moe_align(topk_ids: torch.Tensor, num_local_experts: int, cap: Optional[int] = None,
               expert_map: Optional[torch.Tensor] = None,
               valid_tokens: Optional[torch.Tensor] = None,
-              tile_rows: Optional[torch.Tensor] = None):
+              tile_rows: Optional[torch.Tensor] = None, topk_w: Optional[torch.Tensor] = None,
+              row_w: Optional[torch.Tensor] = None):
     """Returns (sorted_ids [cap], expert_ids [cap/128], num_post_pad [1], pos_of [T*k]);
-    ``tile_rows [cap/128]`` int32 takes the rows of every tile that are no padding."""
+    ``tile_rows [cap/128]`` int32 takes the rows of every tile that are no padding, ``row_w [cap]``
+    fp32 the weight ``topk_w [T, k]`` of every row's pair (0 for padding)."""
     T, k = topk_ids.shape
     numel = T * k
     cap = cap or moe_align_cap(numel, num_local_experts)
@@ -1519,8 +1521,8 @@ def moe_align(topk_ids: torch.Tensor, num_local_experts: int, cap: Optional[int]
     npp = torch.empty(1, device=dev, dtype=torch.int32)
     pos_of = torch.empty(max(numel, 1), device=dev, dtype=torch.int32)
     call("b200_moe_align", ptr(topk_ids), ptr(expert_map), ptr(valid_tokens), ptr(sorted_ids),
-         ptr(expert_ids), ptr(npp), ptr(pos_of), ptr(tile_rows), numel, k, num_local_experts, cap,
-         stream_ptr())
+         ptr(expert_ids), ptr(npp), ptr(pos_of), ptr(tile_rows), ptr(topk_w), ptr(row_w), numel, k,
+         num_local_experts, cap, stream_ptr())
     return sorted_ids, expert_ids, npp, pos_of
 
 
@@ -1579,14 +1581,12 @@ def fused_experts(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_w: 
     numel = T * k
     cap = moe_align_cap(numel, E)
     tile_rows = torch.empty(cap // GROUP_ROWS, device=x.device, dtype=torch.int32)
-    sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap, expert_map, valid_tokens,
-                                                    tile_rows)
-    a_sorted = torch.empty((cap, H), device=x.device, dtype=x.dtype)
-    call("b200_moe_permute", ptr(x), x.stride(0), ptr(a_sorted), H, ptr(sorted_ids), ptr(npp),
-         numel, k, H, cap, 0, DTYPE_CODE[x.dtype], stream_ptr())
     row_w = torch.empty(cap, device=x.device, dtype=torch.float32)
-    call("b200_moe_row_weights", ptr(sorted_ids), ptr(topk_w), ptr(npp), ptr(row_w), numel, cap,
-         stream_ptr())
+    sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap, expert_map, valid_tokens,
+                                                    tile_rows, topk_w, row_w)
+    a_sorted = torch.empty((cap, H), device=x.device, dtype=x.dtype)
+    call("b200_moe_scatter", ptr(x), x.stride(0), ptr(a_sorted), H, ptr(pos_of), T, k, H,
+         DTYPE_CODE[x.dtype], stream_ptr())
     pairs = dict(sorted_ids=sorted_ids, pairs=numel, tile_rows=tile_rows)
     h = gemm_bf16_grouped(a_sorted, w13, expert_ids, npp, silu_mul=True, **pairs)
     y = gemm_bf16_grouped(h, w2, expert_ids, npp, row_scale=row_w, **pairs)
@@ -1700,13 +1700,12 @@ def fused_experts_fp8(x: torch.Tensor, w13: torch.Tensor, w13_scale: torch.Tenso
     E = w13.shape[0]
     numel = T * k
     cap = moe_align_cap(numel, E)
-    sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap, expert_map, valid_tokens)
+    row_w = torch.empty(cap, device=x.device, dtype=torch.float32)
+    sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap, expert_map, valid_tokens,
+                                                    topk_w=topk_w, row_w=row_w)
     a_sorted = torch.empty((cap, H), device=x.device, dtype=x.dtype)
     call("b200_moe_permute", ptr(x), x.stride(0), ptr(a_sorted), H, ptr(sorted_ids), ptr(npp),
          numel, k, H, cap, 1, DTYPE_CODE[x.dtype], stream_ptr())
-    row_w = torch.empty(cap, device=x.device, dtype=torch.float32)
-    call("b200_moe_row_weights", ptr(sorted_ids), ptr(topk_w), ptr(npp), ptr(row_w), numel, cap,
-         stream_ptr())
     aq, a_s = activation(a_sorted, "identity", "plain", quant="fp8_group128", valid_rows=npp)
     h = gemm_q8_grouped(aq, a_s, w13, w13_scale, expert_ids, npp, kind=1)
     hq, h_s = activation(h, "silu", "act_mul", quant="fp8_group128", valid_rows=npp)
@@ -1771,13 +1770,12 @@ def fused_experts_wna16(x: torch.Tensor, q13: torch.Tensor, s13: torch.Tensor, z
     E, N13 = q13.shape[0], q13.shape[1]
     numel = T * k
     cap = moe_align_cap(numel, E)
-    sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap, expert_map, valid_tokens)
+    row_w = torch.empty(cap, device=x.device, dtype=torch.float32)
+    sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap, expert_map, valid_tokens,
+                                                    topk_w=topk_w, row_w=row_w)
     a_sorted = torch.empty((cap, H), device=x.device, dtype=x.dtype)
     call("b200_moe_permute", ptr(x), x.stride(0), ptr(a_sorted), H, ptr(sorted_ids), ptr(npp),
          numel, k, H, cap, 1, DTYPE_CODE[x.dtype], stream_ptr())
-    row_w = torch.empty(cap, device=x.device, dtype=torch.float32)
-    call("b200_moe_row_weights", ptr(sorted_ids), ptr(topk_w), ptr(npp), ptr(row_w), numel, cap,
-         stream_ptr())
     if numel <= WNA16_GROUPED_MAX_ROWS_PER_EXPERT * E:
         h = gemm_wna16_grouped(a_sorted, q13, s13, z13, expert_ids, npp, group, bits)
         hm = activation(h, "silu", "act_mul", valid_rows=npp)
@@ -1816,13 +1814,12 @@ def fused_experts_q8(x: torch.Tensor, w13: torch.Tensor, w13_scale: torch.Tensor
     kind = 2 if w13.dtype == torch.int8 else 0
     qname = "int8" if kind == 2 else "fp8"
     cap = moe_align_cap(numel, E)
-    sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap, expert_map, valid_tokens)
+    row_w = torch.empty(cap, device=x.device, dtype=torch.float32)
+    sorted_ids, expert_ids, npp, pos_of = moe_align(topk_ids, E, cap, expert_map, valid_tokens,
+                                                    topk_w=topk_w, row_w=row_w)
     a_sorted = torch.empty((cap, H), device=x.device, dtype=x.dtype)
     call("b200_moe_permute", ptr(x), x.stride(0), ptr(a_sorted), H, ptr(sorted_ids), ptr(npp),
          numel, k, H, cap, 1, DTYPE_CODE[x.dtype], stream_ptr())
-    row_w = torch.empty(cap, device=x.device, dtype=torch.float32)
-    call("b200_moe_row_weights", ptr(sorted_ids), ptr(topk_w), ptr(npp), ptr(row_w), numel, cap,
-         stream_ptr())
     aq, a_s = per_token_quant(a_sorted, qname, valid_rows=npp)
     h = gemm_q8_grouped(aq, a_s.view(-1), w13, w13_scale, expert_ids, npp, kind=kind)
     hm = activation(h, "silu", "act_mul", valid_rows=npp)
