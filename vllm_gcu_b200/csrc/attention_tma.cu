@@ -67,8 +67,6 @@ __device__ __forceinline__ uint32_t lds32(uint32_t smem_addr) {
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(smem_addr));
   return v;
 }
-__device__ __forceinline__ void consumer_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-
 struct Args {
   const void* q;
   void* out;
@@ -83,8 +81,69 @@ struct Args {
   float softcap;         // kShaped kernels: see b200_paged_decode_sink
   int chunk, window, OD;
   const float* alibi;    // kShaped kernels: [Hq] slopes or null
+  int cluster;           // the splits of a request and key head are a cluster and merge in shared memory
   unsigned int* status;
 };
+
+__device__ __forceinline__ void cluster_arrive_wait() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_peer(const float* p, uint32_t rank) {
+  uint32_t addr;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+// Share of the keys beside a sink in the denominator (maximum M and sum L of the keys in the log2 domain)
+__device__ __forceinline__ float sink_part(float M, float L, float sink) {
+  const float s2 = sink * kLog2e;
+  const float top = fmaxf(M, s2);
+  const float keys = L * exp2f(M - top);
+  return keys / (keys + exp2f(s2 - top));
+}
+// The splits of a cluster, each with maximum, sum and unscaled output of its keys in shared memory: every CTA
+// adds up a share of the numbers.  All threads of the cluster call it.
+template <typename T>
+__device__ __forceinline__ void merge_cluster(const Args& a, const float* m, const float* l, const float* o,
+                                              int b, int kvh, int G, int OD) {
+  cluster_arrive_wait();
+  uint32_t rank;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  if (threadIdx.x < kConsumers) {
+    for (int idx = static_cast<int>(rank) * kConsumers + threadIdx.x; idx < G * HD;
+         idx += a.num_splits * kConsumers) {
+      const int r = idx / HD, d = idx % HD;
+      float pm[8], pl[8], po[8], M = -INFINITY, L = 0.0f, val = 0.0f;
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        pm[s] = -INFINITY;
+        if (s >= a.num_splits) continue;
+        pm[s] = ld_peer(m + r, s);
+        pl[s] = ld_peer(l + r, s);
+        po[s] = ld_peer(o + idx, s);
+      }
+#pragma unroll
+      for (int s = 0; s < 8; ++s) M = fmaxf(M, pm[s]);
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        if (pm[s] == -INFINITY) continue;       // nothing seen: its output was never written
+        const float f = exp2f(pm[s] - M);
+        L += pl[s] * f;
+        val += po[s] * f;
+      }
+      val = L > 0.0f ? val / L : 0.0f;
+      const int head = kvh * G + r;
+      if (a.sink != nullptr && L > 0.0f) val *= sink_part(M, L, a.sink[head]);
+      if (d < OD)
+        static_cast<T*>(a.out)[static_cast<long long>(b) * a.ldo + head * OD + d] = from_f32<T>(val);
+    }
+  }
+  cluster_arrive_wait();           // nobody leaves while another CTA may still read its numbers
+}
+__device__ __forceinline__ void consumer_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+
 
 // kShaped: soft cap, chunk, window, slopes and output columns are in force
 template <typename T, bool kShaped>
@@ -114,7 +173,16 @@ __global__ void __launch_bounds__(kThreads)
   const int start = first + split * chunk;
   const int end = min(seq_len, start + chunk);
 
+  // what a split of a cluster leaves to the others (behind the buffers of its own merge)
+  float* part_m = reinterpret_cast<float*>(smem) + 128 + 4 * 16 * HD;
+  float* part_l = part_m + 16;
+  float* part_o = part_l + 16;
   if (start >= end) {
+    if (a.cluster) {
+      if (threadIdx.x < 16) part_m[threadIdx.x] = -INFINITY;
+      merge_cluster<T>(a, part_m, part_l, part_o, b, kvh, G, OD);
+      return;
+    }
     for (int r = 0; r < G; ++r) {
       const int head = kvh * G + r;
       if (a.num_splits > 1) {
@@ -168,7 +236,10 @@ __global__ void __launch_bounds__(kThreads)
         if (++stage == kStages) { stage = 0; phase ^= 1u; }
       }
     }
-    return;   // the producer warp takes no part in the merge
+    // the producer warp takes no part in the merge
+    __syncwarp();
+    if (a.cluster) merge_cluster<T>(a, part_m, part_l, part_o, b, kvh, G, OD);
+    return;
   }
 
   // ---------------- consumers (warps 0..3) ----------------
@@ -326,14 +397,17 @@ __global__ void __launch_bounds__(kThreads)
       L += sm_l[w * 16 + r] * f;
       o += sm_o[(w * 16 + r) * HD + d] * f;
     }
+    if (a.cluster) {
+      part_o[idx] = o;
+      if (d == 0) {
+        part_m[r] = ok && L > 0.0f ? M : -INFINITY;
+        part_l[r] = L;
+      }
+      continue;
+    }
     float val = (ok && L > 0.0f) ? o / L : 0.0f;
     const int head = kvh * G + r;
-    if (a.sink != nullptr && a.num_splits == 1 && ok && L > 0.0f) {
-      const float s2 = a.sink[head] * kLog2e;
-      const float top = fmaxf(M, s2);
-      const float keys = L * exp2f(M - top);
-      val *= keys / (keys + exp2f(s2 - top));
-    }
+    if (a.sink != nullptr && a.num_splits == 1 && ok && L > 0.0f) val *= sink_part(M, L, a.sink[head]);
     if (a.num_splits > 1) {
       const long long base = (static_cast<long long>(b) * a.Hq + head) * a.num_splits + split;
       a.tmp_out[base * HD + d] = val;
@@ -342,6 +416,28 @@ __global__ void __launch_bounds__(kThreads)
       static_cast<T*>(a.out)[static_cast<long long>(b) * a.ldo + head * OD + d] = from_f32<T>(val);
     }
   }
+  __syncwarp();
+  if (a.cluster) merge_cluster<T>(a, part_m, part_l, part_o, b, kvh, G, OD);
+}
+
+// Launch with the splits of a request and key head as a cluster, or as CTAs on their own
+template <typename... P, typename... A>
+static int launch_splits(void (*kernel)(P...), dim3 grid, size_t smem, bool cluster, cudaStream_t stream, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 1;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = grid.z;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster ? 2 : 1;
+  return launch_code(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
 }
 
 // Tensor maps are cached per (cache base, rows, row elements, dtype): encoding costs a few
@@ -423,12 +519,17 @@ static int paged_decode_tma_impl(const void* q, long long ldq, void* out, long l
   a.num_splits = num_splits; a.max_blocks = max_blocks; a.block_size = block_size;
   a.scale = scale; a.sink = sink; a.softcap = softcap; a.chunk = chunk; a.OD = OD > 0 ? OD : HD;
   a.window = window; a.alibi = alibi;
+  // Up to eight splits merge in shared memory: no partial results in global memory and no second kernel.  us in a
+  // cluster : with both, 1 request of 640 keys and 8 key heads, 3 splits 7.1 : 8.4, 6 splits 5.5 : 7.9, 12 requests
+  // of 900, 2 splits 13.4 : 14.5; but where two rounds of CTAs wait for one another 64 of 1500, 2 splits 75 : 74, 8
+  // splits 134 : 99.
+  a.cluster = num_splits > 1 && num_splits <= 8 && static_cast<long long>(B) * Hkv * num_splits <= 2 * sm_count();
   a.status = status_ptr();
   const bool shaped = softcap > 0.0f || chunk > 0 || window > 0 || alibi != nullptr || a.OD != HD;
   if (shaped && dtype != 0) return -20;
   constexpr int smem = kStages * kStageBytes + 256 + 1024;
-  static_assert(kStages * kStageBytes >= (128 + 4 * 16 * b200::attn_tma::HD) * 4,
-                "merge buffer must fit");
+  static_assert(kStages * kStageBytes >= (128 + 4 * 16 * b200::attn_tma::HD + 32 + 16 * b200::attn_tma::HD) * 4,
+                "merge buffers must fit");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   dim3 grid(B, Hkv, num_splits);
   static bool done0[64] = {false}, done1[64] = {false}, done2[64] = {false};
@@ -442,7 +543,7 @@ static int paged_decode_tma_impl(const void* q, long long ldq, void* out, long l
       if (set != cudaSuccess) return static_cast<int>(set);
       done2[dev] = true;
     }
-    e = launch_overlapped(kern, grid, dim3(kThreads), smem, s, tmK, tmV, a);
+    e = launch_splits(kern, grid, smem, a.cluster != 0, s, tmK, tmV, a);
   } else if (dtype == 0) {
     auto kern = paged_decode_tma_kernel<__nv_bfloat16, false>;
     if (dev >= 0 && dev < 64 && !done0[dev]) {
@@ -451,7 +552,7 @@ static int paged_decode_tma_impl(const void* q, long long ldq, void* out, long l
       if (set != cudaSuccess) return static_cast<int>(set);
       done0[dev] = true;
     }
-    e = launch_overlapped(kern, grid, dim3(kThreads), smem, s, tmK, tmV, a);
+    e = launch_splits(kern, grid, smem, a.cluster != 0, s, tmK, tmV, a);
   } else {
     auto kern = paged_decode_tma_kernel<__half, false>;
     if (dev >= 0 && dev < 64 && !done1[dev]) {
@@ -460,11 +561,29 @@ static int paged_decode_tma_impl(const void* q, long long ldq, void* out, long l
       if (set != cudaSuccess) return static_cast<int>(set);
       done1[dev] = true;
     }
-    e = launch_overlapped(kern, grid, dim3(kThreads), smem, s, tmK, tmV, a);
+    e = launch_splits(kern, grid, smem, a.cluster != 0, s, tmK, tmV, a);
   }
-  if (e != 0 || num_splits <= 1) return e;
+  if (e != 0 || num_splits <= 1 || a.cluster) return e;
   return b200_decode_reduce(out, ldo, tmp_out, tmp_lse, num_splits, B, Hq, HD, dtype, sink,
                             a.OD, stream);
+}
+
+// Number of splits for the kernel of this file (as b200_decode_num_splits).  One CTA has 96 KB of keys on their way,
+// which is its SM's share of the copy bandwidth, and every further CTA costs 10 ns of the whole: splits pay only
+// while SMs are idle.  us by splits 1, 2, 4: 64 requests of 2304 keys and 4 key heads (256 CTAs) 49 : 58 : 68, 32 of
+// 800 and 8 key heads (256) 20 : 27 : 35, 12 of 900 (96) 15 : 13 : 18, 1 of 4000 (8) 41 : 25 : 15, with 8 or 16
+// splits 10.3.  128 keys are enough for a CTA of a cluster; more splits than a cluster has pay from 2048 on (the
+// bound of a captured step's length is the model's, and most requests are shorter).
+B200_API int b200_decode_num_splits_tma(int B, int Hkv, int max_seq_len) {
+  const long long ctas = static_cast<long long>(B) * Hkv;
+  const int target = b200::sm_count();
+  if (ctas <= 0 || ctas >= target || max_seq_len <= 256) return 1;
+  long long s = (target + ctas - 1) / ctas;
+  const long long by_len = (max_seq_len + 127) / 128;
+  if (s > by_len) s = by_len;
+  if (s > 8 && max_seq_len < 8 * 2048) s = 8;
+  if (s > 32) s = 32;
+  return static_cast<int>(s);
 }
 
 B200_API int b200_paged_decode_tma(const void* q, long long ldq, void* out, long long ldo,

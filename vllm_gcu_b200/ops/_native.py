@@ -108,6 +108,7 @@ class _Sigs:
     b200_copy_blocks = [P, I, P, I, L, P]
     b200_swap_blocks = [P, P, P, I, L, P]
     b200_decode_num_splits = [I, I, I]
+    b200_decode_num_splits_tma = [I, I, I]
     b200_paged_decode = [P, L, P, L, P, P, L, L, L, P, I, I, P, P, P, I, I, I, I, I, F, I, P]
     b200_paged_decode_alibi = [P, L, P, L, P, P, L, L, L, P, I, I, P, P, P, I, I, I, I, I, F, I, P,
                                P]
