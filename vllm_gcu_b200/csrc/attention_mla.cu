@@ -45,8 +45,13 @@
 // what a design may have at this point, in fp32: a learnt sink per head in the denominator and an
 // output gate per token and head.
 //
-// Warp roles: warp 0 TMA producer, warp 1 MMA issuer and TMEM owner, warps 2..9 softmax and
-// epilogue.  Every wait is bounded and reports through the status word.
+// A tile's 36 score products and four output products take 2450 cycles when nothing waits; their issue takes
+// as long again, so scores and P V have a thread each, with descriptors that step by constants, and the two
+// threads of a row exchange maxima at a barrier of their two warps: 128 requests x 1536 keys, 128 heads 107 -> 100
+// us, 256 x 1152 keys 166 -> 155, 2 x 1024 new tokens 644 -> 602.
+//
+// Warp roles: warp 0 TMA producer, warp 1 scores and TMEM owner, warps 2..9 softmax and epilogue, warp 10
+// P V.  Every wait is bounded and reports through the status word.
 #include <mutex>
 #include <unordered_map>
 
@@ -63,7 +68,7 @@ constexpr int kMaxW = 576;     // key width, at most
 constexpr int kPage = 16;      // tokens that are neighbours in the cache
 constexpr int kGroup = 8;      // tokens per TMA copy
 constexpr int kQTmem = 6;      // 64-wide chunks of Q in tensor memory, where they are there
-constexpr int kThreads = 320;
+constexpr int kThreads = 352;
 constexpr int kKChunk = BKV * 128;        // [64 x 64] bf16: 8 KB
 constexpr uint32_t kColS = 0;      // one or two score buffers of 64 columns, then the output
                                    // (up to 256 columns), then Q
@@ -77,7 +82,7 @@ struct Lay {
 };
 constexpr int kOffBar = 0;         // barriers first: Q may be read past its end
 constexpr int kOffX = 128;
-constexpr int kOffQ = 2048;
+constexpr int kOffQ = 3072;
 static Lay make_lay(int qrows, int n_q, int n_w) {
   Lay l;
   const int q_chunk = qrows * 128;
@@ -312,81 +317,58 @@ __global__ void __launch_bounds__(kThreads, kResident)
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
+    // ---------------- scores ----------------
     if (elect_one()) {
       constexpr uint32_t kIdescS = make_idesc(BQ, BKV, 1, 1);
-      const uint32_t idesc_o = make_idesc(BQ, nc * 64, 1, 1) | kIdescBMajorMN;
-      const uint32_t q_addr = smem_u32(smem + kOffQ);
-      const uint32_t p_addr = smem_u32(p_smem);
-      auto issue_s = [&](int j) -> bool {
+      const uint64_t q_desc = make_desc_k_sw128(smem_u32(smem + kOffQ));
+      const uint64_t k_desc = make_desc_k_sw128(smem_u32(smem + a.off_k), group);
+      bool ok = mbar_wait(q_full, 0, a.status, kKernelId, 0x200u, abort_flag);
+      for (int j = 0; ok && j < nt; ++j) {
         const int st = j % kStages;
-        const uint32_t use = static_cast<uint32_t>(j / kStages);
-        if (!mbar_wait(&k_full[st], use & 1u, a.status, kKernelId, 0x210u + st, abort_flag))
-          return false;
-        if (j >= kSBufs &&
-            !mbar_wait(&s_empty[j % kSBufs], static_cast<uint32_t>(j / kSBufs - 1) & 1u, a.status,
-                       kKernelId, 0x230u + st, abort_flag))
-          return false;
+        ok = mbar_wait(&k_full[st], static_cast<uint32_t>(j / kStages) & 1u, a.status, kKernelId, 0x210u + st,
+                       abort_flag) &&
+             (j < kSBufs || mbar_wait(&s_empty[j % kSBufs], static_cast<uint32_t>(j / kSBufs - 1) & 1u, a.status,
+                                      kKernelId, 0x230u + st, abort_flag));
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t k_addr = smem_u32(smem + a.off_k + st * k_tile);
+        const uint64_t kd = k_desc + static_cast<uint32_t>(st * (k_tile >> 4));
         const uint32_t col = tmem_base + kColS + j % kSBufs * BKV;
-        if constexpr (kQT > 0) {
 #pragma unroll
-          for (int c = 0; c < kQT; ++c) {
+        for (int c = 0; c < kMaxW / 64; ++c) {
+          if (c >= kQT && c >= n_w) break;
 #pragma unroll
-            for (int ks = 0; ks < 4; ++ks)
-              umma_f16_ts(col, tmem_base + kColQ + c * 32 + ks * 8,
-                          make_desc_k_sw128(k_addr + c * 1024, group) + static_cast<uint64_t>(ks * 2),
+          for (int ks = 0; ks < 4; ++ks) {
+            if (c < kQT)
+              umma_f16_ts(col, tmem_base + kColQ + c * 32 + ks * 8, kd + static_cast<uint32_t>(c * 64 + ks * 2),
                           kIdescS, (c > 0 || ks > 0) ? 1u : 0u);
+            else
+              umma_f16(col, q_desc + static_cast<uint32_t>((c - kQT) * (kQChunk >> 4) + ks * 2),
+                       kd + static_cast<uint32_t>(c * 64 + ks * 2), kIdescS, (c > 0 || ks > 0) ? 1u : 0u);
           }
-        }
-#pragma unroll 1
-        for (int c = kQT; c < n_w; ++c) {
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            umma_f16(col, make_desc_k_sw128(q_addr + (c - kQT) * kQChunk) + static_cast<uint64_t>(ks * 2),
-                     make_desc_k_sw128(k_addr + c * 1024, group) + static_cast<uint64_t>(ks * 2),
-                     kIdescS, (c > 0 || ks > 0) ? 1u : 0u);
         }
         umma_commit(&s_full[j % kSBufs]);
-        return true;
-      };
-      bool ok = mbar_wait(q_full, 0, a.status, kKernelId, 0x200u, abort_flag);
-      ok = ok && issue_s(0);
-      for (int j = 0; ok && j < nt; ++j) {
-        // The scores of tile j + 1 and P V of tile j are issued in whichever order their inputs
-        // arrive.  (The key tile j + 1 could only be requested after P V of tile j - 1 had
-        // finished; waiting for it first would hold back P V of tile j.)
-        bool s_pending = j + 1 < nt;
+      }
+    }
+  } else if (warp == 10) {
+    // ---------------- P V, by a thread of its own: its four products wait for no issue of scores ----------------
+    if (elect_one()) {
+      const uint32_t idesc_o = make_idesc(BQ, nc * 64, 1, 1) | kIdescBMajorMN;
+      const uint64_t p_desc = make_desc_k_sw128(smem_u32(p_smem));
+      const uint64_t v_desc = make_desc_mn_sw128(smem_u32(smem + a.off_k + c0 * 1024), 1024, group);
+      for (int j = 0; j < nt; ++j) {
         const int st = j % kStages;
-        if (s_pending) {
-          const int st1 = (j + 1) % kStages;
-          const uint32_t use1 = static_cast<uint32_t>((j + 1) / kStages);
-          const uint32_t s_phase = static_cast<uint32_t>((j + 1) / kSBufs - 1) & 1u;
-          for (uint32_t it = 0; it < kMbarSpinLimit; ++it) {
-            if (mbar_test(&k_full[st1], use1 & 1u) &&
-                (j + 1 < kSBufs || mbar_test(&s_empty[(j + 1) % kSBufs], s_phase))) {
-              ok = issue_s(j + 1);            // its waits return at once
-              s_pending = false;
-              break;
-            }
-            if (mbar_test(p_full, j & 1)) break;
-            if ((it & 1023u) == 1023u && *abort_flag != 0u) { ok = false; break; }
-          }
-        }
-        if (!ok) break;
-        if (!mbar_wait(p_full, j & 1, a.status, kKernelId, 0x220u, abort_flag)) break;
+        if (!mbar_wait(&k_full[st], static_cast<uint32_t>(j / kStages) & 1u, a.status, kKernelId, 0x218u + st,
+                       abort_flag) ||
+            !mbar_wait(p_full, j & 1, a.status, kKernelId, 0x220u, abort_flag))
+          break;
         tc_fence_after();
-        const uint32_t k_addr = smem_u32(smem + a.off_k + st * k_tile);
-        const uint64_t vdesc = make_desc_mn_sw128(k_addr + c0 * 1024, 1024, group);
+        const uint64_t vd = v_desc + static_cast<uint32_t>(st * (k_tile >> 4));
 #pragma unroll
         for (int ks = 0; ks < BKV / 16; ++ks)
-          umma_f16(tmem_base + kColO, make_desc_k_sw128(p_addr) + static_cast<uint64_t>(ks * 2),
-                   vdesc + static_cast<uint64_t>(ks) * (group >> 3), idesc_o,
-                   (j > 0 || ks > 0) ? 1u : 0u);
+          umma_f16(tmem_base + kColO, p_desc + static_cast<uint32_t>(ks * 2),
+                   vd + static_cast<uint32_t>(ks) * (group >> 3), idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
         umma_commit(&k_empty[st]);
         umma_commit(o_done);
-        if (s_pending) ok = issue_s(j + 1);
       }
     }
   } else {
@@ -427,7 +409,7 @@ __global__ void __launch_bounds__(kThreads, kResident)
       if (lane == 0) mbar_arrive(q_full);
     }
     float m_used = -INFINITY, l = 0.0f;
-    float* xch = reinterpret_cast<float*>(smem + kOffX);    // [2][128]
+    float* xch = reinterpret_cast<float*>(smem + kOffX);    // [2][2][128], two tiles in turn
     for (int j = 0; j < nt; ++j) {
       const int st = j % kSBufs;
       mbar_pass_warp(&s_full[st], static_cast<uint32_t>(j / kSBufs) & 1u, a.status, kKernelId, 0x300u + st,
@@ -451,10 +433,11 @@ __global__ void __launch_bounds__(kThreads, kResident)
 #pragma unroll
         for (int i = 0; i < 32; ++i) mt = fmaxf(mt, __uint_as_float(v[i]));
       }
-      xch[g * BQ + r] = mt;
-      asm volatile("bar.sync 2, 256;" ::: "memory");
-      mt = fmaxf(mt, xch[(g ^ 1) * BQ + r]);
-      asm volatile("bar.sync 3, 256;" ::: "memory");
+      // (the two warps that share rows; the next but one tile's maxima come behind another barrier)
+      float* both = xch + (j & 1) * 2 * BQ;
+      both[g * BQ + r] = mt;
+      asm volatile("bar.sync %0, 64;" ::"r"(2 + qd) : "memory");
+      mt = fmaxf(mt, both[(g ^ 1) * BQ + r]);
       float alpha = 1.0f;
       float m_new = m_used;
       if (mt > m_used && (m_used == -INFINITY || (mt - m_used) * sl2 > 8.0f)) {
@@ -505,9 +488,10 @@ __global__ void __launch_bounds__(kThreads, kResident)
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
     }
-    xch[g * BQ + r] = l;
-    asm volatile("bar.sync 2, 256;" ::: "memory");
-    l += xch[(g ^ 1) * BQ + r];
+    float* both = xch + (nt & 1) * 2 * BQ;
+    both[g * BQ + r] = l;
+    asm volatile("bar.sync %0, 64;" ::"r"(2 + qd) : "memory");
+    l += both[(g ^ 1) * BQ + r];
     if (mbar_wait_warp(o_done, (nt - 1) & 1, a.status, kKernelId, 0x320u, abort_flag)) {
       tc_fence_after();
       const long long grow = row0 + r;
