@@ -30,14 +30,41 @@ def test_full_tiles_and_few_weight_tiles_go_elsewhere(M, monkeypatch):
     assert not C._pair_rows(M, 28672, 4096) and not C._pair_rows(301, 24 * 256 - 256, 4096)
 
 
-# us of tiles on pairs and of the kernel with 128-row tiles as measured: the rule takes the faster one
-@pytest.mark.parametrize("M,N,K,pair,other", [
-    (4096, 5120, 2048, 65.0, 85.4), (2945, 5120, 2048, 59.2, 78.8), (2433, 8192, 3072, 91.0, 111.1),
-    (3862, 2560, 14336, 243.9, 304.9), (7098, 10240, 11264, 1108.1, 1280.3), (1025, 14336, 4096, 96.6, 117.9),
-    (1375, 10240, 3072, 83.1, 80.1), (2118, 768, 4096, 29.5, 20.3), (1569, 3072, 256, 16.2, 13.1),
-    (3248, 512, 14336, 72.5, 52.6), (1065, 1024, 1536, 14.0, 9.2)])
-def test_pairs_or_tiles_of_128_rows(monkeypatch, M, N, K, pair, other):
-    monkeypatch.setattr(C, "_sms", lambda: 148)
-    C._pair_pays.cache_clear()
-    assert C._pair_pays(M, N, K) == (pair < other)
-    C._pair_pays.cache_clear()
+# us as measured with weights beyond L2, by kernel: tiles of 128, 160, 192, 224 and 256 rows with the weights on
+# the M side, 256 x 256 tiles on pairs, 128-row tiles.  The plan's choice is within 12 per cent of the fastest.
+@pytest.mark.parametrize("M,N,K,rows,pair,tiles", [
+    (301, 4096, 4096, (19.6, 20.1, 20.1, 20.1, 19.8), 26.1, 18.4),
+    (400, 5120, 2048, (18.8, 13.7, 13.7, 16.5, 16.5), 19.5, 19.3),
+    (520, 4096, 14336, (95.4, 57.0, 61.3, 61.3, 60.3), 76.7, 91.0),
+    (700, 28672, 4096, (148.1, 133.0, 128.3, 128.1, 121.7), 122.8, 145.6),
+    (700, 2048, 4096, (22.8, 22.3, 24.8, 24.8, 30.7), 28.3, 20.2),
+    (1024, 6144, 4096, (51.6, 51.9, 43.1, 48.3, 52.4), 53.7, 57.0),
+    (1500, 4096, 14336, (174.1, 179.2, 143.1, 160.2, 181.8), 181.0, 182.8),
+    (2048, 2112, 7168, (65.0, 63.7, 72.9, 83.7, 55.5), None, 69.1),
+    (2048, 4096, 4096, (78.8, 63.7, 62.7, 70.3, 58.0), 57.1, 67.3),
+    (2048, 32768, 512, (83.9, 80.5, 72.9, 80.0, 68.2), 81.6, 128.3),
+])
+def test_kernel_for_more_rows(monkeypatch, M, N, K, rows, pair, tiles):
+    monkeypatch.setattr(C, "_SM_COUNT", 148)
+    C._large_plan.cache_clear()
+    kind, r = C._large_plan(M, N, K)
+    C._large_plan.cache_clear()
+    took = {"pair": pair, "tiles": tiles}.get(kind) if kind != "rows" else None
+    if kind == "rows":
+        assert r % 32 == 0 and 32 <= r <= 256
+        # (equal tiles: the smallest of the timed sizes that gives as many)
+        same = [t for size, t in zip((128, 160, 192, 224, 256), rows) if -(-M // size) == -(-M // r)]
+        took = min(same)
+    assert took <= 1.12 * min(t for t in (*rows, pair, tiles) if t is not None)
+
+
+def test_plans_cover_every_shape(monkeypatch):
+    monkeypatch.setattr(C, "_SM_COUNT", 148)
+    C._large_plan.cache_clear()
+    for M in (257, 300, 1000, 5000, 100000):
+        for N in (8, 264, 1000, 4096, 151936):
+            for K in (8, 72, 512, 16384):
+                kind, rows = C._large_plan(M, N, K)
+                assert kind in ("rows", "pair", "tiles") and rows % 32 == 0 and rows <= 256
+                assert kind != "pair" or N % 256 == 0 and K % 64 == 0
+    C._large_plan.cache_clear()

@@ -110,7 +110,7 @@ struct Args {
   int layer_norm;
 };
 
-template <typename T, int QMODE, bool ADD>
+template <typename T, int QMODE, bool ADD, bool KEEP>
 __global__ void __launch_bounds__(1024) rms_norm_kernel(const Args a) {
   __shared__ float red[32];
   grid_release_small();
@@ -122,11 +122,15 @@ __global__ void __launch_bounds__(1024) rms_norm_kernel(const Args a) {
   const T* w = static_cast<const T*>(a.weight);
   const int nvec = a.H >> 3;
 
-  // pass 1: (residual add) + statistics
+  // pass 1: (residual add) + statistics.  KEEP: the first eight columns of a thread (all of a row up to 8192 wide)
+  // and their weights stay in registers; read again from where they were just stored they cost a
+  // trip through the cache.
   float sumsq = 0.0f, sum = 0.0f;
+  uint4 first, first_w;
   for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
     float f[8];
     load8<T>(x + v * 8, f);
+    if (KEEP && v == static_cast<int>(threadIdx.x)) first_w = *reinterpret_cast<const uint4*>(w + v * 8);
     if constexpr (ADD) {
       float r[8];
       load8<T>(res + v * 8, r);
@@ -139,6 +143,7 @@ __global__ void __launch_bounds__(1024) rms_norm_kernel(const Args a) {
       sumsq += f[i] * f[i];
       sum += f[i];
     }
+    if (KEEP && v == static_cast<int>(threadIdx.x)) store8<T>(reinterpret_cast<T*>(&first), f);    // (exact)
   }
   sumsq = block_sum(sumsq, red);
   float mean = 0.0f, rstd;
@@ -154,8 +159,13 @@ __global__ void __launch_bounds__(1024) rms_norm_kernel(const Args a) {
 
   auto normed = [&](int v, float (&f)[8]) {
     float wv[8];
-    load8<T>(src + v * 8, f);
-    load8<T>(w + v * 8, wv);
+    if (KEEP && v == static_cast<int>(threadIdx.x)) {
+      load8<T>(reinterpret_cast<const T*>(&first), f);
+      load8<T>(reinterpret_cast<const T*>(&first_w), wv);
+    } else {
+      load8<T>(src + v * 8, f);
+      load8<T>(w + v * 8, wv);
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i) f[i] = round_to<T>((f[i] - mean) * rstd * wv[i]);
     if (bias != nullptr) {
@@ -240,8 +250,13 @@ int launch2(const Args& a, bool add, cudaStream_t s) {
   int threads = ((a.H >> 3) + 31) & ~31;
   if (threads > 1024) threads = 1024;
   if (threads < 32) threads = 32;
-  return launch_overlapped(add ? rms_norm_kernel<T, QMODE, true> : rms_norm_kernel<T, QMODE, false>,
-                           dim3(a.T), dim3(threads), 0, s, a);
+  // The registers it takes leave an SM two CTAs of 512 threads in place of four: for grids of one round only.
+  // us of 256 x 4096 3.8 : 2.8, 128 x 7168 3.5 : 2.7, 500 x 2048 3.8 : 3.0, but 64 x 4096 2.4 : 2.5 (8-bit rows 3.2 :
+  // 3.3), 600 x 4096 5.0 : 6.2, 8192 x 4096 49 : 70.
+  const bool keep = 2 * a.T > sm_count() && a.T <= 2 * sm_count();
+  auto kernel = add ? (keep ? rms_norm_kernel<T, QMODE, true, true> : rms_norm_kernel<T, QMODE, true, false>)
+                    : (keep ? rms_norm_kernel<T, QMODE, false, true> : rms_norm_kernel<T, QMODE, false, false>);
+  return launch_overlapped(kernel, dim3(a.T), dim3(threads), 0, s, a);
 }
 
 template <typename T>

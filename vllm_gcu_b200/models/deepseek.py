@@ -133,7 +133,7 @@ class MLAAttention(nn.Module):
         if cfg.q_lora_rank > 0:
             qkv_a = self.qkv_a_proj(x)
             q_c, kv = qkv_a.split([cfg.q_lora_rank, L + R], dim=-1)
-            q = self.q_b_proj(self.q_a_layernorm(q_c.contiguous()))
+            q = self.q_b_proj(self.q_a_layernorm(q_c))
         else:
             q = self.q_proj(x)
             kv = self.kv_a_proj_with_mqa(x)

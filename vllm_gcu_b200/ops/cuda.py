@@ -114,19 +114,38 @@ def _wide2_pays(M: int, Nn: int) -> bool:
     return eff2 * 1.15 >= eff1
 
 
-@functools.lru_cache(maxsize=1024)
-def _pair_pays(M: int, Nn: int, K: int) -> bool:
-    """Whether 256 x 256 tiles on CTA pairs (gemm_pair.cu) take less time from 1024 rows on than 128-row tiles
-    of the width that gemm_bf16.cu picks: rounds of the SMs times (K blocks times a rate, and the way out of
-    a tile), as in ``_pair_rows_gain``; beyond a few rounds the 128-row tiles take 1.2 times what those constants
-    say, at the power limit.  Of 110 timed shapes (799 .. 8192 rows, N 512 .. 28672, K 256 .. 14336) it is
-    wrong by more than 3 per cent for one (1962 x 2560 x 768 19.6 : 18.3); a rule by the share of a last wave
-    that tiles fill was for 26, by up to 1.4 (2945 x 5120 x 2048 59 : 79, 4096 x 5120 x 2048 65 : 85)."""
-    kb, sms = K // 64, _sms()
-    pair = 5.13 + -(-(-(-M // 256)) * (Nn // 256) // (sms // 2)) * (2.64 + kb * 0.324)
-    waves = {c: -(-(-(-M // 128)) * -(-Nn // c) // sms) for c in (256, 128, 96, 64)}
+@functools.lru_cache(maxsize=4096)
+def _large_plan(M: int, Nn: int, K: int) -> tuple[str, int]:
+    """Kernel for more than 256 rows, by its estimated time: ``("rows", r)`` the pair kernel with the weights
+    on the M side in tiles of r rows (gemm_pair_rows.cu), ``("pair", 0)`` 256 x 256 tiles on CTA pairs
+    (gemm_pair.cu), ``("tiles", 0)`` 128 rows by the width that fills the SMs best (gemm_bf16.cu).
+
+    Each estimate is rounds of the SMs times (K blocks times a rate that grows with the tile, and a way out),
+    or the rate at the power limit where that is lower.  Fitted to 200 shapes of 257 .. 8192 rows, N 240 .. 28672
+    and K 256 .. 16384 with weights beyond L2; over them it takes 0.85 of the time that rules by filled waves
+    and full tiles took (1.01 of the fastest kernel's), with 5 shapes slower by 3 to 11 per cent.  us, those rules'
+    choice : this one's: 1500 x 4096 x 14336 181 : 143, 2048 x 2112 x 7168 68 : 56, 4096 x 5120 x 2048 81 : 59, 700 x
+    7168 x 16384 169 : 128, 400 x 5120 x 2048 20 : 14, 2183 x 10672 x 7168 420 : 289."""
+    sms, kb = _sms(), -(-K // 64)
+    pairs, w_tiles = sms // 2, -(-Nn // 256)
+    best, plan = float("inf"), ("tiles", 0)
+    for rows in (256, 224, 192, 160, 128, 96, 64):
+        tiles = -(-M // rows)
+        rows = -(-(-(-M // tiles)) // 32) * 32
+        rounds = -(-w_tiles * -(-M // rows) // pairs)
+        us = 5.98 + max(rounds * (0.0132 + 0.00986 * rows + kb * max(0.2092, 0.1698 + 0.00034 * rows)),
+                        rounds * rows * K * 2.2678e-5)
+        if us < best:
+            best, plan = us, ("rows", rows)
+    if Nn % 256 == 0 and K % 64 == 0:
+        tiles = -(-M // 256) * w_tiles
+        us = 6.85 + max(-(-tiles // pairs) * (2.07 + kb * 0.3254), tiles * K * 8.13e-5)
+        if 0.93 * us < best:           # (in a long step the estimates lie within what the power limit makes of them)
+            best, plan = us, ("pair", 0)
+    waves = {c: -(-(-(-M // 128)) * -(-Nn // c) // sms) for c in (256, 128, 96, 64) if c != 256 or Nn % 256 == 0}
     c = min(waves, key=lambda c: waves[c] * (c + 32))
-    return pair <= 1.13 * (2.96 + waves[c] * (c * 0.0202 + kb * (0.181 + c * 0.00039)))
+    us = 4.54 + waves[c] * max(-0.356 + 0.025 * c + kb * (0.1441 + 0.00066 * c), c * K * 2.771e-5)
+    return ("tiles", 0) if us < best else plan
 
 
 def _stream_pays(M: int, Nn: int, K: int) -> bool:
@@ -293,6 +312,22 @@ def _gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = N
                 return out
             if rc != -20:
                 raise N.NativeError(f"b200_gemm_pair_rows failed with code {rc}")
+    if (USE_PAIR_GEMM and not USE_PAIR_SPLIT and M > 256 and epilogue in _PAIR_EPI
+            and (epilogue not in _GATED or Nn % 64 == 0) and not (K % 8 or Nn % 8)):
+        kind, rows = _large_plan(M, Nn, K)
+        args = (ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out), out.stride(0), M, Nn, K, ptr(bias), epilogue)
+        rc = -20
+        if kind == "rows":
+            rc = N.lib().b200_gemm_pair_rows(*args, rows, stream_ptr())
+        elif kind == "pair":
+            rc = N.lib().b200_gemm_pair(*args, stream_ptr())
+        if rc == 0:
+            N.launch_count += 1
+            return out
+        if rc != -20:
+            raise N.NativeError(f"GEMM of {M} x {Nn} x {K} failed with code {rc}")
+        call("b200_gemm_bf16", *args[:-1], None, 0, epilogue, stream_ptr())
+        return out
     if (USE_PAIR_GEMM and PAIR_MIN_M <= M < WIDE2_MIN_M and Nn % 256 == 0 and K % 64 == 0
             and epilogue in _PAIR_EPI
             and -(-M // 256) * (Nn // 256) >= PAIR_MIN_TILES):
@@ -334,19 +369,8 @@ def _gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = N
             return out
         if rc != -20:
             raise N.NativeError(f"b200_gemm_skinny failed with code {rc}")
-    on_pairs = USE_PAIR_GEMM and Nn % 256 == 0 and K % 64 == 0 and epilogue in _PAIR_EPI
-    wide_pays = M >= WIDE2_MIN_M and Nn % 256 == 0 and (
-        _pair_pays(M, Nn, K) if on_pairs else _wide2_pays(M, Nn))
-    if on_pairs and wide_pays:
-        # one 256 x 256 tile per pair of CTAs (gemm_pair.cu); -20 = shape or device not covered
-        rc = N.lib().b200_gemm_pair(ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out),
-                                    out.stride(0), M, Nn, K, ptr(bias), epilogue, stream_ptr())
-        N.launch_count += 1
-        if rc == 0:
-            return out
-        if rc != -20:
-            raise N.NativeError(f"b200_gemm_pair failed with code {rc}")
-    if USE_WIDE2_GEMM and wide_pays and epilogue in _WIDE_EPI:
+    if (USE_WIDE2_GEMM and M >= WIDE2_MIN_M and Nn % 256 == 0
+            and epilogue in _WIDE_EPI and _wide2_pays(M, Nn)):
         rc = N.lib().b200_gemm_wide2(ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out),
                                      out.stride(0), M, Nn, K, ptr(bias), epilogue, stream_ptr())
         N.launch_count += 1
