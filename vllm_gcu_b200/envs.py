@@ -9,7 +9,19 @@ import os
 from typing import Any, Callable
 
 
+# The mapping behind os.environ: a flag that is not set costs a look-up in it, 0.2 us, where os.environ.get
+# encodes the name and raises and catches inside, 2 us; every kernel wrapper asks for one.
+_RAW = getattr(os.environ, "_data", None)
+_KEYS: dict[str, tuple[bytes, ...]] = {}
+
+
 def _get(name: str, default: str | None = None) -> str | None:
+    if _RAW is not None and os.name == "posix":
+        keys = _KEYS.get(name)
+        if keys is None:
+            keys = _KEYS[name] = tuple(os.fsencode(p + name) for p in ("VLLM_B200_", "VLLM_GCU_"))
+        if keys[0] not in _RAW and keys[1] not in _RAW:
+            return default
     for prefix in ("VLLM_B200_", "VLLM_GCU_"):
         v = os.environ.get(prefix + name)
         if v is not None:

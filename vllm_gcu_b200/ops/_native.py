@@ -222,7 +222,9 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device (0.3 us; building the Stream object
+    around it takes 5)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 DTYPE_CODE = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}

@@ -12,6 +12,7 @@ from typing import Optional, Sequence
 
 import torch
 
+from .. import envs
 from . import _native as N
 from ._native import DTYPE_CODE, call, ptr, stream_ptr
 
@@ -57,7 +58,6 @@ def oracle_enabled(name: str) -> bool:
     The reference compiles the same idea into its extension as a debug layer: CPU
     re-implementations and ``*Check`` comparators wrapped around 22 ops
     (csrc/src/native_vllm.h:37-446)."""
-    from .. import envs
     sel = envs.ORACLE
     return sel is not None and ("all" in sel or name in sel)
 
