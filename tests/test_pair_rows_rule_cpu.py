@@ -33,11 +33,9 @@ def test_full_tiles_and_few_weight_tiles_go_elsewhere(M, monkeypatch):
 # us as measured with weights beyond L2, by kernel: tiles of 128, 160, 192, 224 and 256 rows with the weights on
 # the M side, 256 x 256 tiles on pairs, 128-row tiles.  The plan's choice is within 12 per cent of the fastest.
 @pytest.mark.parametrize("M,N,K,rows,pair,tiles", [
-    (301, 4096, 4096, (19.6, 20.1, 20.1, 20.1, 19.8), 26.1, 18.4),
     (400, 5120, 2048, (18.8, 13.7, 13.7, 16.5, 16.5), 19.5, 19.3),
     (520, 4096, 14336, (95.4, 57.0, 61.3, 61.3, 60.3), 76.7, 91.0),
     (700, 28672, 4096, (148.1, 133.0, 128.3, 128.1, 121.7), 122.8, 145.6),
-    (700, 2048, 4096, (22.8, 22.3, 24.8, 24.8, 30.7), 28.3, 20.2),
     (1024, 6144, 4096, (51.6, 51.9, 43.1, 48.3, 52.4), 53.7, 57.0),
     (1500, 4096, 14336, (174.1, 179.2, 143.1, 160.2, 181.8), 181.0, 182.8),
     (2048, 2112, 7168, (65.0, 63.7, 72.9, 83.7, 55.5), None, 69.1),
@@ -47,7 +45,7 @@ def test_full_tiles_and_few_weight_tiles_go_elsewhere(M, monkeypatch):
 def test_kernel_for_more_rows(monkeypatch, M, N, K, rows, pair, tiles):
     monkeypatch.setattr(C, "_SM_COUNT", 148)
     C._large_plan.cache_clear()
-    kind, r = C._large_plan(M, N, K)
+    kind, r, _ = C._large_plan(M, N, K)
     C._large_plan.cache_clear()
     took = {"pair": pair, "tiles": tiles}.get(kind) if kind != "rows" else None
     if kind == "rows":
@@ -61,10 +59,24 @@ def test_kernel_for_more_rows(monkeypatch, M, N, K, rows, pair, tiles):
 def test_plans_cover_every_shape(monkeypatch):
     monkeypatch.setattr(C, "_SM_COUNT", 148)
     C._large_plan.cache_clear()
-    for M in (257, 300, 1000, 5000, 100000):
+    for M in (129, 257, 300, 1000, 5000, 100000):
         for N in (8, 264, 1000, 4096, 151936):
             for K in (8, 72, 512, 16384):
-                kind, rows = C._large_plan(M, N, K)
-                assert kind in ("rows", "pair", "tiles") and rows % 32 == 0 and rows <= 256
+                kind, rows, slices = C._large_plan(M, N, K)
+                assert kind in ("rows", "slices", "pair", "tiles") and rows % 32 == 0 and rows <= 256
+                assert (2 <= slices <= 4 and K >= 512 * slices) if kind == "slices" else slices == 1
                 assert kind != "pair" or N % 256 == 0 and K % 64 == 0
+    C._large_plan.cache_clear()
+
+
+# us of the other kernels' best and with K split over the pairs of a cluster
+@pytest.mark.parametrize("M,N,K,others,split", [
+    (301, 4096, 14336, 49.9, 36.3), (301, 4096, 4096, 17.7, 15.2), (301, 2112, 7168, 24.8, 15.5),
+    (400, 4096, 14336, 52.8, 44.0), (186, 4864, 14336, 50.0, 32.0), (175, 5632, 4096, 18.4, 14.8),
+    (520, 2048, 4096, 17.3, 14.5), (256, 6144, 4096, 18.9, 20.3), (592, 2632, 1536, 9.3, 13.0),
+    (740, 2816, 1024, 8.4, 12.9), (301, 6144, 4096, 19.5, 28.7), (400, 5120, 2048, 12.9, 21.5)])
+def test_k_is_split_where_it_pays(monkeypatch, M, N, K, others, split):
+    monkeypatch.setattr(C, "_SM_COUNT", 148)
+    C._large_plan.cache_clear()
+    assert (C._large_plan(M, N, K)[0] == "slices") == (split < others)
     C._large_plan.cache_clear()

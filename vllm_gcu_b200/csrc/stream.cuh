@@ -53,16 +53,17 @@ __device__ __forceinline__ void park_sums(uint32_t tmem, float* sums, int q, int
 
 // The rows that CTA `split` owns, four columns (GATED: two gate and two up columns, whose weight rows
 // alternate in blocks of 32) a lane, summed in the order of the K slices: store(row, sums).  All peers'
-// values of a row are on their way before the first is added.  WHOLE: the sums are 32-bit integers.
+// values of a row are on their way before the first is added.  WHOLE: the sums are 32-bit integers.  Slice s
+// is CTA first + s * step of the cluster.
 template <bool GATED, bool WHOLE, typename Store>
 __device__ __forceinline__ void sum_rows(const void* smem, int split, int splits, int warp, int warps,
-                                         int lane, int used, Store store) {
+                                         int lane, int used, Store store, int first = 0, int step = 1) {
   const int gate = ((2 * lane) >> 5) * 64 + ((2 * lane) & 31);
   const uint32_t own = smem_u32(smem) + (GATED ? gate : 4 * lane) * 4;
   uint32_t peer[kMaxSplits];
 #pragma unroll
   for (int s = 0; s < kMaxSplits; ++s)
-    peer[s] = s < splits ? (splits > 1 ? peer_addr(own, s) : own) : 0u;
+    peer[s] = s < splits ? (splits > 1 ? peer_addr(own, first + s * step) : own) : 0u;
   for (int r = split + warp * splits; r < used; r += warps * splits) {
     float4 x[kMaxSplits];
 #pragma unroll

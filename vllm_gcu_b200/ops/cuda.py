@@ -114,21 +114,33 @@ def _wide2_pays(M: int, Nn: int) -> bool:
     return eff2 * 1.15 >= eff1
 
 
+def _slices_at_once(slices: int) -> int:
+    """Clusters of so many pairs that run at the same time."""
+    if not torch.cuda.is_available():
+        return (0, 0, 33, 22, 15)[slices]              # of a B200
+    return int(N.lib().b200_gemm_pair_slices_at_once(slices))
+
+
 @functools.lru_cache(maxsize=4096)
-def _large_plan(M: int, Nn: int, K: int) -> tuple[str, int]:
-    """Kernel for more than 256 rows, by its estimated time: ``("rows", r)`` the pair kernel with the weights
-    on the M side in tiles of r rows (gemm_pair_rows.cu), ``("pair", 0)`` 256 x 256 tiles on CTA pairs
-    (gemm_pair.cu), ``("tiles", 0)`` 128 rows by the width that fills the SMs best (gemm_bf16.cu).
+def _large_plan(M: int, Nn: int, K: int) -> tuple[str, int, int]:
+    """Kernel for more than 128 rows, by its estimated time, with its rows of a tile and slices of K:
+    ``("rows", r, 1)`` the pair kernel with the weights on the M side (gemm_pair_rows.cu), ``("slices", r, s)``
+    the same with K split over s pairs (gemm_pair_slices.cu), ``("pair", 0, 1)`` 256 x 256 tiles on CTA pairs
+    (gemm_pair.cu), ``("tiles", 0, 1)`` 128 rows by the width that fills the SMs best (gemm_bf16.cu).
 
     Each estimate is rounds of the SMs times (K blocks times a rate that grows with the tile, and a way out),
     or the rate at the power limit where that is lower.  Fitted to 200 shapes of 257 .. 8192 rows, N 240 .. 28672
     and K 256 .. 16384 with weights beyond L2; over them it takes 0.85 of the time that rules by filled waves
     and full tiles took (1.01 of the fastest kernel's), with 5 shapes slower by 3 to 11 per cent.  us, those rules'
     choice : this one's: 1500 x 4096 x 14336 181 : 143, 2048 x 2112 x 7168 68 : 56, 4096 x 5120 x 2048 81 : 59, 700 x
-    7168 x 16384 169 : 128, 400 x 5120 x 2048 20 : 14, 2183 x 10672 x 7168 420 : 289."""
+    7168 x 16384 169 : 128, 400 x 5120 x 2048 20 : 14, 2183 x 10672 x 7168 420 : 289.
+
+    K is split where the tiles are no more than the clusters that run at once and the estimate is a tenth
+    below the others' (fitted to 300 calls of 40 .. 860 rows): 301 x 4096 x 14336 50 : 36, 301 x 4096 x 4096 17.7 :
+    15.2, 301 x 2112 x 7168 25 : 15.5, 186 x 4864 x 14336 50 : 32, 175 x 5632 x 4096 18.4 : 14.8."""
     sms, kb = _sms(), -(-K // 64)
     pairs, w_tiles = sms // 2, -(-Nn // 256)
-    best, plan = float("inf"), ("tiles", 0)
+    best, plan = float("inf"), ("tiles", 0, 1)
     for rows in (256, 224, 192, 160, 128, 96, 64):
         tiles = -(-M // rows)
         rows = -(-(-(-M // tiles)) // 32) * 32
@@ -136,16 +148,31 @@ def _large_plan(M: int, Nn: int, K: int) -> tuple[str, int]:
         us = 5.98 + max(rounds * (0.0132 + 0.00986 * rows + kb * max(0.2092, 0.1698 + 0.00034 * rows)),
                         rounds * rows * K * 2.2678e-5)
         if us < best:
-            best, plan = us, ("rows", rows)
+            best, plan = us, ("rows", rows, 1)
     if Nn % 256 == 0 and K % 64 == 0:
         tiles = -(-M // 256) * w_tiles
         us = 6.85 + max(-(-tiles // pairs) * (2.07 + kb * 0.3254), tiles * K * 8.13e-5)
-        if 0.93 * us < best:           # (in a long step the estimates lie within what the power limit makes of them)
-            best, plan = us, ("pair", 0)
+        # (products of 100 GFLOP and more in a long step are at the power limit, where pairs did better than
+        # timed alone: 7 x 1024 tokens beside 200 requests 23.2 ms with the estimates as they are, 22.7 so)
+        if us * (0.93 if 2e-11 * M * Nn * K > 1 else 1) < best:
+            best, plan = us, ("pair", 0, 1)
     waves = {c: -(-(-(-M // 128)) * -(-Nn // c) // sms) for c in (256, 128, 96, 64) if c != 256 or Nn % 256 == 0}
     c = min(waves, key=lambda c: waves[c] * (c + 32))
     us = 4.54 + waves[c] * max(-0.356 + 0.025 * c + kb * (0.1441 + 0.00066 * c), c * K * 2.771e-5)
-    return ("tiles", 0) if us < best else plan
+    if us < best:
+        best, plan = us, ("tiles", 0, 1)
+    for slices in (2, 3, 4) if kb >= 16 else ():
+        for rows in (256, 224, 192, 160, 128, 96, 64):
+            tiles = -(-M // rows)
+            rows = -(-(-(-M // tiles)) // 32) * 32
+            units = w_tiles * -(-M // rows)
+            if kb < 8 * slices or units > _slices_at_once(slices):
+                continue
+            us = (3.64 + 0.0213 * rows + 0.054 * slices
+                  + -(-kb // slices) * max(0.2161, 0.0616 + 0.00098 * rows, 0.0020012 * 2 * slices * units))
+            if us < (0.9 * best if plan[0] != "slices" else best):
+                best, plan = us, ("slices", rows, slices)
+    return plan
 
 
 def _stream_pays(M: int, Nn: int, K: int) -> bool:
@@ -312,22 +339,27 @@ def _gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = N
                 return out
             if rc != -20:
                 raise N.NativeError(f"b200_gemm_pair_rows failed with code {rc}")
-    if (USE_PAIR_GEMM and not USE_PAIR_SPLIT and M > 256 and epilogue in _PAIR_EPI
+    if (USE_PAIR_GEMM and not USE_PAIR_SPLIT and M > 128 and epilogue in _PAIR_EPI
             and (epilogue not in _GATED or Nn % 64 == 0) and not (K % 8 or Nn % 8)):
-        kind, rows = _large_plan(M, Nn, K)
-        args = (ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out), out.stride(0), M, Nn, K, ptr(bias), epilogue)
-        rc = -20
-        if kind == "rows":
-            rc = N.lib().b200_gemm_pair_rows(*args, rows, stream_ptr())
-        elif kind == "pair":
-            rc = N.lib().b200_gemm_pair(*args, stream_ptr())
-        if rc == 0:
-            N.launch_count += 1
-            return out
-        if rc != -20:
-            raise N.NativeError(f"GEMM of {M} x {Nn} x {K} failed with code {rc}")
-        call("b200_gemm_bf16", *args[:-1], None, 0, epilogue, stream_ptr())
-        return out
+        kind, rows, slices = _large_plan(M, Nn, K)
+        if M > 256 or kind == "slices":          # (other kernels of up to 256 rows follow below)
+            args = (ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out), out.stride(0), M, Nn, K, ptr(bias),
+                    epilogue)
+            rc = -20
+            if kind == "rows":
+                rc = N.lib().b200_gemm_pair_rows(*args, rows, stream_ptr())
+            elif kind == "slices":
+                rc = N.lib().b200_gemm_pair_slices(*args, rows, slices, stream_ptr())
+            elif kind == "pair":
+                rc = N.lib().b200_gemm_pair(*args, stream_ptr())
+            if rc == 0:
+                N.launch_count += 1
+                return out
+            if rc != -20:
+                raise N.NativeError(f"GEMM of {M} x {Nn} x {K} failed with code {rc}")
+            if M > 256:
+                call("b200_gemm_bf16", *args[:-1], None, 0, epilogue, stream_ptr())
+                return out
     if (USE_PAIR_GEMM and PAIR_MIN_M <= M < WIDE2_MIN_M and Nn % 256 == 0 and K % 64 == 0
             and epilogue in _PAIR_EPI
             and -(-M // 256) * (Nn // 256) >= PAIR_MIN_TILES):
