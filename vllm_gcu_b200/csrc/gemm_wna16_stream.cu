@@ -17,9 +17,10 @@
 // split over a cluster of CTAs that add their partial sums through shared memory (stream.cuh).
 //
 // Roles (384 threads): warp 0 TMA of packed weights, warp 1 tcgen05.mma, warp 2 TMA of activations,
-// warp 3 owner of tensor memory, warps 4..7 and 8..11 de-quantise the even and the odd blocks of 64
-// (warp w can reach the lanes 32 (w mod 4) .. + 31); warps 4..7 move the accumulators out.  Every wait
-// is bounded.
+// warp 3 owner of tensor memory, warps 4..7 and 8..11 de-quantise the first and second half of a packed tile
+// (warp w can reach the lanes 32 (w mod 4) .. + 31); warps 4..7 move the accumulators out.  A buffer of
+// de-quantised weights belongs to one group of warps: with a third group that shared them a warp could be two
+// uses ahead of a barrier's parity.  Every wait is bounded.
 #include "stream.cuh"
 
 namespace b200 {
@@ -31,7 +32,8 @@ constexpr unsigned int kKernelId = 71;
 constexpr int kThreads = 384;
 constexpr int kPackedBytes = BW * 128;   // a packed tile
 constexpr int kMaxPacked = 8, kMaxX = 16;
-constexpr int kBufs = 4;                 // de-quantised blocks in tensor memory, 32 columns each
+constexpr int kEarlyRows = 64;           // see the kernel
+constexpr int kACols = 128;              // columns of de-quantised weights in tensor memory
 
 struct Args {
   const __nv_bfloat16* scales;    // [N, K / g]
@@ -65,27 +67,35 @@ __device__ __forceinline__ void dequant8(uint32_t q, __nv_bfloat162 s2, __nv_bfl
   }
 }
 
-// SMALL: layers of few packed tiles, whose rows may be dealt out over blockIdx.z, and which set up before
-// they wait for the kernel in front (a twentieth of their time; the others gain as much with few rows, but
-// lose it with 96 and more: 128 x 4096 x 14336 of 8 bits 35.9 -> 38.5 us).
-template <int BITS, bool SMALL>
+// SMALL: layers of few packed tiles, whose rows may be dealt out over blockIdx.z.  They, and tiles of up to
+// kEarlyRows rows, set up and bring their first packed tiles into L2 before they wait for the kernel in
+// front (12 rows, the four products of a layer 76.8 -> 73.4 us); with 128 rows a kernel that already holds its place takes issue
+// slots from the de-quantising warps of the one in front (93.1 : 95.1).
+// VEC: the scales of eight groups of 128 come in one 16-byte load, a row a lane.  One by one, a row's
+// scales lie in lines that do not stay in what the ring leaves of the cache, and as many bytes of them as
+// of weights came from L2 (96 rows, the four products of a layer 96.2 -> 88.3 us, 12 rows 82.8 -> 76.8).
+template <int BITS, bool SMALL, bool VEC>
 __global__ void __launch_bounds__(kThreads, 2)
     gemm_wna16_stream_kernel(const __grid_constant__ CUtensorMap tmW,
                              const __grid_constant__ CUtensorMap tmA, const Args p) {
-  constexpr int kBlocks = BITS == 4 ? 4 : 2;          // blocks of 64 in a packed tile
+  // A step is half a packed tile, 64 bytes of every row: one or two blocks of 64 weights.  The two groups
+  // of de-quantising warps take the steps in turn, each with buffers of its own.
+  constexpr int kBlocks = BITS == 4 ? 2 : 1;          // blocks of a step
   constexpr int kVec = BITS == 4 ? 2 : 4;             // 16-byte words of a row in a block
+  constexpr int kBufs = kACols / (32 * kBlocks);      // steps in tensor memory
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* smem_x = smem + p.packed_stages * kPackedBytes;
-  const int x_bytes = p.rows * 128;
+  const int x_block = p.rows * 128, x_bytes = kBlocks * x_block;
   __shared__ uint64_t pfull[kMaxPacked], pempty[kMaxPacked], xfull[kMaxX], xempty[kMaxX];
   __shared__ uint64_t afull[kBufs], aempty[kBufs], done_bar;
   __shared__ uint32_t tmem_slot;
   __shared__ volatile uint32_t abort_word;
   volatile uint32_t* abort_flag = &abort_word;
 
-  if constexpr (!SMALL) grid_wait();
+  const bool early = SMALL || p.rows <= kEarlyRows;
+  if (!early) grid_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int split = static_cast<int>(blockIdx.x);
   const int n0 = static_cast<int>(blockIdx.y) * BW;
@@ -122,15 +132,22 @@ __global__ void __launch_bounds__(kThreads, 2)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot, tmem_a = tmem + acc_cols;
-  if constexpr (SMALL) grid_wait();
 
   // this CTA's packed tiles, and its blocks of 64 (the last tile of a row may hold fewer)
   const int total_blocks = p.K / 64;
-  const int total_tiles = (total_blocks + kBlocks - 1) / kBlocks;
+  const int total_tiles = (total_blocks + 2 * kBlocks - 1) / (2 * kBlocks);
   const int t_lo = static_cast<int>(static_cast<long long>(split) * total_tiles / p.splits);
   const int t_hi = static_cast<int>(static_cast<long long>(split + 1) * total_tiles / p.splits);
-  const int b_lo = t_lo * kBlocks;
-  const int blocks = min(t_hi * kBlocks, total_blocks) - b_lo;
+  const int b_lo = t_lo * 2 * kBlocks;
+  const int blocks = min(t_hi * 2 * kBlocks, total_blocks) - b_lo;
+  const int steps = (blocks + kBlocks - 1) / kBlocks;
+  if (early) {
+    // the first packed tiles come into L2 while the kernels in front still run
+    if (threadIdx.x == 0)
+      for (int t = t_lo; t < t_hi && t < t_lo + p.packed_stages; ++t) tma_prefetch_2d(&tmW, t * 128, n0);
+    __syncwarp();
+    grid_wait();
+  }
 
   if (warp == 0) {
     if (elect_one()) {
@@ -150,10 +167,12 @@ __global__ void __launch_bounds__(kThreads, 2)
     if (elect_one()) {
       int s = 0;
       uint32_t phase = 0;
-      for (int b = 0; b < blocks; ++b) {
+      for (int b = 0; b < blocks; b += kBlocks) {
         if (!mbar_wait(&xempty[s], phase ^ 1u, p.status, kKernelId, 0x200u + s, abort_flag)) break;
-        mbar_expect_tx(&xfull[s], x_bytes);
-        tma_load_2d(smem_x + s * x_bytes, &tmA, &xfull[s], (b_lo + b) * 64, m0);
+        const int n = min(kBlocks, blocks - b);
+        mbar_expect_tx(&xfull[s], n * x_block);
+        for (int i = 0; i < n; ++i)
+          tma_load_2d(smem_x + s * x_bytes + i * x_block, &tmA, &xfull[s], (b_lo + b + i) * 64, m0);
         if (++s == p.x_stages) {
           s = 0;
           phase ^= 1u;
@@ -166,20 +185,26 @@ __global__ void __launch_bounds__(kThreads, 2)
       int s = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int b = 0; b < blocks; ++b) {
-        const int buf = b % kBufs;
+      for (int st = 0; st < steps; ++st) {
+        const int buf = st % kBufs;
         if (!mbar_wait(&xfull[s], phase, p.status, kKernelId, 0x300u + s, abort_flag) ||
-            !mbar_wait(&afull[buf], static_cast<uint32_t>(b / kBufs) & 1u, p.status, kKernelId,
+            !mbar_wait(&afull[buf], static_cast<uint32_t>(st / kBufs) & 1u, p.status, kKernelId,
                        0x320u + buf, abort_flag)) {
           ok = false;
           break;
         }
         tc_fence_after();
         const uint64_t xdesc = make_desc_k_sw128(smem_u32(smem_x + s * x_bytes));
+        const uint32_t ta = tmem_a + buf * (32 * kBlocks);
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          umma_f16_ts(tmem, tmem_a + buf * 32 + k * 8, xdesc + static_cast<uint64_t>(k * 2), idesc,
-                      (b > 0 || k > 0) ? 1u : 0u);
+        for (int i = 0; i < kBlocks; ++i) {
+          if (i > 0 && st * kBlocks + i >= blocks) break;
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            umma_f16_ts(tmem, ta + i * 32 + k * 8,
+                        xdesc + static_cast<uint32_t>(i * (x_block >> 4) + k * 2), idesc,
+                        (st > 0 || i > 0 || k > 0) ? 1u : 0u);
+        }
         umma_commit(&xempty[s]);
         umma_commit(&aempty[buf]);
         if (++s == p.x_stages) {
@@ -197,42 +222,79 @@ __global__ void __launch_bounds__(kThreads, 2)
     // rows past N hold zeros and are never stored: any scale will do
     const __nv_bfloat16* srow = p.scales + (n < p.N ? n : 0) * groups;
     const __nv_bfloat16* zrow = p.zs + (n < p.N ? n : 0) * groups;
-    const bool halves = p.g_shift < 6;                // groups of 32: two per block
-    __nv_bfloat16 sc[2], zz[2];                       // of the next block
-    auto fetch = [&](int b) {
-      const int g0 = ((b_lo + b) * 64) >> p.g_shift;
-      sc[0] = srow[g0];
-      zz[0] = zrow[g0];
-      if (halves) {
-        sc[1] = srow[g0 + 1];
-        zz[1] = zrow[g0 + 1];
+    const bool halves = !VEC && p.g_shift < 6;        // groups of 32: two per block
+    // Scales of the next step.  VEC: groups of 128, one per step, so that the two groups of warps take the two
+    // halves of each 32-bit word of a row's scales: eight groups in one 16-byte load, a word a step.
+    __nv_bfloat16 sc[VEC ? 1 : 2 * kBlocks], zz[VEC ? 1 : 2 * kBlocks];
+    uint4 s8, z8;
+    int word = 0;
+    auto fetch = [&](int st) {
+      if constexpr (VEC) {
+        const int g8 = (t_lo + (st >> 1)) >> 2;          // (a packed tile is two groups)
+        s8 = reinterpret_cast<const uint4*>(srow)[g8];
+        z8 = reinterpret_cast<const uint4*>(zrow)[g8];
+      } else {
+#pragma unroll
+        for (int i = 0; i < kBlocks; ++i) {
+          const int b = min(st * kBlocks + i, blocks - 1);
+          const int g0 = ((b_lo + b) * 64) >> p.g_shift;
+          sc[2 * i] = srow[g0];
+          zz[2 * i] = zrow[g0];
+          if (halves) {
+            sc[2 * i + 1] = srow[g0 + 1];
+            zz[2 * i + 1] = zrow[g0 + 1];
+          }
+        }
       }
     };
-    if (group < blocks) fetch(group);
+    if (group < steps) fetch(group);
+    if constexpr (VEC) word = t_lo & 3;
     int s = 0;
     uint32_t phase = 0;
-    for (int t = t_lo; t < t_hi; ++t) {
+    for (int st = group; st < steps; st += 2) {
       mbar_pass_warp(&pfull[s], phase, p.status, kKernelId, 0x400u + s, abort_flag);
       const uint8_t* tile = smem + s * kPackedBytes + row * 128;
-#pragma unroll 1
-      for (int c = group; c < kBlocks; c += 2) {
-        const int b = (t - t_lo) * kBlocks + c;
-        if (b >= blocks) break;
-        __nv_bfloat162 s2[2], nz2[2];
+      const int buf = st % kBufs;
+      __nv_bfloat162 s2[2 * kBlocks], nz2[2 * kBlocks];
+      if constexpr (VEC) {
+        const uint32_t sw = word < 2 ? (word == 0 ? s8.x : s8.y) : (word == 2 ? s8.z : s8.w);
+        const uint32_t zw = word < 2 ? (word == 0 ? z8.x : z8.y) : (word == 2 ? z8.z : z8.w);
+        const uint32_t pick = group == 0 ? 0x1010u : 0x3232u;
+        const uint32_t sb = __byte_perm(sw, 0u, pick), zb = __byte_perm(zw, 0u, pick) ^ 0x80008000u;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          s2[h] = __bfloat162bfloat162(h == 1 && halves ? sc[1] : sc[0]);
-          nz2[h] = __hneg2(__bfloat162bfloat162(h == 1 && halves ? zz[1] : zz[0]));
+        for (int h = 0; h < 2 * kBlocks; ++h) {
+          s2[h] = *reinterpret_cast<const __nv_bfloat162*>(&sb);
+          nz2[h] = *reinterpret_cast<const __nv_bfloat162*>(&zb);
         }
-        if (b + 2 < blocks) fetch(b + 2);
+      } else {
+#pragma unroll
+        for (int h = 0; h < 2 * kBlocks; ++h) {
+          s2[h] = __bfloat162bfloat162((h & 1) == 1 && halves ? sc[h] : sc[h & ~1]);
+          nz2[h] = __hneg2(__bfloat162bfloat162((h & 1) == 1 && halves ? zz[h] : zz[h & ~1]));
+        }
+      }
+      uint4 u[4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        u[v] = *reinterpret_cast<const uint4*>(tile + (((group * 4 + v) ^ (row & 7)) << 4));
+      if constexpr (VEC) {
+        if (++word == 4) {
+          word = 0;
+          if (st + 2 < steps) fetch(st + 2);
+        }
+      } else if (st + 2 < steps) {
+        fetch(st + 2);
+      }
+#pragma unroll
+      for (int i = 0; i < kBlocks; ++i) {
         uint32_t w[32];
 #pragma unroll
         for (int v = 0; v < kVec; ++v) {
-          const uint4 u = *reinterpret_cast<const uint4*>(tile + (((c * kVec + v) ^ (row & 7)) << 4));
-          const uint32_t words[4] = {u.x, u.y, u.z, u.w};
+          const uint4 x4 = u[i * kVec + v];
+          const uint32_t words[4] = {x4.x, x4.y, x4.z, x4.w};
           if constexpr (BITS == 4) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) dequant8(words[j], s2[v], nz2[v], w + v * 16 + j * 4);
+            for (int j = 0; j < 4; ++j) dequant8(words[j], s2[i * 2 + v], nz2[i * 2 + v], w + v * 16 + j * 4);
           } else {
             const float fs = __bfloat162float(s2[v >> 1].x), fz = __bfloat162float(nz2[v >> 1].x);
 #pragma unroll
@@ -245,23 +307,27 @@ __global__ void __launch_bounds__(kThreads, 2)
             }
           }
         }
-        const int buf = b % kBufs;
-        mbar_pass_warp(&aempty[buf], (static_cast<uint32_t>(b / kBufs) & 1u) ^ 1u, p.status, kKernelId,
-                       0x420u + buf, abort_flag);
-        tc_fence_after();
-        tmem_st_32x32(lane_addr + buf * 32, w);
-        tmem_st_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&afull[buf]);
+        if (i == 0) {
+          mbar_pass_warp(&aempty[buf], (static_cast<uint32_t>(st / kBufs) & 1u) ^ 1u, p.status, kKernelId,
+                         0x420u + buf, abort_flag);
+          tc_fence_after();
+        }
+        tmem_st_32x32(lane_addr + buf * (32 * kBlocks) + i * 32, w);
       }
+      // the packed words are in registers: both barriers of the step at once
+      tmem_st_wait();
+      tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&pempty[s]);
+      if (lane == 0) {
+        mbar_arrive(&afull[buf]);
+        mbar_arrive(&pempty[s]);
+      }
       if (++s == p.packed_stages) {
         s = 0;
         phase ^= 1u;
       }
     }
+    // (a last packed tile of one step: the other group has nothing to wait for)
     __syncwarp();
     // every ring slot has been consumed when done_bar completes, so the partial sums take their place
     // (the other de-quantising group has read its last packed tile before its last block was multiplied)
@@ -308,9 +374,15 @@ static int launch(const void* A, long long lda, const void* qw, Args a, cudaStre
   const int tiles = (a.N + BW - 1) / BW;
   const int packed = (a.K / 64 + (BITS == 4 ? 3 : 1)) / (BITS == 4 ? 4 : 2);
   const bool small = packed <= 8;
-  static AtOnce table[2] = {};
-  auto kernel = small ? gemm_wna16_stream_kernel<BITS, true> : gemm_wna16_stream_kernel<BITS, false>;
-  const int* at_once = clusters_at_once(table[small], kernel, kThreads);
+  // scales of eight groups of 128 in 16 bytes, every row from a boundary
+  const bool vec = BITS == 4 && a.g_shift == 7 && (a.K & 1023) == 0 &&
+                   ((reinterpret_cast<uintptr_t>(a.scales) | reinterpret_cast<uintptr_t>(a.zs)) & 15) == 0;
+  static AtOnce table[4] = {};
+  constexpr bool kVec = BITS == 4;
+  auto kernel = small ? (vec ? gemm_wna16_stream_kernel<BITS, true, kVec> : gemm_wna16_stream_kernel<BITS, true, false>)
+                : vec ? gemm_wna16_stream_kernel<BITS, false, kVec>
+                      : gemm_wna16_stream_kernel<BITS, false, false>;
+  const int* at_once = clusters_at_once(table[small + 2 * vec], kernel, kThreads);
   if (at_once == nullptr) return -20;
   // Bound by the de-quantising warps, so what counts is that every SM has the same share: two CTAs per
   // SM and the largest split that one wave takes, down to two packed tiles a slice (four above 32 rows,
@@ -350,9 +422,10 @@ static int launch(const void* A, long long lda, const void* qw, Args a, cudaStre
   const int per_sm = a.rows > 128 ? 1 : 2;
   a.packed_stages = per_sm == 2 ? 2 : 6;
   const int room = (per_sm == 2 ? kSmemLimit / 2 - 1024 : kSmemLimit) - 1024;
-  a.x_stages = (room - a.packed_stages * kPackedBytes) / (a.rows * 128);
+  const int step = BITS == 4 ? 2 : 1;           // blocks of activations in a stage
+  a.x_stages = (room - a.packed_stages * kPackedBytes) / (a.rows * 128 * step);
   if (a.x_stages > kMaxX) a.x_stages = kMaxX;
-  const int ring = a.packed_stages * kPackedBytes + a.x_stages * a.rows * 128;
+  const int ring = a.packed_stages * kPackedBytes + a.x_stages * a.rows * 128 * step;
   const int sums = a.rows * BW * 4;
   const int bytes = (ring > sums ? ring : sums) + 1024;
   if (a.x_stages < 2 || bytes > kSmemLimit) return -20;
