@@ -1,4 +1,4 @@
-"""The rule that sends 257 .. 890 rows to the pair kernel with the weights on the M side, at shapes that were
+"""The rules that send rows to the pair kernel with the weights on the M side, at shapes that were
 timed on both sides: rows x N x K, and that kernel's time over the other one's (148 SMs)."""
 import pytest
 
@@ -79,4 +79,16 @@ def test_k_is_split_where_it_pays(monkeypatch, M, N, K, others, split):
     monkeypatch.setattr(C, "_SM_COUNT", 148)
     C._large_plan.cache_clear()
     assert (C._large_plan(M, N, K)[0] == "slices") == (split < others)
+    C._large_plan.cache_clear()
+
+
+# 129 .. 256 rows: us of the kernel with the weights on the M side over that of the kernel taken otherwise
+@pytest.mark.parametrize("M,N,K,ratio", [
+    (129, 28672, 4096, 0.90), (160, 10240, 2048, 0.73), (192, 28672, 4096, 0.93), (224, 36864, 7168, 0.96),
+    (256, 10240, 2048, 0.81), (256, 9000, 3000, 0.80), (192, 7168, 1024, 0.80), (144, 16384, 512, 0.89),
+    (256, 28672, 4096, 1.03), (256, 6144, 4096, 1.35)])
+def test_weights_on_the_m_side_up_to_256_rows(monkeypatch, M, N, K, ratio):
+    monkeypatch.setattr(C, "_SM_COUNT", 148)
+    C._large_plan.cache_clear()
+    assert (C._large_plan(M, N, K)[0] == "rows") == (ratio < 1)
     C._large_plan.cache_clear()

@@ -135,6 +135,10 @@ def _large_plan(M: int, Nn: int, K: int) -> tuple[str, int, int]:
     choice : this one's: 1500 x 4096 x 14336 181 : 143, 2048 x 2112 x 7168 68 : 56, 4096 x 5120 x 2048 81 : 59, 700 x
     7168 x 16384 169 : 128, 400 x 5120 x 2048 20 : 14, 2183 x 10672 x 7168 420 : 289.
 
+    From 129 to 256 rows the weights go on the M side where this says so (64 shapes of N 2048 .. 36864: 0.76 to
+    1.00 of the other kernels' time, one 1.05): 160 x 10240 x 2048 19.5 : 14.3, 160 x 12288 x 5120 34 : 29, 192 x
+    28672 x 4096 gated 55 : 52, 256 x 7168 x 1024 11.8 : 9.1, 256 x 9000 x 3000 26.3 : 20.9.
+
     K is split where the tiles are no more than the clusters that run at once and the estimate is a tenth
     below the others' (fitted to 300 calls of 40 .. 860 rows): 301 x 4096 x 14336 50 : 36, 301 x 4096 x 4096 17.7 :
     15.2, 301 x 2112 x 7168 25 : 15.5, 186 x 4864 x 14336 50 : 32, 175 x 5632 x 4096 18.4 : 14.8."""
@@ -342,7 +346,8 @@ def _gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = N
     if (USE_PAIR_GEMM and not USE_PAIR_SPLIT and M > 128 and epilogue in _PAIR_EPI
             and (epilogue not in _GATED or Nn % 64 == 0) and not (K % 8 or Nn % 8)):
         kind, rows, slices = _large_plan(M, Nn, K)
-        if M > 256 or kind == "slices":          # (other kernels of up to 256 rows follow below)
+        # (other kernels of up to 256 rows follow below)
+        if M > 256 or kind in ("slices", "rows"):
             args = (ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out), out.stride(0), M, Nn, K, ptr(bias),
                     epilogue)
             rc = -20
