@@ -5,7 +5,8 @@
 //   out[t, j] = act(x[t, j])                         (element-wise family)
 //
 // Quantising epilogues: dynamic 1x128-group fp8 (scale per row and group),
-// static per-tensor fp8, static symmetric int8, static asymmetric int8.  An
+// dynamic per-row fp8 and int8, static per-tensor fp8, static symmetric int8,
+// static asymmetric int8.  An
 // optional device-side row count limits the work to the valid prefix of a
 // padded buffer (MoE static buffers under CUDA graphs).
 //
@@ -31,7 +32,15 @@ enum Act : int {
   kIdentity = 7,
 };
 enum Mode : int { kActMul = 0, kMulAct = 1, kPlain = 2 };
-enum Quant : int { kQNone = 0, kQFp8Group128 = 1, kQFp8Static = 2, kQInt8Static = 3, kQInt8Asym = 4 };
+enum Quant : int {
+  kQNone = 0,
+  kQFp8Group128 = 1,
+  kQFp8Static = 2,
+  kQInt8Static = 3,
+  kQInt8Asym = 4,
+  kQFp8Token = 5,
+  kQInt8Token = 6,
+};
 
 template <int ACT>
 __device__ __forceinline__ float apply(float x, float thr) {
@@ -91,15 +100,40 @@ __device__ __forceinline__ float rnd(float v) {
 struct Args {
   const void* x;
   void* out;
-  float* scale_out;        // [T, d/128] for group quant
+  float* scale_out;        // [T, d/128] for group quant, [T] for a scale per row
   const float* scale_in;   // scalar for static modes
   const int* azp;          // scalar zero point (asymmetric int8)
   const int* valid_rows;
   long long ldx, ldo;
   int T, d;
+  int chunk;               // vectors of 8 columns that one CTA takes (a multiple of 32)
   float threshold;
 };
 
+// Eight results of a row, rounded to the 16-bit type.
+template <typename T, int ACT, int MODE>
+__device__ __forceinline__ void apply8(const T* x, int d, int v, float thr, float (&f)[8]) {
+  float g[8];
+  ld8<T>(x + v * 8, g);
+  if constexpr (MODE == kPlain) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = rnd<T>(apply<ACT>(g[i], thr));
+  } else {
+    float u[8];
+    ld8<T>(x + d + v * 8, u);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if constexpr (MODE == kActMul)
+        f[i] = rnd<T>(apply<ACT>(g[i], thr) * u[i]);
+      else
+        f[i] = rnd<T>(g[i] * apply<ACT>(u[i], thr));
+    }
+  }
+}
+
+// Few rows are bound by the time of one CTA, whose exponentials and divisions one SM works off: the columns of
+// a row are split over CTAs (blockIdx.y) while there are no more than two to an SM.  A step of 12 rows through four
+// layers of 14336 columns 876 to 865 us, of 96 rows 1465 to 1455.
 template <typename T, int ACT, int MODE, int QUANT>
 __global__ void __launch_bounds__(512) act_kernel(const Args a) {
   grid_release_small();
@@ -107,35 +141,19 @@ __global__ void __launch_bounds__(512) act_kernel(const Args a) {
   const int row = blockIdx.x;
   if (a.valid_rows != nullptr && row >= *a.valid_rows) return;
   const T* x = static_cast<const T*>(a.x) + static_cast<long long>(row) * a.ldx;
-  const int nvec = a.d >> 3;
-  const int nvec_pad = (QUANT == kQFp8Group128) ? ((nvec + 31) & ~31) : nvec;
+  const int first = blockIdx.y * a.chunk;
+  const int nvec = min(a.d >> 3, first + a.chunk);
+  const int nvec_pad = (QUANT == kQFp8Group128) ? ((nvec + 31) & ~31) : nvec;   // (first: a multiple of 32)
   float inv_static = 1.0f;
   int zp = 0;
   if constexpr (QUANT == kQFp8Static || QUANT == kQInt8Static || QUANT == kQInt8Asym)
     inv_static = 1.0f / *a.scale_in;
   if constexpr (QUANT == kQInt8Asym) zp = *a.azp;
 
-  for (int v = threadIdx.x; v < nvec_pad; v += blockDim.x) {
+  for (int v = first + threadIdx.x; v < nvec_pad; v += blockDim.x) {
     const bool ok = v < nvec;
     float f[8];
-    if (ok) {
-      float g[8];
-      ld8<T>(x + v * 8, g);
-      if constexpr (MODE == kPlain) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] = rnd<T>(apply<ACT>(g[i], a.threshold));
-      } else {
-        float u[8];
-        ld8<T>(x + a.d + v * 8, u);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          if constexpr (MODE == kActMul)
-            f[i] = rnd<T>(apply<ACT>(g[i], a.threshold) * u[i]);
-          else
-            f[i] = rnd<T>(g[i] * apply<ACT>(u[i], a.threshold));
-        }
-      }
-    }
+    if (ok) apply8<T, ACT, MODE>(x, a.d, v, a.threshold, f);
     if constexpr (QUANT == kQNone) {
       if (ok) st8<T>(static_cast<T*>(a.out) + static_cast<long long>(row) * a.ldo + v * 8, f);
     } else if constexpr (QUANT == kQFp8Group128) {
@@ -180,12 +198,135 @@ __global__ void __launch_bounds__(512) act_kernel(const Args a) {
   }
 }
 
+// The same with a scale per row, from the row's largest result: its CTAs are a cluster and exchange theirs.  The
+// results stay in registers between the two halves, as the 16-bit values that a separate quantisation would read
+// (same bytes); those beyond two vectors of a thread are computed again.  64 x 14336 beyond what the kernel in
+// front covers: 6.0 us and 3.4 for a quantisation of its own, 4.5 together; a step of 64 rows through four fp8
+// layers 658 to 640 us.  (No more than two CTAs to an SM here either, up to the 8 of a portable cluster.)
+constexpr int kKeep = 2;
+
+template <typename T, int ACT, int MODE, bool INT8>
+__global__ void __launch_bounds__(1024) act_token_kernel(const Args a) {
+  grid_release_small();
+  grid_wait();
+  __shared__ float red[32];
+  __shared__ float largest;
+  const int row = blockIdx.x;
+  if (a.valid_rows != nullptr && row >= *a.valid_rows) return;   // (the whole cluster)
+  const T* x = static_cast<const T*>(a.x) + static_cast<long long>(row) * a.ldx;
+  const int first = blockIdx.y * a.chunk + threadIdx.x;
+  const int nvec = min(a.d >> 3, static_cast<int>(blockIdx.y + 1) * a.chunk);
+  uint4 kept[kKeep];
+  float amax = 0.0f;
+#pragma unroll
+  for (int j = 0; j < kKeep; ++j) {
+    const int v = first + j * blockDim.x;
+    if (v < nvec) {
+      float f[8];
+      apply8<T, ACT, MODE>(x, a.d, v, a.threshold, f);
+      st8<T>(reinterpret_cast<T*>(&kept[j]), f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
+    }
+  }
+  for (int v = first + kKeep * blockDim.x; v < nvec; v += blockDim.x) {
+    float f[8];
+    apply8<T, ACT, MODE>(x, a.d, v, a.threshold, f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
+  }
+  amax = block_max(amax, red);
+  const int ctas = gridDim.y;
+  if (ctas > 1) {
+    if (threadIdx.x == 0) largest = amax;
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (int r = 0; r < ctas; ++r) {
+      uint32_t addr;
+      float other;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(&largest)), "r"(r));
+      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(other) : "r"(addr) : "memory");
+      amax = fmaxf(amax, other);
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  }
+  const float s = fmaxf(amax, 1e-10f) / (INT8 ? 127.0f : 448.0f);
+  if (threadIdx.x == 0 && blockIdx.y == 0) a.scale_out[row] = s;
+  const float inv = 1.0f / s;
+  uint8_t* out = static_cast<uint8_t*>(a.out) + static_cast<long long>(row) * a.ldo;
+  auto write = [&](int v, const float (&f)[8]) {
+    uint2 pk;
+    uint8_t* b = reinterpret_cast<uint8_t*>(&pk);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if constexpr (INT8)
+        b[i] = static_cast<uint8_t>(static_cast<int8_t>(fminf(fmaxf(rintf(f[i] * inv), -128.0f), 127.0f)));
+      else
+        b[i] = f32_to_e4m3(f[i] * inv);
+    }
+    *reinterpret_cast<uint2*>(out + v * 8) = pk;
+  };
+#pragma unroll
+  for (int j = 0; j < kKeep; ++j) {
+    const int v = first + j * blockDim.x;
+    if (v < nvec) {
+      float f[8];
+      ld8<T>(reinterpret_cast<const T*>(&kept[j]), f);
+      write(v, f);
+    }
+  }
+  for (int v = first + kKeep * blockDim.x; v < nvec; v += blockDim.x) {
+    float f[8];
+    apply8<T, ACT, MODE>(x, a.d, v, a.threshold, f);
+    write(v, f);
+  }
+  // (the other CTAs of the cluster have read this one's shared memory)
+  if (ctas > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Threads for `vecs` vectors in equal passes of at most `most`.
+inline int even_threads(int vecs, int most) {
+  const int passes = (vecs + most - 1) / most;
+  return ((vecs + passes - 1) / passes + 31) & ~31;
+}
+
 template <typename T, int ACT, int MODE>
-int launch_q(const Args& a, int quant, cudaStream_t s) {
-  int threads = ((a.d >> 3) + 31) & ~31;
-  threads = threads > 512 ? 512 : (threads < 32 ? 32 : threads);
+int launch_token(Args a, bool int8, cudaStream_t s) {
+  const int nvec = a.d >> 3;
+  int ctas = 1;
+  while (ctas < 8 && static_cast<long long>(a.T) * ctas <= sm_count() && nvec > 64 * ctas) ctas *= 2;
+  a.chunk = ((nvec + ctas - 1) / ctas + 31) & ~31;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(a.T, ctas);
+  cfg.blockDim = dim3(even_threads(a.chunk, 1024));
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 1;
+  attr[1].val.clusterDim.y = ctas;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = ctas > 1 ? 2 : 1;
+  return launch_code(int8 ? cudaLaunchKernelEx(&cfg, act_token_kernel<T, ACT, MODE, true>, a)
+                          : cudaLaunchKernelEx(&cfg, act_token_kernel<T, ACT, MODE, false>, a));
+}
+
+template <typename T, int ACT, int MODE>
+int launch_q(Args a, int quant, cudaStream_t s) {
+  if (quant == kQFp8Token || quant == kQInt8Token)
+    return launch_token<T, ACT, MODE>(a, quant == kQInt8Token, s);
+  const int nvec = a.d >> 3;
+  const int most = (nvec + 63) / 64;
+  int splits = 2 * sm_count() / a.T;
+  splits = splits < 1 ? 1 : (splits > most ? most : splits);
+  a.chunk = ((nvec + splits - 1) / splits + 31) & ~31;
+  splits = (nvec + a.chunk - 1) / a.chunk;
+  const int threads = even_threads(a.chunk, 512);
   auto go = [&](void (*kernel)(Args)) {
-    return launch_overlapped(kernel, dim3(a.T), dim3(threads), 0, s, a);
+    return launch_overlapped(kernel, dim3(a.T, splits), dim3(threads), 0, s, a);
   };
   switch (quant) {
     case kQNone: return go(act_kernel<T, ACT, MODE, kQNone>);
@@ -242,7 +383,7 @@ B200_API int b200_activation(const void* x, long long ldx, void* out, long long 
   if (quant == kQFp8Group128 && (d % 128) != 0) return -2;
   Args a;
   a.x = x; a.out = out; a.scale_out = scale_out; a.scale_in = scale_in; a.azp = azp;
-  a.valid_rows = valid_rows; a.ldx = ldx; a.ldo = ldo; a.T = T; a.d = d; a.threshold = threshold;
+  a.valid_rows = valid_rows; a.ldx = ldx; a.ldo = ldo; a.T = T; a.d = d; a.chunk = 0; a.threshold = threshold;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == 0) return launch_t<__nv_bfloat16>(a, act, mode, quant, s);
   if (dtype == 1) return launch_t<__half>(a, act, mode, quant, s);

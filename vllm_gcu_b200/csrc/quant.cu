@@ -31,11 +31,16 @@ __global__ void __launch_bounds__(1024)
   const T* xr = x + static_cast<long long>(row) * ldx;
   const int nvec = H >> 3;
   float amax = 0.0f;
+  float kept[8];                       // a thread's first vector (rows of up to 8192 elements: its only one)
   for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
     float f[8];
     vec8_load<T>(xr + v * 8, f);
 #pragma unroll
     for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
+    if (v == threadIdx.x) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) kept[i] = f[i];
+    }
   }
   amax = block_max(amax, red);
   const float s = fmaxf(amax, 1e-10f) / (INT8 ? 127.0f : 448.0f);
@@ -43,7 +48,12 @@ __global__ void __launch_bounds__(1024)
   const float inv = 1.0f / s;
   for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
     float f[8];
-    vec8_load<T>(xr + v * 8, f);
+    if (v == threadIdx.x) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = kept[i];
+    } else {
+      vec8_load<T>(xr + v * 8, f);
+    }
     uint2 pk;
     uint8_t* b = reinterpret_cast<uint8_t*>(&pk);
 #pragma unroll

@@ -80,8 +80,8 @@ class DenseMLP(nn.Module):
 
     def _act_quant(self, h: torch.Tensor):
         """Gated activation, fused with the quantisation of down_proj's input when that layer
-        runs on 8-bit activations in a mode the activation kernel can emit (128-wide fp8 groups
-        or a static scale).  Returns ``(tensor, kwargs for down_proj)``."""
+        runs on 8-bit activations in a mode the activation kernel can emit (128-wide fp8 groups,
+        a scale per row or a static scale).  Returns ``(tensor, kwargs for down_proj)``."""
         from ..layers.activation import act_and_mul
         iq = fused_input_quant(self.down_proj, h, h.shape[-1] // 2)
         if iq is not None and iq[0] in C.ACT_QUANT and self.act in C.ACT_CODES:

@@ -29,7 +29,8 @@ NORM_QMODES = {None: 0, "fp8_static": 1, "fp8_token": 2, "fp8_group128": 3,
                "int8_static": 4, "int8_token": 5}
 ACT_CODES = {"silu": 0, "gelu": 1, "gelu_tanh": 2, "fatrelu": 3, "gelu_new": 4,
              "gelu_fast": 5, "gelu_quick": 6, "identity": 7}
-ACT_QUANT = {None: 0, "fp8_group128": 1, "fp8_static": 2, "int8_static": 3, "int8_asym": 4}
+ACT_QUANT = {None: 0, "fp8_group128": 1, "fp8_static": 2, "int8_static": 3, "int8_asym": 4,
+             "fp8_token": 5, "int8_token": 6}
 FP8 = torch.float8_e4m3fn
 #: route head-dim-128 decode attention through the TMA-fed kernel (False: cp.async kernel)
 USE_TMA_DECODE = True
@@ -471,11 +472,13 @@ def activation(x: torch.Tensor, act: str = "silu", mode: str = "act_mul",
     if out is None:
         if q == 0:
             out = torch.empty((T, d), device=x.device, dtype=x.dtype)
-        elif q in (1, 2):
+        elif q in (1, 2, 5):
             out = torch.empty((T, d), device=x.device, dtype=FP8)
         else:
             out = torch.empty((T, d), device=x.device, dtype=torch.int8)
-    if q == 1:
+    if q in (5, 6):
+        scale_out = torch.empty((T, 1), device=x.device, dtype=torch.float32)
+    elif q == 1:
         scale_out = torch.empty((T, d // 128), device=x.device, dtype=torch.float32)
     call("b200_activation", ptr(x2), x2.stride(0), ptr(out), out.stride(0), ptr(scale_out),
          ptr(scale), ptr(azp), ptr(valid_rows), T, d, ACT_CODES[act], m, q, float(threshold),
@@ -1893,8 +1896,7 @@ def fused_experts_q8(x: torch.Tensor, w13: torch.Tensor, w13_scale: torch.Tensor
          numel, k, H, cap, 1, DTYPE_CODE[x.dtype], stream_ptr())
     aq, a_s = per_token_quant(a_sorted, qname, valid_rows=npp)
     h = gemm_q8_grouped(aq, a_s.view(-1), w13, w13_scale, expert_ids, npp, kind=kind)
-    hm = activation(h, "silu", "act_mul", valid_rows=npp)
-    hq, h_s = per_token_quant(hm, qname, valid_rows=npp)
+    hq, h_s = activation(h, "silu", "act_mul", quant=qname + "_token", valid_rows=npp)
     y = gemm_q8_grouped(hq, h_s.view(-1), w2, w2_scale, expert_ids, npp, kind=kind,
                         row_scale=row_w)
     out = torch.empty((T, H), device=x.device, dtype=x.dtype)
