@@ -97,7 +97,7 @@ class FepopelForCausalLM(DecoderLM):
     # CUDA sources with the kernels of this model (a fresh checkout may build only these)
     native_sources = ("activation", "attention", "attention_any", "attention_fmha",
                       "attention_mla", "attention_tma", "cache", "common", "gemm_bf16",
-                      "gemm_pair", "gemm_pair_rows", "gemm_skinny", "gemm_stream", "latent", "moe",
+                      "gemm_pair", "gemm_pair_rows", "gemm_pair_slices", "gemm_skinny", "gemm_stream", "latent", "moe",
                       "residual", "sampler", "step")
 
     def __init__(self, cfg: ModelConfig, device="cpu"):

@@ -56,7 +56,7 @@ class FizunexForCausalLM(DecoderLM):
     # CUDA sources with the kernels of this model (a fresh checkout may build only these)
     native_sources = ("activation", "attention", "attention_any", "attention_fmha",
                       "attention_tma", "cache", "common", "gemm_bf16", "gemm_pair", "gemm_skinny",
-                      "gemm_pair_rows", "gemm_stream", "recurrent", "residual", "sampler", "step")
+                      "gemm_pair_rows", "gemm_pair_slices", "gemm_stream", "recurrent", "residual", "sampler", "step")
     # recurrent states cannot be taken back and are not part of the cache blocks: no draft tokens,
     # no prefix cache, no swapping of blocks
     has_request_state = True
