@@ -11,10 +11,12 @@ vllm_gcu/models/deepseek_v3/deepseek_v3_fusion.py:105-258):
 2. one fused kernel splits the latent, applies RMSNorm to ``kv_c``, RoPE to ``q_pe`` / ``k_pe``
    and writes the latent row into the paged cache (``ops.cuda.mla_rope_cache``);
 3. ``q_nope x W_UK`` -> latent query; attention over the cached latents; ``x W_UV``; ``o_proj``.
+   Prompts long enough for it (``ops.cuda.latent_prefill_plan``) go the other way: the latents they
+   attend to become keys and values of every head, which is 3.4 times less work per pair.
 
 The attention core runs in the tcgen05 latent attention kernel (csrc/attention_mla.cu:
-decode, multi-token verification and prefill chunks in one kernel) for bf16 caches and
-up to 128 heads; other layouts fall back to batched matrix products over
+decode, multi-token verification and prefill chunks in one kernel), expanded prompts in
+csrc/attention_fmha_pair.cuh, for bf16 caches and up to 128 heads; other layouts fall back to batched matrix products over
 gathered latent rows (decode: one padded batch; prefill: per sequence).
 """
 from __future__ import annotations

@@ -75,11 +75,12 @@ def oracle_compare(name: str, got: torch.Tensor, want: torch.Tensor, rtol: float
             f"want {w.flatten()[idx].item():.6g})")
 
 
-# Few rows go to gemm_stream.cu (_stream_pays), 257 rows and more that fill tiles of 256 badly to
-# gemm_pair_rows.cu (_pair_rows).  gemm_skinny.cu keeps what these rules leave of up to 256 rows: up to 128 rows
-# with a two-kernel K split (33 .. 64 rows of K < 4096; 65 .. 128 of K < 4096 or N > 8192) or one wave of 256-wide
-# column tiles, and 129 .. 256 rows in one such wave where the pair kernel does not take them (N no multiple
-# of 256 or K none of 64).  Its plans with counters (SKINNY_ALLOW_SPLIT) are off.
+# Few rows go to gemm_stream.cu (_stream_pays), 257 .. 1023 rows that fill tiles of 256 badly to
+# gemm_pair_rows.cu (_pair_rows), more than 128 rows otherwise by estimated time (_large_plan).  gemm_skinny.cu
+# keeps what these rules leave of up to 256 rows: up to 128 rows with a two-kernel K split (33 .. 64 rows of K <
+# 4096; 65 .. 128 of K < 4096 or N > 8192) or one wave of 256-wide column tiles, and 129 .. 256 rows in one such
+# wave where the plan prefers 128-row or pair tiles and the pair kernel does not take them (N no multiple of 256
+# or K none of 64).  Its plans with counters (SKINNY_ALLOW_SPLIT) are off.
 USE_PAIR_GEMM = True            # 256 x 256 tile per CTA pair, cta_group::2 (gemm_pair.cu)
 USE_PAIR_SPLIT = False          # K split over pairs for few-tile decode GEMMs (gemm_pair.cu)
 PAIR_MIN_M = 129                # below the large-M threshold the pair kernel runs when ...
