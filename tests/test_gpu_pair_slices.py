@@ -62,3 +62,28 @@ def test_refused():
     assert call(*args, 64, None, 0, 64, 2, s) == -20           # fewer K blocks than slices
     assert call(*args, 510, None, 0, 64, 2, s) == -2
     assert call(*args, 512, None, 1, 64, 2, s) == -5           # no bias
+
+
+@pytest.mark.parametrize("M,N,K,head", [(160, 840, 520, 256), (301, 28672, 512, 28416), (257, 1088, 1000, 1024)])
+def test_full_rounds_and_a_tail(M, N, K, head):
+    """Two kernels in one call that meet at ``head``; nothing is written beside the result.  (Tolerance as above.)"""
+    from vllm_gcu_b200.ops import cuda as C
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(N, K, device="cuda", generator=g).div_(math.sqrt(K)).to(torch.bfloat16)
+    bias = torch.randn(N, device="cuda", generator=g).to(torch.bfloat16)
+    exact = a.double() @ w.double().t()
+    for epi in (C.EPI_BIAS, C.EPI_SILU_MUL) if N % 64 == 0 else (C.EPI_BIAS,):
+        want = exact + bias.double()
+        if epi == C.EPI_SILU_MUL:
+            p = exact.view(M, N // 64, 2, 32)
+            want = (torch.nn.functional.silu(p[:, :, 0]) * p[:, :, 1]).reshape(M, -1)
+        out = torch.full((M, want.shape[1] + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+        rc = _native.lib().b200_gemm_pair_rows_tail(
+            a.data_ptr(), K, w.data_ptr(), K, out.data_ptr(), out.stride(0), M, N, K, bias.data_ptr(), epi, 160,
+            head, 96, 2, _native.stream_ptr())
+        assert rc == 0
+        err = (out[:, :want.shape[1]].double() - want).abs()
+        slope = 12 if epi == C.EPI_SILU_MUL else 1
+        assert bool((err <= 2.0 ** -8 * want.abs() + slope * K * 2.0 ** -24 + 4e-5).all()), (epi, err.max())
+        assert bool((out[:, want.shape[1]:] == 7.0).all())

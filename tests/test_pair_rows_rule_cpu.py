@@ -44,9 +44,9 @@ def test_full_tiles_and_few_weight_tiles_go_elsewhere(M, monkeypatch):
 ])
 def test_kernel_for_more_rows(monkeypatch, M, N, K, rows, pair, tiles):
     monkeypatch.setattr(C, "_SM_COUNT", 148)
-    C._large_plan.cache_clear()
+    C._large_estimate.cache_clear()
     kind, r, _ = C._large_plan(M, N, K)
-    C._large_plan.cache_clear()
+    C._large_estimate.cache_clear()
     took = {"pair": pair, "tiles": tiles}.get(kind) if kind != "rows" else None
     if kind == "rows":
         assert r % 32 == 0 and 32 <= r <= 256
@@ -58,7 +58,7 @@ def test_kernel_for_more_rows(monkeypatch, M, N, K, rows, pair, tiles):
 
 def test_plans_cover_every_shape(monkeypatch):
     monkeypatch.setattr(C, "_SM_COUNT", 148)
-    C._large_plan.cache_clear()
+    C._large_estimate.cache_clear()
     for M in (129, 257, 300, 1000, 5000, 100000):
         for N in (8, 264, 1000, 4096, 151936):
             for K in (8, 72, 512, 16384):
@@ -66,7 +66,7 @@ def test_plans_cover_every_shape(monkeypatch):
                 assert kind in ("rows", "slices", "pair", "tiles") and rows % 32 == 0 and rows <= 256
                 assert (2 <= slices <= 4 and K >= 512 * slices) if kind == "slices" else slices == 1
                 assert kind != "pair" or N % 256 == 0 and K % 64 == 0
-    C._large_plan.cache_clear()
+    C._large_estimate.cache_clear()
 
 
 # us of the other kernels' best and with K split over the pairs of a cluster
@@ -77,9 +77,9 @@ def test_plans_cover_every_shape(monkeypatch):
     (740, 2816, 1024, 8.4, 12.9), (301, 6144, 4096, 19.5, 28.7), (400, 5120, 2048, 12.9, 21.5)])
 def test_k_is_split_where_it_pays(monkeypatch, M, N, K, others, split):
     monkeypatch.setattr(C, "_SM_COUNT", 148)
-    C._large_plan.cache_clear()
+    C._large_estimate.cache_clear()
     assert (C._large_plan(M, N, K)[0] == "slices") == (split < others)
-    C._large_plan.cache_clear()
+    C._large_estimate.cache_clear()
 
 
 # 129 .. 256 rows: us of the kernel with the weights on the M side over that of the kernel taken otherwise
@@ -89,6 +89,21 @@ def test_k_is_split_where_it_pays(monkeypatch, M, N, K, others, split):
     (256, 28672, 4096, 1.03), (256, 6144, 4096, 1.35)])
 def test_weights_on_the_m_side_up_to_256_rows(monkeypatch, M, N, K, ratio):
     monkeypatch.setattr(C, "_SM_COUNT", 148)
-    C._large_plan.cache_clear()
+    C._large_estimate.cache_clear()
     assert (C._large_plan(M, N, K)[0] == "rows") == (ratio < 1)
-    C._large_plan.cache_clear()
+    C._large_estimate.cache_clear()
+
+
+# us of one kernel, and of full rounds with a tail whose K is split
+@pytest.mark.parametrize("M,N,K,one,tail", [
+    (301, 28672, 4096, 74.5, 71.1), (400, 28672, 4096, 88.8, 83.6), (200, 20480, 4096, 48.7, 43.5),
+    (310, 9728, 4096, 35.2, 30.8), (512, 10240, 5120, 49.3, 46.6),
+    (300, 21504, 2048, 31.4, 34.3), (1000, 4864, 4096, 34.6, 36.2)])
+def test_tail_where_it_pays(monkeypatch, M, N, K, one, tail):
+    monkeypatch.setattr(C, "_SM_COUNT", 148)
+    C._tail_plan.cache_clear(), C._large_estimate.cache_clear()
+    plan = C._tail_plan(M, N, K)
+    C._tail_plan.cache_clear(), C._large_estimate.cache_clear()
+    assert (plan is not None) == (tail < one)
+    if plan:
+        assert plan[0] % 32 == 0 and plan[1] % 256 == 0 and 0 < plan[1] < N and 2 <= plan[3] <= 4

@@ -285,3 +285,30 @@ B200_API int b200_gemm_pair_slices(const void* A, long long lda, const void* W, 
       config(slices, (N + 255) / 256 * a.row_tiles, attr, static_cast<cudaStream_t>(stream));
   return launch_code(cudaLaunchKernelEx(&cfg, gemm_pair_slices_kernel, tmW, tmA, a));
 }
+
+B200_API int b200_gemm_pair_rows(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc,
+                                 int M, int N, int K, const void* bias, int epi, int rows, void* stream);
+
+// The first `head` weight rows (a multiple of 256) in full rounds of gemm_pair_rows.cu in tiles of `rows`, the others
+// here in tiles of `tail_rows`: a last round that a few pairs would work through alone is shared by more.  301 x 28672
+// x 4096 (224 tiles over 74 pairs) 74.5 -> 71.1 us, 200 x 20480 x 4096 48.7 -> 43.5, 310 x 9728 x 4096 35.2 -> 30.8, 600 x
+// 6400 x 4096 39.3 -> 32.8.  (Starting it without a wait for the kernel in front gave another 0.3 us and was left out.)
+B200_API int b200_gemm_pair_rows_tail(const void* A, long long lda, const void* W, long long ldw, void* C,
+                                      long long ldc, int M, int N, int K, const void* bias, int epi, int rows,
+                                      int head, int tail_rows, int slices, void* stream) {
+  using namespace b200;
+  using namespace b200::pair_slices;
+  if (M <= 0 || N <= 0) return 0;
+  if (head <= 0 || head >= N || (head % 256) != 0 || slices < 2 || slices > 4 || tail_rows <= 0 ||
+      tail_rows > kMaxRows || (tail_rows % 32) != 0 || (K + 63) / 64 < slices || clusters_at_once(slices) == 0)
+    return -20;
+  // (the tail's own refusals, before the head runs)
+  const bool gated = epi == kSiluMul || epi == kGeluMul;
+  if ((N % (gated ? 64 : 8)) != 0) return -20;
+  const int rc = b200_gemm_pair_rows(A, lda, W, ldw, C, ldc, M, head, K, bias, epi, rows, stream);
+  if (rc != 0) return rc;
+  return b200_gemm_pair_slices(A, lda, static_cast<const __nv_bfloat16*>(W) + head * ldw, ldw,
+                               static_cast<__nv_bfloat16*>(C) + (gated ? head / 2 : head), ldc, M, N - head, K,
+                               bias == nullptr ? nullptr : static_cast<const __nv_bfloat16*>(bias) + head, epi,
+                               tail_rows, slices, stream);
+}

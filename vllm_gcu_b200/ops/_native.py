@@ -197,6 +197,7 @@ class _Sigs:
     b200_gemm_stream_grouped = [P, L, P, L, P, L, I, I, I, I, P, P, P, I, P, I, P]
     b200_gemm_pair_slices = [P, L, P, L, P, L, I, I, I, P, I, I, I, P]
     b200_gemm_pair_slices_at_once = [I]
+    b200_gemm_pair_rows_tail = [P, L, P, L, P, L, I, I, I, P, I, I, I, I, I, P]
     b200_gemm_pair_rows = [P, L, P, L, P, L, I, I, I, P, I, I, P]
     b200_gemm_pair_rows_grouped = [P, L, P, L, P, L, I, I, I, I, P, P, P, P, I, P]
     b200_gemm_pair = [P, L, P, L, P, L, I, I, I, P, I, P]

@@ -123,7 +123,6 @@ def _slices_at_once(slices: int) -> int:
     return int(N.lib().b200_gemm_pair_slices_at_once(slices))
 
 
-@functools.lru_cache(maxsize=4096)
 def _large_plan(M: int, Nn: int, K: int) -> tuple[str, int, int]:
     """Kernel for more than 128 rows, by its estimated time, with its rows of a tile and slices of K:
     ``("rows", r, 1)`` the pair kernel with the weights on the M side (gemm_pair_rows.cu), ``("slices", r, s)``
@@ -144,15 +143,66 @@ def _large_plan(M: int, Nn: int, K: int) -> tuple[str, int, int]:
     K is split where the tiles are no more than the clusters that run at once and the estimate is a tenth
     below the others' (fitted to 300 calls of 40 .. 860 rows): 301 x 4096 x 14336 50 : 36, 301 x 4096 x 4096 17.7 :
     15.2, 301 x 2112 x 7168 25 : 15.5, 186 x 4864 x 14336 50 : 32, 175 x 5632 x 4096 18.4 : 14.8."""
+    return _large_estimate(M, Nn, K)[1]
+
+
+def _rows_us(rows: int, rounds: int, kb: int, K: int) -> float:
+    """Estimate of gemm_pair_rows.cu for so many rounds of tiles of ``rows`` rows."""
+    return 5.98 + max(rounds * (0.0132 + 0.00986 * rows + kb * max(0.2092, 0.1698 + 0.00034 * rows)),
+                      rounds * rows * K * 2.2678e-5)
+
+
+def _slices_us(rows: int, units: int, slices: int, kb: int) -> float:
+    """Estimate of gemm_pair_slices.cu for ``units`` tiles."""
+    return (3.64 + 0.0213 * rows + 0.054 * slices
+            + -(-kb // slices) * max(0.2161, 0.0616 + 0.00098 * rows, 0.0020012 * 2 * slices * units))
+
+
+def _even_rows(M: int, rows: int) -> int:
+    """Rows, a multiple of 32, of the equal tiles that are as many as ``M`` has of ``rows``."""
+    return -(-(-(-M // -(-M // rows))) // 32) * 32
+
+
+@functools.lru_cache(maxsize=4096)
+def _tail_plan(M: int, Nn: int, K: int):
+    """``(rows, head, rows of the tail's tiles, slices)`` where the first ``head`` weight rows in full rounds of
+    gemm_pair_rows.cu and the others with K split over the pairs of a cluster are estimated faster than one kernel
+    by 4 per cent, by 7 with more than two row tiles, None elsewhere.  (4 us more where the pairs read more weight tiles
+    than one each.)  It is for a last round of a few tiles.  70 shapes of 130 .. 1004 rows whose estimates differ by
+    4 per cent took 0.94 of the time, 0.69 to 1.03, those of 1.00 and more with three row tiles or more: us of 301 x
+    28672 x 4096 74.1 : 71.0, 200 x 20480 x 4096 48.9 : 43.6, 310 x 9728 x 4096 34.9 : 31.0, 231 x 19456 x 14336 173 :
+    120, 620 x 6656 x 8192 74 : 60, but 300 x 21504 x 2048 31.4 : 34.3, 1000 x 4864 x 4096 34.6 : 36.2."""
+    pairs, kb = _sms() // 2, -(-K // 64)
+    w_tiles = -(-Nn // 256)
+    one, plan = _large_estimate(M, Nn, K)[0], None
+    best = one
+    for rows in (256, 224, 192, 160, 128):
+        rows = _even_rows(M, rows)
+        tiles = -(-M // rows)
+        rounds = w_tiles * tiles // pairs
+        head = rounds * pairs // tiles
+        if not 0 < head < w_tiles:
+            continue
+        us = _rows_us(rows, rounds, kb, K) + (4 if w_tiles > pairs else 0)
+        best = min(best, (0.96 if tiles <= 2 else 0.93) * one)
+        for slices in (2, 3, 4):
+            for r in (256, 224, 192, 160, 128, 96, 64) if us < best and kb >= 8 * slices else ():
+                r = _even_rows(M, r)
+                units = (w_tiles - head) * -(-M // r)
+                if units <= _slices_at_once(slices) and us + _slices_us(r, units, slices, kb) < best:
+                    best, plan = us + _slices_us(r, units, slices, kb), (rows, 256 * head, r, slices)
+    return plan
+
+
+@functools.lru_cache(maxsize=4096)
+def _large_estimate(M: int, Nn: int, K: int) -> tuple[float, tuple[str, int, int]]:
+    """us of the kernel that ``_large_plan`` names, and its plan."""
     sms, kb = _sms(), -(-K // 64)
     pairs, w_tiles = sms // 2, -(-Nn // 256)
     best, plan = float("inf"), ("tiles", 0, 1)
     for rows in (256, 224, 192, 160, 128, 96, 64):
-        tiles = -(-M // rows)
-        rows = -(-(-(-M // tiles)) // 32) * 32
-        rounds = -(-w_tiles * -(-M // rows) // pairs)
-        us = 5.98 + max(rounds * (0.0132 + 0.00986 * rows + kb * max(0.2092, 0.1698 + 0.00034 * rows)),
-                        rounds * rows * K * 2.2678e-5)
+        rows = _even_rows(M, rows)
+        us = _rows_us(rows, -(-w_tiles * -(-M // rows) // pairs), kb, K)
         if us < best:
             best, plan = us, ("rows", rows, 1)
     if Nn % 256 == 0 and K % 64 == 0:
@@ -169,16 +219,14 @@ def _large_plan(M: int, Nn: int, K: int) -> tuple[str, int, int]:
         best, plan = us, ("tiles", 0, 1)
     for slices in (2, 3, 4) if kb >= 16 else ():
         for rows in (256, 224, 192, 160, 128, 96, 64):
-            tiles = -(-M // rows)
-            rows = -(-(-(-M // tiles)) // 32) * 32
+            rows = _even_rows(M, rows)
             units = w_tiles * -(-M // rows)
             if kb < 8 * slices or units > _slices_at_once(slices):
                 continue
-            us = (3.64 + 0.0213 * rows + 0.054 * slices
-                  + -(-kb // slices) * max(0.2161, 0.0616 + 0.00098 * rows, 0.0020012 * 2 * slices * units))
+            us = _slices_us(rows, units, slices, kb)
             if us < (0.9 * best if plan[0] != "slices" else best):
                 best, plan = us, ("slices", rows, slices)
-    return plan
+    return best, plan
 
 
 def _stream_pays(M: int, Nn: int, K: int) -> bool:
@@ -333,6 +381,18 @@ def _gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = N
             return out
         if rc != -20:
             raise N.NativeError(f"b200_gemm_stream failed with code {rc}")
+    if (USE_PAIR_GEMM and not USE_PAIR_SPLIT and 128 < M <= WIDE2_MIN_M and epilogue in _PAIR_EPI
+            and (epilogue not in _GATED or Nn % 64 == 0) and not (K % 8 or Nn % 8)):
+        tail = _tail_plan(M, Nn, K)
+        if tail is not None:
+            rc = N.lib().b200_gemm_pair_rows_tail(ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out),
+                                                  out.stride(0), M, Nn, K, ptr(bias), epilogue, *tail,
+                                                  stream_ptr())
+            if rc == 0:
+                N.launch_count += 2
+                return out
+            if rc != -20:
+                raise N.NativeError(f"b200_gemm_pair_rows_tail failed with code {rc}")
     if (USE_PAIR_GEMM and 256 < M < WIDE2_MIN_M and epilogue in _PAIR_EPI
             and (epilogue not in _GATED or Nn % 64 == 0)):
         rows = _pair_rows(M, Nn, K)
