@@ -684,7 +684,7 @@ int launch_prefill(const PrefillArgs& a, int num_q_tiles, cudaStream_t s) {
 using namespace b200;
 using namespace b200::attn;
 
-// Number of KV splits the decode kernels of this file want for this problem (host helper,
+// Number of KV splits a decode step runs with for this problem (host helper,
 // deterministic: callers size the workspace with it).
 B200_API int b200_decode_num_splits(int B, int Hkv, int max_seq_len) {
   const long long ctas = static_cast<long long>(B) * Hkv;

@@ -103,11 +103,12 @@ __device__ __forceinline__ float sink_part(float M, float L, float sink) {
   const float keys = L * exp2f(M - top);
   return keys / (keys + exp2f(s2 - top));
 }
-// The splits of a cluster, each with maximum, sum and unscaled output of its keys in shared memory: every CTA
-// adds up a share of the numbers.  All threads of the cluster call it.
+// The splits of a cluster, each with its keys' log2 sum and scaled output in shared memory: every CTA adds up a
+// share of the numbers, in the same steps as decode_reduce_kernel (attention.cu), so that a request's result
+// does not depend on which of the two merges its splits.  All threads of the cluster call it.
 template <typename T>
-__device__ __forceinline__ void merge_cluster(const Args& a, const float* m, const float* l, const float* o,
-                                              int b, int kvh, int G, int OD) {
+__device__ __forceinline__ void merge_cluster(const Args& a, const float* lse, const float* o, int b, int kvh,
+                                              int G, int OD) {
   cluster_arrive_wait();
   uint32_t rank;
   asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
@@ -115,27 +116,26 @@ __device__ __forceinline__ void merge_cluster(const Args& a, const float* m, con
     for (int idx = static_cast<int>(rank) * kConsumers + threadIdx.x; idx < G * HD;
          idx += a.num_splits * kConsumers) {
       const int r = idx / HD, d = idx % HD;
-      float pm[8], pl[8], po[8], M = -INFINITY, L = 0.0f, val = 0.0f;
+      float pl[8], po[8], M = -INFINITY, acc = 0.0f, wsum = 0.0f;
 #pragma unroll
       for (int s = 0; s < 8; ++s) {
-        pm[s] = -INFINITY;
+        pl[s] = -INFINITY;
         if (s >= a.num_splits) continue;
-        pm[s] = ld_peer(m + r, s);
-        pl[s] = ld_peer(l + r, s);
+        pl[s] = ld_peer(lse + r, s);
         po[s] = ld_peer(o + idx, s);
       }
 #pragma unroll
-      for (int s = 0; s < 8; ++s) M = fmaxf(M, pm[s]);
+      for (int s = 0; s < 8; ++s) M = fmaxf(M, pl[s]);
 #pragma unroll
       for (int s = 0; s < 8; ++s) {
-        if (pm[s] == -INFINITY) continue;       // nothing seen: its output was never written
-        const float f = exp2f(pm[s] - M);
-        L += pl[s] * f;
-        val += po[s] * f;
+        if (pl[s] == -INFINITY) continue;       // nothing seen: its output was never written
+        const float w = exp2f(pl[s] - M);
+        wsum += w;
+        acc += w * po[s];
       }
-      val = L > 0.0f ? val / L : 0.0f;
+      float val = wsum > 0.0f ? acc / wsum : 0.0f;
       const int head = kvh * G + r;
-      if (a.sink != nullptr && L > 0.0f) val *= sink_part(M, L, a.sink[head]);
+      if (a.sink != nullptr && wsum > 0.0f) val *= sink_part(M, wsum, a.sink[head]);
       if (d < OD)
         static_cast<T*>(a.out)[static_cast<long long>(b) * a.ldo + head * OD + d] = from_f32<T>(val);
     }
@@ -174,13 +174,12 @@ __global__ void __launch_bounds__(kThreads)
   const int end = min(seq_len, start + chunk);
 
   // what a split of a cluster leaves to the others (behind the buffers of its own merge)
-  float* part_m = reinterpret_cast<float*>(smem) + 128 + 4 * 16 * HD;
-  float* part_l = part_m + 16;
-  float* part_o = part_l + 16;
+  float* part_lse = reinterpret_cast<float*>(smem) + 128 + 4 * 16 * HD;
+  float* part_o = part_lse + 16;
   if (start >= end) {
     if (a.cluster) {
-      if (threadIdx.x < 16) part_m[threadIdx.x] = -INFINITY;
-      merge_cluster<T>(a, part_m, part_l, part_o, b, kvh, G, OD);
+      if (threadIdx.x < 16) part_lse[threadIdx.x] = -INFINITY;
+      merge_cluster<T>(a, part_lse, part_o, b, kvh, G, OD);
       return;
     }
     for (int r = 0; r < G; ++r) {
@@ -238,7 +237,7 @@ __global__ void __launch_bounds__(kThreads)
     }
     // the producer warp takes no part in the merge
     __syncwarp();
-    if (a.cluster) merge_cluster<T>(a, part_m, part_l, part_o, b, kvh, G, OD);
+    if (a.cluster) merge_cluster<T>(a, part_lse, part_o, b, kvh, G, OD);
     return;
   }
 
@@ -397,15 +396,12 @@ __global__ void __launch_bounds__(kThreads)
       L += sm_l[w * 16 + r] * f;
       o += sm_o[(w * 16 + r) * HD + d] * f;
     }
+    float val = (ok && L > 0.0f) ? o / L : 0.0f;
     if (a.cluster) {
-      part_o[idx] = o;
-      if (d == 0) {
-        part_m[r] = ok && L > 0.0f ? M : -INFINITY;
-        part_l[r] = L;
-      }
+      part_o[idx] = val;
+      if (d == 0) part_lse[r] = (ok && L > 0.0f) ? M + log2f(L) : -INFINITY;
       continue;
     }
-    float val = (ok && L > 0.0f) ? o / L : 0.0f;
     const int head = kvh * G + r;
     if (a.sink != nullptr && a.num_splits == 1 && ok && L > 0.0f) val *= sink_part(M, L, a.sink[head]);
     if (a.num_splits > 1) {
@@ -417,7 +413,7 @@ __global__ void __launch_bounds__(kThreads)
     }
   }
   __syncwarp();
-  if (a.cluster) merge_cluster<T>(a, part_m, part_l, part_o, b, kvh, G, OD);
+  if (a.cluster) merge_cluster<T>(a, part_lse, part_o, b, kvh, G, OD);
 }
 
 // Launch with the splits of a request and key head as a cluster, or as CTAs on their own
@@ -528,7 +524,7 @@ static int paged_decode_tma_impl(const void* q, long long ldq, void* out, long l
   const bool shaped = softcap > 0.0f || chunk > 0 || window > 0 || alibi != nullptr || a.OD != HD;
   if (shaped && dtype != 0) return -20;
   constexpr int smem = kStages * kStageBytes + 256 + 1024;
-  static_assert(kStages * kStageBytes >= (128 + 4 * 16 * b200::attn_tma::HD + 32 + 16 * b200::attn_tma::HD) * 4,
+  static_assert(kStages * kStageBytes >= (128 + 4 * 16 * b200::attn_tma::HD + 16 + 16 * b200::attn_tma::HD) * 4,
                 "merge buffers must fit");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   dim3 grid(B, Hkv, num_splits);
@@ -568,7 +564,9 @@ static int paged_decode_tma_impl(const void* q, long long ldq, void* out, long l
                             a.OD, stream);
 }
 
-// Number of splits for the kernel of this file (as b200_decode_num_splits).  One CTA has 96 KB of keys on their way,
+// Number of splits that takes the kernel of this file the least time.  Not the one that steps run with
+// (b200_decode_num_splits): every split has its own running maximum, to which its probabilities are rounded to 16 bits,
+// so that another number of splits gives other bits of the same accuracy.  One CTA has 96 KB of keys on their way,
 // which is its SM's share of the copy bandwidth, and every further CTA costs 10 ns of the whole: splits pay only
 // while SMs are idle.  us by splits 1, 2, 4: 64 requests of 2304 keys and 4 key heads (256 CTAs) 49 : 58 : 68, 32 of
 // 800 and 8 key heads (256) 20 : 27 : 35, 12 of 900 (96) 15 : 13 : 18, 1 of 4000 (8) 41 : 25 : 15, with 8 or 16

@@ -325,10 +325,7 @@ class ModelRunner:
             return 1
         from ..ops import cuda as C
         spec = self.model.kv_cache_spec()
-        alibi = str(self.cfg.model.extra.get("position_embedding", "ROPE")).upper() == "ALIBI"
-        tma = (spec["type"] == "gqa" and not alibi and bool(self.kv_caches)
-               and C.tma_decode_covers(spec["head_dim"], self.block_size, self.kv_caches[0].dtype))
-        s = C.decode_num_splits(batch, spec["kv_heads"], max_seq_len, tma)
+        s = C.decode_num_splits(batch, spec["kv_heads"], max_seq_len)
         Hq = spec.get("q_heads") or \
             self.cfg.model.num_attention_heads // self.cfg.parallel.tensor_parallel_size
         D = max(self.cfg.model.head_dim, spec["head_dim"])

@@ -693,15 +693,12 @@ def swap_blocks(src: torch.Tensor, dst: torch.Tensor, mapping_cpu: torch.Tensor)
 # attention
 # ---------------------------------------------------------------------------
 def decode_num_splits(B: int, Hkv: int, max_seq_len: int, tma: bool = False) -> int:
-    """``tma``: the step's caches are ones that :func:`tma_decode_covers`."""
+    """Splits of the keys that a step runs with.  ``tma``: the number that takes the TMA-fed kernel
+    (attention_tma.cu) the least time, for callers that choose a number themselves; no step takes it, since
+    another number of splits rounds the probabilities otherwise, which eight layers of 16 bits carry on to
+    1.5 per cent of the logits."""
     fn = N.lib().b200_decode_num_splits_tma if tma else N.lib().b200_decode_num_splits
     return int(fn(B, Hkv, max_seq_len))
-
-
-def tma_decode_covers(head_dim: int, block_size: int, cache_dtype: torch.dtype) -> bool:
-    """Paged caches of 16 bits that the kernel fed by TMA takes (attention_tma.cu), laid out densely."""
-    return (USE_TMA_DECODE and head_dim == 128 and block_size % 16 == 0
-            and cache_dtype in (torch.bfloat16, torch.float16))
 
 
 def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
@@ -752,9 +749,7 @@ def _paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
         out = torch.empty((B, Hq, od), device=q.device, dtype=q.dtype)
     assert out.stride(2) == 1 and out.stride(1) == od
     if num_splits <= 0:
-        dense = k_cache.stride(2) == D and k_cache.stride(1) == Hkv * D and alibi_slopes is None
-        num_splits = decode_num_splits(B, Hkv, max_seq_len or block_tables.shape[1] * bs,
-                                       dense and tma_decode_covers(D, bs, k_cache.dtype))
+        num_splits = decode_num_splits(B, Hkv, max_seq_len or block_tables.shape[1] * bs)
     tmp_out = tmp_lse = None
     if num_splits > 1:
         if workspace is None:

@@ -109,7 +109,6 @@ class B200AttentionMetadataBuilder(AttentionMetadataBuilder[B200AttentionMetadat
         self._init_reorder_batch_threshold(1)
         self.num_kv_heads = kv_cache_spec.num_kv_heads
         self.head_size = kv_cache_spec.head_size
-        self.tma = C.tma_decode_covers(kv_cache_spec.head_size, kv_cache_spec.block_size, kv_cache_spec.dtype)
         pc = vllm_config.parallel_config
         self.num_heads = vllm_config.model_config.get_num_attention_heads(pc)
         self.max_model_len = vllm_config.model_config.max_model_len
@@ -124,7 +123,7 @@ class B200AttentionMetadataBuilder(AttentionMetadataBuilder[B200AttentionMetadat
                         device=device))
 
     def _splits(self, batch: int, max_seq_len: int) -> int:
-        s = C.decode_num_splits(batch, self.num_kv_heads, max_seq_len, self.tma)
+        s = C.decode_num_splits(batch, self.num_kv_heads, max_seq_len)
         while s > 1 and batch * self.num_heads * s * self.head_size > self.workspace[0].numel():
             s -= 1
         return s
