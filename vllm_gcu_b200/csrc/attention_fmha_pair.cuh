@@ -476,6 +476,11 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     const float sl2 = a.scale * 1.4426950408889634f;
     const uint64_t sl2_2 = f2_pack(sl2, sl2);
     uint32_t s_phase = 0, o_phase = 0, t_phase = 0;
+    // Turns: key tiles that both slots have, one after the other over all pieces of work: slot 0, slot 1, slot 0 ...
+    // Each slot waits for the other's turn before every one of them (the very first excepted), also across
+    // pieces: a slot that went on without could complete the next turn before a warp of the other has looked at this
+    // one, and that warp would wait for a parity that has come back.
+    int both_before = 0;                        // such tiles in the pieces so far
     for (int it = 0;; ++it) {
       if (!mbar_wait_warp(&w_full[it & 1], (it >> 1) & 1, a.status, kKernelId, 0x640u, abort_flag)) break;
       const volatile Work* k = works + (it & 1);
@@ -557,7 +562,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
           }
         }
         const uint64_t mb2 = f2_pack(-mb, -mb);
-        if (h == 0 ? j > 0 && j < nt_both : j < nt_both) {
+        if (j < nt_both && both_before + j + h > 0) {
           mbar_pass_warp(&turn[h ^ 1], t_phase, a.status, kKernelId, 0x644u + h, abort_flag);
           t_phase ^= 1u;
         }
@@ -577,7 +582,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             sum2[c & 1] = f2_add(sum2[c & 1], f2_pack(p0, p1));
             pk[i >> 1] = pack_bf16x2(p0, p1);
           }
-          if (c == 3 && lane == 0 && (h == 0 ? j < nt_both : j + 1 < nt_both)) mbar_arrive(&turn[h]);
+          if (c == 3 && lane == 0 && j < nt_both) mbar_arrive(&turn[h]);
           tmem_st_32x16(s_addr + c * 16, pk);
           if (c == 1) {
             tmem_st_wait();
@@ -594,6 +599,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         f2_unpack(f2_add(sum2[0], sum2[1]), s0, s1);
         l = l * alpha + (s0 + s1);
       }
+      both_before += nt_both;
       if (ok) ok = mbar_wait_warp(&o_done[h], o_phase, a.status, kKernelId, 0x650u + h, abort_flag);
       if (!ok) break;
       o_phase ^= 1u;
