@@ -239,9 +239,7 @@ __global__ void __launch_bounds__(1024) act_token_kernel(const Args a) {
   const int ctas = gridDim.y;
   if (ctas > 1) {
     if (threadIdx.x == 0) largest = amax;
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_sync();
     for (int r = 0; r < ctas; ++r) {
       uint32_t addr;
       float other;
@@ -249,7 +247,7 @@ __global__ void __launch_bounds__(1024) act_token_kernel(const Args a) {
       asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(other) : "r"(addr) : "memory");
       amax = fmaxf(amax, other);
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    cluster_arrive();
   }
   const float s = fmaxf(amax, 1e-10f) / (INT8 ? 127.0f : 448.0f);
   if (threadIdx.x == 0 && blockIdx.y == 0) a.scale_out[row] = s;
@@ -282,7 +280,7 @@ __global__ void __launch_bounds__(1024) act_token_kernel(const Args a) {
     write(v, f);
   }
   // (the other CTAs of the cluster have read this one's shared memory)
-  if (ctas > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (ctas > 1) cluster_wait();
 }
 
 // Threads for `vecs` vectors in equal passes of at most `most`.

@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(kThreads, kResident)
       // (the two warps that share rows; the next but one tile's maxima come behind another barrier)
       float* both = xch + (j & 1) * 2 * BQ;
       both[g * BQ + r] = mt;
-      asm volatile("bar.sync %0, 64;" ::"r"(2 + qd) : "memory");
+      pair_sync(2 + qd);
       mt = fmaxf(mt, both[(g ^ 1) * BQ + r]);
       float alpha = 1.0f;
       float m_new = m_used;
@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(kThreads, kResident)
     }
     float* both = xch + (nt & 1) * 2 * BQ;
     both[g * BQ + r] = l;
-    asm volatile("bar.sync %0, 64;" ::"r"(2 + qd) : "memory");
+    pair_sync(2 + qd);
     l += both[(g ^ 1) * BQ + r];
     if (mbar_wait_warp(o_done, (nt - 1) & 1, a.status, kKernelId, 0x320u, abort_flag)) {
       tc_fence_after();

@@ -85,10 +85,6 @@ struct Args {
   unsigned int* status;
 };
 
-__device__ __forceinline__ void cluster_arrive_wait() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float ld_peer(const float* p, uint32_t rank) {
   uint32_t addr;
   float v;
@@ -109,7 +105,7 @@ __device__ __forceinline__ float sink_part(float M, float L, float sink) {
 template <typename T>
 __device__ __forceinline__ void merge_cluster(const Args& a, const float* lse, const float* o, int b, int kvh,
                                               int G, int OD) {
-  cluster_arrive_wait();
+  cluster_sync();
   uint32_t rank;
   asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   if (threadIdx.x < kConsumers) {
@@ -140,7 +136,7 @@ __device__ __forceinline__ void merge_cluster(const Args& a, const float* lse, c
         static_cast<T*>(a.out)[static_cast<long long>(b) * a.ldo + head * OD + d] = from_f32<T>(val);
     }
   }
-  cluster_arrive_wait();           // nobody leaves while another CTA may still read its numbers
+  cluster_sync();                  // nobody leaves while another CTA may still read its numbers
 }
 __device__ __forceinline__ void consumer_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 

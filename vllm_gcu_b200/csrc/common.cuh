@@ -164,6 +164,30 @@ __device__ __forceinline__ void grid_release_small() {
 }
 
 // ---------------------------------------------------------------------------
+// Barriers of whole warps
+// ---------------------------------------------------------------------------
+// Both halves of the cluster's barrier.  In this form all lanes of a warp execute them together, and those that
+// took different ways in front of it are not together again by themselves.
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Both at once.
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Barrier `id` of two warps, likewise.
+__device__ __forceinline__ void pair_sync(int id) {
+  __syncwarp();
+  asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
+}
+
+// ---------------------------------------------------------------------------
 // TMA (tiled bulk tensor copies, never with cluster multicast)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {

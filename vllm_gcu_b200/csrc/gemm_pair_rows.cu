@@ -279,10 +279,10 @@ __global__ void __launch_bounds__(kThreads, 1)
           released = true;
         }
         if (gated) {
-          asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");       // the last chunk has been read
+          pair_sync(pair_bar);       // the last chunk has been read
 #pragma unroll
           for (int i = 0; i < 16; ++i) xch[(up ? 0 : 512) + i * 32] = __uint_as_float(up ? r[i] : r[16 + i]);
-          asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");
+          pair_sync(pair_bar);
           float f[16], g[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {

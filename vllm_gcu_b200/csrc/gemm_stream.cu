@@ -218,7 +218,6 @@ __global__ void __launch_bounds__(kThreads)
     if (ok)
       park_sums(tmem, reinterpret_cast<float*>(smem), q, lane, used);
   }
-  __syncwarp();
   tc_fence_before();
   if (splits > 1) cluster_arrive_wait();
   else __syncthreads();

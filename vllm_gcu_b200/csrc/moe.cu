@@ -214,10 +214,7 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const AlignArgs a) {
     a.pos_of[i] = e >= 0 ? atomicAdd(&count[e], 1) : -1;
   }
   __syncthreads();
-  if (ctas > 1) {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-  }
+  if (ctas > 1) cluster_sync();
   // sums over the CTAs and padded offsets: a thread takes neighbouring experts
   const int per = (E + static_cast<int>(blockDim.x) - 1) / static_cast<int>(blockDim.x);
   int mine = 0;
@@ -240,7 +237,7 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const AlignArgs a) {
     mine += (all + kTileM - 1) / kTileM * kTileM;
   }
   // (the others may still read this CTA's counts: it leaves behind the wait at the end)
-  if (ctas > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  if (ctas > 1) cluster_arrive();
   int inc = mine;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
@@ -307,7 +304,7 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const AlignArgs a) {
     if (first + c * stride < a.numel) put(first + c * stride, expert[c], place[c]);
   for (int i = first + kKeep * stride; i < a.numel; i += stride)
     put(i, i < n ? expert_of(i) : -1, i < n ? a.pos_of[i] : 0);
-  if (ctas > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (ctas > 1) cluster_wait();
 }
 
 // A_sorted[pos_of[t, s]] = x[t] for every pair of a token, which is read once; rows of padding stay as they are,

@@ -11,10 +11,7 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void cluster_sync_all() { cluster_sync(); }
 // Address of `local` (a shared-memory location of this CTA) in CTA `rank` of the cluster.
 __device__ __forceinline__ uint32_t map_to_cta(const void* local, uint32_t rank) {
   uint32_t out;

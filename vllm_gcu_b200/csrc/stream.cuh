@@ -14,10 +14,7 @@ constexpr int BW = 128;                 // weight rows of a tile
 constexpr int kMaxSplits = 8;
 constexpr int kSmemLimit = 231424;      // of one CTA, 1 KB of it for the alignment of the ring
 
-__device__ __forceinline__ void cluster_arrive_wait() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void cluster_arrive_wait() { cluster_sync(); }
 __device__ __forceinline__ uint32_t peer_addr(uint32_t local, uint32_t rank) {
   uint32_t out;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(local), "r"(rank));
