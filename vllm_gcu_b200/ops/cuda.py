@@ -83,6 +83,10 @@ def oracle_compare(name: str, got: torch.Tensor, want: torch.Tensor, rtol: float
 # or K none of 64).  Its plans with counters (SKINNY_ALLOW_SPLIT) are off.
 USE_PAIR_GEMM = True            # 256 x 256 tile per CTA pair, cta_group::2 (gemm_pair.cu)
 USE_PAIR_SPLIT = False          # K split over pairs for few-tile decode GEMMs (gemm_pair.cu)
+# K split over the pairs of a cluster for 129 rows and more (gemm_pair_slices.cu): 301 x 4096 x 14336 50 -> 36 us.  Off:
+# partial sums round otherwise than one sum over K, as exactly, but eight layers of 16 bits carry that on to 1.3
+# per cent of the logits of a decoding request (150 requests, or 40 of them beside two prompts of 200).
+USE_SPLIT_SUMS = False
 PAIR_MIN_M = 129                # below the large-M threshold the pair kernel runs when ...
 PAIR_MIN_TILES = 48             # ... its tiles can occupy most of the 74 SM pairs
 USE_WIDE2_GEMM = True           # persistent 256 x 256 tiles for large M (gemm_skinny.cu)
@@ -123,11 +127,12 @@ def _slices_at_once(slices: int) -> int:
     return int(N.lib().b200_gemm_pair_slices_at_once(slices))
 
 
-def _large_plan(M: int, Nn: int, K: int) -> tuple[str, int, int]:
+def _large_plan(M: int, Nn: int, K: int, split: bool = True) -> tuple[str, int, int]:
     """Kernel for more than 128 rows, by its estimated time, with its rows of a tile and slices of K:
     ``("rows", r, 1)`` the pair kernel with the weights on the M side (gemm_pair_rows.cu), ``("slices", r, s)``
     the same with K split over s pairs (gemm_pair_slices.cu), ``("pair", 0, 1)`` 256 x 256 tiles on CTA pairs
-    (gemm_pair.cu), ``("tiles", 0, 1)`` 128 rows by the width that fills the SMs best (gemm_bf16.cu).
+    (gemm_pair.cu), ``("tiles", 0, 1)`` 128 rows by the width that fills the SMs best (gemm_bf16.cu).  Without
+    ``split`` every sum over K is one (USE_SPLIT_SUMS).
 
     Each estimate is rounds of the SMs times (K blocks times a rate that grows with the tile, and a way out),
     or the rate at the power limit where that is lower.  Fitted to 200 shapes of 257 .. 8192 rows, N 240 .. 28672
@@ -143,7 +148,7 @@ def _large_plan(M: int, Nn: int, K: int) -> tuple[str, int, int]:
     K is split where the tiles are no more than the clusters that run at once and the estimate is a tenth
     below the others' (fitted to 300 calls of 40 .. 860 rows): 301 x 4096 x 14336 50 : 36, 301 x 4096 x 4096 17.7 :
     15.2, 301 x 2112 x 7168 25 : 15.5, 186 x 4864 x 14336 50 : 32, 175 x 5632 x 4096 18.4 : 14.8."""
-    return _large_estimate(M, Nn, K)[1]
+    return _large_estimate(M, Nn, K, split)[1]
 
 
 def _rows_us(rows: int, rounds: int, kb: int, K: int) -> float:
@@ -195,7 +200,7 @@ def _tail_plan(M: int, Nn: int, K: int):
 
 
 @functools.lru_cache(maxsize=4096)
-def _large_estimate(M: int, Nn: int, K: int) -> tuple[float, tuple[str, int, int]]:
+def _large_estimate(M: int, Nn: int, K: int, split: bool = True) -> tuple[float, tuple[str, int, int]]:
     """us of the kernel that ``_large_plan`` names, and its plan."""
     sms, kb = _sms(), -(-K // 64)
     pairs, w_tiles = sms // 2, -(-Nn // 256)
@@ -217,7 +222,7 @@ def _large_estimate(M: int, Nn: int, K: int) -> tuple[float, tuple[str, int, int
     us = 4.54 + waves[c] * max(-0.356 + 0.025 * c + kb * (0.1441 + 0.00066 * c), c * K * 2.771e-5)
     if us < best:
         best, plan = us, ("tiles", 0, 1)
-    for slices in (2, 3, 4) if kb >= 16 else ():
+    for slices in (2, 3, 4) if split and kb >= 16 else ():
         for rows in (256, 224, 192, 160, 128, 96, 64):
             rows = _even_rows(M, rows)
             units = w_tiles * -(-M // rows)
@@ -381,7 +386,7 @@ def _gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = N
             return out
         if rc != -20:
             raise N.NativeError(f"b200_gemm_stream failed with code {rc}")
-    if (USE_PAIR_GEMM and not USE_PAIR_SPLIT and 128 < M <= WIDE2_MIN_M and epilogue in _PAIR_EPI
+    if (USE_SPLIT_SUMS and USE_PAIR_GEMM and not USE_PAIR_SPLIT and 128 < M <= WIDE2_MIN_M and epilogue in _PAIR_EPI
             and (epilogue not in _GATED or Nn % 64 == 0) and not (K % 8 or Nn % 8)):
         tail = _tail_plan(M, Nn, K)
         if tail is not None:
@@ -407,7 +412,7 @@ def _gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = N
                 raise N.NativeError(f"b200_gemm_pair_rows failed with code {rc}")
     if (USE_PAIR_GEMM and not USE_PAIR_SPLIT and M > 128 and epilogue in _PAIR_EPI
             and (epilogue not in _GATED or Nn % 64 == 0) and not (K % 8 or Nn % 8)):
-        kind, rows, slices = _large_plan(M, Nn, K)
+        kind, rows, slices = _large_plan(M, Nn, K, USE_SPLIT_SUMS)
         # (other kernels of up to 256 rows follow below)
         if M > 256 or kind in ("slices", "rows"):
             args = (ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out), out.stride(0), M, Nn, K, ptr(bias),
