@@ -456,14 +456,18 @@ __device__ __forceinline__ float2 unpack_bf16x2(uint32_t u) {
   return __bfloat1622float2(v);
 }
 // x / y for y >= 1 without a branch, where a loop of IEEE divisions waits for each one in turn (16 gated values
-// of a GEMM's epilogue 2440 cycles, so 700): the quotient by the approximate reciprocal and one Newton step
-// on its residual, an ulp at most from the rounded quotient for y < 2^126 and zero beyond.  Infinities and
-// NaN as in the division (the residual is NaN there, and the first quotient stands).
+// of a GEMM's epilogue 2440 cycles, so 700): the quotient by the approximate reciprocal, and two Newton steps on
+// its residual.  After the first it is within an ulp, its residual exact, and the second rounds it as
+// the division does, but where x / y lies within 2^-24 of an ulp of the middle between two numbers.  (The reciprocal of a
+// quarter of y is not flushed to zero up to the largest y.)  Infinities and NaN as in the division: the residual
+// is NaN there, and the first quotient stands.
 __device__ __forceinline__ float div_from_one(float x, float y) {
   float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(0.25f * y));
+  r *= 0.25f;
   const float q = x * r, rest = fmaf(-q, y, x);
-  return fabsf(rest) < INFINITY ? fmaf(rest, r, q) : q;
+  const float near = fmaf(rest, r, q);
+  return fabsf(rest) < INFINITY ? fmaf(fmaf(-near, y, x), r, near) : q;
 }
 __device__ __forceinline__ float silu_f(float x) { return div_from_one(x, 1.0f + __expf(-x)); }
 // tanh through one exponential and one division: absolute error below 1e-6, exact limits
