@@ -59,11 +59,6 @@ __device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
-__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 // (three operands: half the instructions of a row maximum)
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
@@ -566,7 +561,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
           mbar_pass_warp(&turn[h ^ 1], t_phase, a.status, kKernelId, 0x644u + h, abort_flag);
           t_phase ^= 1u;
         }
-        uint64_t sum2[2] = {0ull, 0ull};
+        float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};      // of 32 keys each
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           uint32_t pk[16];
@@ -579,7 +574,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             f2_unpack(x, p0, p1);
             p0 = ex2_approx(p0);
             p1 = ex2_approx(p1);
-            sum2[c & 1] = f2_add(sum2[c & 1], f2_pack(p0, p1));
+            sum[c] += p0 + p1;
             pk[i >> 1] = pack_bf16x2(p0, p1);
           }
           if (c == 3 && lane == 0 && j < nt_both) mbar_arrive(&turn[h]);
@@ -595,9 +590,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_full[h]);
-        float s0, s1;
-        f2_unpack(f2_add(sum2[0], sum2[1]), s0, s1);
-        l = l * alpha + (s0 + s1);
+        l = l * alpha + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
       }
       both_before += nt_both;
       if (ok) ok = mbar_wait_warp(&o_done[h], o_phase, a.status, kKernelId, 0x650u + h, abort_flag);
