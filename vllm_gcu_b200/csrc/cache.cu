@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(256) mla_rope_cache_kernel(const MlaArgs a) {
 
 // The same for rows that 16-byte accesses can take (16-bit cache, widths and pitches multiples of eight, R of 16):
 // a thread rotates eight neighbouring columns of a head, or of the two halves, and eight columns of the
-// latent stay in registers between sum and store.  128 tokens of 128 heads 7.7 -> 3.3 us, 2048 tokens 31.6 ->
+// latent stay in registers between sum and store.  Sums and products are rounded as there.  128 tokens of 128 heads 7.7 -> 3.3 us, 2048 tokens 31.6 ->
 // 13.0 (element by element before, and started behind the end of the kernel in front).
 template <typename T, bool NEOX>
 __device__ __forceinline__ void rotate8(const T* src, T* dst, const float* cs, int half, int j) {
@@ -485,8 +485,8 @@ __device__ __forceinline__ void rotate8(const T* src, T* dst, const float* cs, i
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const float c = cs[8 * j + i], s = cs[half + 8 * j + i];
-      u[i] = x[i] * c - y[i] * s;
-      v[i] = y[i] * c + x[i] * s;
+      u[i] = fmaf(x[i], c, -(y[i] * s));
+      v[i] = fmaf(x[i], s, y[i] * c);
     }
     vec8_store<T>(dst + 8 * j, u);
     vec8_store<T>(dst + half + 8 * j, v);
@@ -496,8 +496,8 @@ __device__ __forceinline__ void rotate8(const T* src, T* dst, const float* cs, i
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const float c = cs[4 * j + i], s = cs[half + 4 * j + i];
-      u[2 * i] = x[2 * i] * c - x[2 * i + 1] * s;
-      u[2 * i + 1] = x[2 * i + 1] * c + x[2 * i] * s;
+      u[2 * i] = fmaf(x[2 * i], c, -(x[2 * i + 1] * s));
+      u[2 * i + 1] = fmaf(x[2 * i], s, x[2 * i + 1] * c);
     }
     vec8_store<T>(dst + 8 * j, u);
   }
@@ -515,10 +515,11 @@ __global__ void __launch_bounds__(256) mla_rope_cache_vec_kernel(const MlaArgs a
   const long long slot = a.slot_mapping != nullptr ? a.slot_mapping[t] : -1;
   float x[8], ss = 0.0f;
   const bool latent = static_cast<int>(threadIdx.x) < n_l;
-  if (latent) {
-    vec8_load<T>(kv + 8 * threadIdx.x, x);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) ss += x[i] * x[i];
+  if (latent) vec8_load<T>(kv + 8 * threadIdx.x, x);
+  // (columns a block apart, as the other kernel adds them up: the same bits from both)
+  for (int i = threadIdx.x; i < a.L; i += blockDim.x) {
+    const float v = to_f32<T>(kv[i]);
+    ss += v * v;
   }
   if (a.q_pe != nullptr) {
     const T* qin = static_cast<const T*>(a.q_pe) + static_cast<long long>(t) * a.ldq;
