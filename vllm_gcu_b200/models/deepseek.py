@@ -11,8 +11,9 @@ vllm_gcu/models/deepseek_v3/deepseek_v3_fusion.py:105-258):
 2. one fused kernel splits the latent, applies RMSNorm to ``kv_c``, RoPE to ``q_pe`` / ``k_pe``
    and writes the latent row into the paged cache (``ops.cuda.mla_rope_cache``);
 3. ``q_nope x W_UK`` -> latent query; attention over the cached latents; ``x W_UV``; ``o_proj``.
-   Prompts long enough for it (``ops.cuda.latent_prefill_plan``) go the other way: the latents they
-   attend to become keys and values of every head, which is 3.4 times less work per pair.
+   With ``USE_EXPANDED_PROMPTS`` prompts long enough for it (``ops.cuda.latent_prefill_plan``) go the
+   other way: the latents they attend to become keys and values of every head, which is 3.4 times less
+   work per pair.
 
 The attention core runs in the tcgen05 latent attention kernel (csrc/attention_mla.cu:
 decode, multi-token verification and prefill chunks in one kernel), expanded prompts in
@@ -40,6 +41,11 @@ from .moe_models import MoeDecoderLM
 
 
 USE_MLA_KERNEL = True     # tcgen05 latent attention (csrc/attention_mla.cu) where the layout allows
+# Prompts over keys and values expanded per head (MLAAttention._forward_runs): two of 1024 tokens 4.7 ms a step in
+# place of 5.9.  Off: it rounds keys and values where the other form rounds queries and outputs, as exactly (200 rows of
+# logits, error against 64 bits 0.0096, 0.0106 in the other form), but where a router's scores nearly tie another
+# expert is chosen, and the logits of 7 of 48 steps differ from the other form's by 1.1 to 3 per cent.
+USE_EXPANDED_PROMPTS = False
 
 
 mla_attention_ref = ref.latent_attention
@@ -143,7 +149,7 @@ class MLAAttention(nn.Module):
         q_nope, q_pe = q[..., : self.nope], q[..., self.nope:]
         nd = md.num_decode_tokens
         B = md.num_decodes + md.num_prefills
-        if (USE_MLA_KERNEL and ops.use_native(x) and md.num_prefills > 0
+        if (USE_EXPANDED_PROMPTS and USE_MLA_KERNEL and ops.use_native(x) and md.num_prefills > 0
                 and C.mla_attention_supported(q.new_empty((0, N, L + R)), kv_cache, L)):
             o = self._forward_runs(q, kv, kv_cache, md)
             if o is not None:
