@@ -134,6 +134,9 @@ class MLAAttention(nn.Module):
         if kv_cache is None or md.is_dummy:
             # idle data-parallel rank / memory profile: identical zero input for the MoE
             # (vllm_gcu/attention/backends/mla_v1_fusion.py:106-110)
+            # (part of the profile: latent rows and expanded keys and values of a run of prompts)
+            keys = C.LATENT_PREFILL_BYTES // (2 * N * (self.nope + self.vdim)) if USE_EXPANDED_PROMPTS and x.is_cuda else 0
+            held = x.new_empty((keys, N * (self.nope + self.vdim) + L + R))  # noqa: F841
             return self.o_proj(torch.zeros((T, N * self.vdim), dtype=x.dtype, device=x.device))
         if self.w_uk_t is None:
             self.finalize()
