@@ -10,13 +10,15 @@ from typing import Any, Callable
 
 
 # The mapping behind os.environ: a flag that is not set costs a look-up in it, 0.2 us, where os.environ.get
-# encodes the name and raises and catches inside, 2 us; every kernel wrapper asks for one.
-_RAW = getattr(os.environ, "_data", None)
+# encodes the name and raises and catches inside, 2 us; every kernel wrapper asks for one.  (Of this os.environ:
+# one that a program puts in its place is asked itself.)
+_ENVIRON = os.environ
+_RAW = getattr(_ENVIRON, "_data", None)
 _KEYS: dict[str, tuple[bytes, ...]] = {}
 
 
 def _get(name: str, default: str | None = None) -> str | None:
-    if _RAW is not None and os.name == "posix":
+    if _RAW is not None and os.environ is _ENVIRON and os.name == "posix":
         keys = _KEYS.get(name)
         if keys is None:
             keys = _KEYS[name] = tuple(os.fsencode(p + name) for p in ("VLLM_B200_", "VLLM_GCU_"))
