@@ -144,7 +144,8 @@ class MLAAttention(nn.Module):
         if cfg.q_lora_rank > 0:
             qkv_a = self.qkv_a_proj(x)
             q_c, kv = qkv_a.split([cfg.q_lora_rank, L + R], dim=-1)
-            q = self.q_b_proj(self.q_a_layernorm(q_c))
+            # (rows of the latent from 16-byte boundaries are normed where they lie)
+            q = self.q_b_proj(self.q_a_layernorm(q_c if qkv_a.shape[-1] % 8 == 0 else q_c.contiguous()))
         else:
             q = self.q_proj(x)
             kv = self.kv_a_proj_with_mqa(x)
