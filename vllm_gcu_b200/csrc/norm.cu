@@ -250,10 +250,10 @@ int launch2(const Args& a, bool add, cudaStream_t s) {
   int threads = ((a.H >> 3) + 31) & ~31;
   if (threads > 1024) threads = 1024;
   if (threads < 32) threads = 32;
-  // The registers it takes leave an SM two CTAs of 512 threads in place of four: for grids of one round only.
-  // us of 256 x 4096 3.8 : 2.8, 128 x 7168 3.5 : 2.7, 500 x 2048 3.8 : 3.0, but 64 x 4096 2.4 : 2.5 (8-bit rows 3.2 :
-  // 3.3), 600 x 4096 5.0 : 6.2, 8192 x 4096 49 : 70.
-  const bool keep = 2 * a.T > sm_count() && a.T <= 2 * sm_count();
+  // The registers it takes leave an SM two CTAs of 512 threads in place of four, and one of more: for grids of one round
+  // only.  us read again : kept, 256 x 4096 3.8 : 2.8, 128 x 7168 3.5 : 2.7, 272 x 3072 3.6 : 2.9, 148 x 12288 3.9 : 4.0, but
+  // 64 x 4096 2.4 : 2.5 (8-bit rows 3.2 : 3.3), 256 x 7168 3.7 : 4.8, 600 x 4096 5.0 : 6.2, 8192 x 4096 49 : 70.
+  const bool keep = 2 * a.T > sm_count() && a.T <= (threads <= 512 ? 2 : 1) * sm_count();
   auto kernel = add ? (keep ? rms_norm_kernel<T, QMODE, true, true> : rms_norm_kernel<T, QMODE, true, false>)
                     : (keep ? rms_norm_kernel<T, QMODE, false, true> : rms_norm_kernel<T, QMODE, false, false>);
   return launch_overlapped(kernel, dim3(a.T), dim3(threads), 0, s, a);
