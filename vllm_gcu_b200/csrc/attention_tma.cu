@@ -81,7 +81,6 @@ struct Args {
   float softcap;         // kShaped kernels: see b200_paged_decode_sink
   int chunk, window, OD;
   const float* alibi;    // kShaped kernels: [Hq] slopes or null
-  int cluster;           // the splits of a request and key head are a cluster and merge in shared memory
   unsigned int* status;
 };
 
@@ -141,8 +140,10 @@ __device__ __forceinline__ void merge_cluster(const Args& a, const float* lse, c
 __device__ __forceinline__ void consumer_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 
-// kShaped: soft cap, chunk, window, slopes and output columns are in force
-template <typename T, bool kShaped>
+// kShaped: soft cap, chunk, window, slopes and output columns are in force.  kCluster: the splits of a request and
+// key head are a cluster and merge in shared memory (a kernel of its own: its code behind the loop costs the other
+// 2 to 5 per cent)
+template <typename T, bool kShaped, bool kCluster>
 __global__ void __launch_bounds__(kThreads)
     paged_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK,
                             const __grid_constant__ CUtensorMap tmV, const Args a) {
@@ -173,7 +174,7 @@ __global__ void __launch_bounds__(kThreads)
   float* part_lse = reinterpret_cast<float*>(smem) + 128 + 4 * 16 * HD;
   float* part_o = part_lse + 16;
   if (start >= end) {
-    if (a.cluster) {
+    if constexpr (kCluster) {
       if (threadIdx.x < 16) part_lse[threadIdx.x] = -INFINITY;
       merge_cluster<T>(a, part_lse, part_o, b, kvh, G, OD);
       return;
@@ -232,8 +233,10 @@ __global__ void __launch_bounds__(kThreads)
       }
     }
     // the producer warp takes no part in the merge
-    __syncwarp();
-    if (a.cluster) merge_cluster<T>(a, part_lse, part_o, b, kvh, G, OD);
+    if constexpr (kCluster) {
+      __syncwarp();
+      merge_cluster<T>(a, part_lse, part_o, b, kvh, G, OD);
+    }
     return;
   }
 
@@ -393,7 +396,7 @@ __global__ void __launch_bounds__(kThreads)
       o += sm_o[(w * 16 + r) * HD + d] * f;
     }
     float val = (ok && L > 0.0f) ? o / L : 0.0f;
-    if (a.cluster) {
+    if constexpr (kCluster) {
       part_o[idx] = val;
       if (d == 0) part_lse[r] = (ok && L > 0.0f) ? M + log2f(L) : -INFINITY;
       continue;
@@ -408,8 +411,10 @@ __global__ void __launch_bounds__(kThreads)
       static_cast<T*>(a.out)[static_cast<long long>(b) * a.ldo + head * OD + d] = from_f32<T>(val);
     }
   }
-  __syncwarp();
-  if (a.cluster) merge_cluster<T>(a, part_lse, part_o, b, kvh, G, OD);
+  if constexpr (kCluster) {
+    __syncwarp();
+    merge_cluster<T>(a, part_lse, part_o, b, kvh, G, OD);
+  }
 }
 
 // Launch with the splits of a request and key head as a cluster, or as CTAs on their own
@@ -511,11 +516,16 @@ static int paged_decode_tma_impl(const void* q, long long ldq, void* out, long l
   a.num_splits = num_splits; a.max_blocks = max_blocks; a.block_size = block_size;
   a.scale = scale; a.sink = sink; a.softcap = softcap; a.chunk = chunk; a.OD = OD > 0 ? OD : HD;
   a.window = window; a.alibi = alibi;
-  // Up to eight splits merge in shared memory: no partial results in global memory and no second kernel.  us in a
-  // cluster : with both, 1 request of 640 keys and 8 key heads, 3 splits 7.1 : 8.4, 6 splits 5.5 : 7.9, 12 requests
-  // of 900, 2 splits 13.4 : 14.5; but where two rounds of CTAs wait for one another 64 of 1500, 2 splits 75 : 74, 8
-  // splits 134 : 99.
-  a.cluster = num_splits > 1 && num_splits <= 8 && static_cast<long long>(B) * Hkv * num_splits <= 2 * sm_count();
+  // Up to eight splits merge in shared memory: no partial results in global memory and no second kernel.  Where there
+  // are few CTAs, or more than one an SM that all run at once: a cluster's CTAs come two to an SM while other SMs are
+  // idle.  us in a cluster : with both kernels, 8 key heads, 1 request of 640 keys, 3 splits 7.3 : 8.5, 1 of 1500, 8
+  // splits 6.6 : 8.5, 8 of 1500, 4 splits (256 CTAs) 10.4 : 11.3; but 4 of 700, 2 splits (64) 9.5 : 9.1, 4 of 1000, 4 splits
+  // (128) 8.6 : 8.0, 8 of 700, 2 splits (128) 10.4 : 9.3, and in two rounds 6 of 1500, 6 splits (288) 14.9 : 10.4.
+  const long long ctas = static_cast<long long>(B) * Hkv * num_splits;
+  const int sms = sm_count();
+  const bool cluster = num_splits > 1 && num_splits <= 8 &&
+                       (ctas <= sms / 3 || (ctas <= sms * 13 / 30 && num_splits > 2) ||
+                        (ctas > sms && ctas <= sms * 7 / 4));
   a.status = status_ptr();
   const bool shaped = softcap > 0.0f || chunk > 0 || window > 0 || alibi != nullptr || a.OD != HD;
   if (shaped && dtype != 0) return -20;
@@ -524,38 +534,29 @@ static int paged_decode_tma_impl(const void* q, long long ldq, void* out, long l
                 "merge buffers must fit");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   dim3 grid(B, Hkv, num_splits);
-  static bool done0[64] = {false}, done1[64] = {false}, done2[64] = {false};
-  int dev = 0, e = 0;
+  static bool done[6][64] = {};
+  int dev = 0;
   cudaGetDevice(&dev);
-  if (shaped) {
-    auto kern = paged_decode_tma_kernel<__nv_bfloat16, true>;
-    if (dev >= 0 && dev < 64 && !done2[dev]) {
+  auto go = [&](auto kern, int which) -> int {
+    if (dev >= 0 && dev < 64 && !done[which][dev]) {
       const cudaError_t set =
           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
       if (set != cudaSuccess) return static_cast<int>(set);
-      done2[dev] = true;
+      done[which][dev] = true;
     }
-    e = launch_splits(kern, grid, smem, a.cluster != 0, s, tmK, tmV, a);
-  } else if (dtype == 0) {
-    auto kern = paged_decode_tma_kernel<__nv_bfloat16, false>;
-    if (dev >= 0 && dev < 64 && !done0[dev]) {
-      const cudaError_t set =
-          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (set != cudaSuccess) return static_cast<int>(set);
-      done0[dev] = true;
-    }
-    e = launch_splits(kern, grid, smem, a.cluster != 0, s, tmK, tmV, a);
-  } else {
-    auto kern = paged_decode_tma_kernel<__half, false>;
-    if (dev >= 0 && dev < 64 && !done1[dev]) {
-      const cudaError_t set =
-          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (set != cudaSuccess) return static_cast<int>(set);
-      done1[dev] = true;
-    }
-    e = launch_splits(kern, grid, smem, a.cluster != 0, s, tmK, tmV, a);
-  }
-  if (e != 0 || num_splits <= 1 || a.cluster) return e;
+    return launch_splits(kern, grid, smem, cluster, s, tmK, tmV, a);
+  };
+  int e;
+  if (shaped)
+    e = cluster ? go(paged_decode_tma_kernel<__nv_bfloat16, true, true>, 0)
+                : go(paged_decode_tma_kernel<__nv_bfloat16, true, false>, 1);
+  else if (dtype == 0)
+    e = cluster ? go(paged_decode_tma_kernel<__nv_bfloat16, false, true>, 2)
+                : go(paged_decode_tma_kernel<__nv_bfloat16, false, false>, 3);
+  else
+    e = cluster ? go(paged_decode_tma_kernel<__half, false, true>, 4)
+                : go(paged_decode_tma_kernel<__half, false, false>, 5);
+  if (e != 0 || num_splits <= 1 || cluster) return e;
   return b200_decode_reduce(out, ldo, tmp_out, tmp_lse, num_splits, B, Hq, HD, dtype, sink,
                             a.OD, stream);
 }
