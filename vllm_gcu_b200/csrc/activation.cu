@@ -317,12 +317,12 @@ int launch_q(Args a, int quant, cudaStream_t s) {
   if (quant == kQFp8Token || quant == kQInt8Token)
     return launch_token<T, ACT, MODE>(a, quant == kQInt8Token, s);
   const int nvec = a.d >> 3;
-  const int most = (nvec + 63) / 64;
+  const int most = nvec < 128 ? 1 : (nvec + 63) / 64;
   int splits = 2 * sm_count() / a.T;
   splits = splits < 1 ? 1 : (splits > most ? most : splits);
   a.chunk = ((nvec + splits - 1) / splits + 31) & ~31;
   splits = (nvec + a.chunk - 1) / a.chunk;
-  const int threads = even_threads(a.chunk, 512);
+  const int threads = splits > 1 ? even_threads(a.chunk, 512) : (a.chunk < 512 ? a.chunk : 512);
   auto go = [&](void (*kernel)(Args)) {
     return launch_overlapped(kernel, dim3(a.T, splits), dim3(threads), 0, s, a);
   };
