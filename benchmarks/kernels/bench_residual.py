@@ -70,7 +70,7 @@ def cases(T: int, H: int, L: int = 512, D: int = 4096, k: int = 4, E: int = 32, 
              k, H, H, cap, 0, stream_ptr())
 
     def permute():
-        call("b200_moe_permute", ptr(xb), H, ptr(yo), H, ptr(sid), ptr(npp), T * k, k, H, cap, 1, 0,
+        call("b200_moe_permute", ptr(xb), H, ptr(yo), H, ptr(sid), ptr(npp), T * k, k, H, cap, 0,
              stream_ptr())
 
     def unpermute():

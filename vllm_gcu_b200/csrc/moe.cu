@@ -325,18 +325,16 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// A_sorted[pos] = x[sorted_ids[pos] / k]; padding rows are zeroed, or left as they are (zero_pads = 0) for
-// products that do not store them.  One CTA per row.
+// A_sorted[pos] = x[sorted_ids[pos] / k]; padding rows are zeroed.  One CTA per row.
 template <typename T>
 __global__ void __launch_bounds__(256)
     moe_permute_kernel(const T* x, long long ldx, T* out, long long ldo, const int* sorted_ids,
-                       const int* num_post_pad, int numel, int k, int H, int zero_pads) {
+                       const int* num_post_pad, int numel, int k, int H) {
   grid_release_small();
   grid_wait();
   const int pos = blockIdx.x;
   if (pos >= *num_post_pad) return;
   const int pair = sorted_ids[pos];
-  if (pair >= numel && !zero_pads) return;
   uint4* dst = reinterpret_cast<uint4*>(out + static_cast<long long>(pos) * ldo);
   const int nvec = H >> 3;
   if (pair >= numel) {
@@ -635,7 +633,7 @@ B200_API int b200_moe_scatter(const void* x, long long ldx, void* out, long long
 
 B200_API int b200_moe_permute(const void* x, long long ldx, void* out, long long ldo,
                               const int* sorted_ids, const int* num_post_pad, int numel, int k,
-                              int H, int cap, int zero_pads, int dtype, void* stream) {
+                              int H, int cap, int dtype, void* stream) {
   if (cap <= 0) return 0;
   if ((H % 8) != 0) return -2;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -643,11 +641,11 @@ B200_API int b200_moe_permute(const void* x, long long ldx, void* out, long long
     return launch_overlapped(moe_permute_kernel<__nv_bfloat16>, dim3(cap), dim3(256), 0, s,
                              static_cast<const __nv_bfloat16*>(x), ldx,
                              static_cast<__nv_bfloat16*>(out), ldo, sorted_ids, num_post_pad, numel, k,
-                             H, zero_pads);
+                             H);
   if (dtype == 1)
     return launch_overlapped(moe_permute_kernel<__half>, dim3(cap), dim3(256), 0, s,
                              static_cast<const __half*>(x), ldx, static_cast<__half*>(out), ldo,
-                             sorted_ids, num_post_pad, numel, k, H, zero_pads);
+                             sorted_ids, num_post_pad, numel, k, H);
   return -8;
 }
 

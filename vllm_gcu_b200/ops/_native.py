@@ -180,7 +180,7 @@ class _Sigs:
     b200_moe_topk = [P, L, P, P, P, I, I, I, I, I, I, I, F, P, I, P, P, I, P]
     b200_moe_align = [P, P, P, P, P, P, P, P, P, P, I, I, I, I, P]
     b200_moe_scatter = [P, L, P, L, P, I, I, I, I, P]
-    b200_moe_permute = [P, L, P, L, P, P, I, I, I, I, I, I, P]
+    b200_moe_permute = [P, L, P, L, P, P, I, I, I, I, I, P]
     b200_moe_permute_any = [P, L, P, L, P, P, I, I, I, I, I, I, P]
     b200_moe_permute_weighted = [P, L, P, P, L, P, P, I, I, I, I, I, I, P]
     b200_grouped_gemm_f32 = [P, L, P, P, L, I, I, I, I, P, P, P]

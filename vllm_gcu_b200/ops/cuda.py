@@ -1782,7 +1782,7 @@ def ungated_experts(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, topk_id
     a_sorted = torch.empty((cap, Hp), device=x.device, dtype=x.dtype)
     if x.dtype == torch.bfloat16 and H == Hp and H % 8 == 0:
         call("b200_moe_permute", ptr(x), x.stride(0), ptr(a_sorted), Hp, ptr(sorted_ids), ptr(npp),
-             numel, k, H, cap, 1, DTYPE_CODE[x.dtype], stream_ptr())
+             numel, k, H, cap, DTYPE_CODE[x.dtype], stream_ptr())
     else:
         call("b200_moe_permute_any", ptr(x), x.stride(0), ptr(a_sorted), Hp, ptr(sorted_ids),
              ptr(npp), numel, k, H, Hp, cap, DTYPE_CODE[x.dtype], stream_ptr())
@@ -1840,7 +1840,7 @@ def fused_experts_fp8(x: torch.Tensor, w13: torch.Tensor, w13_scale: torch.Tenso
                                                     topk_w=topk_w, row_w=row_w)
     a_sorted = torch.empty((cap, H), device=x.device, dtype=x.dtype)
     call("b200_moe_permute", ptr(x), x.stride(0), ptr(a_sorted), H, ptr(sorted_ids), ptr(npp),
-         numel, k, H, cap, 1, DTYPE_CODE[x.dtype], stream_ptr())
+         numel, k, H, cap, DTYPE_CODE[x.dtype], stream_ptr())
     aq, a_s = activation(a_sorted, "identity", "plain", quant="fp8_group128", valid_rows=npp)
     h = gemm_q8_grouped(aq, a_s, w13, w13_scale, expert_ids, npp, kind=1)
     hq, h_s = activation(h, "silu", "act_mul", quant="fp8_group128", valid_rows=npp)
@@ -1910,7 +1910,7 @@ def fused_experts_wna16(x: torch.Tensor, q13: torch.Tensor, s13: torch.Tensor, z
                                                     topk_w=topk_w, row_w=row_w)
     a_sorted = torch.empty((cap, H), device=x.device, dtype=x.dtype)
     call("b200_moe_permute", ptr(x), x.stride(0), ptr(a_sorted), H, ptr(sorted_ids), ptr(npp),
-         numel, k, H, cap, 1, DTYPE_CODE[x.dtype], stream_ptr())
+         numel, k, H, cap, DTYPE_CODE[x.dtype], stream_ptr())
     if numel <= WNA16_GROUPED_MAX_ROWS_PER_EXPERT * E:
         h = gemm_wna16_grouped(a_sorted, q13, s13, z13, expert_ids, npp, group, bits)
         hm = activation(h, "silu", "act_mul", valid_rows=npp)
@@ -1954,7 +1954,7 @@ def fused_experts_q8(x: torch.Tensor, w13: torch.Tensor, w13_scale: torch.Tensor
                                                     topk_w=topk_w, row_w=row_w)
     a_sorted = torch.empty((cap, H), device=x.device, dtype=x.dtype)
     call("b200_moe_permute", ptr(x), x.stride(0), ptr(a_sorted), H, ptr(sorted_ids), ptr(npp),
-         numel, k, H, cap, 1, DTYPE_CODE[x.dtype], stream_ptr())
+         numel, k, H, cap, DTYPE_CODE[x.dtype], stream_ptr())
     aq, a_s = per_token_quant(a_sorted, qname, valid_rows=npp)
     h = gemm_q8_grouped(aq, a_s.view(-1), w13, w13_scale, expert_ids, npp, kind=kind)
     hq, h_s = activation(h, "silu", "act_mul", quant=qname + "_token", valid_rows=npp)
