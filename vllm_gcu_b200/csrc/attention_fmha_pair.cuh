@@ -4,7 +4,8 @@
 //            the tiles are 128 rows of two heads.  No soft cap, chunk or bias.
 //   latent   latent attention over keys and values that were expanded per head into [keys, heads * 256] (128
 //            columns of a key, 128 of a value), with 64 rotated key columns that all heads share; queries
-//            have 192 columns; the tiles are 2 x 128 rows of one head.  Causal.
+//            have 192 columns; the tiles are 2 x 128 rows of one head.  Causal.  Off by default
+//            (models/deepseek.py, USE_EXPANDED_PROMPTS).
 //
 // What bounds it: per 128 x 128 scores the tensor cores need 1024 cycles (Q K^T and P V; 1280 with 192
 // columns) and the exponentials 1024 cycles of the special-function pipe, and one tile's chain scores ->
@@ -30,9 +31,9 @@
 //
 // Warps: 0 finds work and loads (lane = page and half of a key tile), 1 and 2 tcgen05.mma of the two tiles, 1
 // owns tensor memory, 4..7 softmax and epilogue of the first tile, 8..11 of the second.
-// Measured against the kernel that went before (one issuing thread, no turns, a CTA for each piece of work),
-// 32 heads, us: 8192 tokens 600 -> 509, 2 x 2048 tokens 127 -> 92, 7 x 1024 tokens 137 -> 99, 2048 tokens 73 ->
-// 47.  Latent form, 2 x 1024 tokens of 128 heads with the expansion in front 206, where the absorbed form
+// Measured against the kernel that went before (one issuing thread, no turns, a CTA for each piece of work; the
+// same bits from both), 32 heads, us: 8192 tokens 573 -> 488, 2 x 2048 tokens 113 -> 88, 7 x 1024 tokens 125 -> 104, 40
+// requests of 40 tokens behind 100 71 -> 39.  Latent form, 2 x 1024 tokens of 128 heads with the expansion in front 206, where the absorbed form
 // takes 826 with its products per head.
 #pragma once
 

@@ -48,7 +48,7 @@
 // A tile's 36 score products and four output products take 2450 cycles when nothing waits; their issue takes
 // as long again, so scores and P V have a thread each, with descriptors that step by constants, and the two
 // threads of a row exchange maxima at a barrier of their two warps: 128 requests x 1536 keys, 128 heads 107 -> 100
-// us, 256 x 1152 keys 166 -> 155, 2 x 1024 new tokens 644 -> 602.
+// us, 256 x 1152 keys 166 -> 155, 2 x 1024 new tokens 645 -> 607.
 //
 // Warp roles: warp 0 TMA producer, warp 1 scores and TMEM owner, warps 2..9 softmax and epilogue, warp 10
 // P V.  Every wait is bounded and reports through the status word.

@@ -474,8 +474,8 @@ __global__ void __launch_bounds__(256) mla_rope_cache_kernel(const MlaArgs a) {
 
 // The same for rows that 16-byte accesses can take (16-bit cache, widths and pitches multiples of eight, R of 16):
 // a thread rotates eight neighbouring columns of a head, or of the two halves, and eight columns of the
-// latent stay in registers between sum and store.  Sums and products are rounded as there.  128 tokens of 128 heads 7.7 -> 3.3 us, 2048 tokens 31.6 ->
-// 13.0 (element by element before, and started behind the end of the kernel in front).
+// latent stay in registers between sum and store.  Sums and products are rounded as there.  128 tokens of 128 heads 7.7 -> 3.5 us, 2048 tokens 31.2 ->
+// 14.7 (element by element before, and started behind the end of the kernel in front).
 template <typename T, bool NEOX>
 __device__ __forceinline__ void rotate8(const T* src, T* dst, const float* cs, int half, int j) {
   if constexpr (NEOX) {            // columns 8 j .. 8 j + 7 and their partners half a width further

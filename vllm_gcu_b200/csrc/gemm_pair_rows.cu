@@ -8,8 +8,8 @@
 // tcgen05.mma.cta_group::2) and the activation rows are its N side, any multiple of 32 up to 256, of which
 // each CTA loads one half: 16 KB of weights and at most 16 KB of rows per K block and CTA, the
 // intensity of a 256 x 256 tile when they are full.  Accumulators: 256 columns of tensor memory, two
-// sets, so that the epilogue of a tile (a transposition through shared memory, for rows of 256 bytes)
-// runs under the MMAs of the next.
+// sets, so that the epilogue of a tile (two neighbouring lanes exchange a number for every two rows, and each stores
+// two columns of one) runs under the MMAs of the next.
 //
 // Persistent pairs.  Dense: the row tiles of a weight tile follow each other, so that the weights come
 // from L2 after the first.  Experts: two row tiles of an expert make one (up to 256 rows), its padding is
@@ -17,10 +17,10 @@
 // when it starts.
 //
 // Measured, launches replayed from a graph, weights beyond L2 (the kernels it took over from): 301 rows,
-// 28672 x 4096 76 us (89; 44 at the tensor cores' rate, 63 the vendor library), 6144 x 4096 22 (28), 36864 x
-// 7168 140 (178); 32 experts of 7168 x 2048 with 256 rows each, w13 466 us (633 in row tiles of 128; 321 at
-// the tensor cores' rate), w2 254 (466).
-// What held short K was the epilogue, 3000 cycles for 32 rows of a gated product (IEEE divisions that wait for
+// 28672 x 4096 74 us (89; 44 at the tensor cores' rate, 63 the vendor library), 6144 x 4096 20 (28).  With the first
+// epilogue: 36864 x 7168 140 (178); 32 experts of 7168 x 2048 with 256 rows each, w13 466 us (633 in row tiles of 128;
+// 321 at the tensor cores' rate), w2 254 (466).
+// What held short K was that epilogue, 3000 cycles for 32 rows of a gated product (IEEE divisions that wait for
 // one another, four warps that meet three times a chunk) beside 512 of a K block's products.  Eight warps,
 // no divisions with branches, neighbours' exchange in place of a transposition: 128 experts, 4096 tokens of 8
 // (the same in equal shares): w13 1536 x 2048 260 (216) -> 220 (182), w2 2048 x 768 177 (149) -> 125 (106),

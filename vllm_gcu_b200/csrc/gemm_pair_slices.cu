@@ -8,7 +8,10 @@
 // cluster barrier every CTA adds up a share of the rows out of the others' (stream.cuh): no workspace, no
 // counters, no second kernel.
 //
-// Measured, launches replayed from a graph, weights beyond L2 (the kernels it took over from):
+// Off by default (ops/cuda.py, USE_SPLIT_SUMS): partial sums round otherwise than one sum, as exactly, and layers of 16
+// bits carry that on.
+//
+// Measured, launches replayed from a graph, weights beyond L2 (the kernels that run in its place):
 // 301 rows, 4096 x 14336 50 -> 36 us, 4096 x 4096 17.7 -> 15.2, 2112 x 7168 25 -> 15.5; 186 rows, 4864 x 14336 50 -> 32;
 // 400 rows, 4096 x 14336 53 -> 44.  Not with a second round of clusters (301 rows, 6144 x 4096 19.5 : 28.7) or
 // few K blocks a slice (592 rows, 2632 x 1536 9.3 : 13.0).

@@ -145,7 +145,7 @@ def _large_plan(M: int, Nn: int, K: int, split: bool = True) -> tuple[str, int, 
     1.00 of the other kernels' time, one 1.05): 160 x 10240 x 2048 19.5 : 14.3, 160 x 12288 x 5120 34 : 29, 192 x
     28672 x 4096 gated 55 : 52, 256 x 7168 x 1024 11.8 : 9.1, 256 x 9000 x 3000 26.3 : 20.9.
 
-    K is split where the tiles are no more than the clusters that run at once and the estimate is a tenth
+    With ``split`` K is split where the tiles are no more than the clusters that run at once and the estimate is a tenth
     below the others' (fitted to 300 calls of 40 .. 860 rows): 301 x 4096 x 14336 50 : 36, 301 x 4096 x 4096 17.7 :
     15.2, 301 x 2112 x 7168 25 : 15.5, 186 x 4864 x 14336 50 : 32, 175 x 5632 x 4096 18.4 : 14.8."""
     return _large_estimate(M, Nn, K, split)[1]
@@ -171,8 +171,8 @@ def _even_rows(M: int, rows: int) -> int:
 @functools.lru_cache(maxsize=4096)
 def _tail_plan(M: int, Nn: int, K: int):
     """``(rows, head, rows of the tail's tiles, slices)`` where the first ``head`` weight rows in full rounds of
-    gemm_pair_rows.cu and the others with K split over the pairs of a cluster are estimated faster than one kernel
-    by 4 per cent, by 7 with more than two row tiles, None elsewhere.  (4 us more where the pairs read more weight tiles
+    gemm_pair_rows.cu and the others with K split over the pairs of a cluster (USE_SPLIT_SUMS) are estimated faster
+    than one kernel by 4 per cent, by 7 with more than two row tiles, None elsewhere.  (4 us more where the pairs read more weight tiles
     than one each.)  It is for a last round of a few tiles.  70 shapes of 130 .. 1004 rows whose estimates differ by
     4 per cent took 0.94 of the time, 0.69 to 1.03, those of 1.00 and more with three row tiles or more: us of 301 x
     28672 x 4096 74.1 : 71.0, 200 x 20480 x 4096 48.9 : 43.6, 310 x 9728 x 4096 34.9 : 31.0, 231 x 19456 x 14336 173 :
@@ -254,7 +254,7 @@ def _pair_rows(M: int, Nn: int, K: int = 4096) -> int:
     """Rows of a tile of the pair kernel with the weights on the M side (gemm_pair_rows.cu), 0 where
     another kernel is taken.  It pays for rows that would fill tiles of 256 badly, us at rows x N x K
     against the other kernels: 301 x 28672 x 4096 82 : 104, 301 x 36864 x 7168 143 : 179, 301 x 6144 x 4096
-    22 : 27, 301 x 7168 x 2048 20 : 24, 544 x 28672 x 4096 102 : 130, 610 x 6144 x 4096 28.1 : 28.8, 800 x 7168 x
+    22 : 27, 301 x 7168 x 2048 20 : 24 (all of the kernel with its first epilogue), 544 x 28672 x 4096 102 : 130, 610 x 6144 x 4096 28.1 : 28.8, 800 x 7168 x
     16384 185 : 210, 850 x 12288 x 5120 85 : 91, but 512 x 28672 x 4096 101 : 98, 256 x 28672 x 4096 61 : 57.
     And for enough weight tiles: 301 x 5120 x 2048 17 : 16, 301 x 4096 x 4096 20 : 18.5, 301 x 4096 x 14336
     52.7 : 51.  And where K is long enough for its way out, which is the dearer one, and the other kernel's
@@ -275,7 +275,9 @@ def _pair_rows(M: int, Nn: int, K: int = 4096) -> int:
 @functools.lru_cache(maxsize=1024)
 def _pair_rows_gain(M: int, Nn: int, K: int, rows: int, sms: int) -> float:
     """us by which the pair kernel in tiles of ``rows`` rows is faster than the kernel that would run in
-    its place, estimated: rounds of the SMs times (K blocks times a rate, and the way out of a tile).
+    its place, estimated: rounds of the SMs times (K blocks times a rate, and the way out of a tile).  The rates are
+    those of its first epilogue, and no other tile height is compared: _large_estimate has the present ones, by which
+    about one in six of the shapes that this takes would run 5 per cent faster in other tiles.
     Fitted to 1216 shapes of 257 .. 890 rows, N 5889 .. 49152, K 256 .. 16384 on 148 SMs, where it takes 732 calls
     at 0.86 of the other kernels' time (15 are slower by more than 3 %, all but one of them by less than
     14 %) and leaves out 16 that it would make 5 % faster; without it 393 of the 1216 were slower by 3 to 65 %."""
