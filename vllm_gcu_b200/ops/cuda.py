@@ -127,12 +127,19 @@ def _slices_at_once(slices: int) -> int:
     return int(N.lib().b200_gemm_pair_slices_at_once(slices))
 
 
-def _large_plan(M: int, Nn: int, K: int, split: bool = True) -> tuple[str, int, int]:
+#: us of an epilogue beyond the plain way out: a row of a round of gemm_pair_rows.cu, a round of gemm_pair.cu, a column of
+#: a wave of gemm_bf16.cu.  GELU's error function costs the first the most, whose lanes hold one weight row each.  us of
+#: rows, pair, tiles (16 shapes, weights beyond L2), 700 x 11008 x 1024 plain 16.9, 18.8, 23.8, GELU 26.7, 21.1, 28.5, gated
+#: by GELU 18.6, 16.5, 19.5; 512 x 16384 x 512 13.0, 12.7, 18.7, GELU 23.7, 17.7, 24.7, gated by GELU 16.3, 11.9, 13.2.
+_EPILOGUE_US = {EPI_GELU: (0.023, 1.8, 0.010), EPI_GELU_MUL: (0.006, -0.8, -0.008)}
+
+
+def _large_plan(M: int, Nn: int, K: int, split: bool = True, epilogue: int = 0) -> tuple[str, int, int]:
     """Kernel for more than 128 rows, by its estimated time, with its rows of a tile and slices of K:
     ``("rows", r, 1)`` the pair kernel with the weights on the M side (gemm_pair_rows.cu), ``("slices", r, s)``
     the same with K split over s pairs (gemm_pair_slices.cu), ``("pair", 0, 1)`` 256 x 256 tiles on CTA pairs
     (gemm_pair.cu), ``("tiles", 0, 1)`` 128 rows by the width that fills the SMs best (gemm_bf16.cu).  Without
-    ``split`` every sum over K is one (USE_SPLIT_SUMS).
+    ``split`` every sum over K is one (USE_SPLIT_SUMS).  ``epilogue``: one of _EPILOGUE_US, any other for the plain way out.
 
     Each estimate is rounds of the SMs times (K blocks times a rate that grows with the tile, and a way out),
     or the rate at the power limit where that is lower.  Fitted to 200 shapes of 257 .. 8192 rows, N 240 .. 28672
@@ -148,7 +155,7 @@ def _large_plan(M: int, Nn: int, K: int, split: bool = True) -> tuple[str, int, 
     With ``split`` K is split where the tiles are no more than the clusters that run at once and the estimate is a tenth
     below the others' (fitted to 300 calls of 40 .. 860 rows): 301 x 4096 x 14336 50 : 36, 301 x 4096 x 4096 17.7 :
     15.2, 301 x 2112 x 7168 25 : 15.5, 186 x 4864 x 14336 50 : 32, 175 x 5632 x 4096 18.4 : 14.8."""
-    return _large_estimate(M, Nn, K, split)[1]
+    return _large_estimate(M, Nn, K, split, epilogue if epilogue in _EPILOGUE_US else 0)[1]
 
 
 def _rows_us(rows: int, rounds: int, kb: int, K: int) -> float:
@@ -200,26 +207,29 @@ def _tail_plan(M: int, Nn: int, K: int):
 
 
 @functools.lru_cache(maxsize=4096)
-def _large_estimate(M: int, Nn: int, K: int, split: bool = True) -> tuple[float, tuple[str, int, int]]:
+def _large_estimate(M: int, Nn: int, K: int, split: bool = True, epilogue: int = 0
+                    ) -> tuple[float, tuple[str, int, int]]:
     """us of the kernel that ``_large_plan`` names, and its plan."""
     sms, kb = _sms(), -(-K // 64)
     pairs, w_tiles = sms // 2, -(-Nn // 256)
     best, plan = float("inf"), ("tiles", 0, 1)
+    row_us, pair_us, column_us = _EPILOGUE_US.get(epilogue, (0.0, 0.0, 0.0))
     for rows in (256, 224, 192, 160, 128, 96, 64):
         rows = _even_rows(M, rows)
-        us = _rows_us(rows, -(-w_tiles * -(-M // rows) // pairs), kb, K)
+        rounds = -(-w_tiles * -(-M // rows) // pairs)
+        us = _rows_us(rows, rounds, kb, K) + rounds * rows * row_us
         if us < best:
             best, plan = us, ("rows", rows, 1)
     if Nn % 256 == 0 and K % 64 == 0:
         tiles = -(-M // 256) * w_tiles
-        us = 6.85 + max(-(-tiles // pairs) * (2.07 + kb * 0.3254), tiles * K * 8.13e-5)
+        us = 6.85 + max(-(-tiles // pairs) * (2.07 + pair_us + kb * 0.3254), tiles * K * 8.13e-5)
         # (products of 100 GFLOP and more in a long step are at the power limit, where pairs did better than
         # timed alone: 7 x 1024 tokens beside 200 requests 23.2 ms with the estimates as they are, 22.7 so)
         if us * (0.93 if 2e-11 * M * Nn * K > 1 else 1) < best:
             best, plan = us, ("pair", 0, 1)
     waves = {c: -(-(-(-M // 128)) * -(-Nn // c) // sms) for c in (256, 128, 96, 64) if c != 256 or Nn % 256 == 0}
     c = min(waves, key=lambda c: waves[c] * (c + 32))
-    us = 4.54 + waves[c] * max(-0.356 + 0.025 * c + kb * (0.1441 + 0.00066 * c), c * K * 2.771e-5)
+    us = 4.54 + waves[c] * max(-0.356 + (0.025 + column_us) * c + kb * (0.1441 + 0.00066 * c), c * K * 2.771e-5)
     if us < best:
         best, plan = us, ("tiles", 0, 1)
     for slices in (2, 3, 4) if split and kb >= 16 else ():
@@ -414,7 +424,7 @@ def _gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = N
                 raise N.NativeError(f"b200_gemm_pair_rows failed with code {rc}")
     if (USE_PAIR_GEMM and not USE_PAIR_SPLIT and M > 128 and epilogue in _PAIR_EPI
             and (epilogue not in _GATED or Nn % 64 == 0) and not (K % 8 or Nn % 8)):
-        kind, rows, slices = _large_plan(M, Nn, K, USE_SPLIT_SUMS)
+        kind, rows, slices = _large_plan(M, Nn, K, USE_SPLIT_SUMS, epilogue)
         # (other kernels of up to 256 rows follow below)
         if M > 256 or kind in ("slices", "rows"):
             args = (ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(out), out.stride(0), M, Nn, K, ptr(bias),
